@@ -49,7 +49,7 @@ struct block_context : context_impl {
   std::vector<run_cache<T>> runs;
   std::vector<std::pair<std::pair<int, double>, float2*>> rotations;  // (dims, base) -> table
   // activations [rows_cap]
-  float *xs = nullptr, *y = nullptr, *raw = nullptr, *packed = nullptr, *packed_v = nullptr, *low = nullptr, *hidden = nullptr, *logits = nullptr;
+  float *xs = nullptr, *y = nullptr, *raw = nullptr, *packed = nullptr, *packed_v = nullptr, *scan_part = nullptr, *low = nullptr, *hidden = nullptr, *logits = nullptr;
   T *h = nullptr, *mix = nullptr, *proj = nullptr, *cat = nullptr, *gu = nullptr, *act = nullptr;
   T* shifted[4] = {};
   int ld_raw = 0, ld_shift = 0;
@@ -323,6 +323,7 @@ scan_rows<T> block_context<T>::recurrence(int run, int b, int ld) {
   s.ldo = bs.out_cols();
   s.packed = packed;
   s.packed_v = packed_v;
+  s.part = scan_part;
   s.err = gpus[0].state + 3;
   return s;
 }
@@ -721,7 +722,7 @@ int block_context<T>::create(block_model* model, const context_options& o) {
   // widest rows over the layers
   size_t w_z = 0, w_tiles = 0, w_route = 0, w_staged = 0, w_kv = 0;
   int top = 1;  // experts a token runs at most
-  size_t w_proj = 0, w_cat = 0, w_gu = 0, w_act = 0, w_raw = 0, w_shift = 0, w_low = 0, w_packed = 0, w_values = 0;
+  size_t w_proj = 0, w_cat = 0, w_gu = 0, w_act = 0, w_raw = 0, w_shift = 0, w_low = 0, w_packed = 0, w_values = 0, w_part = 0;
   for (size_t i = 0; i < m->layers.size(); ++i) {
     const block_layer& L = m->layers[i];
     w_proj = std::max(w_proj, (size_t)L.proj_rows);
@@ -747,10 +748,11 @@ int block_context<T>::create(block_model* model, const context_options& o) {
         w_kv = std::max(w_kv, keys * bw.up_rows);
       }
       if (b.kind == BRANCH_WINDOW_ATTN || b.kind == BRANCH_LATENT_ATTN) continue;
-      size_t pk = 0, pv = 0;
-      scan_scratch(b.heads, b.dim, b.vdim, b.kind == BRANCH_WKV, rows_cap, &pk, &pv);
+      size_t pk = 0, pv = 0, pp = 0;
+      scan_scratch(b.heads, b.dim, b.vdim, b.kind == BRANCH_WKV, rows_cap, &pk, &pv, &pp);
       w_packed = std::max(w_packed, pk);
       w_values = std::max(w_values, pv);
+      w_part = std::max(w_part, pp);
     }
   }
   const size_t R = rows_cap, K = m->k_width, es = sizeof(T);
@@ -768,6 +770,7 @@ int block_context<T>::create(block_model* model, const context_options& o) {
     take(raw, R * w_raw * 4);
     take(packed, w_packed * 4);
     take(packed_v, w_values * 4);
+    take(scan_part, w_part * 4);
     take(low, R * w_low * 4);
     take(hidden, (size_t)width * 4);
     take(logits, std::min<size_t>(R, LOGIT_ROWS) * m->n_vocab_pad * 4);

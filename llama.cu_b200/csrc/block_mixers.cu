@@ -219,30 +219,46 @@ __global__ void __launch_bounds__(128) window_pool_kernel(const attn_rows<T> p, 
 }
 
 // ------------------------------------------------------------------ recurrences over rows
-// Two launches.  The first lays a pass's rows out for the second, in binary32: per head and row q, k (rotated and scaled),
+// The first launch lays a pass's rows out for the next, in binary32: per head and row q, k (rotated and scaled),
 // the decays of a wkv layer and its bonus sum_i q_i u_i k_i (the same for every value column) as one run of `stride`
-// floats, and the values by blocks of `cols` columns.  The second walks the rows: a CTA owns `cols` value columns of one
+// floats, and the values by blocks of `cols` columns.  The next walks the rows: a CTA owns `cols` value columns of one
 // head with their whole state in registers - G lanes share NC columns, each lane holding KC channels of each - and rows
 // come in SC_ROWS at a time by bulk copies into a ring of stages.  Lane `sub` of a group holds channels
-// (c / 4) * 4 G + 4 sub + c % 4, so that a warp reads row vectors as contiguous 16-byte pieces.  The state is updated once
-// per row in row order, so neither the cut of a sequence into passes nor the pass length enters the arithmetic.
+// (c / 4) * 4 G + 4 sub + c % 4, so that a warp reads row vectors as contiguous 16-byte pieces.
+//
+// A walk is a chain of dependent rows (about 80 ns each, whatever the width), so long passes are cut into chunks of rows that
+// are walked side by side: one launch (SCAN_STATE) forms what every chunk adds to the state and the product of its decays, the
+// next (SCAN_CHUNK) starts every chunk from the states before it - S <- P S + local, chunk after chunk, in the CTA's registers -
+// and forms the results.  Everything stays products and sums in binary32 (no quotients of decays: a product that underflows is a
+// state that has faded).  A single walk of 2000 rows takes 155 to 160 us; a prompt of 2000 tokens at width 1024 (four layers of 16
+// heads of 64 x 64, four of 4 heads of 128 x 128) went from 3.32 to 2.20 ms.
 constexpr int SC_THREADS = 128;
 constexpr int SC_ROWS = 16;
 constexpr int SC_MAX_STAGES = 4;
-constexpr int SC_NC = 2;
+enum scan_mode { SCAN_WHOLE, SCAN_STATE, SCAN_CHUNK };
+// value columns per group of lanes: two keep a single walk's chain short, four halve the shared-memory reads per state entry
+// once chunks supply the warps
+__host__ __device__ constexpr int scan_nc(int kc, int mode) { return mode != SCAN_WHOLE && kc == 4 ? 4 : 2; }
 
 struct scan_shape {
   int kc, G, dimp, cols, blocks, stride;
 };
-scan_shape scan_shape_of(int dim, int vdim, bool wkv) {
+scan_shape scan_shape_of(int dim, int vdim, bool wkv, int mode) {
   scan_shape s;
   s.kc = dim <= 128 ? 4 : dim <= 256 ? 8 : 16;
   s.G = std::max(2, pow2_at_least((dim + s.kc - 1) / s.kc));
   s.dimp = s.G * s.kc;
-  s.cols = SC_THREADS / s.G * SC_NC;
+  s.cols = SC_THREADS / s.G * scan_nc(s.kc, mode);
   s.blocks = (vdim + s.cols - 1) / s.cols;
   s.stride = (wkv ? 3 : 2) * s.dimp + 4;
   return s;
+}
+// rows per chunk (a multiple of SC_ROWS), 0 = one walk over all rows.  Four CTAs per SM keep its arithmetic busy; both chunk
+// launches walk a chunk, so fewer than three chunks, or chunks shorter than the launch costs, gain nothing.
+constexpr int SC_MAX_CHUNKS = 32, SC_CTAS = 4 * 148;
+int scan_chunk_rows(const scan_shape& z, int heads, int m) {
+  const int chunks = std::min(std::min(SC_MAX_CHUNKS, m / 64), SC_CTAS / std::max(1, heads * z.blocks));
+  return chunks < 3 ? 0 : (m + chunks * SC_ROWS - 1) / (chunks * SC_ROWS) * SC_ROWS;
 }
 
 constexpr int SP_ROWS = 4;  // rows per warp
@@ -309,25 +325,30 @@ __global__ void __launch_bounds__(256) scan_prepare_kernel(const scan_rows<T> p,
   }
 }
 
-struct scan_args {  // what the second launch needs of scan_rows
+struct scan_args {  // what the walks need of scan_rows
   const float *packed, *packed_v, *decay;
   float *state, *out;
+  float* part;  // chunks: [chunk][head][block] {state entries, decays} of every thread; chunk 0: the state before the pass
   int dim, vdim, ldo;
   int* err;
 };
 
-template <int KC, int G, bool WKV>
-__global__ void __launch_bounds__(SC_THREADS) scan_kernel(const scan_args p, const scan_shape z, int m, int pos0, int n_stages) {
+template <int KC, int G, bool WKV, int MODE>
+__global__ void __launch_bounds__(SC_THREADS) scan_kernel(const scan_args p, const scan_shape z, int m, int pos0, int n_stages, int chunk_rows) {
+  constexpr int NC = scan_nc(KC, MODE);
   constexpr int RB = 4;                         // rows reduced together
-  constexpr int SPREAD = G < 8 ? G : 8;         // lanes of a group that end up with results
-  constexpr int KEEP = RB * SC_NC / SPREAD;     // results per such lane
-  constexpr int DIMP = G * KC, STRIDE = (WKV ? 3 : 2) * DIMP + 4, COLS = SC_THREADS / G * SC_NC;
+  constexpr int VALUES = RB * NC;
+  constexpr int SPREAD = G < VALUES ? G : VALUES;  // lanes of a group that end up with results
+  constexpr int KEEP = VALUES / SPREAD;            // results per such lane
+  constexpr int DIMP = G * KC, STRIDE = (WKV ? 3 : 2) * DIMP + 4, COLS = SC_THREADS / G * NC;
+  constexpr int PART = NC * KC + (WKV ? KC : 0);   // floats a thread leaves of a chunk
   extern __shared__ __align__(16) float sm[];
   __shared__ uint64_t bars[SC_MAX_STAGES];
   const int tid = threadIdx.x, sub = tid % G, grp = tid / G;
   const int head = blockIdx.x, v0 = blockIdx.y * COLS, D = p.dim, DV = p.vdim;
+  const int chunk = MODE == SCAN_WHOLE ? 0 : blockIdx.z, first = chunk * chunk_rows, rows_here = MODE == SCAN_WHOLE ? m : min(chunk_rows, m - first);
   constexpr int STAGE = SC_ROWS * (STRIDE + COLS);
-  const int n_tiles = (m + SC_ROWS - 1) / SC_ROWS;
+  const int n_tiles = (rows_here + SC_ROWS - 1) / SC_ROWS;
   if (tid == 0) {
     for (int i = 0; i < n_stages; ++i) mbar_init(smem_u32(&bars[i]), 1);
     fence_mbar_init();
@@ -335,10 +356,10 @@ __global__ void __launch_bounds__(SC_THREADS) scan_kernel(const scan_args p, con
   __syncthreads();
   pdl_launch_dependents();
   pdl_wait();
-  const float* rows = p.packed + (size_t)head * m * STRIDE;
-  const float* vals = p.packed_v + ((size_t)head * z.blocks + blockIdx.y) * m * COLS;
+  const float* rows = p.packed + ((size_t)head * m + first) * STRIDE;
+  const float* vals = p.packed_v + (((size_t)head * z.blocks + blockIdx.y) * m + first) * COLS;
   auto fetch = [&](int tile) {
-    const int s = tile % n_stages, nr = min(SC_ROWS, m - tile * SC_ROWS);
+    const int s = tile % n_stages, nr = min(SC_ROWS, rows_here - tile * SC_ROWS);
     const uint32_t bar = smem_u32(&bars[s]), dst = smem_u32(sm + s * STAGE);
     const uint32_t b0 = (uint32_t)(nr * STRIDE) * 4, b1 = (uint32_t)(nr * COLS) * 4;
     mbar_arrive_expect_tx(bar, b0 + b1);
@@ -348,107 +369,147 @@ __global__ void __launch_bounds__(SC_THREADS) scan_kernel(const scan_args p, con
   if (tid == 0)
     for (int t = 0; t < n_stages && t < n_tiles; ++t) fetch(t);
 
-  float S[SC_NC][KC];
+  float S[NC][KC], P[WKV && MODE == SCAN_STATE ? KC : 1];
   float* st = p.state + (size_t)head * D * DV;
-  const int c0 = v0 + grp * SC_NC;  // first of this group's columns
+  const int c0 = v0 + grp * NC;  // first of this group's columns
+  auto part_of = [&](int slot) { return p.part + (((size_t)slot * gridDim.x + head) * z.blocks + blockIdx.y) * (PART * SC_THREADS) + tid; };
+  const bool from_state = MODE == SCAN_WHOLE || (MODE == SCAN_STATE && chunk == 0);
 #pragma unroll
-  for (int n = 0; n < SC_NC; ++n)
+  for (int n = 0; n < NC; ++n)
 #pragma unroll
     for (int c = 0; c < KC; ++c) {
       const int i = (c >> 2) * 4 * G + 4 * sub + (c & 3);
-      S[n][c] = pos0 > 0 && c0 + n < DV && i < D ? st[(size_t)i * DV + c0 + n] : 0.f;
+      S[n][c] = from_state && pos0 > 0 && c0 + n < DV && i < D ? st[(size_t)i * DV + c0 + n] : 0.f;
     }
   const float dec = WKV ? 0.f : p.decay[head];
-  const bool odd = sub & 1;
+  if (MODE == SCAN_STATE && chunk == 0) {  // (the last chunk overwrites the state while others still start from it)
+    float* o = part_of(0);
+#pragma unroll
+    for (int j = 0; j < NC * KC; ++j) o[j * SC_THREADS] = S[j / KC][j % KC];
+  }
+  if (WKV && MODE == SCAN_STATE)
+#pragma unroll
+    for (int c = 0; c < KC; ++c) P[c] = 1.f;
+  if (MODE == SCAN_CHUNK) {
+    const float through = WKV ? 0.f : powf(dec, (float)chunk_rows);  // decay over a whole chunk
+    const float* o = part_of(chunk == 0 ? 0 : 1);                    // (slot 1 has the whole state behind chunk 0)
+#pragma unroll
+    for (int j = 0; j < NC * KC; ++j) S[j / KC][j % KC] = o[j * SC_THREADS];
+#pragma unroll 4
+    for (int b = 2; b <= chunk; ++b) {
+      o = part_of(b);
+#pragma unroll
+      for (int c = 0; c < KC; ++c) {
+        const float w = WKV ? o[(NC * KC + c) * SC_THREADS] : through;
+#pragma unroll
+        for (int n = 0; n < NC; ++n) S[n][c] = fmaf(w, S[n][c], o[(n * KC + c) * SC_THREADS]);
+      }
+    }
+  }
 
-  // one row: updates the state, leaves this lane's share of both columns' results in o
-  auto advance = [&](const float* row, const float* val, float (&o)[SC_NC]) {
-    const float2 v = *reinterpret_cast<const float2*>(val);
-    o[0] = o[1] = 0.f;
+  // one row: updates the state, leaves this lane's share of its columns' results in o
+  auto advance = [&](const float* row, const float* val, float (&o)[NC]) {
+    float v[NC];
+    if (NC == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(val);
+    else *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(val);
+#pragma unroll
+    for (int n = 0; n < NC; ++n) o[n] = 0.f;
 #pragma unroll
     for (int c4 = 0; c4 < KC / 4; ++c4) {
       const int at = c4 * 4 * G + 4 * sub;
-      const float4 q4 = *reinterpret_cast<const float4*>(row + at), k4 = *reinterpret_cast<const float4*>(row + DIMP + at);
-      float4 w4 = make_float4(dec, dec, dec, dec);
+      const float4 k4 = *reinterpret_cast<const float4*>(row + DIMP + at);
+      float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f), w4 = make_float4(dec, dec, dec, dec);
+      if (MODE != SCAN_STATE) q4 = *reinterpret_cast<const float4*>(row + at);
       if (WKV) w4 = *reinterpret_cast<const float4*>(row + 2 * DIMP + at);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int c = c4 * 4 + e;
         const float q = reinterpret_cast<const float*>(&q4)[e], k = reinterpret_cast<const float*>(&k4)[e], w = reinterpret_cast<const float*>(&w4)[e];
-        if (WKV) {
-          o[0] = fmaf(q, S[0][c], o[0]);
-          o[1] = fmaf(q, S[1][c], o[1]);
-        }
-        S[0][c] = fmaf(w, S[0][c], k * v.x);
-        S[1][c] = fmaf(w, S[1][c], k * v.y);
-        if (!WKV) {
-          o[0] = fmaf(q, S[0][c], o[0]);
-          o[1] = fmaf(q, S[1][c], o[1]);
+        if (WKV && MODE == SCAN_STATE) P[c] *= w;
+#pragma unroll
+        for (int n = 0; n < NC; ++n) {
+          if (WKV && MODE != SCAN_STATE) o[n] = fmaf(q, S[n][c], o[n]);
+          S[n][c] = fmaf(w, S[n][c], k * v[n]);
+          if (!WKV && MODE != SCAN_STATE) o[n] = fmaf(q, S[n][c], o[n]);
         }
       }
     }
   };
   for (int tile = 0; tile < n_tiles; ++tile) {
-    const int s = tile % n_stages, nr = min(SC_ROWS, m - tile * SC_ROWS);
+    const int s = tile % n_stages, nr = min(SC_ROWS, rows_here - tile * SC_ROWS);
     mbar_wait(smem_u32(&bars[s]), (uint32_t)(tile / n_stages) & 1u, p.err, DEV_ERR_FULL_WAIT);  // (expired: the error word is set, results are not used)
     const float* rs = sm + s * STAGE;
-    const float* vs = rs + SC_ROWS * STRIDE + grp * SC_NC;
-    float* out = p.out + (size_t)tile * SC_ROWS * p.ldo + head * DV;
-    // results of RB rows: lanes exchange halves - bit 0 of `sub` keeps one column, bit 1 one row of a pair, bit 2 one pair
-    auto finish = [&](const float (&o)[RB][SC_NC], int r) {
-      float x[RB];
+    const float* vs = rs + SC_ROWS * STRIDE + grp * NC;
+    float* out = p.out + (size_t)(first + tile * SC_ROWS) * p.ldo + head * DV;
+    // results of RB rows, value number row * NC + column: lanes exchange halves, bit after bit of `sub` keeps values with that
+    // bit of their number, until a lane has one left (or the group has no more lanes)
+    auto finish = [&](const float (&o)[RB][NC], int r) {
+      float x[VALUES];
 #pragma unroll
-      for (int b = 0; b < RB; ++b) x[b] = (odd ? o[b][1] : o[b][0]) + __shfl_xor_sync(0xffffffffu, odd ? o[b][0] : o[b][1], 1);
-      if (G >= 4) {
-        const bool up = sub & 2;
+      for (int i = 0; i < VALUES; ++i) x[i] = o[i / NC][i % NC];
 #pragma unroll
-        for (int b = 0; b < RB / 2; ++b) x[b] = (up ? x[2 * b + 1] : x[2 * b]) + __shfl_xor_sync(0xffffffffu, up ? x[2 * b] : x[2 * b + 1], 2);
+      for (int y = 1; y < G; y <<= 1) {
+        if (y < SPREAD) {
+          const bool up = sub & y;
+#pragma unroll
+          for (int i = 0; i < VALUES / (2 * y); ++i) x[i] = (up ? x[2 * i + 1] : x[2 * i]) + __shfl_xor_sync(0xffffffffu, up ? x[2 * i] : x[2 * i + 1], y);
+        } else {
+          x[0] += __shfl_xor_sync(0xffffffffu, x[0], y);
+        }
       }
-      if (G >= 8) {
-        const bool up = sub & 4;
-        x[0] = (up ? x[1] : x[0]) + __shfl_xor_sync(0xffffffffu, up ? x[0] : x[1], 4);
-      }
-#pragma unroll
-      for (int y = 8; y < G; y <<= 1) x[0] += __shfl_xor_sync(0xffffffffu, x[0], y);
-      if (sub < SPREAD && c0 + (sub & 1) < DV) {
+      if (sub < SPREAD && c0 + sub % NC < DV) {
 #pragma unroll
         for (int e = 0; e < KEEP; ++e) {
-          const int b = G >= 8 ? ((sub >> 1) & 1) + 2 * ((sub >> 2) & 1) : G >= 4 ? ((sub >> 1) & 1) + 2 * e : e;
+          const int at = e * SPREAD + sub, b = at / NC, n = at % NC;
+          if (SPREAD < NC && c0 + n >= DV) continue;
           float y = x[e];
-          if (WKV) y = fmaf(rs[(r + b) * STRIDE + STRIDE - 4], vs[(r + b) * COLS + (sub & 1)], y);
-          out[(size_t)(r + b) * p.ldo + c0 + (sub & 1)] = y;
+          if (WKV) y = fmaf(rs[(r + b) * STRIDE + STRIDE - 4], vs[(r + b) * COLS + n], y);
+          out[(size_t)(r + b) * p.ldo + c0 + n] = y;
         }
       }
     };
     int r = 0;
     if (nr == SC_ROWS) {  // whole tiles: the exchange of one row block runs beside the next block's arithmetic
-      float o[2][RB][SC_NC];
+      float o[2][RB][NC];
 #pragma unroll
       for (; r < SC_ROWS; r += RB) {
         const int cur = (r / RB) & 1;
 #pragma unroll
         for (int b = 0; b < RB; ++b) advance(rs + (r + b) * STRIDE, vs + (r + b) * COLS, o[cur][b]);
-        if (r > 0) finish(o[cur ^ 1], r - RB);
+        if (MODE != SCAN_STATE && r > 0) finish(o[cur ^ 1], r - RB);
       }
-      finish(o[(SC_ROWS / RB - 1) & 1], SC_ROWS - RB);
+      if (MODE != SCAN_STATE) finish(o[(SC_ROWS / RB - 1) & 1], SC_ROWS - RB);
     }
 #pragma unroll 1
     for (; r < nr; ++r) {
-      float o[SC_NC];
+      float o[NC];
       advance(rs + r * STRIDE, vs + r * COLS, o);
-      float y = (odd ? o[1] : o[0]) + __shfl_xor_sync(0xffffffffu, odd ? o[0] : o[1], 1);
 #pragma unroll
-      for (int b = 2; b < G; b <<= 1) y += __shfl_xor_sync(0xffffffffu, y, b);
-      if (sub < 2 && c0 + sub < DV) {
-        if (WKV) y = fmaf(rs[r * STRIDE + STRIDE - 4], vs[r * COLS + sub], y);
-        out[(size_t)r * p.ldo + c0 + sub] = y;
+      for (int n = 0; n < NC && MODE != SCAN_STATE; ++n) {
+        float y = o[n];
+#pragma unroll
+        for (int b = 1; b < G; b <<= 1) y += __shfl_xor_sync(0xffffffffu, y, b);
+        if (sub == n % G && c0 + n < DV) {
+          if (WKV) y = fmaf(rs[r * STRIDE + STRIDE - 4], vs[r * COLS + n], y);
+          out[(size_t)r * p.ldo + c0 + n] = y;
+        }
       }
     }
     __syncthreads();  // the stage may be overwritten
     if (tid == 0 && tile + n_stages < n_tiles) fetch(tile + n_stages);
   }
+  if (MODE == SCAN_STATE) {
+    float* o = part_of(chunk + 1);
 #pragma unroll
-  for (int n = 0; n < SC_NC; ++n)
+    for (int j = 0; j < NC * KC; ++j) o[j * SC_THREADS] = S[j / KC][j % KC];
+    if (WKV)
+#pragma unroll
+      for (int c = 0; c < KC; ++c) o[(NC * KC + c) * SC_THREADS] = P[c];
+    return;
+  }
+  if (MODE == SCAN_CHUNK && first + rows_here < m) return;
+#pragma unroll
+  for (int n = 0; n < NC; ++n)
 #pragma unroll
     for (int c = 0; c < KC; ++c) {
       const int i = (c >> 2) * 4 * G + 4 * sub + (c & 3);
@@ -456,24 +517,32 @@ __global__ void __launch_bounds__(SC_THREADS) scan_kernel(const scan_args p, con
     }
 }
 
-template <int KC, int G, bool WKV>
-int launch_scan_shape(const scan_args& a, const scan_shape& z, int heads, int m, int pos0, cudaStream_t stream) {
+template <int KC, int G, bool WKV, int MODE>
+int launch_scan_shape(const scan_args& a, const scan_shape& z, int heads, int m, int pos0, int chunk_rows, cudaStream_t stream) {
   const size_t stage = (size_t)SC_ROWS * (z.stride + z.cols) * sizeof(float);
-  const int n_stages = (int)std::min<size_t>(SC_MAX_STAGES, (200 * 1024) / stage);
+  // (chunks: three stages leave room for four CTAs per SM)
+  const int n_stages = (int)std::min<size_t>(MODE == SCAN_WHOLE ? SC_MAX_STAGES : SC_MAX_STAGES - 1, (200 * 1024) / stage);
   static bool attr_done[16] = {};
   int dev = 0;
   LCU_CUDA(cudaGetDevice(&dev));
   if (dev < 16 && !attr_done[dev]) {
-    LCU_CUDA(cudaFuncSetAttribute((scan_kernel<KC, G, WKV>), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    LCU_CUDA(cudaFuncSetAttribute((scan_kernel<KC, G, WKV, MODE>), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     attr_done[dev] = true;
   }
-  LCU_CUDA(launch_after(scan_kernel<KC, G, WKV>, dim3(heads, z.blocks), dim3(SC_THREADS), stage * n_stages, stream, a, z, m, pos0, n_stages));
+  const int chunks = MODE == SCAN_WHOLE ? 1 : (m + chunk_rows - 1) / chunk_rows - (MODE == SCAN_STATE);  // (nothing follows the last chunk)
+  LCU_CUDA(launch_after(scan_kernel<KC, G, WKV, MODE>, dim3(heads, z.blocks, chunks), dim3(SC_THREADS), stage * n_stages, stream, a, z, m, pos0, n_stages,
+                        chunk_rows));
   return LCU_OK;
 }
 
 template <bool WKV>
-int launch_scan_kernel(const scan_args& a, const scan_shape& z, int heads, int m, int pos0, cudaStream_t stream) {
-#define LCU_SCAN(KC, GG) if (z.kc == KC && z.G == GG) return launch_scan_shape<KC, GG, WKV>(a, z, heads, m, pos0, stream)
+int launch_scan_kernel(const scan_args& a, const scan_shape& z, int heads, int m, int pos0, int chunk_rows, cudaStream_t stream) {
+#define LCU_SCAN(KC, GG)                                                                                        \
+  if (z.kc == KC && z.G == GG) {                                                                                \
+    if (!chunk_rows) return launch_scan_shape<KC, GG, WKV, SCAN_WHOLE>(a, z, heads, m, pos0, 0, stream);        \
+    const int rc = launch_scan_shape<KC, GG, WKV, SCAN_STATE>(a, z, heads, m, pos0, chunk_rows, stream);        \
+    return rc ? rc : launch_scan_shape<KC, GG, WKV, SCAN_CHUNK>(a, z, heads, m, pos0, chunk_rows, stream);      \
+  }
   LCU_SCAN(4, 2);
   LCU_SCAN(4, 4);
   LCU_SCAN(4, 8);
@@ -752,21 +821,27 @@ int launch_window_attention(const attn_rows<T>& p, int m, int pos0, cudaStream_t
 
 template <typename T>
 int launch_scan(const scan_rows<T>& p, bool wkv, int m, int pos0, cudaStream_t stream) {
-  const scan_shape z = scan_shape_of(p.dim, p.vdim, wkv);
+  scan_shape z = scan_shape_of(p.dim, p.vdim, wkv, SCAN_CHUNK);
+  const int chunk_rows = scan_chunk_rows(z, p.heads, m);
+  if (!chunk_rows) z = scan_shape_of(p.dim, p.vdim, wkv, SCAN_WHOLE);
   const dim3 grid((m + SP_ROWS - 1) / SP_ROWS, (p.heads + 7) / 8);
   if (wkv) LCU_CUDA(launch_after(scan_prepare_kernel<T, true>, grid, dim3(256), 0, stream, p, z, m, pos0));
   else LCU_CUDA(launch_after(scan_prepare_kernel<T, false>, grid, dim3(256), 0, stream, p, z, m, pos0));
-  const scan_args a{p.packed, p.packed_v, p.decay, p.state, p.out, p.dim, p.vdim, p.ldo, p.err};
-  return wkv ? launch_scan_kernel<true>(a, z, p.heads, m, pos0, stream) : launch_scan_kernel<false>(a, z, p.heads, m, pos0, stream);
+  const scan_args a{p.packed, p.packed_v, p.decay, p.state, p.out, p.part, p.dim, p.vdim, p.ldo, p.err};
+  return wkv ? launch_scan_kernel<true>(a, z, p.heads, m, pos0, chunk_rows, stream) : launch_scan_kernel<false>(a, z, p.heads, m, pos0, chunk_rows, stream);
 }
 
-void scan_scratch(int heads, int dim, int vdim, bool wkv, size_t rows, size_t* packed_floats, size_t* value_floats) {
-  const scan_shape z = scan_shape_of(dim, vdim, wkv);
+void scan_scratch(int heads, int dim, int vdim, bool wkv, size_t rows, size_t* packed_floats, size_t* value_floats, size_t* part_floats) {
+  const scan_shape whole = scan_shape_of(dim, vdim, wkv, SCAN_WHOLE), z = scan_shape_of(dim, vdim, wkv, SCAN_CHUNK);
   *packed_floats = heads * rows * z.stride;
-  *value_floats = heads * rows * z.blocks * z.cols;
+  *value_floats = heads * rows * std::max(whole.blocks * whole.cols, z.blocks * z.cols);
+  // (passes of fewer rows have no more chunks)
+  const int chunk_rows = scan_chunk_rows(z, heads, (int)rows);
+  const size_t chunks = chunk_rows ? std::min<size_t>(std::min<size_t>(SC_MAX_CHUNKS, rows / 64), SC_CTAS / (heads * z.blocks)) : 0;
+  *part_floats = chunks * heads * z.blocks * SC_THREADS * z.kc * (scan_nc(z.kc, SCAN_CHUNK) + (wkv ? 1 : 0));
 }
 void scan_decay_layout(int dim, int vdim, int m, size_t* head_stride, size_t* row_stride, size_t* offset) {
-  const scan_shape z = scan_shape_of(dim, vdim, true);
+  const scan_shape z = scan_shape_of(dim, vdim, true, SCAN_WHOLE);  // (the same for chunks)
   *head_stride = (size_t)m * z.stride;
   *row_stride = z.stride;
   *offset = 2 * (size_t)z.dimp;

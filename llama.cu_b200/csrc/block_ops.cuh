@@ -179,10 +179,10 @@ struct scan_rows {
   const float* u;         // wkv: [heads][dim]
   float* out;             // [rows][ldo] binary32
   int ldo;
-  float *packed, *packed_v;  // scratch of scan_scratch() floats; wkv: the decays are in `packed` already (scan_decay_layout)
+  float *packed, *packed_v, *part;  // scratch of scan_scratch() floats; wkv: the decays are in `packed` already (scan_decay_layout)
   int* err;
 };
-void scan_scratch(int heads, int dim, int vdim, bool wkv, size_t rows, size_t* packed_floats, size_t* value_floats);
+void scan_scratch(int heads, int dim, int vdim, bool wkv, size_t rows, size_t* packed_floats, size_t* value_floats, size_t* part_floats);
 // where the decay of (head, row, channel) of an m-row pass goes: packed[offset + head * head_stride + row * row_stride + channel]
 void scan_decay_layout(int dim, int vdim, int m, size_t* head_stride, size_t* row_stride, size_t* offset);
 template <typename T>
