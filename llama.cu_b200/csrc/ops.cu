@@ -346,13 +346,19 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 }
 
 // q = u8(roundf(127.5f + x / s)).  For the inputs the quantizer can see - x a finite half, s a positive finite half, |x|
-// within the absmax that rounds to s - the byte comes out of one addition and a truncating conversion instead of the
-// addition and roundf.  quantizer_check_kernel compares the two for every such pair (2 x 10^9 of them) on the device, and
-// tests/test_gpu_kernels.py requires zero differences.
+// within the absmax that rounds to s - the byte is x / s + 128, both operations rounded, without its fraction.  A block's elements
+// share the division r = 1 / s: t = x r is corrected by its remainder (P. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990: with r the rounded reciprocal, t + (x - t s) r is the rounded quotient),
+// and a sum with 2^23 rounded down leaves the byte in the low bits.  Five operations and no branch per element, where the division
+// took about twenty.  quantizer_check_kernel compares the byte with the reference's expression for every such pair (more than 10^9) on
+// the device, and tests/test_gpu_kernels.py requires zero differences.
 __device__ __forceinline__ uint32_t quant_byte_reference(float x, float s) { return static_cast<uint8_t>(roundf(127.5f + x / s)); }
-__device__ __forceinline__ uint32_t quant_byte_fast(float x, float s) {
-  return static_cast<uint8_t>(x / s + 128.0f);  // trunc((127.5f + x / s) + 0.5f) in one addition
+__device__ __forceinline__ uint32_t quant_bits(float x, float s, float r) {  // low byte: q
+  const float t = x * r;
+  return __float_as_uint(__fadd_rd(fmaf(fmaf(-t, s, x), r, t) + 128.0f, 8388608.0f));
 }
+// Scales below the normal halves may be far from absmax / 127.5, and sums then leave 0 .. 255: the reference's own instructions.
+constexpr float QUANT_MIN_SCALE = 6.103515625e-5f;
 
 // every (x, s) pair of the quantizer's domain: s = positive finite half number blockIdx.x * 256 + threadIdx.x..., x every
 // finite half with |x| <= the largest absmax whose scale rounds to s.  counts[0] = pairs checked, counts[1] = differences.
@@ -367,7 +373,8 @@ __global__ void __launch_bounds__(256) quantizer_check_kernel(unsigned long long
       // in the domain iff a block with this absmax would get this scale
       if (__half_as_ushort(__float2half(fabsf(x) / 127.5f)) > sb) continue;
       ++checked;
-      if (quant_byte_reference(x, s) != quant_byte_fast(x, s)) ++diff;
+      const uint32_t got = s < QUANT_MIN_SCALE ? quant_byte_reference(x, s) : quant_bits(x, s, 1.0f / s) & 0xffu;
+      if (quant_byte_reference(x, s) != got) ++diff;
     }
   }
   checked = warp_sum_u64(checked);
@@ -378,58 +385,71 @@ __global__ void __launch_bounds__(256) quantizer_check_kernel(unsigned long long
   }
 }
 
-// The same arithmetic with 16-byte loads: a thread holds eight consecutive halves in registers (read once), the
-// BS / 8 neighbouring lanes that share a block agree on the block's absmax with xor shuffles, and every thread stores
-// its eight bytes at once.  Block sizes 32 .. 256 (4 .. 32 lanes per block); n_vec = elements / 8.
+// The same arithmetic with 16-byte loads: a thread holds sixteen consecutive halves in registers (read once), the
+// BS / 16 neighbouring lanes that share a block agree on the block's absmax with xor shuffles, and every thread stores
+// its sixteen bytes at once (wide_q: q is 16-byte aligned).  Block sizes 32 .. 256 (2 .. 16 lanes per block); n_vec = elements / 16.
+// HBM-bound: 32000 x 4096 in 72 us (5.5 TB/s); with a division per byte it was bound by instructions, 125 us.
 template <int LANES>
-__global__ void __launch_bounds__(256) quantize8_kernel(uint8_t* q, __half* scales, const __half* in, size_t n_vec) {
+__global__ void __launch_bounds__(256) quantize16_kernel(uint8_t* q, __half* scales, const __half* in, size_t n_vec, int wide_q) {
   constexpr int UNROLL = 2;  // vectors per thread whose loads are in flight together
   const size_t stride = (size_t)gridDim.x * 256;
   const size_t n_round = (n_vec + 31) / 32 * 32;  // whole warps take part in the shuffles
   for (size_t v0 = (size_t)blockIdx.x * 256 + threadIdx.x; v0 < n_round; v0 += UNROLL * stride) {
-    uint4 raw[UNROLL];
+    uint4 raw[UNROLL][2];
 #pragma unroll
     for (int r = 0; r < UNROLL; ++r) {
       const size_t v = v0 + r * stride;
-      raw[r] = v < n_vec ? *reinterpret_cast<const uint4*>(in + v * 8) : make_uint4(0, 0, 0, 0);
+      const uint4* src = reinterpret_cast<const uint4*>(in + v * 16);
+      raw[r][0] = v < n_vec ? src[0] : make_uint4(0, 0, 0, 0);
+      raw[r][1] = v < n_vec ? src[1] : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int r = 0; r < UNROLL; ++r) {
       const size_t v = v0 + r * stride;
       if (v >= n_round) break;  // (warp-uniform: v and n_round are multiples of 32 apart from the lane)
       const bool valid = v < n_vec;
-      const __half2* h2 = reinterpret_cast<const __half2*>(&raw[r]);
-      float f[8];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 p = __half22float2(h2[e]);
-        f[2 * e] = p.x;
-        f[2 * e + 1] = p.y;
-      }
+      const __half2* h2 = reinterpret_cast<const __half2*>(&raw[r][0]);
       // absmax on the packed halves (the maximum of halves is exact in any format; NaNs are passed over as fmaxf does)
       __half2 am2 = __hmax2(__hmax2(__habs2(h2[0]), __habs2(h2[1])), __hmax2(__habs2(h2[2]), __habs2(h2[3])));
+      am2 = __hmax2(am2, __hmax2(__hmax2(__habs2(h2[4]), __habs2(h2[5])), __hmax2(__habs2(h2[6]), __habs2(h2[7]))));
       float absmax_val = fmaxf(0.f, fmaxf(__low2float(am2), __high2float(am2)));
 #pragma unroll
       for (int o = LANES / 2; o > 0; o >>= 1) absmax_val = fmaxf(absmax_val, __shfl_xor_sync(0xffffffffu, absmax_val, o));
       const __half s_absmax = __float2half(absmax_val / 127.5f);
       const float sf = __half2float(s_absmax);
+      // a NaN among finite values is passed over by the maximum, but not by this sum (0 x infinity is one as well)
+      __half2 zero = __hmul2(h2[0], __float2half2_rn(0.f));
+#pragma unroll
+      for (int e = 1; e < 8; ++e) zero = __hfma2(h2[e], __float2half2_rn(0.f), zero);
       if (!valid) continue;
       if ((v & (LANES - 1)) == 0) scales[v / LANES] = s_absmax;
-      uint32_t lo = 0, hi = 0;
-      if (sf > 0.f && absmax_val < CUDART_INF_F) {  // (block-uniform) the checked domain: finite values, positive scale
+      uint32_t word[4];
+      // outside the checked domain - scales that are not normal halves (all-zero blocks: 0 / 0), infinities, NaNs - the
+      // reference's own instructions
+      if (sf >= QUANT_MIN_SCALE && absmax_val < CUDART_INF_F && __low2float(zero) == 0.f && __high2float(zero) == 0.f) {
+        const float inv = 1.0f / sf;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          lo |= quant_byte_fast(f[e], sf) << (8 * e);
-          hi |= quant_byte_fast(f[e + 4], sf) << (8 * e);
+        for (int w = 0; w < 4; ++w) {
+          const float2 a = __half22float2(h2[2 * w]), b = __half22float2(h2[2 * w + 1]);
+          const uint32_t b0 = quant_bits(a.x, sf, inv), b1 = quant_bits(a.y, sf, inv), b2 = quant_bits(b.x, sf, inv), b3 = quant_bits(b.y, sf, inv);
+          word[w] = __byte_perm(__byte_perm(b0, b1, 0x0040), __byte_perm(b2, b3, 0x0040), 0x5410);
         }
-      } else {  // an all-zero block (0 / 0), infinities or NaNs: the reference's own instructions
+      } else {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          lo |= quant_byte_reference(f[e], sf) << (8 * e);
-          hi |= quant_byte_reference(f[e + 4], sf) << (8 * e);
+        for (int w = 0; w < 4; ++w) {
+          const float2 a = __half22float2(h2[2 * w]), b = __half22float2(h2[2 * w + 1]);
+          const float f[4] = {a.x, a.y, b.x, b.y};
+          word[w] = 0;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) word[w] |= quant_byte_reference(f[e], sf) << (8 * e);
         }
       }
-      *reinterpret_cast<uint2*>(q + v * 8) = make_uint2(lo, hi);
+      if (wide_q) {
+        *reinterpret_cast<uint4*>(q + v * 16) = make_uint4(word[0], word[1], word[2], word[3]);
+      } else {
+        *reinterpret_cast<uint2*>(q + v * 16) = make_uint2(word[0], word[1]);
+        *reinterpret_cast<uint2*>(q + v * 16 + 8) = make_uint2(word[2], word[3]);
+      }
     }
   }
 }
@@ -736,13 +756,14 @@ int launch_quantize_absmax_uint8(uint8_t* q, __half* scales, const __half* in, s
   if (n_blocks == 0) return LCU_OK;
   const bool vec_ok = (((uintptr_t)in & 15) | ((uintptr_t)q & 7)) == 0;
   if (vec_ok && (bs == 32 || bs == 64 || bs == 128 || bs == 256)) {
-    const size_t n_vec = n_blocks * (size_t)(bs / 8);
-    size_t grid8 = (n_vec + 255) / 256;
-    if (grid8 > 148 * 8) grid8 = 148 * 8;
-    if (bs == 32) quantize8_kernel<4><<<(unsigned)grid8, 256, 0, stream>>>(q, scales, in, n_vec);
-    else if (bs == 64) quantize8_kernel<8><<<(unsigned)grid8, 256, 0, stream>>>(q, scales, in, n_vec);
-    else if (bs == 128) quantize8_kernel<16><<<(unsigned)grid8, 256, 0, stream>>>(q, scales, in, n_vec);
-    else quantize8_kernel<32><<<(unsigned)grid8, 256, 0, stream>>>(q, scales, in, n_vec);
+    const size_t n_vec = n_blocks * (size_t)(bs / 16);
+    const int wide_q = ((uintptr_t)q & 15) == 0;
+    // (a CTA per 512 vectors: persistent CTAs took 5 % longer)
+    const size_t grid16 = std::min<size_t>((n_vec + 511) / 512, 1u << 30);
+    if (bs == 32) quantize16_kernel<2><<<(unsigned)grid16, 256, 0, stream>>>(q, scales, in, n_vec, wide_q);
+    else if (bs == 64) quantize16_kernel<4><<<(unsigned)grid16, 256, 0, stream>>>(q, scales, in, n_vec, wide_q);
+    else if (bs == 128) quantize16_kernel<8><<<(unsigned)grid16, 256, 0, stream>>>(q, scales, in, n_vec, wide_q);
+    else quantize16_kernel<16><<<(unsigned)grid16, 256, 0, stream>>>(q, scales, in, n_vec, wide_q);
     LCU_CUDA(cudaGetLastError());
     return LCU_OK;
   }

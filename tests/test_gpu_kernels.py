@@ -50,6 +50,30 @@ def test_quantizer_bit_exact(lcu, h, w, bs):
     assert (dq == do).all()
 
 
+@pytest.mark.parametrize("bs", [32, 64, 128, 256])
+@pytest.mark.parametrize("blocks", [1, 3, 9, 517])
+def test_quantizer_equal_on_every_alignment(lcu, bs, blocks):
+    """The vector kernel (16-byte aligned input; whole and halved stores) against the plain one, which input at 8 bytes takes: any
+    bit patterns, ordinary values, sparse rows, values half way between two bytes."""
+    rng = np.random.default_rng(bs + blocks)
+    x = rng.integers(0, 1 << 16, (blocks, bs)).astype(np.uint16)
+    x[::3] = f16(rng.standard_normal(x[::3].shape) * 0.02)
+    x[1::6] = f16(rng.standard_normal(x[1::6].shape) * (rng.random(x[1::6].shape) < 0.1))
+    half = rng.integers(-127, 127, x[4::6].shape)  # (scale 1/64: every other value is a whole or a half number of scales)
+    half[:, 0] = 255
+    x[4::6] = f16(half / 128)
+    raw = lcu.DeviceBuffer(x.nbytes + 32)
+    outs = []
+    for at, q_at in ((0, 0), (16, 8), (8, 0)):
+        lcu.check(lcu.lib.lcu_memcpy_h2d(raw.ptr.value + at, x.ctypes.data, x.nbytes))
+        q, s = lcu.DeviceBuffer(x.size + 32), lcu.DeviceBuffer(blocks * 2)
+        lcu.check(lcu.lib.lcu_quantize_absmax_uint8(q.ptr.value + q_at, s.ptr, raw.ptr.value + at, blocks, bs, bs, None))
+        lcu.check(lcu.lib.lcu_synchronize())
+        outs.append((q.to_host(np.uint8, (x.size + 32,))[q_at:q_at + x.size], s.to_host(np.uint16, (blocks,))))
+    for q, s in outs[:2]:
+        assert (q == outs[2][0]).all() and (s == outs[2][1]).all()
+
+
 def test_quantizer_empty_and_bad_block(lcu):
     q, s = lcu.quantize(np.zeros((0, 128), np.uint16), 128)
     assert q.shape == (0, 128) and s.shape == (0, 1)
@@ -231,8 +255,8 @@ def test_gate_arithmetic_against_the_division_for_every_half(lcu):
 
 
 def test_quantizer_arithmetic_on_its_whole_domain(lcu):
-    """The quantizer truncates x / scale + 128 instead of rounding 127.5f + x / scale (transform.cu:60-80).  The device
-    compares the two for every pair the quantizer can meet - every positive finite half as scale, every finite half within
+    """The quantizer truncates x / scale + 128, the quotient formed from the block's 1 / scale, instead of rounding
+    127.5f + x / scale (transform.cu:60-80).  The device compares the two for every pair the quantizer can meet - every positive finite half as scale, every finite half within
     the absmax that rounds to it: about two billion pairs - and must find no differing byte."""
     import ctypes as C
     checked, diff = C.c_uint64(0), C.c_uint64(0)
