@@ -81,4 +81,12 @@ inline int launch_gemm_tc_gated(__half* out, const __half* lhs, int ldx, const _
   return launch_gemm_tc_gated(TC_F16, out, lhs, ldx, w13, m, f, K, err, stream, tile_n);
 }
 
+// 8-bit weights expanded inside the product (gemm_u8.cu): out[m][N] = half(x[m][K] . half((q - 127.5) * scale)^T + beta * out), x and out
+// dense.  From 2 rows, K a multiple of 256, N even, blocks of 32 / 64 / 128; no workspace.
+// gemm_u8_plan: activation rows per tile and CTAs that share a tile's K.  Pure host arithmetic.
+bool gemm_u8_supported(int m, int N, int K, int bs, const void* lhs, const void* q, const void* scales);
+void gemm_u8_plan(int m, int N, int K, int sms, int* tile_rows, int* splits);
+int launch_gemm_u8(__half* out, const __half* lhs, const uint8_t* q, const __half* scales, int bs, int m, int N, int K, float beta, int* err,
+                   cudaStream_t stream);
+
 }  // namespace lcu

@@ -37,6 +37,11 @@ int matmul_rows(__half* out, const __half* lhs, const dev_matrix& w, int m, floa
   }
   const int pass_rows = gemv_max_rows(K);  // 8, fewer where the activation rows are long
   LCU_REQUIRE(pass_rows >= 1, "matmul_nt: a row of K=%d does not fit in shared memory", K);
+  // u8 without scratch.  A single GEMV pass is as fast while K is short (2 rows of 1024 x 1024: 5.8 us against 6.8; 2 of 4096 x 4096:
+  // 10.5 against 10.6; 4 of 11008 x 512: 23.6 against 11.5); every further pass reads the matrix again (400 of 4096 x 4096: 994 against 21).
+  if (w.bs > 0 && pt.u8_deq_min_rows > 0 && m >= pt.u8_deq_min_rows && (m > pass_rows || K > 2048) &&
+      gemm_u8_supported(m, N, K, w.bs, lhs, w.w, w.sc))
+    return launch_gemm_u8(out, lhs, (const uint8_t*)w.w, w.sc, w.bs, m, N, K, beta, err, stream);
   for (int t = 0; t < m; t += pass_rows) {
     gemv_params p{};
     p.w[0] = w.w;

@@ -29,7 +29,8 @@ prefill_tuning& prefill_tuning_ref();
 int& matmul_type_ref();
 
 // Dispatch: fp16 weights with at least tc_min_rows (2) rows of a shape the tcgen05 GEMM takes go to it (gemm_tc.cu);
-// one row, other shapes, and u8 weights without scratch (in passes of 8 rows) go through the weight-streaming GEMV.
+// u8 weights without scratch expand inside the product (gemm_u8.cu, from u8_deq_min_rows rows); one row and other shapes go
+// through the weight-streaming GEMV, in passes of 8 rows.
 // lhs and out are dense row-major ([m][K], [m][N]); err is the device error word.
 // deq / deq_halves: scratch for one dequantized matrix; with it, u8 weights and at least u8_deq_min_rows rows are
 // expanded to fp16 (the values the reference's tile kernel builds in shared memory, llama_cu.cu:222-300) and

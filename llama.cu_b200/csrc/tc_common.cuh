@@ -36,6 +36,44 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
                "l"(map), "r"(x), "r"(y), "r"(bar)
                : "memory");
 }
+// Single-thread instructions (tcgen05.mma, commit, tensor copies) take their operands from uniform registers.  Under
+// `if (lane == 0)` the compiler cannot see that one thread runs and moves every operand over, for each instruction; issuing
+// warps therefore keep their loops, waits and addresses common to the warp and elect a lane around the instructions alone.
+__device__ __forceinline__ bool tc_elect() {  // true for one lane (always the same) of a converged warp
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
+// mbar_wait by a whole warp with one outcome for all lanes
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int* err, int code) {
+  constexpr uint32_t ALL = 0xffffffffu;
+  if (__all_sync(ALL, mbar_try_wait(bar, parity))) return true;
+  const long long t0 = clock64();
+  long long next_check = 400000;
+  for (;;) {
+    if (__all_sync(ALL, mbar_try_wait(bar, parity))) return true;
+    const long long dt = clock64() - t0;
+    if (__any_sync(ALL, dt > next_check)) {
+      if (__any_sync(ALL, *(volatile int*)err != 0)) return false;
+      if (__any_sync(ALL, dt > 2000000000ll)) {
+        atomicCAS(err, 0, code);
+        return false;
+      }
+      next_check += 400000;
+    }
+  }
+}
+// place in a ring of n slots and the parity of its barriers in this round
+struct tc_ring {
+  int slot = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void step(int n) {
+    if (++slot == n) {
+      slot = 0;
+      phase ^= 1u;
+    }
+  }
+};
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {

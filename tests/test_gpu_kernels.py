@@ -139,6 +139,36 @@ def test_matmul_small_shapes(lcu, m, k, n, bs, beta):
     assert np.abs(f32(y) - f32(yo)).max() <= 2e-3 * scale, (m, k, n, bs)
 
 
+@pytest.mark.parametrize("bs", [32, 64, 128])
+@pytest.mark.parametrize("m,k,n,beta", [(2, 4096, 2, 0.0), (17, 256, 128, 1.0), (9, 512, 130, 0.0), (224, 512, 384, 0.0), (225, 1280, 96, 1.0),
+                                        # K split over 2, 4 and 8 CTAs, ragged last tile
+                                        (40, 1024, 1026, 1.0), (300, 2048, 200, 0.0), (9, 11008, 64, 1.0),
+                                        # more tiles than SMs, several row tiles
+                                        (460, 256, 9000, 0.0)])
+def test_product_expands_8_bit_weights(lcu, m, k, n, beta, bs):
+    """Several rows: 8-bit weights are expanded inside the tcgen05 product: against the oracle's product over the same half-rounded
+    weights (binary32 sums in another order, |error| <= k 2^-24 sum|x w|, far below the result's rounding to half), and against the
+    GEMV passes of 8 rows."""
+    rng = np.random.default_rng(m + n + bs)
+    x = f16(rng.standard_normal((m, k)))
+    w = O.synth_f16(n * k, 5, f"u8{n}x{k}", 0.05).reshape(n, k)
+    q, s = O.quantize(w, n, k, bs)
+    prev = f16(rng.standard_normal((m, n)))
+    yo = prev.copy()
+    L.orc_matmul_nt_fp16u8(yo.reshape(-1), x.reshape(-1), q.reshape(-1), s.reshape(-1), m, k, n, bs, beta, 2)
+    y = lcu.matmul_nt(x, q, s, bs, beta=beta, out_u16=prev)
+    assert np.array_equal(y, lcu.matmul_nt(x, q, s, bs, beta=beta, out_u16=prev))
+    lcu.check(lcu.lib.lcu_set_tuning(b"prefill_u8_deq_min_rows", 1000000))
+    try:
+        y_gemv = lcu.matmul_nt(x, q, s, bs, beta=beta, out_u16=prev)
+    finally:
+        lcu.check(lcu.lib.lcu_set_tuning(b"prefill_u8_deq_min_rows", 2))
+    # one unit of the half format at the largest output where the sums round to different sides, and the sums' own error
+    bound = float(np.abs(f32(yo)).max()) * 2.0 ** -10 + k * 2.0 ** -24 * float(np.abs(f32(x)).sum(1).max()) * float(np.abs(f32(w)).max())
+    assert np.abs(f32(y) - f32(yo)).max() <= bound
+    assert np.abs(f32(y) - f32(y_gemv)).max() <= bound
+
+
 @pytest.mark.parametrize("m,k,n,beta,tile", [(9, 64, 32, 0.0, 0), (16, 256, 32, 1.0, 0), (128, 64, 128, 0.0, 128), (129, 512, 192, 1.0, 0),
                                              (200, 1024, 256, 1.0, 64), (77, 4096, 1024, 0.0, 32), (300, 11008, 128, 0.0, 0),
                                              (257, 4096, 4096, 1.0, 0),
