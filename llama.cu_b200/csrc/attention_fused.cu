@@ -118,16 +118,16 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attn_fused_kernel(const __grid_
   const int n_tiles = min(t_tiles, (pos0 + m0 + FA_BM + FA_BN - 1) / FA_BN);       // key tiles that hold a visible key
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---- loads: Q; pass 1: K_0 .. K_{n-1}; pass 2: K_0, V_0, K_1, V_1, ...  (item i lives in ring stage i % FA_RING)
+    if (tc_elect()) {
+      // ---- loads: Q; pass 1: K_0 .. K_{n-1}; pass 2: K_0, V_0, K_1, V_1, ...  (one ring stage each)
       mbar_arrive_expect_tx(smem_u32(&bars[B_Q]), OPERAND);
       for (int kb = 0; kb < NKB; ++kb) tma_load_3d(q_addr + kb * BLOCK_BYTES, &map_q, kb * 64, head, m0, smem_u32(&bars[B_Q]));
       const int items = 3 * n_tiles;
-      for (int it = 0; it < items; ++it) {
-        const int s = it % FA_RING, use = it / FA_RING;
-        if (use > 0 && !mbar_wait(smem_u32(&bars[B_EMPTY + s]), (use - 1) & 1, p.err, DEV_ERR_EMPTY_WAIT)) break;
-        const uint32_t full = smem_u32(&bars[B_FULL + s]);
-        const uint32_t dst = ring_addr + (uint32_t)s * OPERAND;
+      tc_ring r;
+      for (int it = 0; it < items; ++it, r.step(FA_RING)) {
+        if (!mbar_wait(smem_u32(&bars[B_EMPTY + r.slot]), r.phase ^ 1u, p.err, DEV_ERR_EMPTY_WAIT)) break;
+        const uint32_t full = smem_u32(&bars[B_FULL + r.slot]);
+        const uint32_t dst = ring_addr + (uint32_t)r.slot * OPERAND;
         mbar_arrive_expect_tx(full, OPERAND);
         const bool is_v = it >= n_tiles && ((it - n_tiles) & 1);
         const int j = it < n_tiles ? it : (it - n_tiles) >> 1;
@@ -140,17 +140,18 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attn_fused_kernel(const __grid_
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---- MMAs.  sidx counts score tiles over both passes: tile sidx uses accumulator sidx & 1.
-      bool ok = mbar_wait(smem_u32(&bars[B_Q]), 0, p.err, DEV_ERR_FULL_WAIT);
-      int sidx = 0;
-      auto scores = [&](int item) {  // S[sidx & 1] = Q K^T with the K tile of ring item `item`
-        const int s = item % FA_RING, b = sidx & 1;
-        ok = ok && mbar_wait(smem_u32(&bars[B_S_EMPTY + b]), ((uint32_t)(sidx >> 1) & 1u) ^ 1u, p.err, DEV_ERR_TMEM_WAIT);
-        ok = ok && mbar_wait(smem_u32(&bars[B_FULL + s]), (uint32_t)(item / FA_RING) & 1u, p.err, DEV_ERR_FULL_WAIT);
-        if (!ok) return;
-        tc_fence_after();
+    // ---- MMAs.  Score tiles of both passes alternate between two accumulators.
+    bool ok = mbar_wait_warp(smem_u32(&bars[B_Q]), 0, p.err, DEV_ERR_FULL_WAIT);
+    tc_ring sc;
+    auto scores = [&](int item) {  // S[sc.slot] = Q K^T with the K tile of ring item `item`
+      const int s = item % FA_RING, b = sc.slot;
+      ok = ok && mbar_wait_warp(smem_u32(&bars[B_S_EMPTY + b]), sc.phase ^ 1u, p.err, DEV_ERR_TMEM_WAIT);
+      ok = ok && mbar_wait_warp(smem_u32(&bars[B_FULL + s]), (uint32_t)(item / FA_RING) & 1u, p.err, DEV_ERR_FULL_WAIT);
+      if (!ok) return;
+      tc_fence_after();
+      if (tc_elect()) {
 #pragma unroll
         for (int kb = 0; kb < NKB; ++kb) {
           const uint64_t a_desc = smem_desc_sw128(q_addr + kb * BLOCK_BYTES), b_desc = smem_desc_sw128(ring_addr + (uint32_t)s * OPERAND + kb * BLOCK_BYTES);
@@ -159,17 +160,20 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attn_fused_kernel(const __grid_
         }
         tc_commit(smem_u32(&bars[B_EMPTY + s]));
         tc_commit(smem_u32(&bars[B_S_FULL + b]));
-        ++sidx;
-      };
-      for (int j = 0; j < n_tiles && ok; ++j) scores(j);  // pass 1
-      if (ok) scores(n_tiles);                            // pass 2, tile 0
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        if (j + 1 < n_tiles) scores(n_tiles + 2 * (j + 1));
-        const int item = n_tiles + 2 * j + 1, s = item % FA_RING, pb = j & 1;
-        ok = ok && mbar_wait(smem_u32(&bars[B_P_READY + pb]), (uint32_t)(j >> 1) & 1u, p.err, DEV_ERR_FULL_WAIT);
-        ok = ok && mbar_wait(smem_u32(&bars[B_FULL + s]), (uint32_t)(item / FA_RING) & 1u, p.err, DEV_ERR_FULL_WAIT);
-        if (!ok) break;
-        tc_fence_after();
+      }
+      __syncwarp();
+      sc.step(2);
+    };
+    for (int j = 0; j < n_tiles && ok; ++j) scores(j);  // pass 1
+    if (ok) scores(n_tiles);                            // pass 2, tile 0
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      if (j + 1 < n_tiles) scores(n_tiles + 2 * (j + 1));
+      const int item = n_tiles + 2 * j + 1, s = item % FA_RING, pb = j & 1;
+      ok = ok && mbar_wait_warp(smem_u32(&bars[B_P_READY + pb]), (uint32_t)(j >> 1) & 1u, p.err, DEV_ERR_FULL_WAIT);
+      ok = ok && mbar_wait_warp(smem_u32(&bars[B_FULL + s]), (uint32_t)(item / FA_RING) & 1u, p.err, DEV_ERR_FULL_WAIT);
+      if (!ok) break;
+      tc_fence_after();
+      if (tc_elect()) {
 #pragma unroll
         for (int kb2 = 0; kb2 < 2; ++kb2) {
           const uint64_t a_desc = smem_desc_sw128(p_addr + (uint32_t)pb * FA_P_BYTES + kb2 * BLOCK_BYTES);
@@ -181,12 +185,16 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attn_fused_kernel(const __grid_
         tc_commit(smem_u32(&bars[B_EMPTY + s]));
         tc_commit(smem_u32(&bars[B_P_FREE + pb]));
       }
+      __syncwarp();
+    }
+    if (tc_elect()) {
       tc_commit(smem_u32(&bars[B_O_FULL]));  // (also after a failed wait: lets the epilogue warps leave)
       if (!ok) {
         tc_commit(smem_u32(&bars[B_S_FULL]));
         tc_commit(smem_u32(&bars[B_S_FULL + 1]));
       }
     }
+    __syncwarp();
   } else {
     // ---- epilogue: a thread owns row `row` of the tile and the 32 keys [cq * 32, +32) of every key tile.  (With eight
     // warps of 64 keys per thread the kernel was bound by the latency of its own instruction chain: 186 us per 7B layer

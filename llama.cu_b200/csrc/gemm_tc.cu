@@ -173,36 +173,37 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
   bool go = false;
 
   if (warp == 0) {
-    if (lane == 0) {  // ---- TMA producer
-      for (int kb = 0; kb < nk; ++kb) {
-        const int s = kb % nstages, use = kb / nstages;
-        if (use > 0 && !mbar_wait(smem_u32(&bars[MAXS + s]), (use - 1) & 1, err, DEV_ERR_EMPTY_WAIT)) break;
-        const uint32_t full = smem_u32(&bars[s]);
-        const uint32_t dst = base + (uint32_t)s * STAGE;
+    if (tc_elect()) {  // ---- TMA producer
+      tc_ring r;
+      for (int kb = 0; kb < nk; ++kb, r.step(nstages)) {
+        if (!mbar_wait(smem_u32(&bars[MAXS + r.slot]), r.phase ^ 1u, err, DEV_ERR_EMPTY_WAIT)) break;
+        const uint32_t full = smem_u32(&bars[r.slot]);
+        const uint32_t dst = base + (uint32_t)r.slot * STAGE;
         mbar_arrive_expect_tx(full, STAGE);
         tma_load_3d(dst, &map_a, 0, m0, (kb0 + kb) * kbs, full);
         tma_load_3d(dst + (uint32_t)kbs * A_BYTES, &map_b, 0, n_w, (kb0 + kb) * kbs, full);
       }
     }
-  } else if (warp == 1) {
-    if (lane == 0) {  // ---- MMA issuer
-      bool ok = true;
-      for (int kb = 0; kb < nk && ok; ++kb) {
-        const int s = kb % nstages, use = kb / nstages;
-        ok = mbar_wait(smem_u32(&bars[s]), use & 1, err, DEV_ERR_FULL_WAIT);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t a_addr = base + (uint32_t)s * STAGE, b_addr = a_addr + (uint32_t)kbs * A_BYTES;
+    __syncwarp();
+  } else if (warp == 1) {  // ---- MMA issuer
+    tc_ring r;
+    for (int kb = 0; kb < nk; ++kb, r.step(nstages)) {
+      if (!mbar_wait_warp(smem_u32(&bars[r.slot]), r.phase, err, DEV_ERR_FULL_WAIT)) break;
+      tc_fence_after();
+      if (tc_elect()) {
+        const uint32_t a_addr = base + (uint32_t)r.slot * STAGE, b_addr = a_addr + (uint32_t)kbs * A_BYTES;
         for (int j = 0; j < kbs; ++j) {
           const uint64_t a_desc = smem_desc_sw128(a_addr + (uint32_t)j * A_BYTES), b_desc = smem_desc_sw128(b_addr + (uint32_t)j * B_BYTES);
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)  // 16 halves = 32 bytes = 2 descriptor address units per K step
             tc_mma_f16(tmem_base, a_desc + 2 * k, b_desc + 2 * k, IDESC, (kb | j | k) != 0);
         }
-        tc_commit(smem_u32(&bars[MAXS + s]));  // the stage is free once these MMAs have read it
+        tc_commit(smem_u32(&bars[MAXS + r.slot]));  // the stage is free once these MMAs have read it
       }
-      tc_commit(smem_u32(&bars[2 * MAXS]));  // accumulator complete (also on the error path: lets the epilogue leave)
+      __syncwarp();
     }
+    if (tc_elect()) tc_commit(smem_u32(&bars[2 * MAXS]));  // accumulator complete (also on the error path: lets the epilogue leave)
+    __syncwarp();
   } else {
     // ---- epilogue: warp w may touch TMEM lanes 32 * (w % 4) ... + 31 only
     const int quad = warp & 3;
@@ -370,8 +371,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
   }
 
   if (warp == 0) {
-    if (lane == 0) {  // ---- TMA producer (both CTAs)
-      int it = 0;
+    if (tc_elect()) {  // ---- TMA producer (both CTAs)
+      tc_ring r;
       bool ok = true;
       for (int t = cluster_id; t < n_tiles && ok; t += n_clusters) {
         int m0 = (t % tiles_m) * (2 * BM) + (int)rank * BM;
@@ -381,10 +382,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
           m0 = tile.x + (int)rank * BM;
           n0 += tile.z * N;
         }
-        for (int kb = 0; kb < nk; kb += kbs, ++it) {  // (k-blocks past K arrive as zeros)
-          const int s = it % nstages;
-          const uint32_t ph = (uint32_t)(it / nstages) & 1u;
-          ok = mbar_wait(smem_u32(&bars[8 + s]), ph ^ 1u, err, DEV_ERR_EMPTY_WAIT);
+        for (int kb = 0; kb < nk; kb += kbs, r.step(nstages)) {  // (k-blocks past K arrive as zeros)
+          const int s = r.slot;
+          ok = mbar_wait(smem_u32(&bars[8 + s]), r.phase ^ 1u, err, DEV_ERR_EMPTY_WAIT);
           if (!ok) break;
           const uint32_t full_leader = mapa(smem_u32(&bars[s]), 0);
           const uint32_t dst = base + (uint32_t)s * STAGE;
@@ -395,31 +395,31 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {  // ---- MMA issuer (leader CTA only)
-      int it = 0, ti = 0;
+    if (rank == 0) {  // ---- MMA issuer (leader CTA only)
+      tc_ring r, acc;
       bool ok = true;
-      for (int t = cluster_id; t < n_tiles && ok; t += n_clusters, ++ti) {
-        const int b = ti & 1;
-        const uint32_t acc_ph = (uint32_t)(ti >> 1) & 1u;
-        ok = mbar_wait(smem_u32(&bars[18 + b]), acc_ph ^ 1u, err, DEV_ERR_TMEM_WAIT);  // both epilogues have drained buffer b
+      for (int t = cluster_id; t < n_tiles && ok; t += n_clusters, acc.step(2)) {
+        const int b = acc.slot;
+        ok = mbar_wait_warp(smem_u32(&bars[18 + b]), acc.phase ^ 1u, err, DEV_ERR_TMEM_WAIT);  // both epilogues have drained buffer b
         if (!ok) break;
-        tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(b * BN);
-        for (int kb = 0; kb < nk; kb += kbs, ++it) {
-          const int s = it % nstages;
-          const uint32_t ph = (uint32_t)(it / nstages) & 1u;
-          ok = mbar_wait(smem_u32(&bars[s]), ph, err, DEV_ERR_FULL_WAIT);
+        for (int kb = 0; kb < nk; kb += kbs, r.step(nstages)) {
+          ok = mbar_wait_warp(smem_u32(&bars[r.slot]), r.phase, err, DEV_ERR_FULL_WAIT);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t a_addr = base + (uint32_t)s * STAGE, b_addr = a_addr + (uint32_t)kbs * A_BYTES;
-          for (int j = 0; j < kbs && kb + j < nk; ++j) {
-            const uint64_t a_desc = smem_desc_sw128(a_addr + (uint32_t)j * A_BYTES), b_desc = smem_desc_sw128(b_addr + (uint32_t)j * B_BYTES);
+          if (tc_elect()) {
+            const uint32_t a_addr = base + (uint32_t)r.slot * STAGE, b_addr = a_addr + (uint32_t)kbs * A_BYTES;
+            for (int j = 0; j < kbs && kb + j < nk; ++j) {
+              const uint64_t a_desc = smem_desc_sw128(a_addr + (uint32_t)j * A_BYTES), b_desc = smem_desc_sw128(b_addr + (uint32_t)j * B_BYTES);
 #pragma unroll
-            for (int k = 0; k < BK / 16; ++k) tc_mma_f16_pair(d_tmem, a_desc + 2 * k, b_desc + 2 * k, IDESC, (kb | j | k) != 0);
+              for (int k = 0; k < BK / 16; ++k) tc_mma_f16_pair(d_tmem, a_desc + 2 * k, b_desc + 2 * k, IDESC, (kb | j | k) != 0);
+            }
+            tc_commit_pair(smem_u32(&bars[8 + r.slot]), 3);  // frees the stage in both CTAs
           }
-          tc_commit_pair(smem_u32(&bars[8 + s]), 3);  // frees the stage in both CTAs
+          __syncwarp();
         }
-        tc_commit_pair(smem_u32(&bars[16 + b]), 3);  // accumulator b complete (also after a failed wait: lets the epilogues leave)
+        if (tc_elect()) tc_commit_pair(smem_u32(&bars[16 + b]), 3);  // accumulator b complete (also after a failed wait: lets the epilogues leave)
+        __syncwarp();
       }
     }
   } else {

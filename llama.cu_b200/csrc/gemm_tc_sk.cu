@@ -214,18 +214,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SK_THREADS, 1)
   pdl_wait();  // everything above ran under the previous kernel's tail; nothing before this line touches global memory
 
   if (warp == 0) {
-    if (lane == 0) {  // ---- TMA producer (both CTAs)
-      int it = 0;
+    if (tc_elect()) {  // ---- TMA producer (both CTAs)
+      tc_ring r;
       bool ok = true;
       while (ok && sched.next(tile, kb0, kb1, split)) {
         const int m0 = (tile % tiles_m) * (2 * SK_BM) + (int)rank * SK_BM;
         // rows of W for this CTA's 128 columns of accumulator h: n0 + h * n_step
         const int n0 = (tile / tiles_m) * BN_OUT + (int)rank * ((GATE && NB == 1) ? gate_rows : 128);
         const int n_step = GATE ? gate_rows : 256;
-        for (int kb = kb0; kb < kb1; kb += kbs, ++it) {  // (a segment of odd length loads one k-block it does not use)
-          const int s = it % nstages;
-          const uint32_t ph = (uint32_t)(it / nstages) & 1u;
-          ok = mbar_wait(smem_u32(&bars[8 + s]), ph ^ 1u, err, DEV_ERR_EMPTY_WAIT);
+        for (int kb = kb0; kb < kb1; kb += kbs, r.step(nstages)) {  // (a segment of odd length loads one k-block it does not use)
+          const int s = r.slot;
+          ok = mbar_wait(smem_u32(&bars[8 + s]), r.phase ^ 1u, err, DEV_ERR_EMPTY_WAIT);
           if (!ok) break;
           const uint32_t full_leader = mapa(smem_u32(&bars[s]), 0);
           const uint32_t dst = base + (uint32_t)s * STAGE;
@@ -238,36 +237,36 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SK_THREADS, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {  // ---- MMA issuer (leader CTA only)
-      int it = 0, si = 0;
+    if (rank == 0) {  // ---- MMA issuer (leader CTA only)
+      tc_ring r, seg;
       bool ok = true;
-      for (; ok && sched.next(tile, kb0, kb1, split); ++si) {
-        const int b = si % NBUF;
-        const uint32_t acc_ph = (uint32_t)(si / NBUF) & 1u;
-        ok = mbar_wait(smem_u32(&bars[18 + b]), acc_ph ^ 1u, err, DEV_ERR_TMEM_WAIT);  // the epilogues have drained buffer b
+      for (; ok && sched.next(tile, kb0, kb1, split); seg.step(NBUF)) {
+        const int b = seg.slot;
+        ok = mbar_wait_warp(smem_u32(&bars[18 + b]), seg.phase ^ 1u, err, DEV_ERR_TMEM_WAIT);  // the epilogues have drained buffer b
         if (!ok) break;
-        tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(b * BN);
-        for (int kb = kb0; kb < kb1; kb += kbs, ++it) {
-          const int s = it % nstages;
-          const uint32_t ph = (uint32_t)(it / nstages) & 1u;
-          ok = mbar_wait(smem_u32(&bars[s]), ph, err, DEV_ERR_FULL_WAIT);
+        for (int kb = kb0; kb < kb1; kb += kbs, r.step(nstages)) {
+          ok = mbar_wait_warp(smem_u32(&bars[r.slot]), r.phase, err, DEV_ERR_FULL_WAIT);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t a_addr = base + (uint32_t)s * STAGE, b_addr = a_addr + (uint32_t)kbs * A_BYTES;
-          for (int j = 0; j < kbs && kb + j < kb1; ++j) {
-            const uint64_t a_desc = smem_desc_sw128(a_addr + (uint32_t)j * A_BYTES);
+          if (tc_elect()) {
+            const uint32_t a_addr = base + (uint32_t)r.slot * STAGE, b_addr = a_addr + (uint32_t)kbs * A_BYTES;
+            for (int j = 0; j < kbs && kb + j < kb1; ++j) {
+              const uint64_t a_desc = smem_desc_sw128(a_addr + (uint32_t)j * A_BYTES);
 #pragma unroll
-            for (int k = 0; k < SK_BK / 16; ++k) {
+              for (int k = 0; k < SK_BK / 16; ++k) {
 #pragma unroll
-              for (int h = 0; h < NB; ++h)
-                sk_mma_pair(d_tmem + (uint32_t)(h * 256), a_desc + 2 * k, smem_desc_sw128(b_addr + (uint32_t)(h * kbs + j) * B_BYTES) + 2 * k, IDESC,
-                            (kb + j > kb0 || k > 0) ? 1u : 0u);
+                for (int h = 0; h < NB; ++h)
+                  sk_mma_pair(d_tmem + (uint32_t)(h * 256), a_desc + 2 * k, smem_desc_sw128(b_addr + (uint32_t)(h * kbs + j) * B_BYTES) + 2 * k, IDESC,
+                              (kb + j > kb0 || k > 0) ? 1u : 0u);
+              }
             }
+            sk_commit_pair(smem_u32(&bars[8 + r.slot]), 3);  // frees the stage in both CTAs
           }
-          sk_commit_pair(smem_u32(&bars[8 + s]), 3);  // frees the stage in both CTAs
+          __syncwarp();
         }
-        sk_commit_pair(smem_u32(&bars[16 + b]), 3);  // the segment's accumulators are complete (also after a failed wait: lets the epilogues leave)
+        if (tc_elect()) sk_commit_pair(smem_u32(&bars[16 + b]), 3);  // the segment's accumulators are complete (also after a failed wait: lets the epilogues leave)
+        __syncwarp();
       }
     }
   } else {

@@ -39,6 +39,8 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 // Single-thread instructions (tcgen05.mma, commit, tensor copies) take their operands from uniform registers.  Under
 // `if (lane == 0)` the compiler cannot see that one thread runs and moves every operand over, for each instruction; issuing
 // warps therefore keep their loops, waits and addresses common to the warp and elect a lane around the instructions alone.
+// Tiles whose MMAs are short gain most - 509 rows of 4096 x 4096 on 256 x 128 pair tiles: 24.5 -> 19.1 us, 2000 of 2816 x 1024:
+// 18.8 -> 14.5 - 256-wide pair tiles 1 to 2 %.
 __device__ __forceinline__ bool tc_elect() {  // true for one lane (always the same) of a converged warp
   uint32_t one;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
