@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attn_fused_kernel(const __grid_
       const int b = sidx & 1;
       const bool ok = mbar_wait(smem_u32(&bars[B_S_FULL + b]), (uint32_t)(sidx >> 1) & 1u, p.err, DEV_ERR_TMEM_WAIT);
       tc_fence_after();
-      go = __all_sync(0xffffffffu, ok && *(volatile int*)p.err == 0);
+      go = __all_sync(0xffffffffu, ok);  // (the error word is looked at once, before the results are stored: a load from L2 per tile otherwise)
       if (!go) return;
       const int key0 = j * FA_BN + cq * 32;
       uint32_t r[32];
