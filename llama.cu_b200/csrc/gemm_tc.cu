@@ -721,8 +721,8 @@ static void gemm_tc_estimates(int m, int N, int K, int sms, double* whole_us, do
   *t512_us = N >= 2 * K ? balanced(512) : 1e30;
 }
 
-// More than 128 rows: 0 = whole tiles per SM pair, 256 / 512 = the balanced kernel with that tile width (the one whose
-// estimate is lowest; a balanced kernel has to beat whole tiles by 3 %).
+// More than 128 rows, the choice between these two kernels alone (gemm_tc_pick_long has more): 0 = whole tiles per SM pair,
+// 256 / 512 = the balanced kernel with that tile width (the one whose estimate is lowest; a balanced kernel has to beat whole tiles by 3 %).
 int gemm_tc_plan_long(int m, int N, int K, int sms) {
   double whole, t256, t512;
   gemm_tc_estimates(m, N, K, sms, &whole, &t256, &t512);
@@ -734,6 +734,44 @@ int gemm_tc_plan_long(int m, int N, int K, int sms) {
   }
   if (t512 < 0.97 * whole && t512 < best) tile = 512;
   return tile;
+}
+
+// More than 128 rows, operands issued from warp-uniform code: which kernel runs the product.  The estimates (microseconds) follow
+// timings of 16 shapes (K, N from 1024 to 22016) at 129 to 2000 rows on each kernel: a K step of 64 takes 0.26 us on the one-SM kernel
+// (128 x 128 tiles, K split over 2 or 4 CTAs where tiles are few; 0.30 once an SM has several), 0.205 to 0.235 on 256 x 128 pair
+// tiles, 0.34 to 0.42 on 256 x 256 ones; the balanced kernel as in gemm_tc_estimates.  What the choice between whole 256-row tiles and
+// the balanced kernel alone took before, in us: 300 rows of 2048 x 6144 23.3 -> 14.3 (one SM), of 5632 x 2048 23.8 -> 18.4 (one SM),
+// 509 of 11008 x 4096 52.0 -> 43.0 (128-wide pairs), 1000 of 5632 x 2048 34.8 -> 23.4 (128-wide pairs).
+enum tc_long_kernel { TC_ONE_SM, TC_PAIR_128, TC_PAIR_256, TC_BALANCED_256, TC_BALANCED_512 };
+static tc_long_kernel gemm_tc_pick_long(int m, int N, int K, int sms, bool balanced_too, double* best_whole_us = nullptr) {
+  const long C = sms / 2, nk = K / BK, tm = (m + 2 * BM - 1) / (2 * BM);
+  auto ceil_div_l = [](long a, long b) { return (a + b - 1) / b; };
+  double best = 1e30;
+  tc_long_kernel pick = TC_ONE_SM;
+  {
+    const long tiles = (long)((m + BM - 1) / BM) * (N / 128);
+    long sp = tiles * 4 <= sms ? 4 : tiles * 2 <= sms ? 2 : 1;
+    if (nk < 8 * sp) sp = 1;
+    const long waves = ceil_div_l(tiles * sp, sms);
+    best = waves * ((double)nk / sp) * (waves == 1 ? 0.26 : 0.30) + 6.5 + (sp > 1 ? 1 : 0);
+  }
+  {
+    const long waves = ceil_div_l(tm * (N / 128), C);
+    const double est = waves * nk * (waves == 1 ? 0.205 : waves <= (nk < 64 ? 3 : 2) ? 0.215 : 0.235) + 6;
+    if (est < best) best = est, pick = TC_PAIR_128;
+  }
+  if (N % 256 == 0) {
+    const long tiles = tm * (N / 256);
+    const double est = ceil_div_l(tiles, C) * nk * (tiles > 300 && nk <= 80 ? 0.42 : tiles > 40 ? 0.38 : 0.34) + 5;
+    if (est < best) best = est, pick = TC_PAIR_256;
+  }
+  if (best_whole_us) *best_whole_us = best;
+  if (balanced_too) {  // (has to win by 3 %)
+    double whole, t256, t512;
+    gemm_tc_estimates(m, N, K, sms, &whole, &t256, &t512);
+    if (std::min(t256, t512) < 0.97 * best) pick = t256 <= t512 ? TC_BALANCED_256 : TC_BALANCED_512;
+  }
+  return pick;
 }
 
 int& gemm_tc_gate_mode() {
@@ -751,6 +789,7 @@ int gemm_tc_gated_tile(int m, int f, int K) {
   // element at about 5 TB/s, and a launch).  7B shapes: the one launch wins 4 to 8 us per layer from 129 to 1024 rows.
   double whole, t256, t512;
   gemm_tc_estimates(m, 2 * f, K, gemv_sm_count(), &whole, &t256, &t512);
+  if ((2 * f) % 128 == 0) gemm_tc_pick_long(m, 2 * f, K, gemv_sm_count(), false, &whole);
   const double gate_us = (double)m * f * 6.0 / 5.0e6 + 2;
   const double one_launch = t256 + 3 + (m > 1024 ? (m - 1024) * 0.016 : 0.0);
   return one_launch < std::min(whole, t512) + gate_us ? 256 : 0;
@@ -767,27 +806,20 @@ int launch_gemm_shape(void* out, const void* lhs, int ldx, const void* w, int m,
                       int force_bn, int force_pair, int force_split) {
   LCU_REQUIRE(gemm_tc_supported(m, N, K, ldx, lhs, w, out), "gemm_tc: unsupported shape m=%d N=%d K=%d ldx=%d or unaligned pointers", m, N, K, ldx);
   const int sms = gemv_sm_count();
-  // More than 128 rows: three kernels can run the product - whole tiles per SM pair (below), the kernel that deals the
-  // K steps of the last, partial wave evenly over the pairs (gemm_tc_sk.cu, 256-wide tiles), and the same with
-  // 512-wide tiles (a third less operand traffic per multiply-add, no overlap of epilogue and main loop).  Which one is
-  // fastest depends on how the tile count meets the 74 pairs (gemm_tc_estimates).  Mode -1 = that rule; 256 / 512 force
-  // the balanced kernel with that tile width; 0 = never.
-  // (the balanced kernel stores 16-bit results only)
-  if (sizeof(TO) == 2 && force_pair < 0 && !force_bn && (m > BM || gemm_tc_sk_mode() > 0)) {
-    const int mode = gemm_tc_sk_mode();
-    int tile = mode > 0 ? mode : 0;
-    if (mode < 0) tile = gemm_tc_plan_long(m, N, K, sms);
-    if (tile && gemm_tc_sk_supported(m, N, K, ldx, lhs, w, out, tile)) return launch_gemm_tc_sk(tc_type_of<T>(), out, lhs, ldx, w, m, N, K, beta, err, stream, tile);
-  }
-  // Large products: the two-SM kernel, with its 256-wide tile when that still gives (nearly) every SM pair a tile.
-  // Up to 256 rows of a matrix with few tiles stay on the one-SM kernel, which can split K to fill the SMs.
+  // More than 128 rows: gemm_tc_pick_long between the one-SM kernel, whole tiles per SM pair and the kernel that deals the K steps of
+  // the last, partial wave evenly over the pairs (gemm_tc_sk.cu; 16-bit results only), unless a mode forces one of them
+  // (gemm_tc_sk_mode: 256 / 512 = the balanced kernel with that tile width, 0 = never).
   int pair = force_pair;
-  if (pair < 0) {
-    pair = 0;
-    if (m > BM && N % 128 == 0 && !force_bn && (m > 2 * BM || N > 8192)) {
-      const long tiles_m = (m + 2 * BM - 1) / (2 * BM), clusters = sms / 2;
-      pair = (N % 256 == 0 && tiles_m * (N / 256) * 4 >= clusters * 3) ? 256 : 128;
+  if (pair < 0) pair = 0;
+  if (force_pair < 0 && !force_bn && (m > BM || (sizeof(TO) == 2 && gemm_tc_sk_mode() > 0))) {
+    const int mode = sizeof(TO) == 2 ? gemm_tc_sk_mode() : 0;
+    int tile = mode > 0 ? mode : 0;
+    if (N % 128 == 0) {
+      const tc_long_kernel k = gemm_tc_pick_long(m, N, K, sms, mode < 0);
+      if (mode < 0) tile = k == TC_BALANCED_256 ? 256 : k == TC_BALANCED_512 ? 512 : 0;
+      pair = m <= BM ? 0 : k == TC_PAIR_128 ? 128 : k == TC_PAIR_256 ? 256 : 0;
     }
+    if (tile && gemm_tc_sk_supported(m, N, K, ldx, lhs, w, out, tile)) return launch_gemm_tc_sk(tc_type_of<T>(), out, lhs, ldx, w, m, N, K, beta, err, stream, tile);
   }
   if (pair) {
     LCU_REQUIRE((pair == 128 || pair == 256) && N % pair == 0, "gemm_tc: pair tile width %d does not divide N=%d", pair, N);
