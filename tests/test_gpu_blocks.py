@@ -79,6 +79,20 @@ def test_scans_cut_into_chunks(run, rdim, rvdim, heads, dim, dtype):
 
 
 @both
+@pytest.mark.parametrize("rheads,rdim,rvdim,rot_dims,heads,dim", [(9, 24, 12, 16, 11, 8), (1, 136, 132, 8, 8, 12), (4, 8, 4, 8, 2, 132), (3, 64, 260, 64, 16, 4)])
+def test_scan_rows_laid_out_by_fours(run, rheads, rdim, rvdim, rot_dims, heads, dim, dtype):
+    """Head sizes in whole vectors of four: heads that fill a CTA's warps, leave some over or need several CTAs, channels and values
+    past one round of a warp, part of a head turned, odd row counts."""
+    cfg, W = B.case(seed=15, layers=("parallel", "wkv"), mlp_none=(0, 1),
+                    mixer=dict(left_scale=0.0, rheads=rheads, rdim=rdim, rvdim=rvdim, rot_dims=rot_dims), wkv=dict(heads=heads, dim=dim))
+    t = B.tokens(cfg, 75, 5)
+    want = P.forward(t, cfg, W)
+    r = run(cfg, W, dtype)
+    for cuts in (WHOLE, [33, 2, 1, 5]):
+        check(r.feed(t, cuts), want, dtype)
+
+
+@both
 def test_context_is_reused_by_the_next_sequence(run, dtype):
     cfg, W = B.case(seed=4, layers=("parallel", "wkv"))
     r = run(cfg, W, dtype)
