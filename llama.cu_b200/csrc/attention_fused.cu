@@ -34,7 +34,7 @@ constexpr int FA_BN = 128;       // keys per tile
 constexpr int FA_EPI_WARPS = 16;  // four per tensor-memory lane quadrant: a thread owns one row and 32 of a tile's 128 keys
 constexpr int FA_THREADS = 64 + 32 * FA_EPI_WARPS;  // warp 0: TMA, warp 1: MMA + tensor memory, then the epilogue warps
 constexpr int FA_RING = 4;       // ring stages of one 128-key operand each
-constexpr uint32_t FA_P_BYTES = FA_BM * FA_BN * 2;  // one probability tile: two K-major blocks of 128 rows x 64 keys
+constexpr uint32_t FA_P_BYTES = FA_BM * FA_BN * 2;  // one tile of exponentials: two K-major blocks of 128 rows x 64 keys
 
 struct fused_params {
   __half* out;  // [m][ldo]
@@ -50,9 +50,9 @@ constexpr int B_Q = 0;                       // Q landed
 constexpr int B_FULL = 1;                    // [FA_RING] ring stage landed
 constexpr int B_EMPTY = B_FULL + FA_RING;    // [FA_RING] ring stage free
 constexpr int B_S_FULL = B_EMPTY + FA_RING;  // [2] score accumulator ready
-constexpr int B_S_EMPTY = B_S_FULL + 2;      // [2] score accumulator read out (8 warps)
-constexpr int B_P_READY = B_S_EMPTY + 2;     // [2] probability tile written (8 warps)
-constexpr int B_P_FREE = B_P_READY + 2;      // [2] probability tile consumed by its MMAs
+constexpr int B_S_EMPTY = B_S_FULL + 2;      // [2] score accumulator read out (16 warps)
+constexpr int B_P_READY = B_S_EMPTY + 2;     // [2] tile of exponentials written (16 warps)
+constexpr int B_P_FREE = B_P_READY + 2;      // [2] tile of exponentials consumed by its MMAs
 constexpr int B_O_FULL = B_P_FREE + 2;       // output accumulator complete
 constexpr int B_COUNT = B_O_FULL + 1;
 

@@ -65,7 +65,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, in
     }
   }
 }
-// place in a ring of n slots and the parity of its barriers in this round
+// place in a ring of n slots and the parity of its barriers on this lap
 struct tc_ring {
   int slot = 0;
   uint32_t phase = 0;
