@@ -226,7 +226,6 @@ attn_rows<T> block_context<T>::attention(int run, int b, int ld) {
   a.out_scale = bs.out_scale;
   a.out = cat + bw.out_col;
   a.ldo = m->layers[l].out_k;
-  a.err = gpus[0].state + 3;
   return a;
 }
 
@@ -290,7 +289,6 @@ int block_context<T>::latent_attention_rows(int run, int b, int rows, int pos0) 
   a.out_scale = bs.out_scale;
   a.out = cat + bw.out_col;
   a.ldo = m->layers[l].out_k;
-  a.err = gpus[0].state + 3;
   return launch_window_attention(a, rows, pos0, stream());
 }
 

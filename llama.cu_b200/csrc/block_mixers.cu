@@ -900,15 +900,10 @@ int launch_window_append(const attn_rows<T>& p, int m, int pos0, cudaStream_t st
   return LCU_OK;
 }
 
-// up to one tile of the warp-level kernel stays there: half of a 128-row tile would be padding, and its CTAs start faster
-constexpr int WINDOW_TC_ROWS = 64;
 template <typename T>
 int launch_window_attention(const attn_rows<T>& p, int m, int pos0, cudaStream_t stream) {
-  if constexpr (sizeof(T) == 2) {
-    const int mode = window_mma_mode();
-    if ((mode == 3 || (mode == 1 && m > WINDOW_TC_ROWS)) && window_tc_supported(p)) return launch_window_tc(p, m, pos0, stream);
-    if (mode && window_mma_supported(p.dim, p.key2 ? p.dim2 : 0, p.vdim)) return launch_window_mma(p, m, pos0, stream);
-  }
+  if constexpr (sizeof(T) == 2)
+    if (window_mma_mode() && window_mma_supported(p.dim, p.key2 ? p.dim2 : 0, p.vdim)) return launch_window_mma(p, m, pos0, stream);
   const int keys = most_keys(p, pos0 + m - 1);
   const size_t smem = attention_smem(p, keys, false);
   LCU_REQUIRE(smem <= 220 * 1024, "window attention: %d visible keys", keys);

@@ -108,7 +108,6 @@ struct attn_rows {
   float scale, out_scale;
   T* out;
   int ldo;
-  int* err;            // device error word
 };
 // cache rows pos0 .. pos0+m-1, then the blocks they complete, then attention of the rows
 template <typename T>
@@ -116,9 +115,7 @@ int launch_window_append(const attn_rows<T>& p, int m, int pos0, cudaStream_t st
 // (bfloat16 rows with heads of up to 128 take the tensor-core kernel of block_attn.cu)
 bool window_mma_supported(int dim, int dim2, int vdim);
 int launch_window_mma(const attn_rows<__nv_bfloat16>& p, int m, int pos0, cudaStream_t stream);
-bool window_tc_supported(const attn_rows<__nv_bfloat16>& p);
-int launch_window_tc(const attn_rows<__nv_bfloat16>& p, int m, int pos0, cudaStream_t stream);  // block_attn_tc.cu
-int& window_mma_mode();  // 1 (default) = the tensor-core kernel that suits, 0 = neither, 2 / 3 = block_attn.cu / block_attn_tc.cu where supported
+int& window_mma_mode();  // 1 (default) = where supported, 0 = never
 template <typename T>
 int launch_window_attention(const attn_rows<T>& p, int m, int pos0, cudaStream_t stream);
 

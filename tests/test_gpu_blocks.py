@@ -192,21 +192,17 @@ def test_passes_longer_than_the_row_buffers(run):
 @pytest.mark.parametrize("mixer", [dict(heads=4, kv_heads=2, dim=64, vdim=64, window=48, pool=16), dict(heads=3, kv_heads=1, dim=96, vdim=40, window=129, pool=8),
                                    dict(heads=2, kv_heads=2, dim=128, vdim=100, window=1, pool=2), dict(heads=1, kv_heads=1, dim=192, vdim=128, window=300, pool=64),
                                    dict(heads=6, kv_heads=3, dim=8, vdim=5, window=128, pool=1)])
-def test_window_attention_in_tiles_of_128(lcu, run, mixer):
-    """Windows, block means, shared keys and head sizes at the edges of the 128-row tiles, passes of any length."""
+def test_window_attention_at_the_edges_of_tiles(run, mixer):
+    """Windows, block means, shared keys and head sizes at the edges of row and key tiles, passes of any length."""
     cfg, W = B.case(seed=21, layers=("parallel",), mlp_none=(0,), mixer=dict(mixer, right_scale=0.0))
     t = B.tokens(cfg, 420, 7)
     want = P.forward(t, cfg, W)
-    lcu.check(lcu.lib.lcu_set_tuning(b"block_attn_mma", 3))
-    try:
-        r = run(cfg, W, "bfloat16", context_len=448)
-        for cuts in (WHOLE, [127, 2, 128, 129, 1, 33], [256, 1, 163]):
-            check(r.feed(t, cuts), want, "bfloat16")
-    finally:
-        lcu.check(lcu.lib.lcu_set_tuning(b"block_attn_mma", 1))
+    r = run(cfg, W, "bfloat16", context_len=448)
+    for cuts in (WHOLE, [127, 2, 128, 129, 1, 33], [256, 1, 163]):
+        check(r.feed(t, cuts), want, "bfloat16")
 
 
-@pytest.mark.parametrize("keys", [{"block_attn_mma": 0}, {"block_attn_mma": 2}, {"block_row_one_cta": 0}, {"prefill_gate_fused": 256}, {"prefill_gate_fused": 512}, {"prefill_tc_sk": 256},
+@pytest.mark.parametrize("keys", [{"block_attn_mma": 0}, {"block_row_one_cta": 0}, {"prefill_gate_fused": 256}, {"prefill_gate_fused": 512}, {"prefill_tc_sk": 256},
                                   {"prefill_tc_pair": 128}, {"use_graph": 0, "use_pdl": 0}])
 def test_kernel_choices_agree(lcu, run, keys):
     """Other kernels for the same products and attention: balanced and two-SM products, the gate in the product's epilogue,

@@ -63,18 +63,14 @@ def test_against_plain_whole_and_token_by_token(run, name, dtype):  # noqa: F811
 
 @pytest.mark.parametrize("mixer", [dict(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=512, window=200), dict(heads=3, dim=100, rot_dim=28, vdim=96, kv_rank=40),
                                    dict(heads=5, dim=64, rot_dim=32, vdim=64, kv_rank=96, window=129), dict(heads=2, dim=20, rot_dim=6, vdim=12, window=1)])
-def test_attention_in_tiles_of_128(lcu, run, mixer):  # noqa: F811
-    """Keys in two parts, sinks and gates in the 128-row tiles, passes of any length behind any position."""
+def test_attention_at_the_edges_of_tiles(run, mixer):  # noqa: F811
+    """Keys in two parts, sinks and gates at the edges of row and key tiles, passes of any length behind any position."""
     cfg, W = B.latent_case(seed=22, layers=1, mlp_none=(0,), mixer=mixer)
     t = B.tokens(cfg, 420, 7)
     want = P.forward(t, cfg, W)
-    lcu.check(lcu.lib.lcu_set_tuning(b"block_attn_mma", 3))
-    try:
-        r = run(cfg, W, "bfloat16", context_len=448)
-        for cuts in (WHOLE, [127, 2, 128, 129, 1, 33], [256, 1, 163]):
-            check(r.feed(t, cuts), want, "bfloat16")
-    finally:
-        lcu.check(lcu.lib.lcu_set_tuning(b"block_attn_mma", 1))
+    r = run(cfg, W, "bfloat16", context_len=448)
+    for cuts in (WHOLE, [127, 2, 128, 129, 1, 33], [256, 1, 163]):
+        check(r.feed(t, cuts), want, "bfloat16")
 
 
 def test_routing_on_everything_a_row_holds(run):  # noqa: F811
