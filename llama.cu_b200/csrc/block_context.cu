@@ -691,6 +691,7 @@ int block_context<T>::enqueue_prefill(int m_rows, const pass_request& rq) {
       LCU_CUDA(cudaMemcpyAsync(row_list, h_rows, n * sizeof(int), cudaMemcpyHostToDevice, g.stream));
       LCU_TRY(rows_to_logits(done, row_list, 0, n));
       slab.resize((size_t)n * m->n_vocab_pad);
+      LCU_TRY(read_back(g, g.stream, h_stage + 4, 1, "step"));  // (a copy to pageable memory waits without a limit)
       LCU_CUDA(cudaMemcpyAsync(slab.data(), logits, slab.size() * 4, cudaMemcpyDeviceToHost, g.stream));
       LCU_CUDA(cudaStreamSynchronize(g.stream));
       for (int i = 0; i < n; ++i)

@@ -127,6 +127,7 @@ int lcu_set_tuning(const char* key, int value) {
   else if (k == "block_attn_mma") window_mma_mode() = value;
   else if (k == "tp_debug") tp_set_debug(value);
   else if (k == "loader_staged") set_loader_staged(value);
+  else if (k == "host_wait_limit_ms") host_wait_limit_ms() = value < 0 ? 0 : value;
   else if (k == "use_graph") g_default_opts.use_graph = value;
   else if (k == "use_pdl") g_default_opts.use_pdl = value;
   else if (k == "attn_cluster") g_default_opts.attn_cluster = value;

@@ -63,7 +63,7 @@ struct context_impl {
   short* ids = nullptr;                  // token ids on the embedding GPU [context_len]
   __half* probs = nullptr;               // on the output GPU
   short* log = nullptr;                  // generated tokens of a chained run [context_len]
-  int* h_stage = nullptr;                // pinned: [0] position, [1] zero, [2] token read-back
+  int* h_stage = nullptr;                // pinned: [0] position, [1] zero, [2] token read-back, [3] error word; [4], [5] the same in front of logits
   short* h_ids = nullptr;                // pinned token staging [context_len]
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   // captured decode steps, one per variant (decode_variant)
@@ -71,6 +71,8 @@ struct context_impl {
   bool graph_failed = false;
   bool warmed_variant[2] = {false, false};
   int last_row = 0;                      // row of the activations that holds the last token's residual stream
+  // a wait for the GPU ran out (read_back): the streams may still be running, and what the caches hold is not known
+  bool unfinished = false, place_lost = false;
 
   virtual ~context_impl() = default;
   gpu_state& first() { return gpus.front(); }
@@ -98,6 +100,12 @@ struct context_impl {
   int build_graph(int variant);
   int run_decode_step(int n_keys);
   int stage_inputs(const short* tokens, int n);
+  // Two state words of `from` (token, error word) to pinned memory, and the wait for everything before them on `stream`: at most
+  // host_wait_limit_ms() for the call and again for every thousand steps in it, then LCU_ERR_DEVICE_WAIT.  (Kernels bound their
+  // waits on barriers and flags themselves; this bounds whatever else keeps a stream from ending.)
+  int read_back(const gpu_state& from, cudaStream_t stream, int* to, int n_steps, const char* who);
+  bool running();                        // some stream has work left
+  int settled(const char* who);          // after a wait that ran out: refuses until the streams are empty and the tokens cleared
 };
 
 }  // namespace lcu

@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cstdarg>
 #include <cstring>
 #include <thread>
@@ -507,6 +508,10 @@ struct llama_context_impl : context_impl {
 context::~context() {
   if (!impl) return;
   context_impl& c = *impl;
+  if (c.unfinished && c.running()) {  // freeing would wait for the GPU without a limit: the memory stays with the process
+    impl.release();
+    return;
+  }
   for (int v = 0; v < 2; ++v)
     if (c.graph[v]) cudaGraphExecDestroy(c.graph[v]);
   for (size_t i = 0; i < c.gpus.size(); ++i) {
@@ -655,7 +660,10 @@ int context_impl::open_streams(int context_len) {
   return LCU_OK;
 }
 
-void context::clear_tokens() { impl->start_pos = 0; }  // the reference re-allocates everything here (llama_cu.cu:1004-1049)
+void context::clear_tokens() {  // the reference re-allocates everything here (llama_cu.cu:1004-1049)
+  impl->start_pos = 0;
+  impl->place_lost = false;
+}
 
 size_t context::memory_usage() const {
   size_t n = impl->kv_bytes;
@@ -669,6 +677,7 @@ int context::kernels_per_step() const { return impl->kernels_per_step(); }
 int context::set_sampling(int mode, uint64_t seed) {
   LCU_REQUIRE(mode == 0 || mode == 1, "set_sampling: mode %d (0 = greedy, 1 = multinomial)", mode);
   context_impl& c = *impl;
+  LCU_TRY(c.settled("set_sampling"));
   c.opt.sampling = mode;
   c.opt.sample_seed = seed;
   for (int v = 0; v < 2; ++v)  // the captured steps hold the old choice
@@ -681,7 +690,10 @@ int context::set_sampling(int mode, uint64_t seed) {
   return LCU_OK;
 }
 
-int context::rollover(int keep) { return impl->rollover(keep); }
+int context::rollover(int keep) {
+  LCU_TRY(impl->settled("rollover"));
+  return impl->rollover(keep);
+}
 
 int llama_context_impl::rollover(int keep) {
   LCU_REQUIRE(keep >= 1 && keep < start_pos, "rollover: keep %d of %d cached positions", keep, start_pos);
@@ -714,6 +726,68 @@ int context::device_error() {
     }
   }
   return worst;
+}
+
+int& host_wait_limit_ms() {
+  static int ms = 600 * 1000;
+  return ms;
+}
+
+int context_impl::read_back(const gpu_state& from, cudaStream_t stream, int* to, int n_steps, const char* who) {
+  constexpr int NOT_BACK = -1;  // (error codes are positive)
+  volatile int* word = to + 1;
+  *word = NOT_BACK;
+  LCU_CUDA(cudaMemcpyAsync(to, from.state + 2, 8, cudaMemcpyDeviceToHost, stream));
+  const auto begin = std::chrono::steady_clock::now();
+  const double limit = host_wait_limit_ms() * (1.0 + n_steps / 1000.0);
+  // the word itself is watched; the stream is asked now and then, for errors that keep the word from coming back
+  double next_query = limit > 0 && limit < 10 ? limit : 10;
+  while (*word == NOT_BACK) {
+    const double t = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - begin).count();
+    if (t < next_query) continue;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // (another thread may be capturing)
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaStreamQuery(stream);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaErrorNotReady) break;  // (done, or an error, which the synchronisation returns)
+    cudaGetLastError();
+    if (limit > 0 && t > limit) {
+      unfinished = place_lost = true;
+      set_last_error("%s: the GPU has not finished within %.0f ms", who, limit);
+      return LCU_ERR_DEVICE_WAIT;
+    }
+    next_query = t + 1;
+    std::this_thread::yield();
+  }
+  LCU_CUDA(cudaStreamSynchronize(stream));
+  return LCU_OK;
+}
+
+bool context_impl::running() {
+  bool some = false;
+  for (auto& g : gpus) {
+    device_guard dg(g.device);
+    for (cudaStream_t s : {g.stream, g.side})
+      if (s && cudaStreamQuery(s) == cudaErrorNotReady) {
+        cudaGetLastError();
+        some = true;
+      }
+  }
+  return some;
+}
+
+int context_impl::settled(const char* who) {
+  if (!unfinished) return LCU_OK;
+  if (running() || place_lost) {
+    set_last_error("%s: an earlier call gave up waiting for the GPU; clear the tokens, and call again once the GPU has finished", who);
+    return LCU_ERR_DEVICE_WAIT;
+  }
+  for (auto& g : gpus) {
+    device_guard dg(g.device);
+    LCU_CUDA(cudaMemset(g.state + 3, 0, 4));
+  }
+  unfinished = false;
+  return LCU_OK;
 }
 
 // After the step's stream has been synchronised: the last stage's word came back with the token (h_stage[3]); with
@@ -1046,7 +1120,7 @@ int llama_context_impl::enqueue_prefill(int m_rows, const pass_request& rq) {
   }
   if (rq.n_want) {
     device_guard dg(last().device);
-    LCU_CUDA(cudaStreamSynchronize(last().stream));
+    LCU_TRY(read_back(last(), last().stream, h_stage + 4, 1, "step"));
     LCU_TRY(read_step_logits(rq.logits_out));
   }
   return LCU_OK;
@@ -1139,6 +1213,7 @@ int context::next_token(const short* tokens, int n, int* token_out) { return ste
 int context::step(const short* tokens, int n, const int* want, int n_want, float* logits_out, int* token_out) {
   context_impl& c = *impl;
   LCU_REQUIRE(n >= 1, "next_token: no tokens given");
+  LCU_TRY(c.settled("next_token"));
   LCU_REQUIRE(n + c.start_pos <= c.opt.context_len, "next_token: %d new tokens at position %d exceed the context length %d", n,
               c.start_pos, c.opt.context_len);
   for (int i = 0; i < n; ++i)
@@ -1159,8 +1234,7 @@ int context::step(const short* tokens, int n, const int* want, int n_want, float
   }
   c.last_row = n == 1 ? 0 : n - 1;
   device_guard dg(c.first().device);
-  LCU_CUDA(cudaMemcpyAsync(c.h_stage + 2, c.last().state + 2, 8, cudaMemcpyDeviceToHost, c.first().stream));
-  LCU_CUDA(cudaStreamSynchronize(c.first().stream));
+  LCU_TRY(c.read_back(c.last(), c.first().stream, c.h_stage + 2, 1, "next_token"));
   LCU_TRY(finish_step(*this, "next_token"));
   c.start_pos += n;
   if (single)
@@ -1175,14 +1249,14 @@ int context::decode_chained(short first_token, int n_steps, short* tokens_out, f
               n_steps, c.start_pos, c.opt.context_len);
   LCU_REQUIRE(first_token >= 0 && first_token < c.n_vocab, "decode_chained: token id %d outside the vocabulary", first_token);
   LCU_REQUIRE(!c.rows_only(), "decode_chained: matmul_type 1 runs host-driven steps only (lcu_context_next_token)");
+  LCU_TRY(c.settled("decode_chained"));
   LCU_TRY(c.stage_inputs(&first_token, 1));
   device_guard dg(c.first().device);
   LCU_CUDA(cudaEventRecord(c.t0, c.first().stream));
   for (int i = 0; i < n_steps; ++i) LCU_TRY(c.run_decode_step(c.start_pos + i + 1));
   LCU_CUDA(cudaEventRecord(c.t1, c.first().stream));
   LCU_CUDA(cudaMemcpyAsync(c.h_ids, c.log, (size_t)n_steps * 2, cudaMemcpyDeviceToHost, c.first().stream));
-  LCU_CUDA(cudaMemcpyAsync(c.h_stage + 2, c.last().state + 2, 8, cudaMemcpyDeviceToHost, c.first().stream));
-  LCU_CUDA(cudaStreamSynchronize(c.first().stream));
+  LCU_TRY(c.read_back(c.last(), c.first().stream, c.h_stage + 2, n_steps, "decode_chained"));
   LCU_TRY(finish_step(*this, "decode_chained"));
   c.start_pos += n_steps;
   c.last_row = 0;
@@ -1193,12 +1267,16 @@ int context::decode_chained(short first_token, int n_steps, short* tokens_out, f
 
 int context::read_probs(__half* out_host) {
   context_impl& c = *impl;
+  LCU_TRY(c.settled("read_probs"));
   device_guard dg(c.last().device);
   LCU_CUDA(cudaMemcpy(out_host, c.probs, (size_t)c.n_vocab * 2, cudaMemcpyDeviceToHost));
   return LCU_OK;
 }
 
-int context::read_hidden(__half* out_host) { return impl->read_hidden(out_host); }
+int context::read_hidden(__half* out_host) {
+  LCU_TRY(impl->settled("read_hidden"));
+  return impl->read_hidden(out_host);
+}
 
 int llama_context_impl::read_hidden(__half* out_host) {
   device_guard dg(last().device);
@@ -1209,6 +1287,7 @@ int llama_context_impl::read_hidden(__half* out_host) {
 }
 
 int context::bench_kernel(int which, int reps, float* ms_per_launch, uint64_t* bytes_per_launch) {
+  LCU_TRY(impl->settled("bench_kernel"));
   return impl->bench_kernel(which, reps, ms_per_launch, bytes_per_launch);
 }
 

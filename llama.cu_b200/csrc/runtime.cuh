@@ -22,6 +22,7 @@ struct device_guard {
   device_guard& operator=(const device_guard&) = delete;
 };
 
+int& host_wait_limit_ms();    // how long a call of a context waits for its streams; 0 = no limit
 int* device_scratch_words();  // 64 zeroed ints on the current device (error word of the stand-alone operators)
 
 #pragma pack(push, 1)

@@ -76,6 +76,9 @@ struct tc_ring {
     }
   }
 };
+// Tensor memory beside programmatic launches: tcgen05.alloc waits, without a limit, for the columns it asks for.  Kernels therefore
+// allocate before griddepcontrol.launch_dependents (with a __syncthreads between): a CTA of a later kernel that already holds columns
+// then never stands before an earlier kernel's CTA that still needs some.
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {

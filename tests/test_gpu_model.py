@@ -315,3 +315,50 @@ def test_small_model_against_reference_forward(lcu, bs, u8_mode):
     ref.close()
     ctx.close()
     model.close()
+
+
+@pytest.mark.parametrize("family", ["llama", "block"])
+def test_a_wait_for_the_gpu_that_runs_out_is_an_error_and_not_the_end(lcu, family, tmp_path):
+    """A call that waits longer than "host_wait_limit_ms" returns LCU_ERR_DEVICE_WAIT while the GPU works on; later calls refuse until it
+    has finished and the tokens are cleared, and then give what they gave before."""
+    if family == "llama":
+        model = lcu.Model.synthetic(block_size=0, seed=5, scale=0.08, **SMALL)
+    else:
+        import block_cases as B
+
+        cfg, W = B.case(seed=4, layers=("parallel", "wkv"))
+        B.write(str(tmp_path), cfg, W)
+        model = lcu.Model.load(str(tmp_path), dtype="bfloat16")
+    ctx = lcu.Context(model, context_len=1024)
+    prompt = np.arange(3, 20)
+    first, logits = ctx.next_token(prompt), ctx.step([5], want=[0])
+    ctx.clear_tokens()
+    want = ctx.decode_chained(5, 900)[0]
+    lcu.check(lcu.lib.lcu_set_tuning(b"host_wait_limit_ms", 1))
+    try:
+        ctx.clear_tokens()
+        with pytest.raises(lcu.LcuError, match="not finished within"):  # 900 steps, two milliseconds
+            ctx.decode_chained(5, 900)
+        with pytest.raises(lcu.LcuError, match="clear the tokens"):
+            ctx.next_token([5])
+        with pytest.raises(lcu.LcuError, match="clear the tokens"):
+            ctx.probs()
+    finally:
+        lcu.check(lcu.lib.lcu_set_tuning(b"host_wait_limit_ms", 600000))
+    lcu.check(lcu.lib.lcu_synchronize())
+    with pytest.raises(lcu.LcuError, match="clear the tokens"):
+        ctx.next_token([5])
+    ctx.clear_tokens()
+    assert ctx.next_token(prompt) == first and (ctx.step([5], want=[0]) == logits).all()
+    ctx.clear_tokens()
+    assert (ctx.decode_chained(5, 900)[0] == want).all()
+    # a context that is given up on while it runs is left behind without a wait
+    lcu.check(lcu.lib.lcu_set_tuning(b"host_wait_limit_ms", 1))
+    try:
+        left = lcu.Context(model, context_len=1024)
+        with pytest.raises(lcu.LcuError, match="not finished within"):
+            left.decode_chained(5, 900)
+        left.close()
+    finally:
+        lcu.check(lcu.lib.lcu_set_tuning(b"host_wait_limit_ms", 600000))
+    lcu.check(lcu.lib.lcu_synchronize())
