@@ -72,6 +72,13 @@ int lcu_quantize_host(uint8_t* q_host, uint16_t* scales_host, const uint16_t* in
 int lcu_quantize_model_dir(const char* in_dir, const char* out_dir, int bs);
 
 /* ---- operators (the reference's internal seam) ---------------------------------------------- */
+/* Operators return once their kernels are launched.  A kernel whose bounded wait runs out leaves its results unwritten and a code in
+ * the current device's operator error word.  lcu_operator_status, called after the caller has waited for its stream: 0, or status 4
+ * (LCU_ERR_DEVICE_WAIT) with the code, and the word is clear again.  While a code stands, half-precision products of several rows and
+ * prompt attention stay without results; the other operators do not look at codes of earlier launches.
+ * lcu_operator_error_word: the word's device address, for callers that look at it in stream order. */
+int lcu_operator_status(int* device_code_out);
+int lcu_operator_error_word(void** dev_out);
 /* matmul_nt(out, lhs, rhs, beta, stream), llama_cu.cu:738-742 / 1463-1496:
  * out(m,n) = lhs(m,k) . rhs(n,k)^T + beta * out, fp16 in/out, fp32 accumulation.  No gutter rows needed. */
 int lcu_matmul_nt_f16(void* out_dev, const void* lhs_dev, const void* rhs_dev, int m, int k, int n, float beta, void* stream);

@@ -56,6 +56,8 @@ _SIG = {
     "lcu_attention": (C.c_int, [vp, vp, vp, vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, vp]),
     "lcu_logits_head": (C.c_int, [vp, vp, C.c_int, C.c_float, C.POINTER(C.c_int), vp]),
     "lcu_selftest_bounded_wait": (C.c_int, [C.POINTER(C.c_int)]),
+    "lcu_operator_error_word": (C.c_int, [C.POINTER(vp)]),
+    "lcu_operator_status": (C.c_int, [C.POINTER(C.c_int)]),
     "lcu_selftest_quantizer_arithmetic": (C.c_int, [C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]),
     "lcu_selftest_balanced_schedule": (C.c_int, [C.c_int, C.c_int, C.c_int]),
     "lcu_plan_long_prompt_gemm": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int)]),

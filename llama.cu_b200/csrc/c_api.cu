@@ -234,6 +234,24 @@ int lcu_quantize_model_dir(const char* in_dir, const char* out_dir, int bs) {
 }
 
 // ---- operators
+int lcu_operator_error_word(void** dev_out) {
+  NEED_DEVICE();
+  LCU_REQUIRE(dev_out && scratch_err(), "operator_error_word: no scratch");
+  *dev_out = scratch_err();
+  return LCU_OK;
+}
+int lcu_operator_status(int* device_code_out) {
+  NEED_DEVICE();
+  int* err = scratch_err();
+  LCU_REQUIRE(err != nullptr, "operator_status: no scratch");
+  int code = 0;
+  LCU_CUDA(cudaMemcpy(&code, err, 4, cudaMemcpyDeviceToHost));
+  if (device_code_out) *device_code_out = code;
+  if (code == 0) return LCU_OK;
+  LCU_CUDA(cudaMemset(err, 0, 4));
+  set_last_error("a kernel gave up on a bounded wait (device code 0x%x)", code);
+  return LCU_ERR_DEVICE_WAIT;
+}
 int lcu_matmul_nt_f16(void* out_dev, const void* lhs_dev, const void* rhs_dev, int m, int k, int n, float beta, void* stream) {
   NEED_DEVICE();
   LCU_REQUIRE(m >= 1, "matmul_nt: m must be positive");

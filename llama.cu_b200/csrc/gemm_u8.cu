@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)nstages * STAGE);
   uint64_t *full = bars, *empty = bars + U8_MAX_STAGES, *conv = empty + U8_MAX_STAGES, *freed = conv + U8_BUFS, *done = freed + U8_BUFS;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  volatile float* failed = reinterpret_cast<volatile float*>(tmem_slot + 1);  // 1: a wait of this CTA ran out
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = splits > 1 ? (int)cluster_ctarank() : 0;
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
       mbar_init(smem_u32(&freed[i]), 1);
     }
     mbar_init(smem_u32(done), 1);
+    *failed = 0.f;
     fence_mbar_init();
   }
   if (warp == U8_CONV_WARPS + 1) {
@@ -107,6 +109,8 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
   const uint32_t tmem = *tmem_slot;
   pdl_launch_dependents();
   pdl_wait();
+  // Nobody clears the error word between stand-alone calls: what an earlier launch left there does not concern this one.
+  const int seen = *(volatile int*)err;
 
   // rows of the tile this thread converts and stores; tiles may hang over N
   const int quad = warp & 3, group = warp >> 2, row = quad * 32 + lane, n = n0 + row;
@@ -136,8 +140,8 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
         if (blk >= n_blk) break;
         const uint32_t sw = ahead[u];
         ahead[u] = scales_of(blk + U8_AHEAD * U8_GROUPS);
-        ok = mbar_wait(smem_u32(&full[s]), phase, err, DEV_ERR_FULL_WAIT);
-        if (ok && blk >= U8_BUFS) ok = mbar_wait(smem_u32(&freed[buf]), (blk / U8_BUFS - 1) & 1, err, DEV_ERR_EMPTY_WAIT);
+        ok = mbar_wait(smem_u32(&full[s]), phase, err, DEV_ERR_FULL_WAIT, seen);
+        if (ok && blk >= U8_BUFS) ok = mbar_wait(smem_u32(&freed[buf]), (blk / U8_BUFS - 1) & 1, err, DEV_ERR_EMPTY_WAIT, seen);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
@@ -166,14 +170,15 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
         }
       }
     }
-    ok = mbar_wait(smem_u32(done), 0, err, DEV_ERR_TMEM_WAIT) && ok;
+    ok = mbar_wait(smem_u32(done), 0, err, DEV_ERR_TMEM_WAIT, seen) && ok;
     tc_fence_after();
-    go = __all_sync(0xffffffffu, ok && *(volatile int*)err == 0);
+    go = __all_sync(0xffffffffu, ok && *failed == 0.f);
+    if (!go && lane == 0) *failed = 1.f;
   } else if (warp == U8_CONV_WARPS) {
     if (tc_elect()) {  // ---- TMA producer
       tc_ring r;
       for (int i = 0; i < n_st; ++i, r.step(nstages)) {
-        if (!mbar_wait(smem_u32(&empty[r.slot]), r.phase ^ 1u, err, DEV_ERR_EMPTY_WAIT)) break;
+        if (!mbar_wait(smem_u32(&empty[r.slot]), r.phase ^ 1u, err, DEV_ERR_EMPTY_WAIT, seen)) break;
         const uint32_t bar = smem_u32(&full[r.slot]), dst = base + (uint32_t)r.slot * STAGE;
         mbar_arrive_expect_tx(bar, STAGE);
         tma_load_2d(dst, &map_q, (st0 + i) * (U8_STAGE_K / 2), n0, bar);
@@ -185,12 +190,12 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
     bool ok = true;
     tc_ring r, e;
     for (int i = 0; i < n_st && ok; ++i, r.step(nstages)) {
-      ok = mbar_wait_warp(smem_u32(&full[r.slot]), r.phase, err, DEV_ERR_FULL_WAIT);
+      ok = mbar_wait_warp(smem_u32(&full[r.slot]), r.phase, err, DEV_ERR_FULL_WAIT, seen);
       if (!ok) break;
       const uint64_t x = smem_desc_sw128(base + (uint32_t)r.slot * STAGE + U8_Q_BYTES);
 #pragma unroll
       for (int g = 0; g < 2; ++g, e.step(U8_BUFS)) {
-        ok = ok && mbar_wait_warp(smem_u32(&conv[e.slot]), e.phase, err, DEV_ERR_FULL_WAIT);
+        ok = ok && mbar_wait_warp(smem_u32(&conv[e.slot]), e.phase, err, DEV_ERR_FULL_WAIT, seen);
         if (!ok) break;
         tc_fence_after();
         if (tc_elect()) {
@@ -204,7 +209,11 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
         __syncwarp();
       }
     }
-    if (tc_elect()) tc_commit(smem_u32(done));  // (also after a failed wait: lets the other warps leave)
+    if (tc_elect()) {  // (also after a failed wait: lets the other warps leave, without results)
+      if (!ok) *failed = 1.f;
+      __threadfence_block();
+      tc_commit(smem_u32(done));
+    }
     __syncwarp();
   }
 
@@ -237,7 +246,8 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
       }
     __syncwarp();
     cluster_sync();
-    if (go && *(volatile int*)err == 0)
+    for (int q = 0; q < splits && go; ++q) go = ld_dsmem_f32(mapa(smem_u32((const void*)failed), (uint32_t)q)) == 0.f;
+    if (go)
       for (int c = 16 * (rank + splits * group); c < t; c += 16 * U8_GROUPS * splits) {
         float sum[16];
 #pragma unroll
@@ -333,6 +343,7 @@ bool gemm_u8_supported(int m, int N, int K, int bs, const void* lhs, const void*
 
 int launch_gemm_u8(__half* out, const __half* lhs, const uint8_t* q, const __half* scales, int bs, int m, int N, int K, float beta, int* err,
                    cudaStream_t stream) {
+  LCU_REQUIRE(err != nullptr, "gemm_u8: no error word");
   LCU_REQUIRE(gemm_u8_supported(m, N, K, bs, lhs, q, scales), "gemm_u8: unsupported shape m=%d N=%d K=%d blocks of %d or unaligned pointers", m, N, K, bs);
   int t = 16, splits = 1;
   gemm_u8_plan(m, N, K, gemv_sm_count(), &t, &splits);

@@ -169,6 +169,28 @@ def test_product_expands_8_bit_weights(lcu, m, k, n, beta, bs):
     assert np.abs(f32(y) - f32(y_gemv)).max() <= bound
 
 
+@pytest.mark.parametrize("m,k,n", [(200, 512, 384), (9, 4096, 256)])  # one CTA per tile, and K split over a cluster
+def test_product_with_8_bit_weights_behind_an_earlier_error(lcu, m, k, n):
+    """A code that another operator's launch left in the error word does not keep a product from its results, and is reported."""
+    import ctypes as C
+    rng = np.random.default_rng(m)
+    x = f16(rng.standard_normal((m, k)))
+    q, s = O.quantize(f16(rng.standard_normal((n, k)) * 0.05), n, k, 64)
+    want = lcu.matmul_nt(x, q, s, 64)
+    word, code = C.c_void_p(), C.c_int(-1)
+    lcu.check(lcu.lib.lcu_operator_error_word(C.byref(word)))
+    assert lcu.lib.lcu_operator_status(C.byref(code)) == 0 and code.value == 0
+    stale = np.array([0x103], np.int32)
+    lcu.check(lcu.lib.lcu_memcpy_h2d(word, stale.ctypes.data, 4))
+    try:
+        got = lcu.matmul_nt(x, q, s, 64)
+    finally:
+        rc = lcu.lib.lcu_operator_status(C.byref(code))
+    assert np.array_equal(got, want)
+    assert rc == 4 and code.value == 0x103
+    assert lcu.lib.lcu_operator_status(C.byref(code)) == 0 and code.value == 0
+
+
 @pytest.mark.parametrize("m,k,n,beta,tile", [(9, 64, 32, 0.0, 0), (16, 256, 32, 1.0, 0), (128, 64, 128, 0.0, 128), (129, 512, 192, 1.0, 0),
                                              (200, 1024, 256, 1.0, 64), (77, 4096, 1024, 0.0, 32), (300, 11008, 128, 0.0, 0),
                                              (257, 4096, 4096, 1.0, 0),
