@@ -279,9 +279,9 @@ int lcu_selftest_quantizer_arithmetic(uint64_t* checked_out, uint64_t* differenc
  * a GPU of `sms` SMs - the tile width (96 to 256 columns; the last tile may hang over n) and the split-K factor (1, 2 or 4,
  * 128-wide tiles only) - chosen so that one wave of CTAs streams the matrix in equal shares.  n a multiple of 128, k of 64. */
 int lcu_plan_short_prompt_gemm(int n, int k, int sms, int* tile_n_out, int* split_out);
-/* The same for m > 128 rows: *kernel_out = 0 for whole 256-row tiles per SM pair, 256 or 512 for the kernel that deals the K
- * steps of the last wave's tiles evenly over the pairs, with tiles that wide (estimates fitted to timings on B200).  The choice
- * between these two; the product itself may take narrower tiles or one SM per tile where those are estimated shorter still. */
+/* The same for m > 128 rows: *kernel_out = 1 for a 128 x 128 tile per SM, 0 or 128 for whole 256-row tiles of 256 or 128 columns per SM
+ * pair, 256 or 512 for the kernel that deals the K steps of the last wave's tiles evenly over the pairs, with tiles that wide
+ * (estimates fitted to timings on B200). */
 int lcu_plan_long_prompt_gemm(int m, int n, int k, int sms, int* kernel_out);
 /* Host walk of that kernel's work list (no device needed) for n_tiles output tiles of k_steps 64-wide K steps on sm_pairs
  * pairs of SMs: 0 when every K step of every tile is run by exactly one pair, a pair hands partial sums over at most once,

@@ -684,25 +684,10 @@ int& gemm_tc_sk_mode() {
   return mode;
 }
 
-// Estimated duration (microseconds) of an [m][K] x [N][K]^T product, m > 128, on the three kernels: whole tiles per SM
-// pair, and the balanced kernel with 256- and 512-wide tiles.  Fitted to timings of the 7B, 13B and 65B products at 200 to
-// 2048 rows (56 shapes; the picks sum to 10.45 ms against 10.26 ms for the best of the three each time, 11.10 ms for whole
-// tiles alone and 10.51 ms for the balanced 256-wide kernel alone).
-static void gemm_tc_estimates(int m, int N, int K, int sms, double* whole_us, double* t256_us, double* t512_us) {
+// Estimated duration (microseconds) of an [m][K] x [N][K]^T product, m > 128, on the balanced kernel with 256- and 512-wide tiles.
+// Fitted to timings of the 7B, 13B and 65B products at 200 to 2048 rows (56 shapes).
+static void gemm_tc_balanced_estimates(int m, int N, int K, int sms, double* t256_us, double* t512_us) {
   const long C = sms / 2, nk = K / BK, tm = (m + 2 * BM - 1) / (2 * BM);
-  auto ceil_div_l = [](long a, long b) { return (a + b - 1) / b; };
-  double whole;
-  if ((m > 2 * BM || N > 8192) && N % 128 == 0) {
-    const long n256 = tm * (N / 256);
-    // (several hundred tiles of a short K: the whole-tile kernel's epilogues weigh more, 0.42 us per K step measured)
-    if (N % 256 == 0 && n256 * 4 >= C * 3) whole = ceil_div_l(n256, C) * nk * (n256 > 300 && nk <= 80 ? 0.42 : n256 > 40 ? 0.38 : 0.34) + 5;
-    else whole = ceil_div_l(tm * (N / 128), C) * nk * 0.37 + 5;
-  } else {
-    const long n128 = (long)((m + BM - 1) / BM) * (N / 128);
-    long sp = n128 * 4 <= sms ? 4 : n128 * 2 <= sms ? 2 : 1;
-    if (nk < 8 * sp) sp = 1;
-    whole = ceil_div_l(n128 * sp, sms) * ((double)nk / sp) * 0.40 + 6;
-  }
   auto balanced = [&](int bn) -> double {
     if (N % bn) return 1e30;
     const long n = tm * (N / bn), full = n / C, rest = n - full * C;
@@ -716,34 +701,18 @@ static void gemm_tc_estimates(int m, int N, int K, int sms, double* whole_us, do
     }
     return t;
   };
-  *whole_us = whole;
   *t256_us = balanced(256);
   *t512_us = N >= 2 * K ? balanced(512) : 1e30;
 }
 
-// More than 128 rows, the choice between these two kernels alone (gemm_tc_pick_long has more): 0 = whole tiles per SM pair,
-// 256 / 512 = the balanced kernel with that tile width (the one whose estimate is lowest; a balanced kernel has to beat whole tiles by 3 %).
-int gemm_tc_plan_long(int m, int N, int K, int sms) {
-  double whole, t256, t512;
-  gemm_tc_estimates(m, N, K, sms, &whole, &t256, &t512);
-  double best = whole;
-  int tile = 0;
-  if (t256 < 0.97 * whole && t256 < best) {
-    best = t256;
-    tile = 256;
-  }
-  if (t512 < 0.97 * whole && t512 < best) tile = 512;
-  return tile;
-}
-
-// More than 128 rows, operands issued from warp-uniform code: which kernel runs the product.  The estimates (microseconds) follow
-// timings of 16 shapes (K, N from 1024 to 22016) at 129 to 2000 rows on each kernel: a K step of 64 takes 0.26 us on the one-SM kernel
-// (128 x 128 tiles, K split over 2 or 4 CTAs where tiles are few; 0.30 once an SM has several), 0.205 to 0.235 on 256 x 128 pair
-// tiles, 0.34 to 0.42 on 256 x 256 ones; the balanced kernel as in gemm_tc_estimates.  What the choice between whole 256-row tiles and
+// More than 128 rows, operands issued from warp-uniform code: which kernel runs the product (tc_long_kernel).  The estimates
+// (microseconds) follow timings of 16 shapes (K, N from 1024 to 22016) at 129 to 2000 rows on each kernel: a K step of 64 takes 0.26 us
+// on the one-SM kernel (128 x 128 tiles, K split over 2 or 4 CTAs where tiles are few; 0.30 once an SM has several), 0.205 to 0.235 on
+// 256 x 128 pair tiles, 0.34 to 0.42 on 256 x 256 ones; the balanced kernel as above.  What the choice between whole 256-row tiles and
 // the balanced kernel alone took before, in us: 300 rows of 2048 x 6144 23.3 -> 14.3 (one SM), of 5632 x 2048 23.8 -> 18.4 (one SM),
 // 509 of 11008 x 4096 52.0 -> 43.0 (128-wide pairs), 1000 of 5632 x 2048 34.8 -> 23.4 (128-wide pairs).
-enum tc_long_kernel { TC_ONE_SM, TC_PAIR_128, TC_PAIR_256, TC_BALANCED_256, TC_BALANCED_512 };
-static tc_long_kernel gemm_tc_pick_long(int m, int N, int K, int sms, bool balanced_too, double* best_whole_us = nullptr) {
+// balanced_too: the balanced kernel may run it (16-bit results); best_whole_us: the lowest estimate without it.
+int gemm_tc_plan_long(int m, int N, int K, int sms, bool balanced_too, double* best_whole_us) {
   const long C = sms / 2, nk = K / BK, tm = (m + 2 * BM - 1) / (2 * BM);
   auto ceil_div_l = [](long a, long b) { return (a + b - 1) / b; };
   double best = 1e30;
@@ -767,8 +736,8 @@ static tc_long_kernel gemm_tc_pick_long(int m, int N, int K, int sms, bool balan
   }
   if (best_whole_us) *best_whole_us = best;
   if (balanced_too) {  // (has to win by 3 %)
-    double whole, t256, t512;
-    gemm_tc_estimates(m, N, K, sms, &whole, &t256, &t512);
+    double t256, t512;
+    gemm_tc_balanced_estimates(m, N, K, sms, &t256, &t512);
     if (std::min(t256, t512) < 0.97 * best) pick = t256 <= t512 ? TC_BALANCED_256 : TC_BALANCED_512;
   }
   return pick;
@@ -787,9 +756,10 @@ int gemm_tc_gated_tile(int m, int f, int K) {
   // its duration is the balanced kernel's for the stacked product plus about 3 us measured, more beyond 1024 rows)
   // against the best kernel for the stacked product plus the gate kernel's pass over the result (6 bytes per output
   // element at about 5 TB/s, and a launch).  7B shapes: the one launch wins 4 to 8 us per layer from 129 to 1024 rows.
+  if ((2 * f) % 256) return 0;
   double whole, t256, t512;
-  gemm_tc_estimates(m, 2 * f, K, gemv_sm_count(), &whole, &t256, &t512);
-  if ((2 * f) % 128 == 0) gemm_tc_pick_long(m, 2 * f, K, gemv_sm_count(), false, &whole);
+  gemm_tc_balanced_estimates(m, 2 * f, K, gemv_sm_count(), &t256, &t512);
+  gemm_tc_plan_long(m, 2 * f, K, gemv_sm_count(), false, &whole);
   const double gate_us = (double)m * f * 6.0 / 5.0e6 + 2;
   const double one_launch = t256 + 3 + (m > 1024 ? (m - 1024) * 0.016 : 0.0);
   return one_launch < std::min(whole, t512) + gate_us ? 256 : 0;
@@ -806,7 +776,7 @@ int launch_gemm_shape(void* out, const void* lhs, int ldx, const void* w, int m,
                       int force_bn, int force_pair, int force_split) {
   LCU_REQUIRE(gemm_tc_supported(m, N, K, ldx, lhs, w, out), "gemm_tc: unsupported shape m=%d N=%d K=%d ldx=%d or unaligned pointers", m, N, K, ldx);
   const int sms = gemv_sm_count();
-  // More than 128 rows: gemm_tc_pick_long between the one-SM kernel, whole tiles per SM pair and the kernel that deals the K steps of
+  // More than 128 rows: gemm_tc_plan_long between the one-SM kernel, whole tiles per SM pair and the kernel that deals the K steps of
   // the last, partial wave evenly over the pairs (gemm_tc_sk.cu; 16-bit results only), unless a mode forces one of them
   // (gemm_tc_sk_mode: 256 / 512 = the balanced kernel with that tile width, 0 = never).
   int pair = force_pair;
@@ -815,7 +785,7 @@ int launch_gemm_shape(void* out, const void* lhs, int ldx, const void* w, int m,
     const int mode = sizeof(TO) == 2 ? gemm_tc_sk_mode() : 0;
     int tile = mode > 0 ? mode : 0;
     if (N % 128 == 0) {
-      const tc_long_kernel k = gemm_tc_pick_long(m, N, K, sms, mode < 0);
+      const int k = gemm_tc_plan_long(m, N, K, sms, mode < 0);
       if (mode < 0) tile = k == TC_BALANCED_256 ? 256 : k == TC_BALANCED_512 ? 512 : 0;
       pair = m <= BM ? 0 : k == TC_PAIR_128 ? 128 : k == TC_PAIR_256 ? 256 : 0;
     }

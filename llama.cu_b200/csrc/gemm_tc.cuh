@@ -48,9 +48,10 @@ int launch_gemm_tc_grouped(tc_type type, void* out, const void* lhs, int ldx, co
 // -1 (default) = launch_gemm_tc uses it, with 256- or 512-wide tiles, where its estimate says it wins; 256 / 512 =
 // always, with that tile width, where it divides N; 0 = never
 int& gemm_tc_sk_mode();
-// more than 128 rows: the choice between whole tiles per SM pair (0) and the balanced kernel (256 / 512: its tile width) on a GPU
-// of `sms` SMs; launch_gemm_tc weighs narrower tiles and the one-SM kernel besides.  Pure host arithmetic.
-int gemm_tc_plan_long(int m, int N, int K, int sms);
+// more than 128 rows, N a multiple of 128: the kernel launch_gemm_tc takes on a GPU of `sms` SMs - 128 x 128 tiles on one SM each,
+// whole 256-row tiles per SM pair, or the balanced kernel - with its tile width.  Pure host arithmetic.
+enum tc_long_kernel { TC_PAIR_256 = 0, TC_ONE_SM = 1, TC_PAIR_128 = 128, TC_BALANCED_256 = 256, TC_BALANCED_512 = 512 };
+int gemm_tc_plan_long(int m, int N, int K, int sms, bool balanced_too = true, double* best_whole_us = nullptr);
 // one-SM kernel, up to 128 rows, N a multiple of 128: the tile width (96 to 256) and split-K factor (1, 2, 4; 128-wide
 // tiles only) launch_gemm_tc uses on a GPU of `sms` SMs.  Pure host arithmetic.
 void gemm_tc_plan_short(int N, int K, int sms, int* tile_n, int* split);

@@ -86,9 +86,9 @@ def test_short_prompt_gemm_plan_fills_one_wave():
 
 
 def test_long_prompt_gemm_plan_follows_the_measurements():
-    """Host arithmetic behind lcu_matmul_nt_f16 for more than 128 rows: whole tiles per SM pair (0) or the kernel that
-    deals the last wave's K steps evenly (256).  Pinned where the two were measured more than 5 % apart on a B200 (7B
-    shapes, microseconds whole / balanced in the comments)."""
+    """Host arithmetic behind lcu_matmul_nt_f16 for more than 128 rows: a 128 x 128 tile per SM (1), whole 256-row tiles of 256 (0) or
+    128 columns per SM pair, or the kernel that deals the last wave's K steps evenly (256, 512).  Pinned where the best two were
+    measured more than 5 % apart on a B200 (microseconds on one SM / 128-wide / 256-wide / balanced 256 in the comments)."""
     lcu = load_package()
 
     def plan(m, n, k, sms=148):
@@ -96,15 +96,20 @@ def test_long_prompt_gemm_plan_follows_the_measurements():
         lcu.check(lcu.lib.lcu_plan_long_prompt_gemm(m, n, k, sms, C.byref(out)))
         return out.value
 
-    assert plan(512, 22016, 4096) == 256    # 83.1 / 78.5: 172 tiles for 74 pairs, the third wave is a third full
-    assert plan(2048, 22016, 4096) == 256   # 278 / 259
-    assert plan(512, 4096, 4096) == 0       # 28.9 / 33.4: every tile would be handed over
-    assert plan(768, 4096, 4096) == 256     # 48.9 / 34.3
-    assert plan(512, 4096, 11008) == 256    # 82.4 / 66.1
-    assert plan(1024, 4096, 11008) == 0     # 72.3 / 83.3: 64 tiles, one wave
+    assert plan(256, 2048, 5632) == 1       # 14.1 / 22.6 / 33.7 / 23.7: 32 tiles, K split over four CTAs
+    assert plan(300, 6144, 2048) == 1       # 13.9 / 19.1 / 19.1 / 22.6: 144 tiles, one wave
+    assert plan(509, 4096, 4096) == 128     # 20.8 / 19.2 / 27.8 / 29.8: 64 tiles for 74 pairs
+    assert plan(509, 4096, 11008) == 128    # 49.6 / 42.8 / 61.1 / 51.8
+    assert plan(1000, 5632, 1024) == 128    # 22.9 / 17.9 / 19.6 / 23.6
+    assert plan(777, 4096, 4096) == 0       # 37.0 / 30.8 / 28.2 / 34.5
+    assert plan(1300, 6144, 2048) == 0      # 45.2 / 33.5 / 30.7 / 35.0
+    assert plan(300, 22016, 4096) == 256    # 107.5 / 77.9 / 76.8 / 71.0: 172 tiles for 74 pairs, the third wave is a third full
+    assert plan(777, 15360, 5120) == 256    # 189.9 / 133.6 / 131.2 / 119.6
+    assert plan(1600, 4096, 11008) == 256   # 154.8 / 148.0 / 133.6 / 117.6
     for m in (129, 300, 777, 2048, 8192):
-        for n, k in ((4096, 4096), (12288, 4096), (22016, 4096), (27648, 5120), (8192, 22016), (32000, 4096)):
-            assert plan(m, n, k) in (0, 256, 512)
+        for n, k in ((4096, 4096), (12288, 4096), (22016, 4096), (27648, 5120), (8192, 22016), (32000, 4096), (1024, 64), (128, 320)):
+            assert plan(m, n, k) in (0, 1, 128, 256, 512)
+            assert n % 256 == 0 or plan(m, n, k) in (1, 128)
     with pytest.raises(lcu.LcuError):
         plan(128, 4096, 4096)
 
