@@ -706,11 +706,12 @@ static void gemm_tc_balanced_estimates(int m, int N, int K, int sms, double* t25
 }
 
 // More than 128 rows, operands issued from warp-uniform code: which kernel runs the product (tc_long_kernel).  The estimates
-// (microseconds) follow timings of 16 shapes (K, N from 1024 to 22016) at 129 to 2000 rows on each kernel: a K step of 64 takes 0.26 us
-// on the one-SM kernel (128 x 128 tiles, K split over 2 or 4 CTAs where tiles are few; 0.30 once an SM has several), 0.205 to 0.235 on
-// 256 x 128 pair tiles, 0.34 to 0.42 on 256 x 256 ones; the balanced kernel as above.  What the choice between whole 256-row tiles and
-// the balanced kernel alone took before, in us: 300 rows of 2048 x 6144 23.3 -> 14.3 (one SM), of 5632 x 2048 23.8 -> 18.4 (one SM),
-// 509 of 11008 x 4096 52.0 -> 43.0 (128-wide pairs), 1000 of 5632 x 2048 34.8 -> 23.4 (128-wide pairs).
+// (microseconds) are fitted to device times of 27 shapes (K from 64 to 22016, N from 1024 to 27648) at 13 row counts from 129 to 2000 on
+// each of the five kernels: a K step of 64 takes 0.26 us on the one-SM kernel (128 x 128 tiles, K split over 2 or 4 CTAs where tiles are
+// few; 0.365 once an SM has several), 0.215 to 0.235 on 256 x 128 pair tiles, 0.38 to 0.42 on 256 x 256 ones; the balanced kernel as
+// above.  The picks take 0.2 % longer than the best kernel each time, 0.3 % over 120 random shapes that were not fitted (13 % at the
+// worst, K = 192); with the constants of whole shapes alone, short K went to wide pair tiles: 200 rows of 64 x 1024 6.4 us (one SM: 3.7),
+// of 512 x 4096 6.5 (5.6), of 1024 x 3072 9.2 (8.0).
 // balanced_too: the balanced kernel may run it (16-bit results); best_whole_us: the lowest estimate without it.
 int gemm_tc_plan_long(int m, int N, int K, int sms, bool balanced_too, double* best_whole_us) {
   const long C = sms / 2, nk = K / BK, tm = (m + 2 * BM - 1) / (2 * BM);
@@ -722,16 +723,16 @@ int gemm_tc_plan_long(int m, int N, int K, int sms, bool balanced_too, double* b
     long sp = tiles * 4 <= sms ? 4 : tiles * 2 <= sms ? 2 : 1;
     if (nk < 8 * sp) sp = 1;
     const long waves = ceil_div_l(tiles * sp, sms);
-    best = waves * ((double)nk / sp) * (waves == 1 ? 0.26 : 0.30) + 6.5 + (sp > 1 ? 1 : 0);
+    best = waves * ((double)nk / sp) * (waves == 1 ? 0.26 : 0.365) + 5.4 + (sp > 1 ? 1 : 0);
   }
   {
     const long waves = ceil_div_l(tm * (N / 128), C);
-    const double est = waves * nk * (waves == 1 ? 0.205 : waves <= (nk < 64 ? 3 : 2) ? 0.215 : 0.235) + 6;
+    const double est = waves * nk * (waves == 1 ? 0.22 : waves <= (nk < 64 ? 3 : 2) ? 0.215 : 0.235) + 6.5;
     if (est < best) best = est, pick = TC_PAIR_128;
   }
   if (N % 256 == 0) {
     const long tiles = tm * (N / 256);
-    const double est = ceil_div_l(tiles, C) * nk * (tiles > 300 && nk <= 80 ? 0.42 : tiles > 40 ? 0.38 : 0.34) + 5;
+    const double est = ceil_div_l(tiles, C) * nk * (tiles > 300 && nk <= 80 ? 0.42 : tiles > 40 ? 0.39 : 0.38) + 7.5;
     if (est < best) best = est, pick = TC_PAIR_256;
   }
   if (best_whole_us) *best_whole_us = best;

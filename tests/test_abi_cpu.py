@@ -98,6 +98,12 @@ def test_long_prompt_gemm_plan_follows_the_measurements():
 
     assert plan(256, 2048, 5632) == 1       # 14.1 / 22.6 / 33.7 / 23.7: 32 tiles, K split over four CTAs
     assert plan(300, 6144, 2048) == 1       # 13.9 / 19.1 / 19.1 / 22.6: 144 tiles, one wave
+    # short K: what a launch takes apart from its K steps decides
+    assert plan(200, 1024, 64) == 1         # 3.7 / 5.1 / 6.4 / 6.5
+    assert plan(256, 4096, 512) == 1        # 5.6 / 6.5 / 8.8 / 15.1
+    assert plan(200, 3072, 1024) == 1       # 8.0 / 9.2 / 13.1 / 15.2
+    assert plan(2000, 4096, 512) == 0       # 21.1 / 16.8 / 14.4 / 22.1
+    assert plan(509, 5632, 1024) == 128     # 15.6 / 13.3 / 14.5 / 19.0
     assert plan(509, 4096, 4096) == 128     # 20.8 / 19.2 / 27.8 / 29.8: 64 tiles for 74 pairs
     assert plan(509, 4096, 11008) == 128    # 49.6 / 42.8 / 61.1 / 51.8
     assert plan(1000, 5632, 1024) == 128    # 22.9 / 17.9 / 19.6 / 23.6
