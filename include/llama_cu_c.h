@@ -283,7 +283,10 @@ int lcu_plan_short_prompt_gemm(int n, int k, int sms, int* tile_n_out, int* spli
  * pair, 256 or 512 for the kernel that deals the K steps of the last wave's tiles evenly over the pairs, with tiles that wide
  * (estimates fitted to timings on B200). */
 int lcu_plan_long_prompt_gemm(int m, int n, int k, int sms, int* kernel_out);
-/* Host walk of that kernel's work list (no device needed) for n_tiles output tiles of k_steps 64-wide K steps on sm_pairs
+/* Products with 8-bit weights that are expanded inside (lcu_matmul_nt_fp16u8 from 2 rows): activation rows per tile (a multiple of 16
+ * up to 224) and the CTAs that share a tile's K (1, 2, 4 or 8).  n even, k a multiple of 256. */
+int lcu_plan_u8_gemm(int m, int n, int k, int sms, int* tile_rows_out, int* splits_out);
+/* Host walk of the balanced kernel's work list (no device needed) for n_tiles output tiles of k_steps 64-wide K steps on sm_pairs
  * pairs of SMs: 0 when every K step of every tile is run by exactly one pair, a pair hands partial sums over at most once,
  * and each shared tile's owner finds exactly the pairs that ran the rest of it, in order; a positive code names the rule
  * that failed, -1 bad arguments. */

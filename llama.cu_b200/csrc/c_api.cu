@@ -635,6 +635,11 @@ int lcu_plan_short_prompt_gemm(int n, int k, int sms, int* tile_n_out, int* spli
   gemm_tc_plan_short(n, k, sms, tile_n_out, split_out);
   return LCU_OK;
 }
+int lcu_plan_u8_gemm(int m, int n, int k, int sms, int* tile_rows_out, int* splits_out) {
+  LCU_REQUIRE(m >= 2 && n >= 2 && n % 2 == 0 && k >= 256 && k % 256 == 0 && sms >= 1 && tile_rows_out && splits_out, "plan_u8_gemm: bad arguments");
+  gemm_u8_plan(m, n, k, sms, tile_rows_out, splits_out);
+  return LCU_OK;
+}
 int lcu_selftest_silu_arithmetic(uint64_t* checked_out, uint64_t* differences_out) {
   NEED_DEVICE();
   unsigned long long a = 0, b = 0;

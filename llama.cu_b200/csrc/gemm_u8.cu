@@ -324,7 +324,7 @@ void gemm_u8_plan(int m, int N, int K, int sms, int* tile_rows, int* splits) {
     const double per_block = std::max(0.235, 0.06 + 0.00156 * t);
     for (int sp = 1; sp <= 8; sp *= 2) {
       if (K / U8_STAGE_K < 2 * sp) continue;
-      const long at_once = sp <= 2 ? sms : sp == 4 ? sms - 12 : sms - 36;
+      const long at_once = std::max(1, sp <= 2 ? sms : sp == 4 ? sms - 12 : sms - 36);
       const long ctas = (long)((N + U8_ROWS - 1) / U8_ROWS) * ((m + t - 1) / t) * sp, waves = (ctas + at_once - 1) / at_once;
       const double est = waves * (5.4 + (double)K / U8_KB / sp * per_block + (sp > 1 ? 0.5 * sp : 0.0));
       if (est < best - 0.2) {  // (ties stay with fewer tiles and no split)

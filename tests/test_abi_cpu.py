@@ -120,6 +120,29 @@ def test_long_prompt_gemm_plan_follows_the_measurements():
         plan(128, 4096, 4096)
 
 
+def test_8_bit_product_plan_on_any_number_of_sms():
+    """Host arithmetic behind lcu_matmul_nt_fp16u8 for several rows: tiles within the kernel's limits, every CTA of a cluster with K of
+    its own, also on a slice of a GPU; and the splits that the shapes of test_product_expands_8_bit_weights stand for."""
+    lcu = load_package()
+
+    def plan(m, n, k, sms=148):
+        t, s = C.c_int(0), C.c_int(0)
+        lcu.check(lcu.lib.lcu_plan_u8_gemm(m, n, k, sms, C.byref(t), C.byref(s)))
+        return t.value, s.value
+
+    for sms in (1, 12, 18, 36, 37, 74, 148):
+        for m in (2, 16, 17, 200, 224, 225, 600, 65535):
+            for n, k in ((2, 256), (64, 11008), (130, 512), (1026, 1024), (4096, 4096), (11008, 4096), (22016, 8192)):
+                t, s = plan(m, n, k, sms)
+                assert t % 16 == 0 and 16 <= t <= 224 and s in (1, 2, 4, 8) and (s == 1 or k // 128 >= 2 * s), (m, n, k, sms, t, s)
+    # without SMs to spare there is nothing to gain from sharing a tile
+    assert plan(200, 4096, 4096, 12)[1] == 1 and plan(200, 4096, 4096, 36)[1] == 1
+    for m, k, n, splits in ((17, 256, 128, 1), (40, 1024, 1026, 2), (225, 1280, 96, 4), (300, 2048, 200, 4), (9, 11008, 64, 8), (460, 256, 9000, 1)):
+        assert plan(m, n, k)[1] == splits, (m, k, n)
+    with pytest.raises(lcu.LcuError):
+        plan(2, 64, 128)
+
+
 def test_balanced_gemm_schedule_covers_every_k_step_once():
     """The prompt GEMM that deals the last wave's K steps evenly over the SM pairs: its work list, walked on the host for
     every pair of a launch.  Every K step of every tile must be run by exactly one pair; a pair may start inside a tile
