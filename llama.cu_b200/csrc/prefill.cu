@@ -37,10 +37,13 @@ int matmul_rows(__half* out, const __half* lhs, const dev_matrix& w, int m, floa
   }
   const int pass_rows = gemv_max_rows(K);  // 8, fewer where the activation rows are long
   LCU_REQUIRE(pass_rows >= 1, "matmul_nt: a row of K=%d does not fit in shared memory", K);
-  // u8 without scratch.  A single GEMV pass is as fast while K is short (2 rows of 1024 x 1024: 5.8 us against 6.8; 2 of 4096 x 4096:
-  // 10.5 against 10.6; 4 of 11008 x 512: 23.6 against 11.5); every further pass reads the matrix again (400 of 4096 x 4096: 994 against 21).
-  if (w.bs > 0 && pt.u8_deq_min_rows > 0 && m >= pt.u8_deq_min_rows && (m > pass_rows || K > 2048) &&
-      gemm_u8_supported(m, N, K, w.bs, lhs, w.w, w.sc))
+  // u8 without scratch: expanded inside the product, except where a single GEMV pass is as fast (us, GEMV / product).  That is while K
+  // is short (2 rows of 1024 x 1024: 5.8 / 6.8); for two rows of a few thousand (4096 x 1024: 8.4 / 9.3, 4096 x 4096: 10.5 / 10.5, but
+  // 4096 x 8192 16.5 / 14.3 and 5120 x 1024 10.5 / 8.9); and where the product's tiles need a second wave while the rows leave the GEMV
+  // all its CTAs (4 of 4096 x 22016: 33.1 / 38.0, 2 of 8192 x 22016: 57.8 / 62.7, but 6 of 4096 x 22016 51.5 / 38.0).  Every further pass
+  // reads the matrix again (400 of 4096 x 4096: 994 / 21).
+  const bool one_pass = m <= pass_rows && (K <= 2048 || (m == 2 && K <= 4096 && N <= 4096) || (m * K <= 16384 && N > 128 * gemv_sm_count()));
+  if (w.bs > 0 && pt.u8_deq_min_rows > 0 && m >= pt.u8_deq_min_rows && !one_pass && gemm_u8_supported(m, N, K, w.bs, lhs, w.w, w.sc))
     return launch_gemm_u8(out, lhs, (const uint8_t*)w.w, w.sc, w.bs, m, N, K, beta, err, stream);
   for (int t = 0; t < m; t += pass_rows) {
     gemv_params p{};

@@ -140,7 +140,7 @@ def test_matmul_small_shapes(lcu, m, k, n, bs, beta):
 
 
 @pytest.mark.parametrize("bs", [32, 64, 128])
-@pytest.mark.parametrize("m,k,n,beta", [(2, 4096, 2, 0.0), (17, 256, 128, 1.0), (9, 512, 130, 0.0), (224, 512, 384, 0.0), (225, 1280, 96, 1.0),
+@pytest.mark.parametrize("m,k,n,beta", [(3, 4096, 2, 0.0), (17, 256, 128, 1.0), (9, 512, 130, 0.0), (224, 512, 384, 0.0), (225, 1280, 96, 1.0),
                                         # K split over 2, 4 and 8 CTAs, ragged last tile
                                         (40, 1024, 1026, 1.0), (300, 2048, 200, 0.0), (9, 11008, 64, 1.0),
                                         # more tiles than SMs, several row tiles
