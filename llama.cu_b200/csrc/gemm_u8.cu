@@ -109,8 +109,7 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
   const uint32_t tmem = *tmem_slot;
   pdl_launch_dependents();
   pdl_wait();
-  // Nobody clears the error word between stand-alone calls: what an earlier launch left there does not concern this one.
-  const int seen = *(volatile int*)err;
+  constexpr bool HEED = false;  // nobody clears the error word between stand-alone calls: what stands there may be an earlier launch's
 
   // rows of the tile this thread converts and stores; tiles may hang over N
   const int quad = warp & 3, group = warp >> 2, row = quad * 32 + lane, n = n0 + row;
@@ -140,8 +139,8 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
         if (blk >= n_blk) break;
         const uint32_t sw = ahead[u];
         ahead[u] = scales_of(blk + U8_AHEAD * U8_GROUPS);
-        ok = mbar_wait(smem_u32(&full[s]), phase, err, DEV_ERR_FULL_WAIT, seen);
-        if (ok && blk >= U8_BUFS) ok = mbar_wait(smem_u32(&freed[buf]), (blk / U8_BUFS - 1) & 1, err, DEV_ERR_EMPTY_WAIT, seen);
+        ok = mbar_wait(smem_u32(&full[s]), phase, err, DEV_ERR_FULL_WAIT, HEED);
+        if (ok && blk >= U8_BUFS) ok = mbar_wait(smem_u32(&freed[buf]), (blk / U8_BUFS - 1) & 1, err, DEV_ERR_EMPTY_WAIT, HEED);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
@@ -170,7 +169,7 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
         }
       }
     }
-    ok = mbar_wait(smem_u32(done), 0, err, DEV_ERR_TMEM_WAIT, seen) && ok;
+    ok = mbar_wait(smem_u32(done), 0, err, DEV_ERR_TMEM_WAIT, HEED) && ok;
     tc_fence_after();
     go = __all_sync(0xffffffffu, ok && *failed == 0.f);
     if (!go && lane == 0) *failed = 1.f;
@@ -178,7 +177,7 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
     if (tc_elect()) {  // ---- TMA producer
       tc_ring r;
       for (int i = 0; i < n_st; ++i, r.step(nstages)) {
-        if (!mbar_wait(smem_u32(&empty[r.slot]), r.phase ^ 1u, err, DEV_ERR_EMPTY_WAIT, seen)) break;
+        if (!mbar_wait(smem_u32(&empty[r.slot]), r.phase ^ 1u, err, DEV_ERR_EMPTY_WAIT, HEED)) break;
         const uint32_t bar = smem_u32(&full[r.slot]), dst = base + (uint32_t)r.slot * STAGE;
         mbar_arrive_expect_tx(bar, STAGE);
         tma_load_2d(dst, &map_q, (st0 + i) * (U8_STAGE_K / 2), n0, bar);
@@ -190,12 +189,12 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
     bool ok = true;
     tc_ring r, e;
     for (int i = 0; i < n_st && ok; ++i, r.step(nstages)) {
-      ok = mbar_wait_warp(smem_u32(&full[r.slot]), r.phase, err, DEV_ERR_FULL_WAIT, seen);
+      ok = mbar_wait_warp(smem_u32(&full[r.slot]), r.phase, err, DEV_ERR_FULL_WAIT, HEED);
       if (!ok) break;
       const uint64_t x = smem_desc_sw128(base + (uint32_t)r.slot * STAGE + U8_Q_BYTES);
 #pragma unroll
       for (int g = 0; g < 2; ++g, e.step(U8_BUFS)) {
-        ok = ok && mbar_wait_warp(smem_u32(&conv[e.slot]), e.phase, err, DEV_ERR_FULL_WAIT, seen);
+        ok = ok && mbar_wait_warp(smem_u32(&conv[e.slot]), e.phase, err, DEV_ERR_FULL_WAIT, HEED);
         if (!ok) break;
         tc_fence_after();
         if (tc_elect()) {
@@ -246,7 +245,7 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
       }
     __syncwarp();
     cluster_sync();
-    for (int q = 0; q < splits && go; ++q) go = ld_dsmem_f32(mapa(smem_u32((const void*)failed), (uint32_t)q)) == 0.f;
+    go = __all_sync(0xffffffffu, go && (lane >= splits || ld_dsmem_f32(mapa(smem_u32((const void*)failed), (uint32_t)lane)) == 0.f));
     if (go)
       for (int c = 16 * (rank + splits * group); c < t; c += 16 * U8_GROUPS * splits) {
         float sum[16];

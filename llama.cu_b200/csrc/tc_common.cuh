@@ -47,7 +47,7 @@ __device__ __forceinline__ bool tc_elect() {  // true for one lane (always the s
   return one != 0;
 }
 // mbar_wait by a whole warp with one outcome for all lanes
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int* err, int code, int seen = 0) {
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int* err, int code, bool heed = true) {
   constexpr uint32_t ALL = 0xffffffffu;
   if (__all_sync(ALL, mbar_try_wait(bar, parity))) return true;
   const long long t0 = clock64();
@@ -56,7 +56,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, in
     if (__all_sync(ALL, mbar_try_wait(bar, parity))) return true;
     const long long dt = clock64() - t0;
     if (__any_sync(ALL, dt > next_check)) {
-      if (__any_sync(ALL, *(volatile int*)err != seen)) return false;
+      if (heed && __any_sync(ALL, *(volatile int*)err != 0)) return false;
       if (__any_sync(ALL, dt > 2000000000ll)) {
         atomicCAS(err, 0, code);
         return false;
