@@ -286,6 +286,10 @@ int lcu_plan_long_prompt_gemm(int m, int n, int k, int sms, int* kernel_out);
 /* Products with 8-bit weights that are expanded inside (lcu_matmul_nt_fp16u8 from 2 rows): activation rows per tile (a multiple of 16
  * up to 224) and the CTAs that share a tile's K (1, 2, 4 or 8).  n even, k a multiple of 256. */
 int lcu_plan_u8_gemm(int m, int n, int k, int sms, int* tile_rows_out, int* splits_out);
+/* How the recurrences of a block model walk a pass of `rows` rows (heads of dim x vdim; wkv != 0: decays per channel) on a GPU of `sms`
+ * SMs: rows per chunk (0: one walk over all rows), CTAs of the walk, and for chunks the CTAs an SM holds and the shared memory of each. */
+int lcu_plan_recurrence(int heads, int dim, int vdim, int wkv, int rows, int sms, int* chunk_rows_out, int* ctas_out, int* ctas_per_sm_out,
+                        int* smem_per_cta_out);
 /* Host walk of the balanced kernel's work list (no device needed) for n_tiles output tiles of k_steps 64-wide K steps on sm_pairs
  * pairs of SMs: 0 when every K step of every tile is run by exactly one pair, a pair hands partial sums over at most once,
  * and each shared tile's owner finds exactly the pairs that ran the rest of it, in order; a positive code names the rule

@@ -6,6 +6,7 @@
 
 #include "block_ops.cuh"
 #include "elem.cuh"
+#include "gemv.cuh"
 
 namespace lcu {
 namespace {
@@ -230,8 +231,8 @@ __global__ void __launch_bounds__(128) window_pool_kernel(const attn_rows<T> p, 
 // are walked side by side: one launch (SCAN_STATE) forms what every chunk adds to the state and the product of its decays, the
 // next (SCAN_CHUNK) starts every chunk from the states before it - S <- P S + local, chunk after chunk, in the CTA's registers -
 // and forms the results.  Everything stays products and sums in binary32 (no quotients of decays: a product that underflows is a
-// state that has faded).  A single walk of 2000 rows takes 155 to 160 us; a prompt of 2000 tokens at width 1024 (four layers of 16
-// heads of 64 x 64, four of 4 heads of 128 x 128) went from 3.32 to 2.20 ms.
+// state that has faded).  2000 rows, one walk -> the two launches, in us: retention, 4 heads of 128 x 128 154 -> 15.6 + 31.5, 16 heads
+// 180 -> 47 + 112 (four chunks); wkv, 16 heads of 64 x 64 159 -> 18.6 + 34.0, 64 heads 205 -> 55 + 117.
 constexpr int SC_THREADS = 128;
 constexpr int SC_ROWS = 16;
 constexpr int SC_MAX_STAGES = 4;
@@ -253,12 +254,23 @@ scan_shape scan_shape_of(int dim, int vdim, bool wkv, int mode) {
   s.stride = (wkv ? 3 : 2) * s.dimp + 4;
   return s;
 }
-// rows per chunk (a multiple of SC_ROWS), 0 = one walk over all rows.  Four CTAs per SM keep its arithmetic busy; both chunk
-// launches walk a chunk, so fewer than three chunks, or chunks shorter than the launch costs, gain nothing.
-constexpr int SC_MAX_CHUNKS = 32, SC_CTAS = 4 * 148;
-int scan_chunk_rows(const scan_shape& z, int heads, int m) {
-  const int chunks = std::min(std::min(SC_MAX_CHUNKS, m / 64), SC_CTAS / std::max(1, heads * z.blocks));
-  return chunks < 3 ? 0 : (m + chunks * SC_ROWS - 1) / (chunks * SC_ROWS) * SC_ROWS;
+size_t scan_stage_bytes(const scan_shape& z) { return (size_t)SC_ROWS * (z.stride + z.cols) * sizeof(float); }
+// Stages of a chunk's ring and CTAs of an SM: three stages where four CTAs fit an SM with them (heads up to 64, retention up to 128),
+// else two (four CTAs of wkv heads of 128 or retention heads of 192, two or three up to 256, one above).
+constexpr size_t SC_SM_SMEM = 228 * 1024, SC_CTA_SMEM = 1024 + 64;  // an SM's shared memory; what a CTA takes of it beside its stages
+int scan_chunk_stages(const scan_shape& z) { return 4 * (3 * scan_stage_bytes(z) + SC_CTA_SMEM) <= SC_SM_SMEM ? 3 : 2; }
+int scan_ctas_per_sm(const scan_shape& z) { return (int)std::min<size_t>(4, SC_SM_SMEM / (scan_chunk_stages(z) * scan_stage_bytes(z) + SC_CTA_SMEM)); }
+// rows per chunk (a multiple of SC_ROWS), 0 = one walk over all rows.  The CTAs of all chunks are resident at once, four per SM where
+// they fit: that keeps its arithmetic busy, and a second wave would be a second walk.  Both chunk launches walk a chunk, so fewer than
+// three chunks, or chunks shorter than the launch costs, gain nothing: prompts of four-layer models, one walk / chunks, in us - wkv heads
+// of 128 at width 1024 with 192, 240, 320 rows 567 / 598, 595 / 621, 652 / 629; of 64 595 / 597, 626 / 627, 667 / 622.
+constexpr int SC_MAX_CHUNKS = 32, SC_MIN_ROWS = 256;
+int scan_most_chunks(const scan_shape& z, int heads, int m, int sms) {
+  return std::min(std::min(SC_MAX_CHUNKS, m / 64), scan_ctas_per_sm(z) * sms / std::max(1, heads * z.blocks));
+}
+int scan_chunk_rows(const scan_shape& z, int heads, int m, int sms) {
+  const int chunks = scan_most_chunks(z, heads, m, sms);
+  return m < SC_MIN_ROWS || chunks < 3 ? 0 : (m + chunks * SC_ROWS - 1) / (chunks * SC_ROWS) * SC_ROWS;
 }
 
 constexpr int SP_ROWS = 4;  // rows per warp
@@ -618,9 +630,8 @@ __global__ void __launch_bounds__(SC_THREADS) scan_kernel(const scan_args p, con
 
 template <int KC, int G, bool WKV, int MODE>
 int launch_scan_shape(const scan_args& a, const scan_shape& z, int heads, int m, int pos0, int chunk_rows, cudaStream_t stream) {
-  const size_t stage = (size_t)SC_ROWS * (z.stride + z.cols) * sizeof(float);
-  // (chunks: three stages leave room for four CTAs per SM)
-  const int n_stages = (int)std::min<size_t>(MODE == SCAN_WHOLE ? SC_MAX_STAGES : SC_MAX_STAGES - 1, (200 * 1024) / stage);
+  const size_t stage = scan_stage_bytes(z);
+  const int n_stages = (int)std::min<size_t>(MODE == SCAN_WHOLE ? SC_MAX_STAGES : scan_chunk_stages(z), (200 * 1024) / stage);
   static bool attr_done[16] = {};
   int dev = 0;
   LCU_CUDA(cudaGetDevice(&dev));
@@ -921,7 +932,7 @@ int launch_window_attention(const attn_rows<T>& p, int m, int pos0, cudaStream_t
 template <typename T>
 int launch_scan(const scan_rows<T>& p, bool wkv, int m, int pos0, cudaStream_t stream) {
   scan_shape z = scan_shape_of(p.dim, p.vdim, wkv, SCAN_CHUNK);
-  const int chunk_rows = scan_chunk_rows(z, p.heads, m);
+  const int chunk_rows = scan_chunk_rows(z, p.heads, m, gemv_sm_count());
   if (!chunk_rows) z = scan_shape_of(p.dim, p.vdim, wkv, SCAN_WHOLE);
   const dim3 grid((m + SP_ROWS - 1) / SP_ROWS, (p.heads + 7) / 8);
   if (scan_prepare4_suits(p, z, wkv)) {
@@ -940,9 +951,16 @@ void scan_scratch(int heads, int dim, int vdim, bool wkv, size_t rows, size_t* p
   *packed_floats = heads * rows * z.stride;
   *value_floats = heads * rows * std::max(whole.blocks * whole.cols, z.blocks * z.cols);
   // (passes of fewer rows have no more chunks)
-  const int chunk_rows = scan_chunk_rows(z, heads, (int)rows);
-  const size_t chunks = chunk_rows ? std::min<size_t>(std::min<size_t>(SC_MAX_CHUNKS, rows / 64), SC_CTAS / (heads * z.blocks)) : 0;
+  const int sms = gemv_sm_count();
+  const size_t chunks = scan_chunk_rows(z, heads, (int)rows, sms) ? scan_most_chunks(z, heads, (int)rows, sms) : 0;
   *part_floats = chunks * heads * z.blocks * SC_THREADS * z.kc * (scan_nc(z.kc, SCAN_CHUNK) + (wkv ? 1 : 0));
+}
+void scan_plan(int heads, int dim, int vdim, bool wkv, int m, int sms, int* chunk_rows, int* ctas, int* ctas_per_sm, int* smem_per_cta) {
+  const scan_shape z = scan_shape_of(dim, vdim, wkv, SCAN_CHUNK);
+  *chunk_rows = scan_chunk_rows(z, heads, m, sms);
+  *ctas = *chunk_rows ? heads * z.blocks * ((m + *chunk_rows - 1) / *chunk_rows) : heads * scan_shape_of(dim, vdim, wkv, SCAN_WHOLE).blocks;
+  *ctas_per_sm = scan_ctas_per_sm(z);
+  *smem_per_cta = (int)(scan_chunk_stages(z) * scan_stage_bytes(z));
 }
 void scan_decay_layout(int dim, int vdim, int m, size_t* head_stride, size_t* row_stride, size_t* offset) {
   const scan_shape z = scan_shape_of(dim, vdim, true, SCAN_WHOLE);  // (the same for chunks)

@@ -183,6 +183,9 @@ struct scan_rows {
   int* err;
 };
 void scan_scratch(int heads, int dim, int vdim, bool wkv, size_t rows, size_t* packed_floats, size_t* value_floats, size_t* part_floats);
+// how a pass of m rows is walked on a GPU of `sms` SMs: rows per chunk (0: one walk), CTAs of the walk, and for chunks the CTAs an SM
+// holds and their shared memory.  Pure host arithmetic.
+void scan_plan(int heads, int dim, int vdim, bool wkv, int m, int sms, int* chunk_rows, int* ctas, int* ctas_per_sm, int* smem_per_cta);
 // where the decay of (head, row, channel) of an m-row pass goes: packed[offset + head * head_stride + row * row_stride + channel]
 void scan_decay_layout(int dim, int vdim, int m, size_t* head_stride, size_t* row_stride, size_t* offset);
 template <typename T>

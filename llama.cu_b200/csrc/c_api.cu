@@ -640,6 +640,12 @@ int lcu_plan_u8_gemm(int m, int n, int k, int sms, int* tile_rows_out, int* spli
   gemm_u8_plan(m, n, k, sms, tile_rows_out, splits_out);
   return LCU_OK;
 }
+int lcu_plan_recurrence(int heads, int dim, int vdim, int wkv, int rows, int sms, int* chunk_rows_out, int* ctas_out, int* ctas_per_sm_out, int* smem_per_cta_out) {
+  LCU_REQUIRE(heads >= 1 && dim >= 1 && dim <= 512 && vdim >= 1 && rows >= 1 && sms >= 1 && chunk_rows_out && ctas_out && ctas_per_sm_out && smem_per_cta_out,
+              "plan_recurrence: bad arguments");
+  scan_plan(heads, dim, vdim, wkv != 0, rows, sms, chunk_rows_out, ctas_out, ctas_per_sm_out, smem_per_cta_out);
+  return LCU_OK;
+}
 int lcu_selftest_silu_arithmetic(uint64_t* checked_out, uint64_t* differences_out) {
   NEED_DEVICE();
   unsigned long long a = 0, b = 0;

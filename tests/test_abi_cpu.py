@@ -143,6 +143,31 @@ def test_8_bit_product_plan_on_any_number_of_sms():
         plan(2, 64, 128)
 
 
+def test_recurrence_chunks_are_resident_at_once():
+    """Host arithmetic behind the recurrences of block models: the CTAs of all chunks fit the SMs side by side (a second wave would be a
+    second walk), on any number of SMs; chunks cover the rows in whole steps of 16."""
+    lcu = load_package()
+
+    def plan(heads, dim, vdim, wkv, rows, sms=148):
+        out = [C.c_int(-1) for _ in range(4)]
+        lcu.check(lcu.lib.lcu_plan_recurrence(heads, dim, vdim, wkv, rows, sms, *map(C.byref, out)))
+        return [o.value for o in out]
+
+    for sms in (12, 18, 36, 74, 148):
+        for wkv in (0, 1):
+            for heads in (1, 2, 4, 8, 16, 64):
+                for dim in (4, 32, 64, 100, 128, 160, 256, 300, 512):
+                    for rows in (16, 192, 255, 256, 640, 2000, 2048):
+                        chunk, ctas, per_sm, smem = plan(heads, dim, dim, wkv, rows, sms)
+                        assert 1 <= per_sm <= 4 and per_sm * (smem + 1024) <= 228 * 1024 and smem <= 200 * 1024
+                        if chunk:
+                            assert rows >= 256 and chunk % 16 == 0 and 2 * chunk < rows and ctas <= per_sm * sms, (sms, wkv, heads, dim, rows)
+    assert plan(16, 64, 64, 1, 2000)[:3] == [112, 576, 4]
+    assert plan(4, 128, 128, 0, 2000)[:3] == [112, 576, 4]
+    assert plan(8, 128, 128, 1, 2000)[:3] == [224, 576, 4]  # (with two stages: three leave room for two CTAs)
+    assert plan(4, 256, 256, 1, 2000)[0] == 0
+
+
 def test_balanced_gemm_schedule_covers_every_k_step_once():
     """The prompt GEMM that deals the last wave's K steps evenly over the SM pairs: its work list, walked on the host for
     every pair of a launch.  Every K step of every tile must be run by exactly one pair; a pair may start inside a tile

@@ -67,14 +67,14 @@ def test_portions(run, cuts, dtype):
 @both
 @pytest.mark.parametrize("rdim,rvdim,heads,dim", [(128, 100, 3, 64), (200, 36, 5, 16), (16, 256, 1, 128), (300, 8, 2, 4)])
 def test_scans_cut_into_chunks(run, rdim, rvdim, heads, dim, dtype):
-    """Passes long enough for recurrences to walk chunks of rows side by side (from 192 rows, last chunks of any length), from the
+    """Passes long enough for recurrences to walk chunks of rows side by side (from 256 rows, last chunks of any length), from the
     beginning and from a state, against the plain walk; the state behind them against single steps and a short pass."""
     cfg, W = B.case(seed=12, layers=("parallel", "wkv"), mlp_none=(0, 1), mixer=dict(left_scale=0.0, rheads=2, rdim=rdim, rvdim=rvdim, rot_dims=rdim),
                     wkv=dict(heads=heads, dim=dim))
     t = B.tokens(cfg, 640, 5)
     want = P.forward(t, cfg, W)
     r = run(cfg, W, dtype, context_len=704)
-    for cuts in (WHOLE, [192, 1, 201, 7, 239], [1, 447, 192]):
+    for cuts in (WHOLE, [192, 1, 201, 7, 239], [1, 447, 192], [256, 1, 271, 112]):
         check(r.feed(t, cuts), want, dtype)
 
 
