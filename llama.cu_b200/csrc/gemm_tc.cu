@@ -5,17 +5,18 @@
 // in tensor memory, one rounding to fp16 on the way out (with the residual add when beta = 1).
 //
 // One CTA computes one 128 x BN output tile (BN = the widest of 128, 64, 32 weight rows that divides N).  Warp roles:
-//   warp 0  - one lane issues the TMA loads: per 64-wide K step a 128 x 64 activation box and a
+//   warp 0  - an elected lane issues the TMA loads: per 64-wide K step a 128 x 64 activation box and a
 //             BN x 64 weight box (cp.async.bulk.tensor.2d, 128-byte swizzle, zero fill past the last row)
 //             into a ring of shared-memory stages, completion on `full` mbarriers;
-//   warp 1  - allocates BN tensor-memory columns; one lane issues tcgen05.mma (M = 128, N = BN, K = 16,
-//             four per stage) from shared-memory descriptors and releases each stage with
+//   warp 1  - allocates BN tensor-memory columns; an elected lane issues tcgen05.mma (M = 128, N = BN, K = 16,
+//             four per stage; loops and waits are common to the warp) from shared-memory descriptors and releases each stage with
 //             tcgen05.commit on its `empty` mbarrier; a last commit signals the epilogue;
 //   warps 2-5 - epilogue: each warp reads its 32-lane quadrant of the accumulator with tcgen05.ld
 //             (32 columns at a time), adds beta * out, rounds to half and stores 64-byte row pieces.
 // Two kernels share these roles: gemm_tc_kernel (one SM per tile, optionally a cluster of 2 or 4 CTAs that
-// splits K and reduces through distributed shared memory - for few rows) and gemm_tc_pair_kernel (two SMs per
-// 256-row tile with tcgen05.mma.cta_group::2, persistent, two accumulators in tensor memory - for many rows).
+// splits K and reduces through distributed shared memory) and gemm_tc_pair_kernel (two SMs per
+// 256-row tile with tcgen05.mma.cta_group::2, persistent, two accumulators in tensor memory).  Up to 128 rows take the
+// first; above, gemm_tc_plan_long picks between them and the balanced kernel (gemm_tc_sk.cu).
 // No TMA multicast anywhere.  Every mbarrier wait is bounded: on expiry the kernel records a code in the error
 // word, skips ahead and still frees its tensor memory.
 #include <cuda.h>
