@@ -21,7 +21,7 @@
 // multi-row kernel (gemv.cu) the producer does not depend on the activations, so under programmatic
 // dependent launch the rings of kernel n+1 fill while kernel n drains; every wait is bounded; int8
 // weights are de-quantised in registers bit-identically to half((q - 127.5f) * scale)
-// (reference llama_cu.cu:287-289); the RMSNorm prologue keeps the reference's summation order.
+// (reference llama_cu.cu:287-289); the RMSNorm prologue rounds where the reference does (llama_cu.cu:72-106) and sums in an order of its own.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -51,7 +51,29 @@ constexpr int MAX_SW = 4;                   // ring depth per warp
 constexpr int NACC = 4;                     // independent accumulator sets (no chain on one result)
 constexpr int EMPTY_BASE = NW_MAX * MAX_SW;  // barriers: full[w * MAX_SW + s], empty[EMPTY_BASE + w * MAX_SW + s]
 constexpr int BAR_BYTES = 2 * EMPTY_BASE * 8;
-constexpr int SMEM_FIXED = BAR_BYTES + 64;  // barriers; scratch of the RMSNorm reduction
+constexpr int SMEM_FIXED = BAR_BYTES + 64;  // barriers; the activation row's barrier and the CTA's count (tensor-parallel)
+
+// u8 kernels read 32 activation bytes per 16 weight bytes; with the row stored flat, the two segments of a
+// quarter warp would meet on the same banks.  The activations of every segment are therefore shifted by 16 more
+// bytes than those of the one before (vector i of eight halves lives at byte 16 * (i + i / (SEG / 8))).
+template <int WT>
+__host__ __device__ __forceinline__ int row_offset(int vec_index) {
+  return is16<WT> ? vec_index * 16 : (vec_index + (vec_index >> (geom<WT>::SEG_SHIFT - 3))) * 16;
+}
+// the activation row in shared memory: the row itself, sums over aligned groups of 64 (factored u8), sums of squares over
+// aligned blocks of 256 (RMSNorm)
+struct row_layout {
+  int sums, squares, total;  // byte offsets
+};
+template <int WT>
+__host__ __device__ __forceinline__ row_layout row_layout_of(int K, bool norm) {
+  row_layout r;
+  const int xbytes = is16<WT> ? K * 2 : K * 2 + (K >> geom<WT>::SEG_SHIFT) * 16 + 16;
+  r.sums = (xbytes + 127) & ~127;
+  r.squares = r.sums + (WT == 2 ? (K / 64 * 4 + 127) & ~127 : 0);
+  r.total = r.squares + (norm ? (K / 256 * 4 + 127) & ~127 : 0);
+  return r;
+}
 
 template <int EPI>
 __device__ __forceinline__ void map_row(const gemv_params& p, int vrow, int& mat, int& row) {
@@ -193,6 +215,89 @@ __device__ __forceinline__ void step_pair_factored(float (&accs)[NACC][4], const
   acc[3] += sh * (ta[3] + tb[3]);
 }
 
+// ---- the activation row: global -> shared memory, normalised, with the group sums of the factored u8 kernels.
+// This is what a launch does between its predecessor's end and its first product, with nothing to hide it behind, and most of
+// its instructions run once: their fetch counts as much as their latency, so loops that need no register array stay rolled.
+// Squares are added per vector, by shuffles over aligned blocks of 256 and over the blocks (an order that does not depend on the
+// number of threads); group sums come from the same pass as the normalised values.  Decode step, 8 layers, with the epilogue by
+// batches below, in us: 1024 wide fp16 219 -> 196, 2048 wide 274 -> 253, 4096 wide 630 -> 620, with u8 weights 480 -> 468.
+constexpr int ROW_VEC = 4;  // vectors of eight halves a thread requests at once
+
+__device__ __forceinline__ float square_sum8(const uint4& q) {
+  const __half2* h = reinterpret_cast<const __half2*>(&q);
+  float s = 0.f;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 f = __half22float2(h[e]);
+    s = fmaf(f.x, f.x, s);
+    s = fmaf(f.y, f.y, s);
+  }
+  return s;
+}
+// x_i <- norm_w_i *h half(x_i * rinv)
+__device__ __forceinline__ uint4 norm8(uint4 xq, const uint4& wq, float rinv) {
+  __half2* x2 = reinterpret_cast<__half2*>(&xq);
+  const __half2* w2 = reinterpret_cast<const __half2*>(&wq);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 f = __half22float2(x2[e]);
+    x2[e] = __hmul2(w2[e], __floats2half2_rn(f.x * rinv, f.y * rinv));
+  }
+  return xq;
+}
+// vector i of the row is final: the sum of its group of 64 (eight neighbouring lanes)
+__device__ __forceinline__ void row_sums8(const uint4& q, int i, int lane, float* xs64) {
+  const __half2* h = reinterpret_cast<const __half2*>(&q);
+  float s = 0.f;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 f = __half22float2(h[e]);
+    s += f.x + f.y;
+  }
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  s += __shfl_xor_sync(0xffffffffu, s, 4);
+  if ((lane & 7) == 0) xs64[i >> 3] = s;
+}
+// The row is in shared memory (each thread reads back the vectors it wrote itself, or all of them are visible): normalise
+// it and form its group sums.  K is a multiple of 256, so a warp's 32 vectors are all inside the row or all outside.
+template <int WT>
+__device__ __forceinline__ void row_finish(const gemv_params& p, bool norm, uint8_t* xs, float* xs64, float* squares, int tid, int threads,
+                                           const uint4 (&nw)[ROW_VEC]) {
+  const int vec = p.K >> 3, lane = tid & 31;
+  float rinv = 1.f;
+  if (norm) {
+#pragma unroll 2
+    for (int i = tid; i < vec; i += threads) {
+      const float s = warp_sum(square_sum8(*reinterpret_cast<const uint4*>(xs + row_offset<WT>(i))));
+      if (lane == 0) squares[i >> 5] = s;
+    }
+    bar_sync(1, threads);
+    float t = 0.f;
+    for (int b = lane; b < vec >> 5; b += 32) t += squares[b];
+    rinv = rsqrtf(warp_sum(t) / p.K + p.eps);
+  }
+  auto finish = [&](int i, const uint4& w) {
+    uint4 q = *reinterpret_cast<const uint4*>(xs + row_offset<WT>(i));
+    if (norm) {
+      q = norm8(q, w, rinv);
+      *reinterpret_cast<uint4*>(xs + row_offset<WT>(i)) = q;
+    }
+    if (WT == 2) row_sums8(q, i, lane, xs64);
+  };
+  if (norm) {
+#pragma unroll
+    for (int j = 0; j < ROW_VEC; ++j)
+      if (tid + j * threads < vec) finish(tid + j * threads, nw[j]);
+#pragma unroll 1
+    for (int i = tid + ROW_VEC * threads; i < vec; i += threads) finish(i, *reinterpret_cast<const uint4*>(p.norm_w + i * 8));
+  } else if (WT == 2) {
+#pragma unroll 4
+    for (int i = tid; i < vec; i += threads) finish(i, nw[0]);
+  }
+  bar_sync(1, threads);
+}
+
 // Weight types (WT): 0 = fp16; 1 = u8, every weight rounded to half((q - 127.5) * scale) before the
 // product exactly as the reference's tensor-core kernel does (llama_cu.cu:287-289, 332-341); 2 = u8
 // with the scale factored out of each 64-weight group: sum_k x_k (q_k - 127.5) s = s * (sum_k x_k
@@ -204,7 +309,7 @@ template <int WT, int EPI, int NW>
 __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(const gemv_params p, const int sw, const int pf_bytes,
                                                                                         const __grid_constant__ gemv_batch bt) {
   constexpr int NCONS = NW * 32;
-  static_assert(NW >= 4 && NW <= NW_MAX, "the RMSNorm reduction uses the first four consumer warps");
+  static_assert(NW <= NW_MAX, "barriers");
   constexpr int ESZ = is16<WT> ? 2 : 1;
   constexpr int ROWB = geom<WT>::ROWB, SEG = geom<WT>::SEG, NSTEPS = geom<WT>::NSTEPS;
   constexpr int CHUNK_K = ROWB / ESZ;        // weights of one row per stage
@@ -212,19 +317,14 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
 
   extern __shared__ __align__(128) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);  // full: [w * MAX_SW + s], empty: [EMPTY_BASE + w * MAX_SW + s]
-  float* scratch = reinterpret_cast<float*>(smem + BAR_BYTES);  // [8] floats of the RMSNorm reduction, then the activation row's barrier
   const uint32_t xbar = smem_u32(smem + BAR_BYTES + 32);
   int* cta_done = reinterpret_cast<int*>(smem + BAR_BYTES + 40);  // consumer warps of this CTA that are through (tensor-parallel)
-  uint8_t* xs = smem + SMEM_FIXED;                     // activation row, K halves (u8 kernels: skewed, see xoff)
-  // u8 kernels read 32 activation bytes per 16 weight bytes; with the row stored flat, the two segments of a
-  // quarter warp would meet on the same banks.  The activations of every segment are therefore shifted by 16 more
-  // bytes than those of the one before (vector i of eight halves lives at byte 16 * (i + i / (SEG / 8))).
-  auto xoff = [](int vec_index) { return is16<WT> ? vec_index * 16 : (vec_index + (vec_index >> (geom<WT>::SEG_SHIFT - 3))) * 16; };
-  const int xbytes = is16<WT> ? p.K * 2 : p.K * 2 + (p.K >> geom<WT>::SEG_SHIFT) * 16 + 16;
-  float* xs64 = reinterpret_cast<float*>(xs + ((xbytes + 127) & ~127));  // sums of x over aligned groups of 64
-  // norm weights beyond what the consumers hold in registers (rows longer than NVEC * 8 * consumer threads) are staged here
-  uint8_t* nws = reinterpret_cast<uint8_t*>(xs64) + ((p.K / 64 * 4 + 127) & ~127);
-  uint8_t* stages = nws + (p.norm_w != nullptr && p.K > 4096 ? (((p.K - 4096) * 2 + 127) & ~127) : 0);  // [NW][sw][STAGE_BYTES]
+  uint8_t* xs = smem + SMEM_FIXED;                     // activation row, K halves (row_offset)
+  const row_layout rl = row_layout_of<WT>(p.K, WT != 3 && p.norm_w != nullptr);
+  float* xs64 = reinterpret_cast<float*>(xs + rl.sums);
+  float* squares = reinterpret_cast<float*>(xs + rl.squares);
+  uint8_t* stages = xs + rl.total;                     // [NW][sw][STAGE_BYTES]
+  auto xoff = [](int vec_index) { return row_offset<WT>(vec_index); };
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (WT != 3 || !bt.hold) pdl_launch_dependents();
@@ -245,21 +345,24 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
     return row;
   };
   const __half* x_row = WT == 3 && EPI == EPI_PLAIN ? reinterpret_cast<const __half*>(bt.x[bi]) : p.x;
-  const int pr0 = (int)(((long long)pairs * cta) / n_ctas);
-  const int npairs = (int)(((long long)pairs * (cta + 1)) / n_ctas) - pr0;
+  // first pair of a CTA: floor(pairs * cta / n_ctas), without the 64-bit division
+  const int per_cta = pairs / n_ctas, more = pairs - per_cta * n_ctas;
+  const int pr0 = per_cta * cta + more * cta / n_ctas;
+  const int npairs = per_cta * (cta + 1) + more * (cta + 1) / n_ctas - pr0;
   const int rowbytes = p.K * ESZ;
   const int nchunks = (rowbytes + ROWB - 1) / ROWB;
 
   // Scales of a row chunk are one contiguous run; when rows start 16-byte aligned they travel as one more bulk copy
   // per row on the same barrier, otherwise as 4-byte cp.async pieces issued by all lanes (32 more barrier arrivals).
   const bool sc_bulk = !is16<WT> && ((p.K / p.bs) & 7) == 0 && ((ROWB / p.bs) & 7) == 0;
-  if (tid == 0) {
-    for (int i = 0; i < NW * MAX_SW; ++i) {
-      mbar_init(smem_u32(&bars[i]), (is16<WT> || sc_bulk) ? 1 : 33);
-      mbar_init(smem_u32(&bars[EMPTY_BASE + i]), 1);
+  if (warp == NW && lane < NW * MAX_SW) {
+    static_assert(NW * MAX_SW <= 32, "a barrier of each kind per lane");
+    mbar_init(smem_u32(&bars[lane]), (is16<WT> || sc_bulk) ? 1 : 33);
+    mbar_init(smem_u32(&bars[EMPTY_BASE + lane]), 1);
+    if (lane == 0) {
+      mbar_init(xbar, 1);
+      *cta_done = 0;
     }
-    mbar_init(xbar, 1);
-    *cta_done = 0;
     fence_mbar_init();
   }
   __syncthreads();
@@ -358,46 +461,36 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
   }
 
   // -------------------------------------------------------------- consumers
-  // The norm weights do not depend on the previous kernel: their loads are in flight while this one waits for it.
-  constexpr int NVEC = 4;  // 16-byte vectors of norm weights per thread kept in registers (covers K <= 4096 with four warps)
+  // The norm weights do not depend on the previous kernel: they are brought close while this one waits for it.
   const int vec = p.K >> 3;
-  uint4 nw[NVEC];
-  if (WT != 3 && p.norm_w != nullptr && npairs > 0) {
+  const bool norm = WT != 3 && p.norm_w != nullptr;
+  uint4 nw[ROW_VEC];
+  if (norm) {
 #pragma unroll
-    for (int j = 0; j < NVEC; ++j) {
-      const int i = tid + j * NCONS;
-      nw[j] = i < vec ? *reinterpret_cast<const uint4*>(p.norm_w + i * 8) : make_uint4(0, 0, 0, 0);
-    }
-    // the rest of a long row's norm weights: asynchronous 16-byte copies into shared memory, no registers held
-    for (int i = tid + NVEC * NCONS; i < vec; i += NCONS) cp_async16(smem_u32(nws) + (uint32_t)(i - NVEC * NCONS) * 16, p.norm_w + i * 8);
-    cp_async_commit();
+    for (int j = 0; j < ROW_VEC; ++j)
+      if (tid + j * NCONS < vec) nw[j] = *reinterpret_cast<const uint4*>(p.norm_w + (tid + j * NCONS) * 8);
   }
   pdl_wait();
   if (WT == 3 && bt.hold) pdl_launch_dependents();
   const float gate_scale = WT == 3 && EPI == EPI_SILU && bt.n > 0 ? bt.gate_scale[bi] : 1.0f;
+  const int pos = EPI == EPI_ROPE_KV ? *p.pos : 0;
   if (npairs > 0) {
-    // Rows that fit the consumers' registers (NVEC vectors per thread: K <= 4096 with four warps) are loaded by the
-    // threads themselves and stay in registers for the normalisation.  Longer rows come in as bulk copies of one
-    // 512-element segment each: one trip to L2 whatever the row length, where per-thread loads paid a round trip per
-    // batch of vectors - several microseconds for rows of 8192 and more.  Both read past L1 (L2 is where another GPU's
-    // peer stores land).
-    const bool row_in_regs = vec <= NVEC * NCONS;
-    uint4 xv[NVEC];
-    if (row_in_regs) {
+    // Rows of up to ROW_VEC vectors per thread are loaded by the threads themselves.  Longer rows come in as bulk copies of one
+    // 512-element segment each: one trip to L2 whatever the row length, where per-thread loads would pay a round trip per
+    // batch of vectors.  Both read past L1 (L2 is where another GPU's peer stores land).
+    if (vec <= ROW_VEC * NCONS) {
       if (p.n_wait > 0) {
         // tensor-parallel: parts of the row come from other GPUs; wait for their flags first
         if (tid < p.n_wait) flag_wait_at_least(p.wait_flags + tid, *p.seq * TP_EXCHANGES_PER_STEP + p.wait_id, p.err);
         bar_sync(1, NCONS);
       }
+      uint4 xv[ROW_VEC];
 #pragma unroll
-      for (int j = 0; j < NVEC; ++j) {
-        const int i = tid + j * NCONS;
-        if (i < vec) {
-          xv[j] = __ldcg(reinterpret_cast<const uint4*>(x_row + i * 8));
-          *reinterpret_cast<uint4*>(xs + xoff(i)) = xv[j];
-        }
-      }
-      bar_sync(1, NCONS);
+      for (int j = 0; j < ROW_VEC; ++j)
+        if (tid + j * NCONS < vec) xv[j] = __ldcg(reinterpret_cast<const uint4*>(x_row + (tid + j * NCONS) * 8));
+#pragma unroll
+      for (int j = 0; j < ROW_VEC; ++j)
+        if (tid + j * NCONS < vec) *reinterpret_cast<uint4*>(xs + xoff(tid + j * NCONS)) = xv[j];
     } else {
       if (warp == 0) {
         if (p.n_wait > 0) {
@@ -412,146 +505,87 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
       }
       mbar_wait(xbar, 0, p.err, DEV_ERR_FULL_WAIT);
     }
-    if (WT != 3 && p.norm_w != nullptr) {
-      // RMSNorm with the reference's summation order (llama_cu.cu:72-106): 256 strided partial sums,
-      // xor trees inside 8 warps, xor tree over the 8 warp sums.  Each of the 128 threads here plays
-      // two of the reference's threads (t and t + 128), each warp two of its warps (w and w + 4).
-      auto xat = [&](int i) { return __half2float(*reinterpret_cast<const __half*>(xs + xoff(i >> 3) + (i & 7) * 2)); };
-      if (warp < 4) {  // (a fifth consumer warp only joins the barriers and the normalisation below)
-        float s0 = 0.f, s1 = 0.f;
-        for (int i = tid; i < p.K; i += 256) {
-          float v = xat(i);
-          s0 += v * v;
-        }
-        for (int i = tid + 128; i < p.K; i += 256) {
-          float v = xat(i);
-          s1 += v * v;
-        }
-        s0 = warp_sum(s0);
-        s1 = warp_sum(s1);
-        if (lane == 0) {
-          scratch[warp] = s0;
-          scratch[warp + 4] = s1;
-        }
-      }
-      bar_sync(1, NCONS);
-      float t = lane < 8 ? scratch[lane] : 0.f;  // every warp repeats the last tree: no second hand-over
-      for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      const float rinv = rsqrtf(__shfl_sync(0xffffffffu, t, 0) / p.K + p.eps);
-      // x_i <- norm_w_i *h half(x_i * rinv), eight elements at a time from the registers filled above
-      auto norm8 = [&](uint4 xq, uint4 wq) {
-        __half2* xq2 = reinterpret_cast<__half2*>(&xq);
-        const __half2* wq2 = reinterpret_cast<const __half2*>(&wq);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = __half22float2(xq2[e]);
-          xq2[e] = __hmul2(wq2[e], __floats2half2_rn(f.x * rinv, f.y * rinv));
-        }
-        return xq;
-      };
-#pragma unroll
-      for (int j = 0; j < NVEC; ++j) {
-        const int i = tid + j * NCONS;
-        if (i < vec) *reinterpret_cast<uint4*>(xs + xoff(i)) = norm8(row_in_regs ? xv[j] : *reinterpret_cast<const uint4*>(xs + xoff(i)), nw[j]);
-      }
-      cp_async_wait<0>();  // (each thread reads back the staged norm weights it copied itself)
-      for (int i = tid + NVEC * NCONS; i < vec; i += NCONS)
-        *reinterpret_cast<uint4*>(xs + xoff(i)) =
-            norm8(*reinterpret_cast<const uint4*>(xs + xoff(i)), *reinterpret_cast<const uint4*>(nws + (size_t)(i - NVEC * NCONS) * 16));
-      bar_sync(1, NCONS);
-    }
-    if (WT == 2) {  // sums of the (normalised) activations over aligned groups of 64: eight lanes per group, 16 bytes per lane
-#pragma unroll 3
-      for (int grp64 = warp * 4 + (lane >> 3); grp64 < p.K / 64; grp64 += NW * 4) {
-        const uint4 q = *reinterpret_cast<const uint4*>(xs + xoff(grp64 * 8 + (lane & 7)));
-        const __half2* h = reinterpret_cast<const __half2*>(&q);
-        float s = 0.f;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = __half22float2(h[e]);
-          s += f.x + f.y;
-        }
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        s += __shfl_xor_sync(0xffffffffu, s, 4);
-        if ((lane & 7) == 0) xs64[grp64] = s;
-      }
-      bar_sync(1, NCONS);
-    }
+    row_finish<WT>(p, norm, xs, xs64, squares, tid, NCONS, nw);
   }
 
   const int g = lane >> 2, c = lane & 3;
   const int flip = g & 1;
-  const bool diag = c == (g >> 1);
-  int pos = 0;
-  if (EPI == EPI_ROPE_KV) pos = *p.pos;
 
+  // A warp's row pairs are taken BATCH at a time: of each pair the diagonal lane of every quad holds its segment's sums, and the
+  // quad's lane c keeps those of the batch's pair c, so that one tree over the segments and one epilogue (lanes 0 .. 3, a
+  // pair each) serve four pairs.  A tree and an epilogue per pair were 900 of the 2900 cycles a pair of 4096 u8 weights took.
+  constexpr int BATCH = 4;
+  const int diag_lane = 4 * g + (g >> 1);
   int slot = 0;
   uint32_t par = 0;
-  for (int i = warp; i < npairs; i += NW) {
-    float accs[NACC][4];
-#pragma unroll
-    for (int a = 0; a < NACC; ++a) accs[a][0] = accs[a][1] = accs[a][2] = accs[a][3] = 0.f;
-    // u8 kernels (latency-bound): what the epilogue reads from global memory is requested now, one address for the
-    // whole warp, so that its latency passes under the row's products instead of after them.  The fp16 kernels run at
-    // the memory roofline, where the early loads measured no difference; they fetch in the epilogue.
-    constexpr bool EARLY = !is16<WT>;
-    const int vrow = 2 * (pr0 + i);
+  for (int i0 = warp; i0 < npairs; i0 += BATCH * NW) {
+    // what the epilogue reads from global memory is requested ahead of the products
+    const int i = i0 + c * NW, vrow = 2 * (pr0 + i);
+    const bool mine = g == 0 && i < npairs;
     __half2 prev = __half2half2(__ushort_as_half(0));
     float2 cs = make_float2(1.f, 0.f);
     int mat = 0, row = vrow, head = 0, j = 0;
-    auto fetch_epilogue_operands = [&]() {
+    if (mine) {
       if (EPI == EPI_PLAIN) {
-        if (p.beta != 0.f) prev = *reinterpret_cast<const __half2*>(p.out + vrow);
+        if (WT != 3 && p.beta != 0.f) prev = *reinterpret_cast<const __half2*>(p.out + vrow);
       } else if (EPI == EPI_ROPE_KV) {
         map_row<EPI_ROPE_KV>(p, vrow, mat, row);
         head = row / p.head_dim;
         j = row - head * p.head_dim;
         if (mat < 2) cs = p.rope[(size_t)pos * (p.head_dim >> 1) + (j >> 1)];
       }
-    };
-    if (EARLY) fetch_epilogue_operands();
-    for (int ci = 0; ci < nchunks; ++ci) {
-      mbar_wait(smem_u32(&bars[warp * MAX_SW + slot]), par, p.err, DEV_ERR_FULL_WAIT);
-      const int cbytes = min(ROWB, rowbytes - ci * ROWB);
-      const int vb = min(max(cbytes - g * SEG, 0), SEG);  // valid bytes of this lane's segment
-      const uint8_t* st = stages + (size_t)(warp * sw + slot) * STAGE_BYTES;
-      const uint8_t* seg0 = st + g * SEG;
-      const uint8_t* xseg = xs + xoff((ci * CHUNK_K + g * (SEG / ESZ)) >> 3);
-      // A full chunk (every chunk but possibly the last of a row) takes the branch-free path, so that the
-      // shared loads of all eight steps can be issued ahead of the tensor-core instructions.
-      if (WT == 2 && cbytes == ROWB && bs_shift >= 7) {
-#pragma unroll
-        for (int sp = 0; sp < NSTEPS / 2; ++sp) step_pair_factored<true>(accs, sp, flip, c, g, SEG, seg0, xseg, st, xs64, ci, bs_shift);
-      } else if (WT == 2 && bs_shift >= 7) {
-#pragma unroll
-        for (int sp = 0; sp < NSTEPS / 2; ++sp) step_pair_factored<false>(accs, sp, flip, c, g, vb, seg0, xseg, st, xs64, ci, bs_shift);
-      } else if (cbytes == ROWB) {
-#pragma unroll
-        for (int s = 0; s < NSTEPS; ++s) step<WT, true>(accs, s, flip, c, g, SEG, seg0, xseg, st, xs64, ci, bs_shift);
-      } else {
-#pragma unroll
-        for (int s = 0; s < NSTEPS; ++s) step<WT, false>(accs, s, flip, c, g, vb, seg0, xseg, st, xs64, ci, bs_shift);
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&bars[EMPTY_BASE + warp * MAX_SW + slot]));
-      if (++slot == sw) {
-        slot = 0;
-        par ^= 1;
-      }
     }
-
-    // the diagonal lanes hold segment g of row 0 (d0/d1) and of row 1 (d2/d3): fixed-order shuffle tree
     float v0 = 0.f, v1 = 0.f;
-    if (diag) {
+#pragma unroll 1
+    for (int k = 0; k < BATCH && i0 + k * NW < npairs; ++k) {
+      float accs[NACC][4];
+#pragma unroll
+      for (int a = 0; a < NACC; ++a) accs[a][0] = accs[a][1] = accs[a][2] = accs[a][3] = 0.f;
+      for (int ci = 0; ci < nchunks; ++ci) {
+        mbar_wait(smem_u32(&bars[warp * MAX_SW + slot]), par, p.err, DEV_ERR_FULL_WAIT);
+        const int cbytes = min(ROWB, rowbytes - ci * ROWB);
+        const int vb = min(max(cbytes - g * SEG, 0), SEG);  // valid bytes of this lane's segment
+        const uint8_t* st = stages + (size_t)(warp * sw + slot) * STAGE_BYTES;
+        const uint8_t* seg0 = st + g * SEG;
+        const uint8_t* xseg = xs + xoff((ci * CHUNK_K + g * (SEG / ESZ)) >> 3);
+        // A full chunk (every chunk but possibly the last of a row) takes the branch-free path, so that the
+        // shared loads of all eight steps can be issued ahead of the tensor-core instructions.
+        if (WT == 2 && cbytes == ROWB && bs_shift >= 7) {
+#pragma unroll
+          for (int sp = 0; sp < NSTEPS / 2; ++sp) step_pair_factored<true>(accs, sp, flip, c, g, SEG, seg0, xseg, st, xs64, ci, bs_shift);
+        } else if (WT == 2 && bs_shift >= 7) {
+#pragma unroll
+          for (int sp = 0; sp < NSTEPS / 2; ++sp) step_pair_factored<false>(accs, sp, flip, c, g, vb, seg0, xseg, st, xs64, ci, bs_shift);
+        } else if (cbytes == ROWB) {
+#pragma unroll
+          for (int s = 0; s < NSTEPS; ++s) step<WT, true>(accs, s, flip, c, g, SEG, seg0, xseg, st, xs64, ci, bs_shift);
+        } else {
+#pragma unroll
+          for (int s = 0; s < NSTEPS; ++s) step<WT, false>(accs, s, flip, c, g, vb, seg0, xseg, st, xs64, ci, bs_shift);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bars[EMPTY_BASE + warp * MAX_SW + slot]));
+        if (++slot == sw) {
+          slot = 0;
+          par ^= 1;
+        }
+      }
+      // segment g of row 0 is in d0/d1, of row 1 in d2/d3 of the quad's diagonal lane
       const float a0 = (accs[0][0] + accs[1][0]) + (accs[2][0] + accs[3][0]), a1 = (accs[0][1] + accs[1][1]) + (accs[2][1] + accs[3][1]);
       const float a2 = (accs[0][2] + accs[1][2]) + (accs[2][2] + accs[3][2]), a3 = (accs[0][3] + accs[1][3]) + (accs[2][3] + accs[3][3]);
-      v0 = (g & 1) ? a1 : a0;
-      v1 = (g & 1) ? a3 : a2;
+      const float s0 = __shfl_sync(0xffffffffu, (g & 1) ? a1 : a0, diag_lane);
+      const float s1 = __shfl_sync(0xffffffffu, (g & 1) ? a3 : a2, diag_lane);
+      if (c == k) {
+        v0 = s0;
+        v1 = s1;
+      }
     }
-    v0 = warp_sum(v0);
-    v1 = warp_sum(v1);
-    if (lane == 0) {
+#pragma unroll
+    for (int o = 16; o >= 4; o >>= 1) {  // fixed-order tree over the segments
+      v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+      v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+    }
+    if (mine) {
       const int pr = pr0 + i;
       if (WT == 3) {
         if (EPI == EPI_PLAIN) {
@@ -562,10 +596,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
           const float z = gate_scale * v0;
           o[pr] = __float2bfloat16(z / (1.0f + expf(-z)) * (gate_scale * v1));
         }
-        continue;
-      }
-      if (!EARLY) fetch_epilogue_operands();
-      if (EPI == EPI_PLAIN) {
+      } else if (EPI == EPI_PLAIN) {
         float a0 = v0, a1 = v1;
         __half* o = p.out + vrow;
         if (p.beta != 0.f) {
@@ -603,11 +634,12 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
     }
   }
   // tensor-parallel: the last consumer warp of the launch to get here publishes this GPU's slice (every result went into
-  // the other GPUs' rows as a peer store in the epilogue above, made by lane 0 of its warp).  The fences widen with the
+  // the other GPUs' rows as a peer store in the epilogue above, made by the warp's first lanes).  The fences widen with the
   // counting: a warp counts itself inside its CTA behind a CTA-scope fence (shared memory), the last warp of a CTA
   // counts the CTA behind a device-scope fence (global memory), and only the last warp of the launch pays for the
   // system-scope fence - cumulative over everything counted before it - ahead of the flags it writes into the waiting
   // GPUs' memory.  (A system-scope fence in every warp serialises for more than 10 us per launch.)
+  if (p.done_count != nullptr) __syncwarp();  // (lanes 0 .. 3 made the stores)
   if (p.done_count != nullptr && lane == 0) {
     __threadfence_block();
     if (atomicAdd_block(cta_done, 1) == NW - 1) {
@@ -658,10 +690,8 @@ int configure(const gemv_params& p, int sms, gemv1_config& c) {
   // weight type of the kernel: fp16; u8 with the reference's per-weight rounding; u8 with factored scales
   const int wt = !q ? 0 : ((t.int8_factored && p.bs >= 64) ? 2 : 1);
   const size_t stage_bytes = wt == 2 ? 2 * geom<2>::ROWB + 2 * geom<2>::SC_ROW : wt == 1 ? 2 * geom<1>::ROWB + 2 * geom<1>::SC_ROW : 2 * geom<0>::ROWB;
-  const int seg_shift = wt == 2 ? geom<2>::SEG_SHIFT : geom<1>::SEG_SHIFT;
-  const size_t xbytes = wt == 0 ? (size_t)p.K * 2 : (size_t)p.K * 2 + ((size_t)p.K >> seg_shift) * 16 + 16;  // u8: skewed activation row
-  const size_t nw_stage = p.norm_w != nullptr && p.K > 4096 ? ((((size_t)p.K - 4096) * 2 + 127) & ~(size_t)127) : 0;
-  const size_t fixed = SMEM_FIXED + ((xbytes + 127) & ~(size_t)127) + (((size_t)p.K / 64 * 4 + 127) & ~(size_t)127) + nw_stage;
+  const bool norm = p.norm_w != nullptr;
+  const size_t fixed = SMEM_FIXED + (wt == 0 ? row_layout_of<0>(p.K, norm) : wt == 1 ? row_layout_of<1>(p.K, norm) : row_layout_of<2>(p.K, norm)).total;
   // CTAs per SM: as many as asked for that still fit with a two-deep ring per warp (the factored u8 kernel is
   // latency-bound and compiled for three); then the deepest ring that keeps them resident
   int cps = wt == 2 ? t.ctas_per_sm_int8 : t.ctas_per_sm;
