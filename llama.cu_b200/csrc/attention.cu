@@ -1,21 +1,21 @@
 // Fused attention over the fp16 KV cache for sm_100a.
 //
 // Replaces the reference's matmul_qk -> softmax_rows -> matmul_qkv chain (llama_cu.cu:400-531,
-// called at 1161-1171) and its per-layer score tensor with one kernel that keeps scores and
-// probabilities on chip.  The reference's rounding points are kept ("parity" arithmetic):
+// called at 1161-1171) and its per-layer score tensor with one kernel that keeps scores on chip:
 //   score  s_t = half( (sum_i q_i k_ti) / sqrtf(head_dim) )                    llama_cu.cu:420-425
-//   prob   p_t = half( expf(s_t - max) / sum_t' expf(s_t' - max) )             llama_cu.cu:443-498
-//   out    o_j = half( sum_t float(p_t) float(v_tj) )                          llama_cu.cu:524-529
-// which needs the row's max and sum before any probability is formed, so the kernel is two-pass
-// over the scores (held in shared memory as halves), not an online-softmax.
+//   out    o_j = half( sum_t e^(s_t - max) v_tj / sum_t e^(s_t - max) )        llama_cu.cu:443-529
+// (the reference rounds each quotient e^(s_t - max) / sum to half; here exponentials and sums stay in binary32).
 //
 // One thread-block cluster of CS CTAs serves one (query row, head): each CTA takes a contiguous
 // slice of the cached positions.  K and V are stored head-major ([head][position][head_dim], keys
-// already rotated), so a slice is one contiguous run of 2*head_dim-byte rows.  Latency plan for
-// decode (short slices): the K rows AND the V rows of the first rounds are requested up front, so
-// there is one trip to memory instead of two; every CTA pushes its (max, sum) pair into all peers'
-// shared memory (st.shared::cluster) and its partial output into CTA 0's, which leaves two cluster
-// barriers in the kernel.  Slice sums are combined as sum_r lsum_r * expf(lmax_r - max) in rank order.
+// already rotated), so a slice is one contiguous run of 2*head_dim-byte rows.  A short decode step is a chain of
+// dependent steps, not bytes, so the chain is kept short: every warp runs over its rows with a running maximum, sum
+// and output of its own - no barrier before the end - then a CTA's warps meet once in shared memory and the
+// cluster's CTAs once in rank 0's (st.shared::cluster).  Rows older than the pass's first position do not depend on
+// the kernel before this one: they, and the position itself, are read before griddepcontrol.wait.
+// With two passes over the slice, three block and two cluster barriers a launch took 4.6 / 5.9 us from its wait to its last
+// store at 20 / 300 positions (32 heads).  Decode step of 8 layers, before -> now, at 40 / 430 positions, in us: 4096 wide with u8
+// weights 472 -> 443 / 484 -> 444, 4096 wide fp16 620 -> 610 / 627 -> 616, 1024 wide 194 -> 185 / 197 -> 186.
 #include "attention.cuh"
 
 namespace lcu {
@@ -23,8 +23,7 @@ namespace {
 
 constexpr int ATT_THREADS = 256;
 constexpr int ATT_WARPS = ATT_THREADS / 32;
-constexpr int PRE_ROUNDS = 4;  // rounds of K and V rows requested together at kernel start
-constexpr int BATCH = 4;       // rounds whose row loads are issued before the first of them is used
+constexpr int AS_CH = 64;  // rows a CTA takes at a time
 
 __device__ __forceinline__ void st_dsmem_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
@@ -46,209 +45,239 @@ __device__ __forceinline__ void publish_when_last(const attn_params& p, int tid,
   }
 }
 
+// What a warp has seen so far: maximum of its scores, sum of exponentials and sum of exponentials x V relative to it.  A row
+// is shared by LPR lanes (8 halves = 16 bytes each); lanes of all row groups hold the same maximum, sums per group.
 template <int HD>
-__global__ void __launch_bounds__(ATT_THREADS) attn_kernel(const attn_params p) {
-  constexpr int LPR = HD / 8;    // lanes that share one cached row (8 halves = 16 bytes each)
-  constexpr int RPW = 32 / LPR;  // rows a warp handles per round
-  constexpr int RPR = ATT_WARPS * RPW;  // rows per round of the whole CTA
-  extern __shared__ __align__(16) uint8_t smem[];
-  float* xmax = reinterpret_cast<float*>(smem);  // [8] slice maxima of all ranks (pushed by the peers)
-  float* xsum = xmax + 8;                        // [8] slice exp-sums relative to the slice maximum
-  float* rpart = xsum + 8;                       // [8][HD] partial outputs of all ranks (used on rank 0)
-  float* wpart = rpart + 8 * HD;                 // [ATT_WARPS][HD]
-  float* wred = wpart + ATT_WARPS * HD;          // [2 * ATT_WARPS] scratch
-  __half* sc = reinterpret_cast<__half*>(wred + 2 * ATT_WARPS);  // [chunk] scores of this CTA's slice
+struct warp_rows {
+  static constexpr int LPR = HD / 8;             // lanes that share one cached row
+  static constexpr int RPW = 32 / LPR;           // rows a warp handles per round
+  static constexpr int RPR = ATT_WARPS * RPW;    // rows per round of the whole CTA
+  static constexpr int ROUNDS = AS_CH / RPR;     // rounds of one chunk
+  float m, sum, acc[8], e[ROUNDS];
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int grp = lane / LPR, gl = lane % LPR;
-  const uint32_t rank = cluster_ctarank(), cs = cluster_nctarank();
-  const int head = blockIdx.y, qrow = blockIdx.z;
-
-  pdl_launch_dependents();
-  // Remote shared-memory stores need the target CTA to have started: arrive now, wait right before
-  // the first push (split-phase, so the wait is free by then).
-  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-  pdl_wait();
-
-  const int start_pos = p.pos ? *p.pos : p.pos_value;
-  const int T = start_pos + qrow + 1;  // causal: row r sees positions 0 .. start_pos + r
-  const int chunk = (T + (int)cs - 1) / (int)cs;
-  const int t0 = min(T, (int)rank * chunk), t1 = min(T, t0 + chunk);
-  const int n = t1 - t0;
-
-  const __half* kbase = p.k_cache + ((size_t)head * p.ctx_len + t0) * HD + gl * 8;
-  const __half* vbase = p.v_cache + ((size_t)head * p.ctx_len + t0) * HD + gl * 8;
-
-  // requests for the first rounds of K and V go out together
-  uint4 kreg[PRE_ROUNDS], vreg[PRE_ROUNDS];
+  __device__ __forceinline__ void clear() {
+    m = -CUDART_INF_F;
+    sum = 0.f;
 #pragma unroll
-  for (int r = 0; r < PRE_ROUNDS; ++r) {
-    const int t = r * RPR + warp * RPW + grp;
-    kreg[r] = make_uint4(0, 0, 0, 0);
-    vreg[r] = make_uint4(0, 0, 0, 0);
-    if (t < n) {
-      kreg[r] = *reinterpret_cast<const uint4*>(kbase + (size_t)t * HD);
-      vreg[r] = *reinterpret_cast<const uint4*>(vbase + (size_t)t * HD);
-    }
+    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
   }
-  float q[8];
-  {
-    const uint4 qv = *reinterpret_cast<const uint4*>(p.q + (size_t)qrow * p.ldq + head * HD + gl * 8);
-    const __half2* h = reinterpret_cast<const __half2*>(&qv);
+  // scores of one chunk, rounded to half, and their exponentials (kept for `values`); valid(j): round j's row exists
+  template <class Key, class Valid>
+  __device__ __forceinline__ void scores(const float (&q)[8], float scale_div, Key key, Valid valid) {
+    float top = -CUDART_INF_F;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float2 f = __half22float2(h[i]);
-      q[2 * i] = f.x;
-      q[2 * i + 1] = f.y;
-    }
-  }
-  const float scale_div = sqrtf((float)HD);
-
-  // ---- pass 1: scores of the slice, rounded to half, and the slice maximum.  Rounds are taken BATCH at a time with
-  // all their row loads issued before the first use (long slices would otherwise pay one memory latency per round).
-  float lmax = -CUDART_INF_F;
-  for (int base = 0; base < n; base += BATCH * RPR) {
-    uint4 kv[BATCH];
-#pragma unroll
-    for (int j = 0; j < BATCH; ++j) {
-      const int t = base + j * RPR + warp * RPW + grp;
-      if (base == 0 && j < PRE_ROUNDS) kv[j] = kreg[j < PRE_ROUNDS ? j : 0];
-      else if (t < n) kv[j] = *reinterpret_cast<const uint4*>(kbase + (size_t)t * HD);
-      else kv[j] = make_uint4(0, 0, 0, 0);
-    }
-#pragma unroll
-    for (int j = 0; j < BATCH; ++j) {
-      const int t = base + j * RPR + warp * RPW + grp;
+    for (int j = 0; j < ROUNDS; ++j) {
+      const uint4 kv = key(j);
+      const __half2* h = reinterpret_cast<const __half2*>(&kv);
       float s = 0.f;
-      const __half2* h = reinterpret_cast<const __half2*>(&kv[j]);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        float2 f = __half22float2(h[i]);
+        const float2 f = __half22float2(h[i]);
         s += q[2 * i] * f.x;
         s += q[2 * i + 1] * f.y;
       }
 #pragma unroll
       for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (t < n) {
-        const __half sh = __float2half(s / scale_div);
-        if (gl == 0) sc[t] = sh;
-        lmax = fmaxf(lmax, __half2float(sh));
+      e[j] = valid(j) ? __half2float(__float2half(s / scale_div)) : -CUDART_INF_F;
+      top = fmaxf(top, e[j]);
+    }
+#pragma unroll
+    for (int o = LPR; o < 32; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    top = fmaxf(top, m);
+    const float keep = top > -CUDART_INF_F ? expf(m - top) : 1.f;
+    m = top;
+    sum *= keep;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] *= keep;
+#pragma unroll
+    for (int j = 0; j < ROUNDS; ++j) {
+      e[j] = valid(j) && m > -CUDART_INF_F ? expf(e[j] - m) : 0.f;
+      sum += e[j];
+    }
+  }
+  template <class Value, class Valid>
+  __device__ __forceinline__ void values(Value value, Valid valid) {
+#pragma unroll
+    for (int j = 0; j < ROUNDS; ++j) {
+      if (!valid(j)) continue;
+      const uint4 vv = value(j);
+      const __half2* h = reinterpret_cast<const __half2*>(&vv);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 f = __half22float2(h[i]);
+        acc[2 * i] += e[j] * f.x;
+        acc[2 * i + 1] += e[j] * f.y;
       }
     }
   }
-  lmax = warp_max(lmax);
-  if (lane == 0) wred[warp] = lmax;
-  __syncthreads();
-  lmax = wred[0];
-#pragma unroll
-  for (int w = 1; w < ATT_WARPS; ++w) lmax = fmaxf(lmax, wred[w]);
+};
 
-  // slice exp-sum relative to the slice maximum (fixed order: lanes, then warps)
-  float lsum = 0.f;
-  for (int t = tid; t < n; t += ATT_THREADS) lsum += expf(__half2float(sc[t]) - lmax);
-  lsum = warp_sum(lsum);
-  if (lane == 0) wred[ATT_WARPS + warp] = lsum;
-  __syncthreads();
-  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-  if (tid < (int)cs) {  // thread r pushes this slice's pair into rank r's table
-    float s = 0.f;
-    for (int w = 0; w < ATT_WARPS; ++w) s += wred[ATT_WARPS + w];
-    st_dsmem_f32(mapa(smem_u32(&xmax[rank]), tid), lmax);
-    st_dsmem_f32(mapa(smem_u32(&xsum[rank]), tid), s);
-  }
-  cluster_sync();
-  float gmax = -CUDART_INF_F;
-  for (uint32_t r = 0; r < cs; ++r) gmax = fmaxf(gmax, xmax[r]);
-  float gsum = 0.f;
-  for (uint32_t r = 0; r < cs; ++r) {
-    const float m = xmax[r];
-    if (m > -CUDART_INF_F) gsum += xsum[r] * expf(m - gmax);  // an empty slice contributes nothing
-  }
+// Shared memory where the warps of a CTA and the CTAs of a cluster meet.
+template <int HD>
+struct meeting {
+  float cta_max[8], cta_sum[8];  // of all ranks (rank 0's copy is used)
+  float cta_out[8][HD];
+  float warp_max[ATT_WARPS], warp_sum[ATT_WARPS];
+  float warp_out[ATT_WARPS][HD];
+};
 
-  // ---- pass 2: probabilities rounded to half, times V (rounds in batches, as above)
-  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int base = 0; base < n; base += BATCH * RPR) {
-    uint4 vv[BATCH];
+// combines warps, then ranks, in fixed order; `threads` consumer threads on named barrier 1; every thread of the CTA has
+// arrived at the cluster's start barrier.  Threads beyond the consumers only take part in cluster_sync().
+template <int HD>
+__device__ __forceinline__ void meet_and_store(const attn_params& p, meeting<HD>& mt, warp_rows<HD>& w, int head, int qrow, uint32_t rank, uint32_t cs) {
+  constexpr int LPR = warp_rows<HD>::LPR;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 #pragma unroll
-    for (int j = 0; j < BATCH; ++j) {
-      const int t = base + j * RPR + warp * RPW + grp;
-      if (base == 0 && j < PRE_ROUNDS) vv[j] = vreg[j < PRE_ROUNDS ? j : 0];
-      else if (t < n) vv[j] = *reinterpret_cast<const uint4*>(vbase + (size_t)t * HD);
-      else vv[j] = make_uint4(0, 0, 0, 0);
-    }
+  for (int o = LPR; o < 32; o <<= 1) {
+    w.sum += __shfl_xor_sync(0xffffffffu, w.sum, o);
 #pragma unroll
-    for (int j = 0; j < BATCH; ++j) {
-      const int t = base + j * RPR + warp * RPW + grp;
-      if (t < n) {
-        const float pr = __half2float(__float2half(expf(__half2float(sc[t]) - gmax) / gsum));
-        const __half2* h = reinterpret_cast<const __half2*>(&vv[j]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float2 f = __half22float2(h[i]);
-          acc[2 * i] += pr * f.x;
-          acc[2 * i + 1] += pr * f.y;
-        }
-      }
-    }
+    for (int i = 0; i < 8; ++i) w.acc[i] += __shfl_xor_sync(0xffffffffu, w.acc[i], o);
   }
-  // combine the row groups of a warp, then the warps, then the cluster ranks (all in fixed order)
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-    for (int o = LPR; o < 32; o <<= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
-  if (grp == 0) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) wpart[warp * HD + gl * 8 + i] = acc[i];
+  if (lane < LPR) {
+    *reinterpret_cast<float4*>(&mt.warp_out[warp][lane * 8]) = make_float4(w.acc[0], w.acc[1], w.acc[2], w.acc[3]);
+    *reinterpret_cast<float4*>(&mt.warp_out[warp][lane * 8 + 4]) = make_float4(w.acc[4], w.acc[5], w.acc[6], w.acc[7]);
   }
-  __syncthreads();
+  if (lane == 0) {
+    mt.warp_max[warp] = w.m;
+    mt.warp_sum[warp] = w.sum;
+  }
+  bar_sync(1, ATT_THREADS);
+  // (an empty part has maximum -inf and adds nothing)
+  auto weight = [](float m, float top) { return m > -CUDART_INF_F ? expf(m - top) : 0.f; };
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // remote stores need the target CTA to have started
   if (tid < HD) {
-    float s = 0.f;
-    for (int w = 0; w < ATT_WARPS; ++w) s += wpart[w * HD + tid];
-    st_dsmem_f32(mapa(smem_u32(&rpart[rank * HD + tid]), 0), s);  // into rank 0's table
+    float top = mt.warp_max[0];
+#pragma unroll
+    for (int i = 1; i < ATT_WARPS; ++i) top = fmaxf(top, mt.warp_max[i]);
+    float o = 0.f, s = 0.f;
+#pragma unroll
+    for (int i = 0; i < ATT_WARPS; ++i) {
+      const float f = weight(mt.warp_max[i], top);
+      o += f * mt.warp_out[i][tid];
+      s += f * mt.warp_sum[i];
+    }
+    st_dsmem_f32(mapa(smem_u32(&mt.cta_out[rank][tid]), 0), o);
+    if (tid == 0) {
+      st_dsmem_f32(mapa(smem_u32(&mt.cta_max[rank]), 0), top);
+      st_dsmem_f32(mapa(smem_u32(&mt.cta_sum[rank]), 0), s);
+    }
   }
   cluster_sync();
   if (rank == 0 && tid < HD) {
-    float s = 0.f;
-    for (uint32_t r = 0; r < cs; ++r) s += rpart[r * HD + tid];
-    const __half o = __float2half(s);
+    float top = -CUDART_INF_F;
+    for (uint32_t r = 0; r < cs; ++r) top = fmaxf(top, mt.cta_max[r]);
+    float o = 0.f, s = 0.f;
+    for (uint32_t r = 0; r < cs; ++r) {
+      const float f = weight(mt.cta_max[r], top);
+      o += f * mt.cta_out[r][tid];
+      s += f * mt.cta_sum[r];
+    }
+    const __half h = __float2half(o / s);
     const size_t at = (size_t)qrow * p.ldo + head * HD + tid;
-    p.out[at] = o;
-    for (int q = 0; q < p.n_peer_out; ++q) p.peer_out[q][at] = o;  // tensor-parallel: into every GPU's row (peer stores)
+    p.out[at] = h;
+    for (int q = 0; q < p.n_peer_out; ++q) p.peer_out[q][at] = h;  // tensor-parallel: into every GPU's row (peer stores)
   }
   if (rank == 0 && p.done_count != nullptr) publish_when_last(p, tid, (int)(gridDim.y * gridDim.z));
+}
+
+__device__ __forceinline__ void load_query(float (&q)[8], const __half* at) {
+  const uint4 qv = __ldcg(reinterpret_cast<const uint4*>(at));
+  const __half2* h = reinterpret_cast<const __half2*>(&qv);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __half22float2(h[i]);
+    q[2 * i] = f.x;
+    q[2 * i + 1] = f.y;
+  }
+}
+
+template <int HD>
+__global__ void __launch_bounds__(ATT_THREADS) attn_kernel(const attn_params p) {
+  using rows = warp_rows<HD>;
+  __shared__ __align__(16) meeting<HD> mt;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int grp = lane / rows::LPR, gl = lane % rows::LPR;
+  const uint32_t rank = cluster_ctarank(), cs = cluster_nctarank();
+  const int head = blockIdx.y, qrow = blockIdx.z;
+
+  pdl_launch_dependents();
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // (split-phase: waited for before the first remote store)
+
+  // the position was settled before this step's first kernel began
+  const int start_pos = p.pos ? *p.pos : p.pos_value;
+  const int T = start_pos + qrow + 1;  // causal: row r sees positions 0 .. start_pos + r
+  const int chunk = (T + (int)cs - 1) / (int)cs;
+  const int t0 = min(T, (int)rank * chunk), t1 = min(T, t0 + chunk);
+  const int n = t1 - t0;
+  const __half* kbase = p.k_cache + ((size_t)head * p.ctx_len + t0) * HD + gl * 8;
+  const __half* vbase = p.v_cache + ((size_t)head * p.ctx_len + t0) * HD + gl * 8;
+  const int row0 = warp * rows::RPW + grp;
+  auto row_of = [&](int base, int j) { return base + j * rows::RPR + row0; };
+  auto load = [&](const __half* b, int t) { return __ldcg(reinterpret_cast<const uint4*>(b + (size_t)t * HD)); };
+
+  uint4 kreg[rows::ROUNDS], vreg[rows::ROUNDS];
+  auto fetch = [&](int base, int from, int to) {  // this thread's rows of a chunk that lie in from .. to - 1
+#pragma unroll
+    for (int j = 0; j < rows::ROUNDS; ++j) {
+      const int t = row_of(base, j);
+      if (t >= from && t < to) {
+        kreg[j] = load(kbase, t);
+        vreg[j] = load(vbase, t);
+      }
+    }
+  };
+#pragma unroll
+  for (int j = 0; j < rows::ROUNDS; ++j) kreg[j] = vreg[j] = make_uint4(0, 0, 0, 0);
+  const int old = min(n, start_pos - t0);  // rows of the slice that earlier passes wrote
+  fetch(0, 0, old);
+  pdl_wait();
+  float q[8];
+  load_query(q, p.q + (size_t)qrow * p.ldq + head * HD + gl * 8);
+  fetch(0, max(old, 0), n);
+  const float scale_div = sqrtf((float)HD);
+
+  rows w;
+  w.clear();
+  for (int base = 0; base < n; base += AS_CH) {
+    if (base > 0) fetch(base, 0, n);
+    auto valid = [&](int j) { return row_of(base, j) < n; };
+    w.scores(q, scale_div, [&](int j) { return kreg[j]; }, valid);
+    w.values([&](int j) { return vreg[j]; }, valid);
+  }
+  meet_and_store(p, mt, w, head, qrow, rank, cs);
 }
 
 // ---------------------------------------------------------------------------------------------------
 // Streaming variant for long slices.  Same arithmetic, same thread-to-row assignment and summation order as
 // attn_kernel (the two give identical bits), but the rows come through shared memory: a producer warp brings the
 // slice in as contiguous bulk copies of up to 64 rows (the cache is head-major, so a slice is one contiguous run),
-// K chunks first, then V chunks, through a ring of three buffers with full/empty mbarriers.  With per-thread
+// K and V chunks in turn, through a ring of buffers with full/empty mbarriers.  With per-thread
 // loads a CTA has at most 4 rows per thread in flight and a 260-row slice pays a memory latency every few rounds;
-// here the ring keeps 48 KB per CTA requested at all times.
-constexpr int AS_CH = 64;  // rows per chunk
-constexpr int AS_NB = 3;   // ring buffers
+// here the ring keeps 64 KB per CTA requested at all times.
+constexpr int AS_NB = 4;   // ring buffers
 constexpr int AS_THREADS = ATT_THREADS + 32;
 
 template <int HD>
 __global__ void __launch_bounds__(AS_THREADS, 3) attn_stream_kernel(const attn_params p) {
-  constexpr int LPR = HD / 8, RPW = 32 / LPR, RPR = ATT_WARPS * RPW;
+  using rows = warp_rows<HD>;
   constexpr int CHUNK_BYTES = AS_CH * HD * 2;
-  extern __shared__ __align__(16) uint8_t smem[];
-  float* xmax = reinterpret_cast<float*>(smem);
-  float* xsum = xmax + 8;
-  float* rpart = xsum + 8;
-  float* wpart = rpart + 8 * HD;
-  float* wred = wpart + ATT_WARPS * HD;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(wred + 2 * ATT_WARPS);  // full[AS_NB], empty[AS_NB]
-  uint8_t* ring = reinterpret_cast<uint8_t*>(bars + 8);                // 16-byte aligned (bulk-copy destination)
-  __half* sc = reinterpret_cast<__half*>(ring + AS_NB * CHUNK_BYTES);  // [slice] scores
+  extern __shared__ __align__(128) uint8_t ring[];
+  __shared__ __align__(16) meeting<HD> mt;
+  __shared__ uint64_t bars[2 * AS_NB];  // full[AS_NB], empty[AS_NB]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int grp = lane / LPR, gl = lane % LPR;
+  const int grp = lane / rows::LPR, gl = lane % rows::LPR;
   const uint32_t rank = cluster_ctarank(), cs = cluster_nctarank();
   const int head = blockIdx.y, qrow = blockIdx.z;
 
   pdl_launch_dependents();
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  const int start_pos = p.pos ? *p.pos : p.pos_value;  // (settled before this step's first kernel began)
+  const int T = start_pos + qrow + 1;
+  const int chunk = (T + (int)cs - 1) / (int)cs;
+  const int t0 = min(T, (int)rank * chunk), t1 = min(T, t0 + chunk);
+  const int n = t1 - t0;
+  const int nch = (n + AS_CH - 1) / AS_CH;
   if (tid == 0) {
     for (int i = 0; i < AS_NB; ++i) {
       mbar_init(smem_u32(&bars[i]), 1);
@@ -257,183 +286,73 @@ __global__ void __launch_bounds__(AS_THREADS, 3) attn_stream_kernel(const attn_p
     fence_mbar_init();
   }
   __syncthreads();
-  pdl_wait();
-
-  const int start_pos = p.pos ? *p.pos : p.pos_value;
-  const int T = start_pos + qrow + 1;
-  const int chunk = (T + (int)cs - 1) / (int)cs;
-  const int t0 = min(T, (int)rank * chunk), t1 = min(T, t0 + chunk);
-  const int n = t1 - t0;
-  const int nch = (n + AS_CH - 1) / AS_CH, total = 2 * nch;
 
   if (warp == ATT_WARPS) {
-    // ---- producer: chunk i < nch is K chunk i, chunk nch + j is V chunk j.  Chunks up to nch + AS_NB - 1 need only
-    // buffers that pass 1 releases; the rest wait for pass 2 and are issued after the first cluster barrier.
+    // ---- producer: copy i is the K (i even) or V (i odd) part of chunk i / 2; chunks of rows that earlier passes wrote are
+    // requested before the kernel ahead of this one has ended
     const __half* kb = p.k_cache + ((size_t)head * p.ctx_len + t0) * HD;
     const __half* vb = p.v_cache + ((size_t)head * p.ctx_len + t0) * HD;
-    auto issue = [&](int i) {
-      const int b = i % AS_NB, use = i / AS_NB;
-      if (use > 0 && !mbar_wait(smem_u32(&bars[AS_NB + b]), (use - 1) & 1, p.err, DEV_ERR_EMPTY_WAIT)) return false;
-      const int c = i < nch ? i : i - nch;
-      const uint32_t bytes = (uint32_t)min(AS_CH, n - c * AS_CH) * (HD * 2);
-      const uint32_t full = smem_u32(&bars[b]);
-      mbar_arrive_expect_tx(full, bytes);
-      bulk_g2s(smem_u32(ring + b * CHUNK_BYTES), (i < nch ? kb : vb) + (size_t)c * AS_CH * HD, bytes, full);
-      return true;
-    };
-    const int first_part = min(total, nch + AS_NB);
-    bool ok = true;
-    if (lane == 0)
-      for (int i = 0; i < first_part && ok; ++i) ok = issue(i);
+    if (lane == 0) {
+      bool waited = false;
+      for (int i = 0; i < 2 * nch; ++i) {
+        const int b = i % AS_NB, use = i / AS_NB, c = i >> 1;
+        const int rows_here = min(AS_CH, n - c * AS_CH);
+        if (!waited && t0 + c * AS_CH + rows_here > start_pos) {
+          pdl_wait();
+          waited = true;
+        }
+        if (use > 0 && !mbar_wait(smem_u32(&bars[AS_NB + b]), (use - 1) & 1, p.err, DEV_ERR_EMPTY_WAIT)) break;
+        const uint32_t bytes = (uint32_t)rows_here * (HD * 2), full = smem_u32(&bars[b]);
+        mbar_arrive_expect_tx(full, bytes);
+        bulk_g2s(smem_u32(ring + b * CHUNK_BYTES), ((i & 1) ? vb : kb) + (size_t)c * AS_CH * HD, bytes, full);
+      }
+    }
     __syncwarp();
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     cluster_sync();
-    if (lane == 0)
-      for (int i = first_part; i < total && ok; ++i) ok = issue(i);
-    __syncwarp();
-    cluster_sync();
+    if (rank == 0 && p.done_count != nullptr) __syncthreads();  // (publish_when_last)
     return;
   }
 
+  pdl_wait();
   float q[8];
-  {
-    const uint4 qv = *reinterpret_cast<const uint4*>(p.q + (size_t)qrow * p.ldq + head * HD + gl * 8);
-    const __half2* h = reinterpret_cast<const __half2*>(&qv);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float2 f = __half22float2(h[i]);
-      q[2 * i] = f.x;
-      q[2 * i + 1] = f.y;
-    }
-  }
+  load_query(q, p.q + (size_t)qrow * p.ldq + head * HD + gl * 8);
   const float scale_div = sqrtf((float)HD);
   bool ok = true;
-
-  // ---- pass 1: scores of the slice, rounded to half, and the slice maximum
-  float lmax = -CUDART_INF_F;
+  rows w;
+  w.clear();
+  const int row0 = warp * rows::RPW + grp;
   for (int c = 0; c < nch; ++c) {
-    const int b = c % AS_NB;
-    ok = ok && mbar_wait(smem_u32(&bars[b]), (c / AS_NB) & 1, p.err, DEV_ERR_FULL_WAIT);
-    const uint8_t* buf = ring + b * CHUNK_BYTES;
-#pragma unroll
-    for (int r0 = 0; r0 < AS_CH; r0 += RPR) {
-      const int r = r0 + warp * RPW + grp;
-      const int t = c * AS_CH + r;
-      uint4 kv = make_uint4(0, 0, 0, 0);
-      if (ok && t < n) kv = *reinterpret_cast<const uint4*>(buf + (size_t)r * (HD * 2) + gl * 16);
-      float s = 0.f;
-      const __half2* h = reinterpret_cast<const __half2*>(&kv);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float2 f = __half22float2(h[i]);
-        s += q[2 * i] * f.x;
-        s += q[2 * i + 1] * f.y;
-      }
-#pragma unroll
-      for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (t < n) {
-        const __half sh = __float2half(s / scale_div);
-        if (gl == 0) sc[t] = sh;
-        lmax = fmaxf(lmax, __half2float(sh));
-      }
-    }
+    auto valid = [&](int j) { return ok && c * AS_CH + j * rows::RPR + row0 < n; };
+    auto at = [&](const uint8_t* buf, int j) { return *reinterpret_cast<const uint4*>(buf + (size_t)(j * rows::RPR + row0) * (HD * 2) + gl * 16); };
+    const int kb = (2 * c) % AS_NB, vb = (2 * c + 1) % AS_NB;
+    const uint32_t parity = (uint32_t)((2 * c) / AS_NB) & 1u;
+    ok = ok && mbar_wait(smem_u32(&bars[kb]), parity, p.err, DEV_ERR_FULL_WAIT);
+    w.scores(q, scale_div, [&](int j) { return valid(j) ? at(ring + kb * CHUNK_BYTES, j) : make_uint4(0, 0, 0, 0); }, valid);
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&bars[AS_NB + b]));
-  }
-  lmax = warp_max(lmax);
-  if (lane == 0) wred[warp] = lmax;
-  bar_sync(1, ATT_THREADS);
-  lmax = wred[0];
-#pragma unroll
-  for (int w = 1; w < ATT_WARPS; ++w) lmax = fmaxf(lmax, wred[w]);
-
-  float lsum = 0.f;
-  for (int t = tid; t < n; t += ATT_THREADS) lsum += expf(__half2float(sc[t]) - lmax);
-  lsum = warp_sum(lsum);
-  if (lane == 0) wred[ATT_WARPS + warp] = lsum;
-  bar_sync(1, ATT_THREADS);
-  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-  if (tid < (int)cs) {
-    float s = 0.f;
-    for (int w = 0; w < ATT_WARPS; ++w) s += wred[ATT_WARPS + w];
-    st_dsmem_f32(mapa(smem_u32(&xmax[rank]), tid), lmax);
-    st_dsmem_f32(mapa(smem_u32(&xsum[rank]), tid), s);
-  }
-  cluster_sync();
-  float gmax = -CUDART_INF_F;
-  for (uint32_t r = 0; r < cs; ++r) gmax = fmaxf(gmax, xmax[r]);
-  float gsum = 0.f;
-  for (uint32_t r = 0; r < cs; ++r) {
-    const float m = xmax[r];
-    if (m > -CUDART_INF_F) gsum += xsum[r] * expf(m - gmax);
-  }
-
-  // ---- pass 2: probabilities rounded to half, times V
-  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int c = 0; c < nch; ++c) {
-    const int i = nch + c, b = i % AS_NB;
-    ok = ok && mbar_wait(smem_u32(&bars[b]), (i / AS_NB) & 1, p.err, DEV_ERR_FULL_WAIT);
-    const uint8_t* buf = ring + b * CHUNK_BYTES;
-#pragma unroll
-    for (int r0 = 0; r0 < AS_CH; r0 += RPR) {
-      const int r = r0 + warp * RPW + grp;
-      const int t = c * AS_CH + r;
-      if (ok && t < n) {
-        const float pr = __half2float(__float2half(expf(__half2float(sc[t]) - gmax) / gsum));
-        const uint4 vv = *reinterpret_cast<const uint4*>(buf + (size_t)r * (HD * 2) + gl * 16);
-        const __half2* h = reinterpret_cast<const __half2*>(&vv);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          float2 f = __half22float2(h[k]);
-          acc[2 * k] += pr * f.x;
-          acc[2 * k + 1] += pr * f.y;
-        }
-      }
-    }
+    if (lane == 0) mbar_arrive(smem_u32(&bars[AS_NB + kb]));
+    ok = ok && mbar_wait(smem_u32(&bars[vb]), parity, p.err, DEV_ERR_FULL_WAIT);
+    w.values([&](int j) { return at(ring + vb * CHUNK_BYTES, j); }, valid);
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&bars[AS_NB + b]));
+    if (lane == 0) mbar_arrive(smem_u32(&bars[AS_NB + vb]));
   }
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-    for (int o = LPR; o < 32; o <<= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
-  if (grp == 0) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) wpart[warp * HD + gl * 8 + i] = acc[i];
-  }
-  bar_sync(1, ATT_THREADS);
-  if (tid < HD) {
-    float s = 0.f;
-    for (int w = 0; w < ATT_WARPS; ++w) s += wpart[w * HD + tid];
-    st_dsmem_f32(mapa(smem_u32(&rpart[rank * HD + tid]), 0), s);
-  }
-  cluster_sync();
-  if (rank == 0 && tid < HD) {
-    float s = 0.f;
-    for (uint32_t r = 0; r < cs; ++r) s += rpart[r * HD + tid];
-    const __half o = __float2half(s);
-    const size_t at = (size_t)qrow * p.ldo + head * HD + tid;
-    p.out[at] = o;
-    for (int q = 0; q < p.n_peer_out; ++q) p.peer_out[q][at] = o;  // tensor-parallel: into every GPU's row (peer stores)
-  }
-  if (rank == 0 && p.done_count != nullptr) publish_when_last(p, tid, (int)(gridDim.y * gridDim.z));
+  meet_and_store(p, mt, w, head, qrow, rank, cs);
+}
+
+// positions a CTA's slice may hold (one half each within 200 KB beside the partial results)
+template <int HD>
+constexpr int most_positions() {
+  return (200 * 1024 - 16 - (int)sizeof(float) * (16 + 8 * HD + ATT_WARPS * HD + 2 * ATT_WARPS)) / 2;
 }
 
 template <int HD>
 int launch_hd(const attn_params& p, int m, int cs, int max_T, cudaStream_t stream, int pdl) {
   const int chunk = (max_T + cs - 1) / cs;
-  const size_t smem = (16 + 8 * HD + ATT_WARPS * HD + 2 * ATT_WARPS) * sizeof(float) + (size_t)chunk * 2 + 16;
-  LCU_REQUIRE(smem <= 200 * 1024, "attention: %d positions per CTA do not fit in shared memory", chunk);
-  static bool attr_done[16] = {};
-  int dev = 0;
-  LCU_CUDA(cudaGetDevice(&dev));
-  if (dev < 16 && !attr_done[dev]) {
-    LCU_CUDA(cudaFuncSetAttribute(attn_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr_done[dev] = true;
-  }
+  LCU_REQUIRE(chunk <= most_positions<HD>(), "attention: %d positions per CTA do not fit in shared memory", chunk);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cs, p.n_heads, m);
   cfg.blockDim = dim3(ATT_THREADS);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = 0;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -451,9 +370,8 @@ int launch_hd(const attn_params& p, int m, int cs, int max_T, cudaStream_t strea
 template <int HD>
 int launch_stream_hd(const attn_params& p, int m, int cs, int max_T, cudaStream_t stream, int pdl) {
   const int chunk = (max_T + cs - 1) / cs;
-  const size_t smem = (16 + 8 * HD + ATT_WARPS * HD + 2 * ATT_WARPS) * sizeof(float) + 64 + (size_t)AS_NB * AS_CH * HD * 2 +
-                      (((size_t)chunk * 2 + 15) & ~(size_t)15);
-  LCU_REQUIRE(smem <= 200 * 1024, "attention: %d positions per CTA do not fit in shared memory", chunk);
+  const size_t smem = (size_t)AS_NB * AS_CH * HD * 2;
+  LCU_REQUIRE(chunk <= most_positions<HD>() - AS_NB * AS_CH * HD, "attention: %d positions per CTA do not fit in shared memory", chunk);
   LCU_REQUIRE(p.err != nullptr, "attention: the streaming kernel needs a device error word");
   static bool attr_done[16] = {};
   int dev = 0;

@@ -425,6 +425,30 @@ def test_attention_streaming_kernel_gives_the_same_bits(lcu, T0, H, hd, cluster)
     assert np.abs(f32(outs[1]) - f32(oo)).max() <= 4e-3
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("T0", [0, 7, 8, 63, 64, 127, 510, 511, 512, 1023, 1024])
+def test_attention_slices_at_the_edges_of_chunks(lcu, T0, hd):
+    """One query row over slices that are empty, end with a chunk of 64 rows or one row behind it, through both decode kernels, for every
+    cluster size: equal bits of the two, and the oracle's row.  Bound: the oracle rounds every probability to half (2^-11 of it), so
+    its row may be off by 2^-11 max|v| < 2.5e-3 here, and both round the result (|row| < 4.5: 2^-9)."""
+    H = 2
+    rng = np.random.default_rng(T0 + hd)
+    dim, T = H * hd, T0 + 1
+    q, k, v = f16(rng.standard_normal((1, dim))), f16(rng.standard_normal((T, dim))), f16(rng.standard_normal((T, dim)))
+    oo = np.zeros_like(q)
+    L.orc_attention(oo.reshape(-1), q.reshape(-1), k.reshape(-1), v.reshape(-1), 1, T, dim, H, T0, 0)
+    for cluster in (1, 2, 4, 8):
+        outs = []
+        try:
+            for mode in (0, 1):
+                lcu.check(lcu.lib.lcu_set_tuning(b"attn_stream", mode))
+                outs.append(lcu.attention(q, k, v, H, T0, cluster))
+        finally:
+            lcu.check(lcu.lib.lcu_set_tuning(b"attn_stream", -1))
+        assert (outs[0] == outs[1]).all()
+        assert np.abs(f32(outs[0]) - f32(oo)).max() <= 2.5e-3 + 2.0**-9, cluster
+
+
 @pytest.mark.parametrize("m,T0,cluster", [(1, 50, 4), (70, 9, 0), (70, 9, -1), (300, 100, -1), (70, 9, -2), (300, 100, -2)])
 def test_attention_head_dim_64(lcu, m, T0, cluster):
     rng = np.random.default_rng(8)
