@@ -139,6 +139,7 @@ __global__ void __cluster_dims__(HC_CLUSTER, 1, 1) __launch_bounds__(HC_THREADS)
         best = x_best[r];
         best_i = x_idx[r];
       }
+    if (best_i >= V) best_i = 0;  // (no probability is a number: the first index, as std::max_element; a chained step feeds it back)
     if (p.token_out) *p.token_out = best_i;
     if (p.next_ids) p.next_ids[0] = (short)best_i;
     if (p.pos) *p.pos += p.advance;

@@ -295,6 +295,7 @@ __global__ void __launch_bounds__(HEAD_THREADS) logits_head_kernel(const head_pa
         best = s_red[w];
         best_i = s_idx[w];
       }
+    if (best_i >= V) best_i = 0;  // (no probability is a number: the first index, as std::max_element; a chained step feeds it back)
     if (p.token_out) *p.token_out = best_i;
     if (p.next_ids) p.next_ids[0] = (short)best_i;
     if (p.pos) *p.pos += p.advance;
