@@ -36,6 +36,7 @@ int lcu_device_count(void);
 int lcu_set_matmul_type(int type);
 /* launch-shape knobs used for the measurements (defaults are the measured best): "gemv_stages", "gemv_ctas_per_sm",
  * "gemv_ctas_per_sm_int8", "gemv_variant", "gemv_warp_stages", "gemv_warp_stages_int8", "gemv_consumer_warps_int8", "gemv_prefetch_kb",
+ * "gemv_held" (0 = weights of small single-row products are streamed like those of large ones, -1 = held in registers by a rule),
  * "int8_factored" (0 = round every dequantized weight to half as the reference does), "prefill_tc_min_rows",
  * "prefill_tc_tile_n", "prefill_tc_pair", "prefill_tc_split", "prefill_tc_sk", "prefill_tc_kb", "prefill_sk_kb" (k-blocks per
  * stage and tensor copy of the one-SM / the pair GEMMs), "prefill_gate_fused", "prefill_u8_deq_min_rows", "prefill_u8_shadow", "prefill_fuse",

@@ -106,6 +106,9 @@ int gemv_sm_count();
 // several passes
 int gemv_max_rows(int K);
 
+// weights of small launches held in registers: -1 = by the rule (default), 0 = never
+void gemv_held_mode(int mode);
+
 // loads all single-row kernels on the current device ahead of their first launch
 int gemv_single_row_preload();
 // consumer warps of the single-row launch these arguments lead to

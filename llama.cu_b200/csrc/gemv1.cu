@@ -98,103 +98,53 @@ __device__ __forceinline__ uint32_t dequant_pair(uint32_t word, uint32_t selecto
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// One 64-byte step of every segment: 16 tile rows x 32 (fp16) or 64 (u8) weights per lane group.
-template <int WT, bool FULL>
-__device__ __forceinline__ void step(float (&accs)[NACC][4], const int s, const int flip, const int c, const int g, const int vb,
-                                     const uint8_t* seg0, const uint8_t* xseg, const uint8_t* st, const float* xs64, const int ci,
-                                     const int bs) {
-  constexpr int ESZ = is16<WT> ? 2 : 1;
-  constexpr int ROWB = geom<WT>::ROWB, SEG = geom<WT>::SEG, NSTEPS = geom<WT>::NSTEPS;
-  constexpr int CHUNK_K = ROWB / ESZ;
+// One 64-byte step of every segment: 16 tile rows x 32 (fp16) or 64 (u8) weights per lane group.  lo / hi: 16 bytes of the pair's
+// rows; x0, x1: the activations they meet; sc_lo / sc_hi: their scales; xsum: sum of the activations of the step (factored u8).
+template <int WT>
+__device__ __forceinline__ void step(float (&accs)[NACC][4], const int s, const uint4& lo, const uint4& hi, const uint4& x0, const uint4& x1, __half sc_lo,
+                                     __half sc_hi, float xsum) {
   float* acc = accs[(2 * s) % NACC];
   float* acc_b = accs[(2 * s + 1) % NACC];
-  const int off = ((s ^ flip) << 6) + c * 16;  // byte offset inside the segment
-  const bool ok = FULL || off < vb;
-  uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
-  if (ok) {
-    lo = *reinterpret_cast<const uint4*>(seg0 + off);
-    hi = *reinterpret_cast<const uint4*>(seg0 + ROWB + off);
-  }
-  if (is16<WT>) {
-    uint4 xb = make_uint4(0, 0, 0, 0);
-    if (ok) xb = *reinterpret_cast<const uint4*>(xseg + off);
-    if (WT == 3) {
-      mma_16816_bf16(acc, lo.x, hi.x, lo.y, hi.y, xb.x, xb.y);
-      mma_16816_bf16(acc_b, lo.z, hi.z, lo.w, hi.w, xb.z, xb.w);
-    } else {
-      mma_16816(acc, lo.x, hi.x, lo.y, hi.y, xb.x, xb.y);
-      mma_16816(acc_b, lo.z, hi.z, lo.w, hi.w, xb.z, xb.w);
-    }
+  if (WT == 3) {
+    mma_16816_bf16(acc, lo.x, hi.x, lo.y, hi.y, x0.x, x0.y);
+    mma_16816_bf16(acc_b, lo.z, hi.z, lo.w, hi.w, x0.z, x0.w);
+  } else if (WT == 0) {
+    mma_16816(acc, lo.x, hi.x, lo.y, hi.y, x0.x, x0.y);
+    mma_16816(acc_b, lo.z, hi.z, lo.w, hi.w, x0.z, x0.w);
+  } else if (WT == 2) {
+    const float corr = 1151.5f * xsum;
+    float ta[4] = {0.f, 0.f, 0.f, 0.f}, tb[4] = {0.f, 0.f, 0.f, 0.f};
+    const uint32_t M = 0x64646464u;  // bytes -> halves 1024 + q
+    mma_16816(ta, __byte_perm(lo.x, M, 0x4140), __byte_perm(hi.x, M, 0x4140), __byte_perm(lo.x, M, 0x4342), __byte_perm(hi.x, M, 0x4342), x0.x, x0.y);
+    mma_16816(tb, __byte_perm(lo.y, M, 0x4140), __byte_perm(hi.y, M, 0x4140), __byte_perm(lo.y, M, 0x4342), __byte_perm(hi.y, M, 0x4342), x0.z, x0.w);
+    mma_16816(ta, __byte_perm(lo.z, M, 0x4140), __byte_perm(hi.z, M, 0x4140), __byte_perm(lo.z, M, 0x4342), __byte_perm(hi.z, M, 0x4342), x1.x, x1.y);
+    mma_16816(tb, __byte_perm(lo.w, M, 0x4140), __byte_perm(hi.w, M, 0x4140), __byte_perm(lo.w, M, 0x4342), __byte_perm(hi.w, M, 0x4342), x1.z, x1.w);
+    // only the diagonal entries (column == this lane's segment) are meaningful, and they share `corr`
+    const float sl = __half2float(sc_lo), sh = __half2float(sc_hi);
+    acc[0] += sl * ((ta[0] + tb[0]) - corr);
+    acc[1] += sl * ((ta[1] + tb[1]) - corr);
+    acc[2] += sh * ((ta[2] + tb[2]) - corr);
+    acc[3] += sh * ((ta[3] + tb[3]) - corr);
   } else {
-    uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
-    __half sc_lo = __ushort_as_half(0), sc_hi = sc_lo;
-    float corr = 0.f;
-    if (ok) {
-      x0 = *reinterpret_cast<const uint4*>(xseg + 2 * off);
-      x1 = *reinterpret_cast<const uint4*>(xseg + 2 * off + 16);
-      const __half* scs = reinterpret_cast<const __half*>(st + 2 * ROWB);
-      const int si = (g * SEG + off) >> bs;  // k offset inside the chunk / block size (bs is log2 of it here)
-      sc_lo = scs[si];
-      sc_hi = scs[geom<WT>::SC_ROW / 2 + si];
-      // WT 2: sum of x over this lane's segment and step (the diagonal column of the tile)
-      if (WT == 2) corr = 1151.5f * xs64[ci * (CHUNK_K / 64) + g * NSTEPS + (s ^ flip)];
-    }
-    if (WT == 2) {
-      float ta[4] = {0.f, 0.f, 0.f, 0.f}, tb[4] = {0.f, 0.f, 0.f, 0.f};
-      const uint32_t M = 0x64646464u;  // bytes -> halves 1024 + q
-      mma_16816(ta, __byte_perm(lo.x, M, 0x4140), __byte_perm(hi.x, M, 0x4140), __byte_perm(lo.x, M, 0x4342), __byte_perm(hi.x, M, 0x4342), x0.x, x0.y);
-      mma_16816(tb, __byte_perm(lo.y, M, 0x4140), __byte_perm(hi.y, M, 0x4140), __byte_perm(lo.y, M, 0x4342), __byte_perm(hi.y, M, 0x4342), x0.z, x0.w);
-      mma_16816(ta, __byte_perm(lo.z, M, 0x4140), __byte_perm(hi.z, M, 0x4140), __byte_perm(lo.z, M, 0x4342), __byte_perm(hi.z, M, 0x4342), x1.x, x1.y);
-      mma_16816(tb, __byte_perm(lo.w, M, 0x4140), __byte_perm(hi.w, M, 0x4140), __byte_perm(lo.w, M, 0x4342), __byte_perm(hi.w, M, 0x4342), x1.z, x1.w);
-      // only the diagonal entries (column == this lane's segment) are meaningful, and they share `corr`
-      const float sl = __half2float(sc_lo), sh = __half2float(sc_hi);
-      acc[0] += sl * ((ta[0] + tb[0]) - corr);
-      acc[1] += sl * ((ta[1] + tb[1]) - corr);
-      acc[2] += sh * ((ta[2] + tb[2]) - corr);
-      acc[3] += sh * ((ta[3] + tb[3]) - corr);
-    } else {
-      const __half2 s_lo = __half2half2(sc_lo), s_hi = __half2half2(sc_hi);
-      mma_16816(acc, dequant_pair(lo.x, 0x4140, s_lo), dequant_pair(hi.x, 0x4140, s_hi), dequant_pair(lo.x, 0x4342, s_lo),
-                dequant_pair(hi.x, 0x4342, s_hi), x0.x, x0.y);
-      mma_16816(acc_b, dequant_pair(lo.y, 0x4140, s_lo), dequant_pair(hi.y, 0x4140, s_hi), dequant_pair(lo.y, 0x4342, s_lo),
-                dequant_pair(hi.y, 0x4342, s_hi), x0.z, x0.w);
-      mma_16816(acc, dequant_pair(lo.z, 0x4140, s_lo), dequant_pair(hi.z, 0x4140, s_hi), dequant_pair(lo.z, 0x4342, s_lo),
-                dequant_pair(hi.z, 0x4342, s_hi), x1.x, x1.y);
-      mma_16816(acc_b, dequant_pair(lo.w, 0x4140, s_lo), dequant_pair(hi.w, 0x4140, s_hi), dequant_pair(lo.w, 0x4342, s_lo),
-                dequant_pair(hi.w, 0x4342, s_hi), x1.z, x1.w);
-    }
+    const __half2 s_lo = __half2half2(sc_lo), s_hi = __half2half2(sc_hi);
+    mma_16816(acc, dequant_pair(lo.x, 0x4140, s_lo), dequant_pair(hi.x, 0x4140, s_hi), dequant_pair(lo.x, 0x4342, s_lo),
+              dequant_pair(hi.x, 0x4342, s_hi), x0.x, x0.y);
+    mma_16816(acc_b, dequant_pair(lo.y, 0x4140, s_lo), dequant_pair(hi.y, 0x4140, s_hi), dequant_pair(lo.y, 0x4342, s_lo),
+              dequant_pair(hi.y, 0x4342, s_hi), x0.z, x0.w);
+    mma_16816(acc, dequant_pair(lo.z, 0x4140, s_lo), dequant_pair(hi.z, 0x4140, s_hi), dequant_pair(lo.z, 0x4342, s_lo),
+              dequant_pair(hi.z, 0x4342, s_hi), x1.x, x1.y);
+    mma_16816(acc_b, dequant_pair(lo.w, 0x4140, s_lo), dequant_pair(hi.w, 0x4140, s_hi), dequant_pair(lo.w, 0x4342, s_lo),
+              dequant_pair(hi.w, 0x4342, s_hi), x1.z, x1.w);
   }
 }
 
 // Factored u8, block size >= 128: the two 64-byte steps of a 128-weight block share their scale, so the eight
 // tensor-core products of both steps are summed before the one multiplication by the scale.
-template <bool FULL>
-__device__ __forceinline__ void step_pair_factored(float (&accs)[NACC][4], const int sp, const int flip, const int c, const int g, const int vb,
-                                                   const uint8_t* seg0, const uint8_t* xseg, const uint8_t* st, const float* xs64, const int ci,
-                                                   const int bs) {
-  constexpr int ROWB = geom<2>::ROWB, SEG = geom<2>::SEG, NSTEPS = geom<2>::NSTEPS;
-  constexpr int CHUNK_K = ROWB;
-  float* acc = accs[sp % NACC];
-  const uint32_t M = 0x64646464u;  // bytes -> halves 1024 + q
-  // a row's last chunk may be short; its length is a multiple of the block size, so a 128-byte pair is valid or not as a whole
-  const bool ok = FULL || (sp << 7) < vb;
-  // the correction term is the start value of one accumulator chain: sum - 1151.5 * sum(x) costs no instruction of its own
-  float negcorr = 0.f;
-  if (ok) {
-    const float2 xs2 = *reinterpret_cast<const float2*>(xs64 + ci * (CHUNK_K / 64) + g * NSTEPS + 2 * sp);
-    negcorr = -1151.5f * (xs2.x + xs2.y);
-  }
+struct factored_pair {
   float ta[4], tb[4];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int off = (((2 * sp + h) ^ flip) << 6) + c * 16;  // odd segments take the two steps in swapped order (bank spread)
-    uint4 lo = make_uint4(0, 0, 0, 0), hi = lo, x0 = lo, x1 = lo;
-    if (ok) {
-      lo = *reinterpret_cast<const uint4*>(seg0 + off);
-      hi = *reinterpret_cast<const uint4*>(seg0 + ROWB + off);
-      x0 = *reinterpret_cast<const uint4*>(xseg + 2 * off);
-      x1 = *reinterpret_cast<const uint4*>(xseg + 2 * off + 16);
-    }
+  // the correction term is the start value of one accumulator chain: sum - 1151.5 * sum(x) costs no instruction of its own
+  __device__ __forceinline__ void half_step(int h, const uint4& lo, const uint4& hi, const uint4& x0, const uint4& x1, float negcorr) {
+    const uint32_t M = 0x64646464u;  // bytes -> halves 1024 + q
     if (h == 0) {  // the block's first products start the two chains
       mma_16816_from(ta, __byte_perm(lo.x, M, 0x4140), __byte_perm(hi.x, M, 0x4140), __byte_perm(lo.x, M, 0x4342), __byte_perm(hi.x, M, 0x4342), x0.x, x0.y, negcorr);
       mma_16816_from(tb, __byte_perm(lo.y, M, 0x4140), __byte_perm(hi.y, M, 0x4140), __byte_perm(lo.y, M, 0x4342), __byte_perm(hi.y, M, 0x4342), x0.z, x0.w, 0.f);
@@ -205,14 +155,80 @@ __device__ __forceinline__ void step_pair_factored(float (&accs)[NACC][4], const
     mma_16816(ta, __byte_perm(lo.z, M, 0x4140), __byte_perm(hi.z, M, 0x4140), __byte_perm(lo.z, M, 0x4342), __byte_perm(hi.z, M, 0x4342), x1.x, x1.y);
     mma_16816(tb, __byte_perm(lo.w, M, 0x4140), __byte_perm(hi.w, M, 0x4140), __byte_perm(lo.w, M, 0x4342), __byte_perm(hi.w, M, 0x4342), x1.z, x1.w);
   }
+  __device__ __forceinline__ void add_to(float* acc, __half sc_lo, __half sc_hi) const {
+    const float sl = __half2float(sc_lo), sh = __half2float(sc_hi);
+    acc[0] += sl * (ta[0] + tb[0]);
+    acc[1] += sl * (ta[1] + tb[1]);
+    acc[2] += sh * (ta[2] + tb[2]);
+    acc[3] += sh * (ta[3] + tb[3]);
+  }
+};
+
+// The segment's sums of both rows, to all lanes of its quad: row 0 is in d0/d1, row 1 in d2/d3 of the quad's diagonal lane.
+__device__ __forceinline__ void segment_sums(const float (&accs)[NACC][4], int lane, float& s0, float& s1) {
+  const float a0 = (accs[0][0] + accs[1][0]) + (accs[2][0] + accs[3][0]), a1 = (accs[0][1] + accs[1][1]) + (accs[2][1] + accs[3][1]);
+  const float a2 = (accs[0][2] + accs[1][2]) + (accs[2][2] + accs[3][2]), a3 = (accs[0][3] + accs[1][3]) + (accs[2][3] + accs[3][3]);
+  const int g = lane >> 2, diag_lane = 4 * g + (g >> 1);
+  s0 = __shfl_sync(0xffffffffu, (g & 1) ? a1 : a0, diag_lane);
+  s1 = __shfl_sync(0xffffffffu, (g & 1) ? a3 : a2, diag_lane);
+}
+
+// The steps of a staged chunk.  Lanes of an odd segment take the steps of a pair in swapped order (bank spread); every place
+// that forms a row's sum takes them in this order, so the sum's bits do not depend on the kernel.
+template <int WT, bool FULL>
+__device__ __forceinline__ void staged_step(float (&accs)[NACC][4], const int s, const int flip, const int c, const int g, const int vb, const uint8_t* seg0,
+                                            const uint8_t* xseg, const uint8_t* st, const float* xs64, const int ci, const int bs) {
+  constexpr int ROWB = geom<WT>::ROWB, SEG = geom<WT>::SEG, NSTEPS = geom<WT>::NSTEPS, CHUNK_K = ROWB / (is16<WT> ? 2 : 1);
+  const int off = ((s ^ flip) << 6) + c * 16;  // byte offset inside the segment
+  uint4 lo = make_uint4(0, 0, 0, 0), hi = lo, x0 = lo, x1 = lo;
+  __half sc_lo = __ushort_as_half(0), sc_hi = sc_lo;
+  float xsum = 0.f;
+  if (FULL || off < vb) {
+    lo = *reinterpret_cast<const uint4*>(seg0 + off);
+    hi = *reinterpret_cast<const uint4*>(seg0 + ROWB + off);
+    if (is16<WT>) {
+      x0 = *reinterpret_cast<const uint4*>(xseg + off);
+    } else {
+      x0 = *reinterpret_cast<const uint4*>(xseg + 2 * off);
+      x1 = *reinterpret_cast<const uint4*>(xseg + 2 * off + 16);
+      const __half* scs = reinterpret_cast<const __half*>(st + 2 * ROWB);
+      const int si = (g * SEG + off) >> bs;  // k offset inside the chunk / block size (bs is log2 of it here)
+      sc_lo = scs[si];
+      sc_hi = scs[geom<WT>::SC_ROW / 2 + si];
+      // WT 2: sum of x over this lane's segment and step (the diagonal column of the tile)
+      if (WT == 2) xsum = xs64[ci * (CHUNK_K / 64) + g * NSTEPS + (s ^ flip)];
+    }
+  }
+  step<WT>(accs, s, lo, hi, x0, x1, sc_lo, sc_hi, xsum);
+}
+template <bool FULL>
+__device__ __forceinline__ void staged_step_pair(float (&accs)[NACC][4], const int sp, const int flip, const int c, const int g, const int vb,
+                                                 const uint8_t* seg0, const uint8_t* xseg, const uint8_t* st, const float* xs64, const int ci, const int bs) {
+  constexpr int ROWB = geom<2>::ROWB, SEG = geom<2>::SEG, NSTEPS = geom<2>::NSTEPS;
+  // a row's last chunk may be short; its length is a multiple of the block size, so a 128-byte pair is valid or not as a whole
+  const bool ok = FULL || (sp << 7) < vb;
+  float negcorr = 0.f;
+  if (ok) {
+    const float2 xs2 = *reinterpret_cast<const float2*>(xs64 + ci * (ROWB / 64) + g * NSTEPS + 2 * sp);
+    negcorr = -1151.5f * (xs2.x + xs2.y);
+  }
+  factored_pair f;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int off = (((2 * sp + h) ^ flip) << 6) + c * 16;
+    uint4 lo = make_uint4(0, 0, 0, 0), hi = lo, x0 = lo, x1 = lo;
+    if (ok) {
+      lo = *reinterpret_cast<const uint4*>(seg0 + off);
+      hi = *reinterpret_cast<const uint4*>(seg0 + ROWB + off);
+      x0 = *reinterpret_cast<const uint4*>(xseg + 2 * off);
+      x1 = *reinterpret_cast<const uint4*>(xseg + 2 * off + 16);
+    }
+    f.half_step(h, lo, hi, x0, x1, negcorr);
+  }
   if (!ok) return;  // (after the warp-wide tensor-core instructions)
   const __half* scs = reinterpret_cast<const __half*>(st + 2 * ROWB);
   const int si = (g * SEG + (sp << 7)) >> bs;
-  const float sl = __half2float(scs[si]), sh = __half2float(scs[geom<2>::SC_ROW / 2 + si]);
-  acc[0] += sl * (ta[0] + tb[0]);
-  acc[1] += sl * (ta[1] + tb[1]);
-  acc[2] += sh * (ta[2] + tb[2]);
-  acc[3] += sh * (ta[3] + tb[3]);
+  f.add_to(accs[sp % NACC], scs[si], scs[geom<2>::SC_ROW / 2 + si]);
 }
 
 // ---- the activation row: global -> shared memory, normalised, with the group sums of the factored u8 kernels.
@@ -263,7 +279,7 @@ __device__ __forceinline__ void row_sums8(const uint4& q, int i, int lane, float
 // it and form its group sums.  K is a multiple of 256, so a warp's 32 vectors are all inside the row or all outside.
 template <int WT>
 __device__ __forceinline__ void row_finish(const gemv_params& p, bool norm, uint8_t* xs, float* xs64, float* squares, int tid, int threads,
-                                           const uint4 (&nw)[ROW_VEC]) {
+                                           const uint4 (&nw)[ROW_VEC], float inv_k) {
   const int vec = p.K >> 3, lane = tid & 31;
   float rinv = 1.f;
   if (norm) {
@@ -273,9 +289,14 @@ __device__ __forceinline__ void row_finish(const gemv_params& p, bool norm, uint
       if (lane == 0) squares[i >> 5] = s;
     }
     bar_sync(1, threads);
+    // over the blocks: every run of `span` lanes adds up all of them, so every lane ends with the whole sum
+    const int blocks = vec >> 5, span = blocks >= 32 ? 32 : 1 << (32 - __clz(blocks - 1));
     float t = 0.f;
-    for (int b = lane; b < vec >> 5; b += 32) t += squares[b];
-    rinv = rsqrtf(warp_sum(t) / p.K + p.eps);
+    for (int b = lane & (span - 1); b < blocks; b += 32) t += squares[b];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      if (o < span) t += __shfl_xor_sync(0xffffffffu, t, o);
+    rinv = rsqrtf(t * inv_k + p.eps);
   }
   auto finish = [&](int i, const uint4& w) {
     uint4 q = *reinterpret_cast<const uint4*>(xs + row_offset<WT>(i));
@@ -285,7 +306,9 @@ __device__ __forceinline__ void row_finish(const gemv_params& p, bool norm, uint
     }
     if (WT == 2) row_sums8(q, i, lane, xs64);
   };
-  if (norm) {
+  if (norm && vec <= threads) {  // (a path of its own: skipping code costs its fetch)
+    if (tid < vec) finish(tid, nw[0]);
+  } else if (norm) {
 #pragma unroll
     for (int j = 0; j < ROW_VEC; ++j)
       if (tid + j * threads < vec) finish(tid + j * threads, nw[j]);
@@ -296,6 +319,81 @@ __device__ __forceinline__ void row_finish(const gemv_params& p, bool norm, uint
     for (int i = tid; i < vec; i += threads) finish(i, nw[0]);
   }
   bar_sync(1, threads);
+}
+
+__device__ __forceinline__ uint4 ld_stream(const void* at) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(at));
+  return v;
+}
+
+// ---- what becomes of a row pair's two sums
+struct pair_operands {  // what the epilogue reads from global memory, and where its results go
+  __half2 prev;
+  float2 cs;
+  int mat, row, head, j;
+  template <int WT, int EPI>
+  __device__ __forceinline__ void fetch(const gemv_params& p, int pr, int pos) {
+    prev = __half2half2(__ushort_as_half(0));
+    cs = make_float2(1.f, 0.f);
+    if (EPI == EPI_PLAIN) {
+      if (WT != 3 && p.beta != 0.f) prev = *reinterpret_cast<const __half2*>(p.out + 2 * pr);
+    } else if (EPI == EPI_ROPE_KV) {
+      map_row<EPI_ROPE_KV>(p, 2 * pr, mat, row);
+      head = row / p.head_dim;
+      j = row - head * p.head_dim;
+      if (mat < 2) cs = p.rope[(size_t)pos * (p.head_dim >> 1) + (j >> 1)];
+    }
+  }
+};
+template <int WT, int EPI>
+__device__ __forceinline__ void store_pair(const gemv_params& p, const gemv_batch& bt, int bi, const pair_operands& po, int pr, float v0, float v1, int pos,
+                                           float gate_scale) {
+  const int vrow = 2 * pr;
+  if (WT == 3) {
+    if (EPI == EPI_PLAIN) {
+      if (bt.f32[bi]) *reinterpret_cast<float2*>(reinterpret_cast<float*>(bt.out[bi]) + vrow) = make_float2(v0, v1);
+      else *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(bt.out[bi]) + vrow) = __floats2bfloat162_rn(v0, v1);
+    } else {  // the gate on the binary32 sums
+      __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(bt.n > 0 ? bt.out[bi] : p.out);
+      const float z = gate_scale * v0;
+      o[pr] = __float2bfloat16(z / (1.0f + expf(-z)) * (gate_scale * v1));
+    }
+  } else if (EPI == EPI_PLAIN) {
+    float a0 = v0, a1 = v1;
+    __half* o = p.out + vrow;
+    if (p.beta != 0.f) {
+      a0 = a0 + p.beta * __low2float(po.prev);
+      a1 = a1 + p.beta * __high2float(po.prev);
+    }
+    const __half2 r2 = __halves2half2(__float2half(a0), __float2half(a1));
+    *reinterpret_cast<__half2*>(o) = r2;
+    if (p.out_peer) *reinterpret_cast<__half2*>(p.out_peer + vrow) = r2;  // peer store over NVLink
+    for (int q = 0; q < p.n_peer_out; ++q) *reinterpret_cast<__half2*>(p.peer_out[q] + vrow) = r2;  // tensor-parallel: into every GPU's row
+  } else {
+    const __half a = __float2half(v0), bq = __float2half(v1);  // the matmul's own output rounding
+    if (EPI == EPI_SILU) {
+      const float val = __half2float(a);  // llama_cu.cu:536-537 on the half-rounded w1 / w3 outputs
+      const __half gated = __float2half(val / (1.0f + expf(-val)) * __half2float(bq));
+      p.out[pr] = gated;
+      for (int q = 0; q < p.n_peer_out; ++q) p.peer_out[q][pr] = gated;
+    } else {
+      __half o0 = a, o1 = bq;
+      if (po.mat < 2) {  // llama_cu.cu:381-387, cos/sin from the context's table
+        const float real = __half2float(a), imag = __half2float(bq);
+        const float a_cos = po.cs.x, a_sin = po.cs.y;
+        o0 = __float2half(real * a_cos - imag * a_sin);
+        o1 = __float2half(real * a_sin + imag * a_cos);
+      }
+      const __half2 pr2 = __halves2half2(o0, o1);
+      if (po.mat == 0) {
+        *reinterpret_cast<__half2*>(p.q_out + po.row) = pr2;
+      } else {
+        __half* cache = po.mat == 1 ? p.k_cache : p.v_cache;
+        *reinterpret_cast<__half2*>(cache + ((size_t)po.head * p.ctx_len + pos) * p.head_dim + po.j) = pr2;
+      }
+    }
+  }
 }
 
 // Weight types (WT): 0 = fp16; 1 = u8, every weight rounded to half((q - 127.5) * scale) before the
@@ -465,6 +563,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
   const int vec = p.K >> 3;
   const bool norm = WT != 3 && p.norm_w != nullptr;
   uint4 nw[ROW_VEC];
+  const float inv_k = 1.0f / p.K;
   if (norm) {
 #pragma unroll
     for (int j = 0; j < ROW_VEC; ++j)
@@ -505,7 +604,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
       }
       mbar_wait(xbar, 0, p.err, DEV_ERR_FULL_WAIT);
     }
-    row_finish<WT>(p, norm, xs, xs64, squares, tid, NCONS, nw);
+    row_finish<WT>(p, norm, xs, xs64, squares, tid, NCONS, nw, inv_k);
   }
 
   const int g = lane >> 2, c = lane & 3;
@@ -515,26 +614,13 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
   // quad's lane c keeps those of the batch's pair c, so that one tree over the segments and one epilogue (lanes 0 .. 3, a
   // pair each) serve four pairs.  A tree and an epilogue per pair were 900 of the 2900 cycles a pair of 4096 u8 weights took.
   constexpr int BATCH = 4;
-  const int diag_lane = 4 * g + (g >> 1);
   int slot = 0;
   uint32_t par = 0;
   for (int i0 = warp; i0 < npairs; i0 += BATCH * NW) {
-    // what the epilogue reads from global memory is requested ahead of the products
-    const int i = i0 + c * NW, vrow = 2 * (pr0 + i);
+    const int i = i0 + c * NW;
     const bool mine = g == 0 && i < npairs;
-    __half2 prev = __half2half2(__ushort_as_half(0));
-    float2 cs = make_float2(1.f, 0.f);
-    int mat = 0, row = vrow, head = 0, j = 0;
-    if (mine) {
-      if (EPI == EPI_PLAIN) {
-        if (WT != 3 && p.beta != 0.f) prev = *reinterpret_cast<const __half2*>(p.out + vrow);
-      } else if (EPI == EPI_ROPE_KV) {
-        map_row<EPI_ROPE_KV>(p, vrow, mat, row);
-        head = row / p.head_dim;
-        j = row - head * p.head_dim;
-        if (mat < 2) cs = p.rope[(size_t)pos * (p.head_dim >> 1) + (j >> 1)];
-      }
-    }
+    pair_operands po;  // requested ahead of the products
+    if (mine) po.fetch<WT, EPI>(p, pr0 + i, pos);
     float v0 = 0.f, v1 = 0.f;
 #pragma unroll 1
     for (int k = 0; k < BATCH && i0 + k * NW < npairs; ++k) {
@@ -552,16 +638,16 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
         // shared loads of all eight steps can be issued ahead of the tensor-core instructions.
         if (WT == 2 && cbytes == ROWB && bs_shift >= 7) {
 #pragma unroll
-          for (int sp = 0; sp < NSTEPS / 2; ++sp) step_pair_factored<true>(accs, sp, flip, c, g, SEG, seg0, xseg, st, xs64, ci, bs_shift);
+          for (int sp = 0; sp < NSTEPS / 2; ++sp) staged_step_pair<true>(accs, sp, flip, c, g, SEG, seg0, xseg, st, xs64, ci, bs_shift);
         } else if (WT == 2 && bs_shift >= 7) {
 #pragma unroll
-          for (int sp = 0; sp < NSTEPS / 2; ++sp) step_pair_factored<false>(accs, sp, flip, c, g, vb, seg0, xseg, st, xs64, ci, bs_shift);
+          for (int sp = 0; sp < NSTEPS / 2; ++sp) staged_step_pair<false>(accs, sp, flip, c, g, vb, seg0, xseg, st, xs64, ci, bs_shift);
         } else if (cbytes == ROWB) {
 #pragma unroll
-          for (int s = 0; s < NSTEPS; ++s) step<WT, true>(accs, s, flip, c, g, SEG, seg0, xseg, st, xs64, ci, bs_shift);
+          for (int s = 0; s < NSTEPS; ++s) staged_step<WT, true>(accs, s, flip, c, g, SEG, seg0, xseg, st, xs64, ci, bs_shift);
         } else {
 #pragma unroll
-          for (int s = 0; s < NSTEPS; ++s) step<WT, false>(accs, s, flip, c, g, vb, seg0, xseg, st, xs64, ci, bs_shift);
+          for (int s = 0; s < NSTEPS; ++s) staged_step<WT, false>(accs, s, flip, c, g, vb, seg0, xseg, st, xs64, ci, bs_shift);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bars[EMPTY_BASE + warp * MAX_SW + slot]));
@@ -570,11 +656,8 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
           par ^= 1;
         }
       }
-      // segment g of row 0 is in d0/d1, of row 1 in d2/d3 of the quad's diagonal lane
-      const float a0 = (accs[0][0] + accs[1][0]) + (accs[2][0] + accs[3][0]), a1 = (accs[0][1] + accs[1][1]) + (accs[2][1] + accs[3][1]);
-      const float a2 = (accs[0][2] + accs[1][2]) + (accs[2][2] + accs[3][2]), a3 = (accs[0][3] + accs[1][3]) + (accs[2][3] + accs[3][3]);
-      const float s0 = __shfl_sync(0xffffffffu, (g & 1) ? a1 : a0, diag_lane);
-      const float s1 = __shfl_sync(0xffffffffu, (g & 1) ? a3 : a2, diag_lane);
+      float s0, s1;
+      segment_sums(accs, lane, s0, s1);
       if (c == k) {
         v0 = s0;
         v1 = s1;
@@ -585,53 +668,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
       v0 += __shfl_xor_sync(0xffffffffu, v0, o);
       v1 += __shfl_xor_sync(0xffffffffu, v1, o);
     }
-    if (mine) {
-      const int pr = pr0 + i;
-      if (WT == 3) {
-        if (EPI == EPI_PLAIN) {
-          if (bt.f32[bi]) *reinterpret_cast<float2*>(reinterpret_cast<float*>(bt.out[bi]) + vrow) = make_float2(v0, v1);
-          else *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(bt.out[bi]) + vrow) = __floats2bfloat162_rn(v0, v1);
-        } else {  // the gate on the binary32 sums
-          __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(bt.n > 0 ? bt.out[bi] : p.out);
-          const float z = gate_scale * v0;
-          o[pr] = __float2bfloat16(z / (1.0f + expf(-z)) * (gate_scale * v1));
-        }
-      } else if (EPI == EPI_PLAIN) {
-        float a0 = v0, a1 = v1;
-        __half* o = p.out + vrow;
-        if (p.beta != 0.f) {
-          a0 = a0 + p.beta * __low2float(prev);
-          a1 = a1 + p.beta * __high2float(prev);
-        }
-        const __half2 r2 = __halves2half2(__float2half(a0), __float2half(a1));
-        *reinterpret_cast<__half2*>(o) = r2;
-        if (p.out_peer) *reinterpret_cast<__half2*>(p.out_peer + vrow) = r2;  // peer store over NVLink
-        for (int q = 0; q < p.n_peer_out; ++q) *reinterpret_cast<__half2*>(p.peer_out[q] + vrow) = r2;  // tensor-parallel: into every GPU's row
-      } else {
-        const __half a = __float2half(v0), bq = __float2half(v1);  // the matmul's own output rounding
-        if (EPI == EPI_SILU) {
-          const float val = __half2float(a);  // llama_cu.cu:536-537 on the half-rounded w1 / w3 outputs
-          const __half gated = __float2half(val / (1.0f + expf(-val)) * __half2float(bq));
-          p.out[pr] = gated;
-          for (int q = 0; q < p.n_peer_out; ++q) p.peer_out[q][pr] = gated;
-        } else {
-          __half o0 = a, o1 = bq;
-          if (mat < 2) {  // llama_cu.cu:381-387, cos/sin from the context's table (fetched above)
-            const float real = __half2float(a), imag = __half2float(bq);
-            const float a_cos = cs.x, a_sin = cs.y;
-            o0 = __float2half(real * a_cos - imag * a_sin);
-            o1 = __float2half(real * a_sin + imag * a_cos);
-          }
-          const __half2 pr2 = __halves2half2(o0, o1);
-          if (mat == 0) {
-            *reinterpret_cast<__half2*>(p.q_out + row) = pr2;
-          } else {
-            __half* cache = mat == 1 ? p.k_cache : p.v_cache;
-            *reinterpret_cast<__half2*>(cache + ((size_t)head * p.ctx_len + pos) * p.head_dim + j) = pr2;
-          }
-        }
-      }
-    }
+    if (mine) store_pair<WT, EPI>(p, bt, bi, po, pr0 + i, v0, v1, pos, gate_scale);
   }
   // tensor-parallel: the last consumer warp of the launch to get here publishes this GPU's slice (every result went into
   // the other GPUs' rows as a peer store in the epilogue above, made by the warp's first lanes).  The fences widen with the
@@ -652,6 +689,155 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
       }
     }
   }
+}
+
+// ---- small matrices: a launch's whole share of the weights is held in registers.
+//
+// A launch over a few megabytes is as long as its chain of dependent steps, not as its bytes: with a ring, CTAs start when the
+// kernel before them gives its shared memory back, set barriers up, wait for their first stage and run two or three row pairs one
+// after the other.  Here a warp requests the one row pair it owns (two pairs where rows fit half a chunk: DUAL) straight into
+// registers as its first act; a CTA needs shared memory for the activation row only, so CTAs start while the kernels before them
+// run, and what follows the wait is the row, one pass of products, one tree, one store: 1.0 us without a norm, 1.6 with one (1024
+// wide).  Rows of NCH chunks of 4 KiB.  Sums are formed in the order of the ring's kernel: the same bits.  Decode step, ring ->
+// held, us: 512 wide, 4 layers, 95 -> 72; 1024 wide, 8 layers, 184 -> 143, with u8 weights 232 -> 176; 2048 wide, 8 layers, 245 -> 235,
+// u8 294 -> 286; Zibovik 1024 wide, 8 layers, 304 -> 278.
+template <int NCH>
+constexpr int held_warps = NCH == 1 ? 8 : 4;  // most warps of a CTA (64 NCH registers of weights per thread)
+
+template <int WT, int EPI, int NCH, bool DUAL>
+__global__ void __launch_bounds__(held_warps<NCH> * 32, NCH == 1 ? 2 : 3) gemv_held_kernel(const gemv_params p, const __grid_constant__ gemv_batch bt) {
+  constexpr int ESZ = is16<WT> ? 2 : 1, ROWB = geom<WT>::ROWB, SEG = geom<WT>::SEG, NSTEPS = geom<WT>::NSTEPS, CHUNK_K = ROWB / ESZ;
+  static_assert(!DUAL || NCH == 1, "two pairs share one chunk");
+  extern __shared__ __align__(128) uint8_t xs[];  // activation row (row_layout)
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, threads = blockDim.x;
+  const int g = lane >> 2, c = lane & 3, flip = g & 1, seg = DUAL ? g & 3 : g;
+  if (WT != 3 || !bt.hold) pdl_launch_dependents();
+
+  int pairs = (p.n_mats * p.rows_per_mat) >> 1, cta = blockIdx.x, bi = 0;
+  if (WT == 3 && bt.n > 0) {  // which of the batch's matrices this CTA works on
+    while (bi + 1 < bt.n && (int)blockIdx.x >= bt.first_cta[bi + 1]) ++bi;
+    cta = blockIdx.x - bt.first_cta[bi];
+    pairs = bt.rows[bi] >> 1;
+  }
+  const int unit = cta * (threads >> 5) + warp, pr = DUAL ? 2 * unit + (g >> 2) : unit;
+  const bool live = pr < pairs;
+  size_t picked = 0;
+  if (WT == 3 && bt.choice != nullptr) {
+    if (!bt.choice_settled) pdl_wait();
+    picked = (size_t)bt.choice[bi] * bt.choice_bytes;
+  }
+  const int rowbytes = p.K * ESZ, shift = is16<WT> ? 0 : 31 - __clz(p.bs);
+  uint4 lo[NCH][NSTEPS], hi[NCH][NSTEPS];  // zero past the row's end
+  uint32_t sc[WT == 2 ? NCH : 1][2][4];    // scales of the lane's segment: with blocks of 64 eight per chunk and row, of 128 four
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    int mat, row;
+    map_row<EPI>(p, 2 * (live ? pr : pairs - 1) + r, mat, row);
+    int place = row;
+    if (WT == 3 && EPI == EPI_SILU && bt.n > 0) place = ((row >> bt.gate_shift) << (bt.gate_shift + 1)) + (mat << bt.gate_shift) + (row & ((1 << bt.gate_shift) - 1));
+    const uint8_t* w = reinterpret_cast<const uint8_t*>(WT == 3 && bt.n > 0 ? bt.w[bi] : p.w[mat]) + (WT == 3 ? picked : 0) + (size_t)place * rowbytes + c * 16;
+#pragma unroll
+    for (int ci = 0; ci < NCH; ++ci) {
+      const uint8_t* at = w + ci * ROWB + seg * SEG;
+      const int vb = rowbytes - ci * ROWB - seg * SEG - c * 16;  // valid bytes from the lane's first on
+#pragma unroll
+      for (int s = 0; s < NSTEPS; ++s) {
+        const int off = (s ^ flip) << 6;
+        (r ? hi : lo)[ci][s] = make_uint4(0, 0, 0, 0);
+        if (off < vb) (r ? hi : lo)[ci][s] = ld_stream(at + off);
+      }
+      if (WT == 2) {  // (rows are multiples of 256 weights: two scales travel together)
+        const int per = SEG >> shift, first = (ci * ROWB + seg * SEG) >> shift;
+        const __half* scs = p.sc[mat] + (size_t)row * (p.K >> shift) + first;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) sc[ci][r][h] = 2 * h < per && first + 2 * h < (p.K >> shift) ? *reinterpret_cast<const uint32_t*>(scs + 2 * h) : 0;
+      }
+    }
+  }
+  const bool norm = WT != 3 && p.norm_w != nullptr;
+  const row_layout rl = row_layout_of<WT>(p.K, norm);
+  float* xs64 = reinterpret_cast<float*>(xs + rl.sums);
+  const int vec = p.K >> 3;
+  const float inv_k = 1.0f / p.K;
+  uint4 nw[ROW_VEC];
+  if (norm) {
+#pragma unroll
+    for (int j = 0; j < ROW_VEC; ++j)
+      if (tid + j * threads < vec) nw[j] = *reinterpret_cast<const uint4*>(p.norm_w + (tid + j * threads) * 8);
+  }
+  pdl_wait();
+  if (WT == 3 && bt.hold) pdl_launch_dependents();
+  const float gate_scale = WT == 3 && EPI == EPI_SILU && bt.n > 0 ? bt.gate_scale[bi] : 1.0f;
+  const int pos = EPI == EPI_ROPE_KV ? *p.pos : 0;
+  const __half* x_row = WT == 3 && EPI == EPI_PLAIN ? reinterpret_cast<const __half*>(bt.x[bi]) : p.x;
+  auto x_at = [&](int i) { return __ldcg(reinterpret_cast<const uint4*>(x_row + i * 8)); };
+  auto x_put = [&](int i, const uint4& v) { *reinterpret_cast<uint4*>(xs + row_offset<WT>(i)) = v; };
+  if (vec <= threads) {
+    if (tid < vec) x_put(tid, x_at(tid));
+  } else {
+    uint4 xv[ROW_VEC];
+#pragma unroll
+    for (int j = 0; j < ROW_VEC; ++j)
+      if (tid + j * threads < vec) xv[j] = x_at(tid + j * threads);
+#pragma unroll
+    for (int j = 0; j < ROW_VEC; ++j)
+      if (tid + j * threads < vec) x_put(tid + j * threads, xv[j]);
+  }
+  const bool mine = live && (DUAL ? (lane & 15) == 0 : lane == 0);
+  pair_operands po;
+  if (mine) po.fetch<WT, EPI>(p, pr, pos);
+  row_finish<WT>(p, norm, xs, xs64, reinterpret_cast<float*>(xs + rl.squares), tid, threads, nw, inv_k);
+
+  float accs[NACC][4];
+#pragma unroll
+  for (int a = 0; a < NACC; ++a) accs[a][0] = accs[a][1] = accs[a][2] = accs[a][3] = 0.f;
+#pragma unroll
+  for (int ci = 0; ci < NCH; ++ci) {
+    const uint8_t* xseg = xs + row_offset<WT>((ci * CHUNK_K + seg * (SEG / ESZ)) >> 3);
+    const int vb = rowbytes - ci * ROWB - seg * SEG;
+    auto x_of = [&](int s, uint4& x0, uint4& x1) {
+      const int off = ((s ^ flip) << 6) + c * 16;
+      x0 = x1 = make_uint4(0, 0, 0, 0);
+      if (ci + 1 < NCH || off < vb) {
+        x0 = *reinterpret_cast<const uint4*>(xseg + (is16<WT> ? off : 2 * off));
+        if (!is16<WT>) x1 = *reinterpret_cast<const uint4*>(xseg + 2 * off + 16);
+      }
+    };
+    const float* sums = xs64 + ci * (CHUNK_K / 64) + seg * NSTEPS;
+    if (WT == 2 && shift >= 7) {
+#pragma unroll
+      for (int sp = 0; sp < NSTEPS / 2; ++sp) {
+        const bool ok = ci + 1 < NCH || (sp << 7) < vb;
+        const float negcorr = ok ? -1151.5f * (sums[2 * sp] + sums[2 * sp + 1]) : 0.f;
+        factored_pair f;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint4 x0, x1;
+          x_of(2 * sp + h, x0, x1);
+          f.half_step(h, lo[ci][2 * sp + h], hi[ci][2 * sp + h], x0, x1, negcorr);
+        }
+        auto pick = [&](int r) { return __ushort_as_half((unsigned short)(sc[ci][r][sp >> 1] >> (16 * (sp & 1)))); };
+        if (ok) f.add_to(accs[sp % NACC], pick(0), pick(1));
+      }
+    } else {
+#pragma unroll
+      for (int s = 0; s < NSTEPS; ++s) {
+        uint4 x0, x1;
+        x_of(s, x0, x1);
+        const bool ok = ci + 1 < NCH || ((s ^ flip) << 6) < vb;
+        auto pick = [&](int r) { return __ushort_as_half((unsigned short)(WT == 2 ? sc[ci][r][s >> 1] >> (16 * ((s ^ flip) & 1)) : 0)); };
+        step<WT>(accs, s, lo[ci][s], hi[ci][s], x0, x1, pick(0), pick(1), WT == 2 && ok ? sums[s ^ flip] : 0.f);
+      }
+    }
+  }
+  float v0, v1;
+  segment_sums(accs, lane, v0, v1);
+#pragma unroll
+  for (int o = DUAL ? 8 : 16; o >= 4; o >>= 1) {  // (DUAL: a row's upper four segments are empty)
+    v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+    v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+  }
+  if (mine) store_pair<WT, EPI>(p, bt, bi, po, pr, v0, v1, pos, gate_scale);
 }
 
 template <int WT, int EPI, int NW>
@@ -675,6 +861,62 @@ int launch_one(const gemv_params& p, cudaStream_t stream, int pdl, size_t smem, 
   cfg.numAttrs = pdl ? 1 : 0;
   LCU_CUDA(cudaLaunchKernelEx(&cfg, gemv1_kernel<WT, EPI, NW>, p, sw, pf_bytes, bt));
   return LCU_OK;
+}
+
+template <int WT, int EPI, int NCH, bool DUAL>
+int launch_held_shape(const gemv_params& p, cudaStream_t stream, int pdl, int warps, int grid, const gemv_batch& bt) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(warps * 32);
+  cfg.dynamicSmemBytes = row_layout_of<WT>(p.K, WT != 3 && p.norm_w != nullptr).total;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  LCU_CUDA(cudaLaunchKernelEx(&cfg, gemv_held_kernel<WT, EPI, NCH, DUAL>, p, bt));
+  return LCU_OK;
+}
+
+// Whether a launch's weights are held in registers, and its shape.
+struct held_plan {
+  int chunks = 0, warps = 0, grid = 0;  // chunks 0: no
+  bool dual = false;
+};
+int g_held_mode = -1;  // -1 = by the rule, 0 = never
+// At most twelve warps per SM, one wave beside the kernels around it (4096 wide u8, 13.8 for wo: 2 % slower held).  Rows: a launch
+// between ring kernels gains nothing, so lengths stop where a model's other launches are too large - bfloat16 rows of 4 KiB
+// (Filulix, 2048 wide) 185 -> 188 us, rows of two chunks of 1536 wide fp16 (8 KiB) 152 -> 173, where 1024 wide ones (5.5 KiB), whose
+// step is held as a whole, gain 156 -> 143.  Tensor-parallel launches stay on the ring.
+constexpr int HELD_WARPS_PER_SM = 12;
+template <class PairsOf>
+held_plan plan_held(int wt, int epi, const gemv_params& p, int n, PairsOf pairs_of, int sms) {
+  held_plan h;
+  if (g_held_mode == 0 || wt == 1 || (wt == 2 && p.bs != 64 && p.bs != 128) || p.n_wait > 0 || p.done_count != nullptr || p.n_peer_out > 0) return h;
+  const int rowbytes = p.K * (wt == 2 ? 1 : 2), chunks = (rowbytes + 4095) / 4096;
+  if (rowbytes > (wt == 3 ? 3072 : epi == EPI_PLAIN ? 6144 : 4096)) return h;
+  long long single = 0, two = 0;
+  for (int i = 0; i < n; ++i) {
+    single += pairs_of(i);
+    two += (pairs_of(i) + 1) / 2;
+  }
+  h.dual = rowbytes <= 2048 && single > 4 * sms;
+  const long long units = h.dual ? two : single;
+  if (units > HELD_WARPS_PER_SM * sms) return h;
+  h.warps = std::max(((int)units + sms - 1) / sms, p.norm_w ? 4 : 2);
+  h.warps = std::max(std::min(h.warps, chunks == 1 ? held_warps<1> : held_warps<2>), (p.K / 8 + ROW_VEC * 32 - 1) / (ROW_VEC * 32));
+  if (h.warps > (chunks == 1 ? held_warps<1> : held_warps<2>)) return h;  // (a thread holds ROW_VEC vectors of the row)
+  for (int i = 0; i < n; ++i) h.grid += ((h.dual ? (pairs_of(i) + 1) / 2 : pairs_of(i)) + h.warps - 1) / h.warps;
+  h.chunks = chunks;
+  return h;
+}
+template <int WT, int EPI>
+int launch_held(const held_plan& h, const gemv_params& p, cudaStream_t stream, int pdl, const gemv_batch& bt = gemv_batch{}) {
+  if (h.dual) return launch_held_shape<WT, EPI, 1, true>(p, stream, pdl, h.warps, h.grid, bt);
+  if constexpr (EPI == EPI_PLAIN && WT != 3)
+    if (h.chunks == 2) return launch_held_shape<WT, EPI, 2, false>(p, stream, pdl, h.warps, h.grid, bt);
+  return launch_held_shape<WT, EPI, 1, false>(p, stream, pdl, h.warps, h.grid, bt);
 }
 
 }  // namespace
@@ -719,6 +961,8 @@ int configure(const gemv_params& p, int sms, gemv1_config& c) {
 }
 }  // namespace
 
+void gemv_held_mode(int mode) { g_held_mode = mode; }
+
 // Loads every single-row kernel on the current device (the CUDA runtime loads a kernel at its first use; a first decode
 // step whose launches stall one after the other in that loading would leave the other GPUs of a tensor-parallel step
 // waiting far longer than their bounded waits allow).
@@ -749,6 +993,17 @@ int launch_gemv_single_row(const gemv_params& p, int epilogue, cudaStream_t stre
   if (rc) return rc;
   const int wt = c.wt, nw = c.nw, sw = c.sw, grid = c.grid, pf = c.pf;
   const size_t smem = c.smem;
+  const held_plan h = plan_held(wt, epilogue, p, 1, [&](int) { return p.n_mats * p.rows_per_mat / 2; }, sms);
+  if (h.chunks) {
+#define LCU_HELD_CASE(E) \
+  case E: return wt == 0 ? launch_held<0, E>(h, p, stream, pdl) : launch_held<2, E>(h, p, stream, pdl);
+    switch (epilogue) {
+      LCU_HELD_CASE(EPI_PLAIN)
+      LCU_HELD_CASE(EPI_ROPE_KV)
+      LCU_HELD_CASE(EPI_SILU)
+    }
+#undef LCU_HELD_CASE
+  }
 #define LCU_GEMV1_CASE(E)                                                                  \
   case E:                                                                                  \
     if (wt == 0) return launch_one<0, E, 4>(p, stream, pdl, smem, grid, sw, pf);           \
@@ -779,11 +1034,17 @@ int launch_gemv_bf16(const gemv_batch& b, int K, int* err, cudaStream_t stream, 
   p.K = K;
   p.m = 1;
   p.err = err;
+  gemv_batch bt = b;
+  const held_plan h = plan_held(3, EPI_PLAIN, p, b.n, [&](int i) { return b.rows[i] / 2; }, gemv_sm_count());
+  if (h.chunks) {
+    bt.first_cta[0] = 0;
+    for (int i = 0; i < b.n; ++i) bt.first_cta[i + 1] = bt.first_cta[i] + ((h.dual ? (b.rows[i] / 2 + 1) / 2 : b.rows[i] / 2) + h.warps - 1) / h.warps;
+    return launch_held<3, EPI_PLAIN>(h, p, stream, pdl, bt);
+  }
   gemv1_config c;
   int rc = configure(p, gemv_sm_count(), c);
   if (rc) return rc;
   // CTAs are dealt to the matrices in proportion to their rows, at least one each
-  gemv_batch bt = b;
   const int spare = c.grid > b.n ? c.grid - b.n : 0;
   long long seen = 0;
   for (int i = 0; i < b.n; ++i) {
@@ -807,6 +1068,8 @@ int launch_gemv_bf16_gated(void* out, const void* x, const void* w13, int f, int
   p.x = reinterpret_cast<const __half*>(x);
   p.out = reinterpret_cast<__half*>(out);
   p.err = err;
+  const held_plan h = plan_held(3, EPI_SILU, p, 1, [&](int) { return f; }, gemv_sm_count());
+  if (h.chunks) return launch_held<3, EPI_SILU>(h, p, stream, pdl);
   gemv1_config c;
   int rc = configure(p, gemv_sm_count(), c);
   if (rc) return rc;
@@ -825,16 +1088,21 @@ int launch_gemv_bf16_gated_picked(const gemv_batch& b, int f, int K, int* err, c
   p.m = 1;
   p.x = reinterpret_cast<const __half*>(b.x[0]);
   p.err = err;
-  gemv1_config c;
-  int rc = configure(p, gemv_sm_count(), c);
-  if (rc) return rc;
   gemv_batch bt = b;
-  const int per = std::max(1, c.grid / b.n);  // every matrix the same share of the CTAs
-  for (int i = 0; i <= b.n; ++i) bt.first_cta[i] = i * per;
   for (int i = 0; i < b.n; ++i) {
     bt.w[i] = b.w[0];
     bt.rows[i] = 2 * f;
   }
+  const held_plan h = plan_held(3, EPI_SILU, p, b.n, [&](int) { return f; }, gemv_sm_count());
+  if (h.chunks) {
+    for (int i = 0; i <= b.n; ++i) bt.first_cta[i] = i * (h.grid / b.n);
+    return launch_held<3, EPI_SILU>(h, p, stream, pdl, bt);
+  }
+  gemv1_config c;
+  int rc = configure(p, gemv_sm_count(), c);
+  if (rc) return rc;
+  const int per = std::max(1, c.grid / b.n);  // every matrix the same share of the CTAs
+  for (int i = 0; i <= b.n; ++i) bt.first_cta[i] = i * per;
   return launch_one<3, EPI_SILU, 4>(p, stream, pdl, c.smem, per * b.n, c.sw, c.pf, bt);
 }
 
