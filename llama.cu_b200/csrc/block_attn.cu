@@ -39,7 +39,7 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 
 // HK, HV: columns of the key (both parts) and value tiles
 template <int HK, int HV>
-__global__ void __launch_bounds__(WA_THREADS, HK == 64 ? 4 : HK == 128 ? 3 : 2) window_mma_kernel(const attn_rows<__nv_bfloat16> p, int m, int pos0) {
+__global__ void __launch_bounds__(WA_THREADS, HK == 64 ? 4 : 2) window_mma_kernel(const attn_rows<__nv_bfloat16> p, int m, int pos0) {
   using T = __nv_bfloat16;
   constexpr int LDK = HK + 8, LDV = HV + 8, STAGE = WA_K * (LDK + LDV), CK = HK / 8, CV = HV / 8;
   extern __shared__ __align__(16) T wa_smem[];  // [2 stages][keys | values]
@@ -93,6 +93,13 @@ __global__ void __launch_bounds__(WA_THREADS, HK == 64 ? 4 : HK == 128 ? 3 : 2) 
   const int win_lo = pos_lo + 1 - p.window, win_hi = pos_hi + 1 - p.window;  // first token of the window (may be negative)
   const int warp_first = pos0 + q0 + warp * 16, warp_last = warp_first + 15;
 
+  // A tile's copies: four neighbouring threads take 64 bytes of a row at a time, and a thread's columns are the same in every tile,
+  // so that a row costs its addresses once and a copy an offset.  (With row and column from a running index the staging took
+  // 700 of the 1590 instructions a warp spends on a tile of 192 + 128 columns, and this kernel is bound by their issue and latency.
+  // Prompts of 2000 tokens, with the scale in the exponent's product and outputs rescaled only when a maximum moves: Zibovik 2048 wide
+  // 1.69 -> 1.57 ms, Filulix 1024 wide 2.07 -> 1.97; 128 columns with three CTAs per SM, 168 registers and spills: 2.05.)
+  const int quad_col = (tid & 3) * 8, row0 = tid >> 2;
+  constexpr int ROWS_AT_ONCE = WA_THREADS / 4;
   auto stage_tile = [&](int tile, int stage) {
     T* ks = wa_smem + (size_t)stage * STAGE;
     T* vs = ks + WA_K * LDK;
@@ -100,20 +107,25 @@ __global__ void __launch_bounds__(WA_THREADS, HK == 64 ? 4 : HK == 128 ? 3 : 2) 
     const int t0 = pooled ? tile * WA_K : lo + (tile - pool_tiles) * WA_K, end = pooled ? n_blocks : last_pos + 1;
     const T *kb = pooled ? kp : kc, *vb = pooled ? vp : vc;
     const int shift = pooled ? 0 : p.cache.first;
-    for (int i = tid; i < WA_K * CK; i += WA_THREADS) {
-      const int r = i / CK, ch = (i % CK) * 8;
+#pragma unroll
+    for (int r = row0; r < WA_K; r += ROWS_AT_ONCE) {
       const bool live = t0 + r < end;
-      const size_t row = live ? t0 + r - shift : 0;
-      const bool second = ch >= k_cols, kv = live && ch < k2_end;
-      const T* src = !kv ? kb : second ? p.key2 + (size_t)(t0 + r - p.first2) * p.ld2 + ch - k_cols : kb + row * ldk + ch;
-      copy16_or_zero(smem_u32(ks + r * LDK + ch), src, kv);
-    }
-    for (int i = tid; i < WA_K * CV; i += WA_THREADS) {
-      const int r = i / CV, ch = (i % CV) * 8;
-      const bool live = t0 + r < end;
-      const size_t row = live ? t0 + r - shift : 0;
-      const bool vv = live && ch < v_cols;
-      copy16_or_zero(smem_u32(vs + r * LDV + ch), vv ? vb + row * ldv + ch : vb, vv);
+      const int row = live ? t0 + r - shift : 0;
+      const T* k1 = kb + (size_t)row * ldk + quad_col;
+      const T* k2 = p.key2 && live ? p.key2 + (size_t)(t0 + r - p.first2) * p.ld2 - k_cols + quad_col : kb;
+      const T* v1 = vb + (size_t)row * ldv + quad_col;
+      const uint32_t kd = smem_u32(ks + r * LDK + quad_col), vd = smem_u32(vs + r * LDV + quad_col);
+#pragma unroll
+      for (int i = 0; i < CK / 4; ++i) {
+        const int ch = i * 32 + quad_col;
+        const bool there = live && ch < k2_end;
+        copy16_or_zero(kd + i * 64, there ? (ch < k_cols ? k1 : k2) + i * 32 : kb, there);
+      }
+#pragma unroll
+      for (int i = 0; i < CV / 4; ++i) {
+        const bool there = live && i * 32 + quad_col < v_cols;
+        copy16_or_zero(vd + i * 64, there ? v1 + i * 32 : vb, there);
+      }
     }
     cp_async_commit();
   };
@@ -122,7 +134,7 @@ __global__ void __launch_bounds__(WA_THREADS, HK == 64 ? 4 : HK == 128 ? 3 : 2) 
 #pragma unroll
   for (int j = 0; j < HV / 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
   float mx_lo = -CUDART_INF_F, mx_hi = -CUDART_INF_F, sum_lo = 0.f, sum_hi = 0.f;
-  const float scale2 = p.scale * LOG2E;
+  const float scale2 = p.scale * LOG2E, by = scale2 > 0.f ? scale2 : 1.f;
 
   stage_tile(0, 0);
   for (int tile = 0; tile < n_tiles; ++tile) {
@@ -155,10 +167,12 @@ __global__ void __launch_bounds__(WA_THREADS, HK == 64 ? 4 : HK == 128 ? 3 : 2) 
       }
       // every key of the tile visible to every row of the warp?
       const bool full = pooled ? t0 + WA_K <= blocks_of(warp_first) : (t0 + WA_K - 1 <= warp_first && t0 >= warp_last + 1 - p.window);
+      if (scale2 <= 0.f) {  // (the largest product is not the largest score then)
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
+        for (int j = 0; j < 8; ++j)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s[j][e] *= scale2;
+          for (int e = 0; e < 4; ++e) s[j][e] *= scale2;
+      }
       if (!full) {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -180,7 +194,7 @@ __global__ void __launch_bounds__(WA_THREADS, HK == 64 ? 4 : HK == 128 ? 3 : 2) 
       tm_lo = fmaxf(tm_lo, __shfl_xor_sync(0xffffffffu, tm_lo, 2));
       tm_hi = fmaxf(tm_hi, __shfl_xor_sync(0xffffffffu, tm_hi, 1));
       tm_hi = fmaxf(tm_hi, __shfl_xor_sync(0xffffffffu, tm_hi, 2));
-      const float nm_lo = fmaxf(mx_lo, tm_lo), nm_hi = fmaxf(mx_hi, tm_hi);
+      const float nm_lo = fmaxf(mx_lo, tm_lo * by), nm_hi = fmaxf(mx_hi, tm_hi * by);
       // a row that has seen nothing yet keeps sum 0 and output 0 (its maximum is still -inf)
       const float ref_lo = nm_lo > -CUDART_INF_F ? nm_lo : 0.f, ref_hi = nm_hi > -CUDART_INF_F ? nm_hi : 0.f;
       const float f_lo = ex2(mx_lo - ref_lo), f_hi = ex2(mx_hi - ref_hi);
@@ -193,7 +207,8 @@ __global__ void __launch_bounds__(WA_THREADS, HK == 64 ? 4 : HK == 128 ? 3 : 2) 
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
           const int j = 2 * kk + b;
-          const float e0 = ex2(s[j][0] - ref_lo), e1 = ex2(s[j][1] - ref_lo), e2 = ex2(s[j][2] - ref_hi), e3 = ex2(s[j][3] - ref_hi);
+          const float e0 = ex2(fmaf(s[j][0], by, -ref_lo)), e1 = ex2(fmaf(s[j][1], by, -ref_lo));
+          const float e2 = ex2(fmaf(s[j][2], by, -ref_hi)), e3 = ex2(fmaf(s[j][3], by, -ref_hi));
           ts_lo += e0 + e1;
           ts_hi += e2 + e3;
           pa[kk][2 * b] = pack2(e0, e1);
@@ -202,12 +217,14 @@ __global__ void __launch_bounds__(WA_THREADS, HK == 64 ? 4 : HK == 128 ? 3 : 2) 
       }
       sum_lo = sum_lo * f_lo + ts_lo;  // (this lane's keys; the lanes of a row are added at the end)
       sum_hi = sum_hi * f_hi + ts_hi;
+      if (__any_sync(0xffffffffu, f_lo != 1.f || f_hi != 1.f)) {  // (some row's maximum has moved)
 #pragma unroll
-      for (int j = 0; j < HV / 8; ++j) {
-        o[j][0] *= f_lo;
-        o[j][1] *= f_lo;
-        o[j][2] *= f_hi;
-        o[j][3] *= f_hi;
+        for (int j = 0; j < HV / 8; ++j) {
+          o[j][0] *= f_lo;
+          o[j][1] *= f_lo;
+          o[j][2] *= f_hi;
+          o[j][3] *= f_hi;
+        }
       }
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
