@@ -148,6 +148,7 @@ int block_context<T>::residual(hyper_params<T>& p, const pending_result& done, i
     p.up_out = done.streams->out;
     p.post_w = done.post;
     p.n_y = done.n_pieces;
+    p.y_rows_in_order = done.pieces == first_rows;
   }
   ++launches;
   return launch_hyper_rows(p, n_rows, stream());
@@ -644,7 +645,7 @@ int block_context<T>::enqueue_decode_step(int) {
     e.ld_copy = m->k_loop;
   }
   ++launches;
-  LCU_TRY(launch_block_embed(e, g.stream));
+  LCU_TRY(launch_block_embed(e, g.stream, true));
   pending_result done;
   LCU_TRY(layers(1, -1, done));
   LCU_TRY(rows_to_logits(done, nullptr, 0, 1));
@@ -677,7 +678,7 @@ int block_context<T>::enqueue_prefill(int m_rows, const pass_request& rq) {
       e.copy = loop_row + width;
       e.ld_copy = m->k_loop;
     }
-    LCU_TRY(launch_block_embed(e, g.stream));
+    LCU_TRY(launch_block_embed(e, g.stream, false));
     pending_result done;
     LCU_TRY(layers(rows, pos0, done));
     // logits of the wanted rows of this pass, LOGIT_ROWS at a time

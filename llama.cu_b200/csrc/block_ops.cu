@@ -315,6 +315,222 @@ int launch_hyper_one(const hyper_params<T>& p, int n_rows, cudaStream_t stream) 
   return launch_clustered(hyper_rows_kernel<T, SM, CL, PRE>, n_rows * CL, CL, HY_THREADS, smem, stream, p, per);
 }
 
+// ------------------------------------------------------------------ the same for a single row
+// In a step this pass sits between two products, one CTA long, and nothing hides it: it is its chain of dependent loads and
+// reductions.  So what does not depend on the kernel before it - the weights of streams, norms, shift and router, the shifted-in row
+// and the position, both of the step before - is in registers when the wait ends; the residual's columns and the result's are
+// requested together after it and stay in registers to the last store (V vectors of four columns per thread).  CTAs of NT threads.
+// Step, kernel of many rows -> this one, us: Filulix 2048 wide (four streams: a cluster of 8 CTAs -> one of 512 threads), 4 layers,
+// 184 -> 162; Zibovik 1024 wide, 8 layers, 278 -> 254.
+template <typename T, int SM, int CL, int NT, int V, bool PRE>
+__global__ void __launch_bounds__(NT) hyper_one_kernel(const hyper_params<T> p, const int per) {
+  extern __shared__ __align__(16) float h_row[];  // with a router: this CTA's columns of h, then partial sums of the experts
+  __shared__ float s_red[2][NT / 32], s_part[2];
+  struct __align__(4 * sizeof(T)) pack { T e[4]; };
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = blockIdx.x;
+  pdl_launch_dependents();
+  const int S = p.streams, W = p.width, c0 = min(W, rank * per), c1 = min(W, c0 + per);
+  const bool res = p.y != nullptr, shift = p.mix != nullptr;
+  int col[V];
+  bool in_row[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    col[i] = c0 + 4 * (tid + i * NT);
+    in_row[i] = col[i] < c1;
+  }
+  auto f4 = [](const float* at) { return *reinterpret_cast<const float4*>(at); };
+  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+  float in[SM], up[SM], mix[SM][SM];
+#pragma unroll
+  for (int s = 0; s < SM; ++s) {
+    in[s] = s < S ? p.in[s] : 0.f;
+    up[s] = res && s < S ? p.up_out[s] : 0.f;
+#pragma unroll
+    for (int t = 0; t < SM; ++t) mix[s][t] = res && s < S && t < S ? p.up_mix[s * S + t] : 0.f;
+  }
+  float4 nw[V], post[V], mu[V][HY_MIX];
+  pack before[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    nw[i] = p.norm_w && in_row[i] ? f4(p.norm_w + col[i]) : none;
+    post[i] = PRE && p.post_w && in_row[i] ? f4(p.post_w + col[i]) : none;
+    if (shift && in_row[i]) {
+#pragma unroll
+      for (int k = 0; k < HY_MIX; ++k) mu[i][k] = f4(p.mu + (size_t)k * W + col[i]);
+      before[i] = *reinterpret_cast<const pack*>(p.prev + col[i]);
+    }
+  }
+  const bool start = shift && *p.pos == 0;
+  constexpr int RV = 16;  // vectors of router weights a lane holds: the first expert of its warp, rows of up to 2048 columns
+  pack rw[RV];
+  if (p.router) {
+#pragma unroll
+    for (int i = 0; i < RV; ++i)
+      if (warp < p.experts && 4 * lane + 128 * i < c1 - c0) rw[i] = *reinterpret_cast<const pack*>(p.router + (size_t)warp * p.ld_router + c0 + 4 * lane + 128 * i);
+  }
+  pdl_wait();
+  const int row = p.rows ? p.rows[0] : 0;
+  float* x = p.xs + (size_t)row * S * W;
+  const float* y = p.y + (PRE && p.y_rows ? 0 : (size_t)row * p.ldy);
+  float4 xv[V][SM], yv[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i)
+#pragma unroll
+    for (int s = 0; s < SM; ++s) xv[i][s] = s < S && in_row[i] ? __ldcg(reinterpret_cast<const float4*>(x + (size_t)s * W + col[i])) : none;
+#pragma unroll
+  for (int i = 0; i < V; ++i) yv[i] = none;
+  if (res) {
+    const int pieces = PRE && p.y_rows ? p.n_y : 1;
+    for (int k = 0; k < pieces; ++k) {
+      const size_t at = PRE && p.y_rows ? (size_t)(p.y_rows_in_order ? k : p.y_rows[(size_t)row * p.n_y + k]) * p.ldy : 0;
+#pragma unroll
+      for (int i = 0; i < V; ++i)
+        if (in_row[i]) {
+          const float4 v = __ldcg(reinterpret_cast<const float4*>(y + at + col[i]));
+          yv[i] = make_float4(yv[i].x + v.x, yv[i].y + v.y, yv[i].z + v.z, yv[i].w + v.w);
+        }
+    }
+  }
+  auto row_total = [&](float v, int which) {  // over the CTA's threads, then the row's CTAs
+    v = warp_sum(v);
+    if (lane == 0) s_red[which][warp] = v;
+    __syncthreads();
+    float t = lane < NT / 32 ? s_red[which][lane] : 0.f;
+    t = warp_sum(t);
+    if (CL > 1) {
+      if (tid == 0) s_part[which] = t;
+      cluster_sync();
+      t = 0.f;
+#pragma unroll
+      for (int r = 0; r < CL; ++r) t += ld_dsmem_f32(mapa(smem_u32(&s_part[which]), r));
+    }
+    return t;
+  };
+  auto sum_squares = [](const float4& a, float s) { return fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(a.z, a.z, fmaf(a.w, a.w, s)))); };
+  const float inv_w = 1.0f / (float)W;
+  if (PRE && res && p.post_w) {
+    float sy = 0.f;
+#pragma unroll
+    for (int i = 0; i < V; ++i) sy = sum_squares(yv[i], sy);
+    const float inv_y = 1.0f / sqrtf(row_total(sy, 0) * inv_w + p.eps);
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+      yv[i] = make_float4(yv[i].x * (inv_y * post[i].x), yv[i].y * (inv_y * post[i].y), yv[i].z * (inv_y * post[i].z), yv[i].w * (inv_y * post[i].w));
+  }
+  float ss = 0.f;
+  float4 u[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    u[i] = none;
+    auto mixed = [&](int e) {
+      float v[SM], n[SM];
+#pragma unroll
+      for (int s = 0; s < SM; ++s) v[s] = reinterpret_cast<const float*>(&xv[i][s])[e];
+      if (res) {
+#pragma unroll
+        for (int t = 0; t < SM; ++t) {
+          n[t] = up[t] * reinterpret_cast<const float*>(&yv[i])[e];
+#pragma unroll
+          for (int s = 0; s < SM; ++s) n[t] = fmaf(mix[s][t], v[s], n[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < SM; ++t) {
+          v[t] = n[t];
+          reinterpret_cast<float*>(&xv[i][t])[e] = n[t];
+        }
+      }
+      float a = 0.f;
+#pragma unroll
+      for (int s = 0; s < SM; ++s) a = fmaf(in[s], v[s], a);
+      return a;
+    };
+#pragma unroll
+    for (int e = 0; e < 4; ++e) reinterpret_cast<float*>(&u[i])[e] = mixed(e);
+    ss = sum_squares(u[i], ss);  // (columns past the row are zero)
+  }
+  const float inv = 1.0f / sqrtf(row_total(ss, 1) * inv_w + p.eps);
+  T* h = p.h;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    if (!in_row[i]) continue;
+    pack o;
+    float4 back;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float ue = reinterpret_cast<const float*>(&u[i])[e];
+      o.e[e] = from_f<T>(p.norm_w ? ue * inv * (p.norm_base + reinterpret_cast<const float*>(&nw[i])[e]) : ue);
+      reinterpret_cast<float*>(&back)[e] = to_f(o.e[e]);
+    }
+    *reinterpret_cast<pack*>(h + col[i]) = o;
+    if (p.router) *reinterpret_cast<float4*>(h_row + col[i] - c0) = back;
+    if (shift) {
+#pragma unroll
+      for (int k = 0; k < HY_MIX; ++k) {
+        pack m;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float hf = reinterpret_cast<const float*>(&back)[e], d = (start ? 0.f : to_f(before[i].e[e])) - hf;
+          m.e[e] = from_f<T>(fmaf(d, reinterpret_cast<const float*>(&mu[i][k])[e], hf));
+        }
+        *reinterpret_cast<pack*>(p.mix + k * p.mix_stride + col[i]) = m;
+      }
+      *reinterpret_cast<pack*>(p.prev + col[i]) = o;
+    }
+    if (p.u_out) *reinterpret_cast<float4*>(p.u_out + col[i]) = u[i];
+    if (res && p.store) {
+#pragma unroll
+      for (int s = 0; s < SM; ++s)
+        if (s < S) *reinterpret_cast<float4*>(x + (size_t)s * W + col[i]) = xv[i][s];
+    }
+  }
+  if (p.router) {  // z = router . h: this CTA's columns of every expert, then the sum over the CTAs in rank 0
+    __syncthreads();
+    float* z = h_row + per;
+    for (int e = warp; e < p.experts; e += NT / 32) {
+      float a = 0.f;
+      auto add = [&](const pack& wv, int c) {
+        const float4 hv = f4(h_row + c);
+        a = fmaf(to_f(wv.e[0]), hv.x, fmaf(to_f(wv.e[1]), hv.y, fmaf(to_f(wv.e[2]), hv.z, fmaf(to_f(wv.e[3]), hv.w, a))));
+      };
+      const T* w = p.router + (size_t)e * p.ld_router + c0;
+      if (e == warp) {
+#pragma unroll
+        for (int i = 0; i < RV; ++i)
+          if (4 * lane + 128 * i < c1 - c0) add(rw[i], 4 * lane + 128 * i);
+      }
+      for (int c = 4 * lane + (e == warp ? 128 * RV : 0); c < c1 - c0; c += 128) add(*reinterpret_cast<const pack*>(w + c), c);
+      a = warp_sum(a);
+      if (lane == 0) z[e] = a;
+    }
+    if (CL > 1) cluster_sync();
+    else __syncthreads();
+    if (rank == 0) {
+      if (CL > 1) {
+        for (int e = tid; e < p.experts; e += NT) {
+          float a = 0.f;
+#pragma unroll
+          for (int r = 0; r < CL; ++r) a += ld_dsmem_f32(mapa(smem_u32(z + e), r));
+          z[p.experts + e] = a;
+        }
+        __syncthreads();
+      }
+      if (warp == 0)
+        pick_largest(CL > 1 ? z + p.experts : z, p.experts, p.top, [&](int k, int e, float v) {
+          p.pick[k] = e;
+          p.pick_weight[k] = sigmoid_f(v);
+        });
+    }
+  }
+  if (CL > 1) cluster_sync();  // nobody leaves while its partial sum may still be read
+}
+
+template <typename T, int SM, int CL, int NT, int V, bool PRE>
+int launch_hyper_single(const hyper_params<T>& p, cudaStream_t stream) {
+  const int per = (int)round_up(ceil_div(p.width, CL), 4);
+  const size_t smem = p.router ? ((size_t)per + 2 * p.experts) * sizeof(float) : 0;
+  return launch_clustered(hyper_one_kernel<T, SM, CL, NT, V, PRE>, CL, CL, NT, smem, stream, p, per);
+}
+
 // ------------------------------------------------------------------ token shift
 // A thread keeps V columns (width a multiple of V) and their mu over TS_ROWS rows.
 constexpr int TS_ROWS = 8, TS_MIX = 5;
@@ -593,10 +809,20 @@ __global__ void __launch_bounds__(256) matmul_f32_tile_kernel(float* out, const 
 }  // namespace
 
 template <typename T>
-int launch_block_embed(const embed_params<T>& p, cudaStream_t stream) {
-  if (p.width % 4 == 0) LCU_CUDA(launch_after(block_embed_kernel<T, 4>, dim3(p.m), dim3(512), 0, stream, p));
-  else LCU_CUDA(launch_after(block_embed_kernel<T, 1>, dim3(p.m), dim3(512), 0, stream, p));
+int launch_block_embed(const embed_params<T>& p, cudaStream_t stream, bool after_all) {
+  auto kernel = p.width % 4 == 0 ? block_embed_kernel<T, 4> : block_embed_kernel<T, 1>;
+  if (after_all) {
+    kernel<<<p.m, 512, 0, stream>>>(p);
+    LCU_CUDA(cudaGetLastError());
+  } else {
+    LCU_CUDA(launch_after(kernel, dim3(p.m), dim3(512), 0, stream, p));
+  }
   return LCU_OK;
+}
+
+int& hyper_row_single() {
+  static int on = 1;
+  return on;
 }
 
 int& hyper_row_one_cta() {
@@ -611,6 +837,21 @@ int launch_hyper_rows(const hyper_params<T>& p, int n_rows, cudaStream_t stream)
   LCU_REQUIRE(p.mix == nullptr || (n_rows == 1 && p.n_mix == HY_MIX), "hyper_rows: the token shift is fused for a single row of %d inputs", HY_MIX);
   LCU_REQUIRE(p.router == nullptr || n_rows == 1, "hyper_rows: experts are picked for a single row");
   const bool pre = p.y && (p.post_w || p.y_rows);
+  // One row of whole vectors, up to four streams: one CTA where a thread holds one vector (two of a single stream), else a cluster.
+  // (Router weights and the row of a router fit the default 48 KB then: 2048 columns and 1024 experts take 16.)
+  if (n_rows == 1 && p.streams <= 4 && p.width % 4 == 0 && p.width <= 8 * HY_CLUSTER * 128 && hyper_row_single()) {
+#define LCU_SINGLE(SM, CL, NT, V) \
+  return pre ? launch_hyper_single<T, SM, CL, NT, V, true>(p, stream) : launch_hyper_single<T, SM, CL, NT, V, false>(p, stream)
+    if (p.streams == 1) {
+      if (p.width <= 1024) LCU_SINGLE(1, 1, 256, 1);
+      if (p.width <= 2048) LCU_SINGLE(1, 1, 512, 1);
+      LCU_SINGLE(1, HY_CLUSTER, 128, 2);
+    }
+    if (p.width <= 1024) LCU_SINGLE(4, 1, 256, 1);
+    if (p.width <= 2048) LCU_SINGLE(4, 1, 512, 1);
+    LCU_SINGLE(4, HY_CLUSTER, 128, 2);
+#undef LCU_SINGLE
+  }
   const int most = hyper_row_one_cta();  // (measured: 7 % of a step at 1024 columns, lost again where a CTA has four vectors per thread to load twice)
   const bool spread = n_rows == 1 && (p.width > most || p.width * p.streams > 2 * most);
 #define LCU_HYPER(SM)                                                                                                                        \
@@ -711,7 +952,7 @@ int launch_matmul_f32_grouped(float* out, const float* x, int ldx, const float* 
 }
 
 #define LCU_BLOCK_OPS(T)                                                                                                             \
-  template int launch_block_embed<T>(const embed_params<T>&, cudaStream_t);                                                          \
+  template int launch_block_embed<T>(const embed_params<T>&, cudaStream_t, bool);                                                        \
   template int launch_hyper_rows<T>(const hyper_params<T>&, int, cudaStream_t);                                                      \
   template int launch_token_shift<T>(const T*, int, T*, const float*, T*, size_t, int, int, int, int, cudaStream_t);                 \
   template int launch_head_gate<T>(T*, int, const float*, int, const T*, int, const float*, int, int, float, float, int, cudaStream_t); \

@@ -28,8 +28,10 @@ struct embed_params {
   T* copy;       // optional: the rows once more, ld_copy apart
   int ld_copy;
 };
+// after_all: begins when everything before it in the stream has ended, so that the kernels of a step may read what earlier steps
+// left (position, shifted-in rows) before they wait for the kernels ahead of them
 template <typename T>
-int launch_block_embed(const embed_params<T>& p, cudaStream_t stream);
+int launch_block_embed(const embed_params<T>& p, cudaStream_t stream, bool after_all);
 
 // One pass over residual rows between two sublayers:
 //   y <- sum_k y[y_rows[row][k]]                     (optional: a result that lies in pieces)
@@ -52,6 +54,7 @@ struct hyper_params {
   const float* post_w;
   const int* y_rows;     // [rows][n_y]
   int n_y;
+  int y_rows_in_order;   // y_rows of a single row are 0 .. n_y - 1
   const int* rows;       // row numbers to work on, or null: 0 .. n-1; results are dense
   T* h;                  // [n][ldh]
   int ldh;
@@ -69,6 +72,7 @@ struct hyper_params {
   int* pick;             // [top]
   float* pick_weight;    // [top]
 };
+int& hyper_row_single();   // 1 = a single row has a kernel of its own, 0 = it takes the one for many
 int& hyper_row_one_cta();  // a single row of up to this many columns (all streams: twice as many) is one CTA's, a longer one a cluster's
 template <typename T>
 int launch_hyper_rows(const hyper_params<T>& p, int n_rows, cudaStream_t stream);

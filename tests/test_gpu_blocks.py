@@ -331,3 +331,24 @@ def test_replay_program(tmp_path, dtype):
         assert f.exists() == bool(len(w))
         if len(w):
             check(np.fromfile(f, np.float32).reshape(len(w), cfg["vocab"]), w, dtype)
+
+
+@pytest.mark.parametrize("kind,width,streams", [("shift", 88, 1), ("shift", 1024, 4), ("shift", 1028, 3), ("shift", 2048, 2), ("shift", 2056, 4),
+                                                ("routed", 1024, 1), ("routed", 1036, 1), ("routed", 2048, 1), ("routed", 2052, 1), ("routed", 4100, 1)])
+def test_single_rows_in_a_kernel_of_their_own(lcu, run, kind, width, streams):  # noqa: F811
+    """Residual pass of one row, with token shift, output norm, pieces and router, at the edges of its thread and cluster shapes, against
+    the kernel of many rows.  Both work in binary32, sums of squares in another order: logits differ by rounding of bfloat16 inputs to
+    the products only where a value lies on a tie, 2^-9 of a few of them - far below the limit against the plain implementation."""
+    if kind == "shift":
+        cfg, W = B.case(seed=3, layers=("wkv",), width=width, ff=64, streams=streams, vocab=64)
+    else:
+        cfg, W = B.latent_case(seed=3, layers=1, width=width, experts=11, top=3, ff=32, vocab=64)
+    t = B.tokens(cfg, 9, 2)
+    out = []
+    try:
+        for single in (0, 1):
+            lcu.check(lcu.lib.lcu_set_tuning(b"block_row_single", single))
+            out.append(run(cfg, W, "bfloat16").feed(t, [1]))
+    finally:
+        lcu.check(lcu.lib.lcu_set_tuning(b"block_row_single", 1))
+    check(out[1], out[0], "bfloat16", 0.1)
