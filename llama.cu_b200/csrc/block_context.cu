@@ -612,6 +612,7 @@ int block_context<T>::pick_token(bool advance_only, int advance, short* next, sh
   hp.log = log_at;
   hp.step = step;
   hp.log_capacity = log_cap;
+  if (next && tells_host()) hp.host_out = h_stage + 8;  // (a single-token step)
   ++launches;
   LCU_TRY(launch_logits_head(hp, g.stream, pdl));
   if (opt.sampling) {

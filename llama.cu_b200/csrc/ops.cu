@@ -303,6 +303,7 @@ __global__ void __launch_bounds__(HEAD_THREADS) logits_head_kernel(const head_pa
       if (*p.step < p.log_capacity) p.log[*p.step] = (short)best_i;
       *p.step += 1;
     }
+    if (p.host_out) tell_host(p.host_out, best_i, __ldcg(p.token_out + 1));
   }
 }
 

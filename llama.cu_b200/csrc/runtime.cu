@@ -734,10 +734,15 @@ int& host_wait_limit_ms() {
 }
 
 int context_impl::read_back(const gpu_state& from, cudaStream_t stream, int* to, int n_steps, const char* who) {
-  constexpr int NOT_BACK = -1;  // (error codes are positive)
-  volatile int* word = to + 1;
-  *word = NOT_BACK;
+  *(volatile int*)(to + 1) = NOT_BACK;
   LCU_CUDA(cudaMemcpyAsync(to, from.state + 2, 8, cudaMemcpyDeviceToHost, stream));
+  LCU_TRY(wait_for(to, stream, n_steps, who, nullptr));
+  LCU_CUDA(cudaStreamSynchronize(stream));
+  return LCU_OK;
+}
+
+int context_impl::wait_for(int* to, cudaStream_t stream, int n_steps, const char* who, bool* came) {
+  volatile int* word = to + 1;
   const auto begin = std::chrono::steady_clock::now();
   const double limit = host_wait_limit_ms() * (1.0 + n_steps / 1000.0);
   // the word itself is watched; the stream is asked now and then, for errors that keep the word from coming back
@@ -759,7 +764,7 @@ int context_impl::read_back(const gpu_state& from, cudaStream_t stream, int* to,
     next_query = t + 1;
     std::this_thread::yield();
   }
-  LCU_CUDA(cudaStreamSynchronize(stream));
+  if (came) *came = *word != NOT_BACK;
   return LCU_OK;
 }
 
@@ -790,11 +795,11 @@ int context_impl::settled(const char* who) {
   return LCU_OK;
 }
 
-// After the step's stream has been synchronised: the last stage's word came back with the token (h_stage[3]); with
+// After the step's stream has been synchronised: the last stage's word came back behind the token (to[1]); with
 // more than one stage the other stages' words are read as well.
-static int finish_step(context& ctx, const char* who) {
+static int finish_step(context& ctx, const int* to, const char* who) {
   context_impl& c = *ctx.impl;
-  int code = c.h_stage[3];
+  int code = to[1];
   if (code != 0 || c.gpus.size() > 1) {
     const int all = ctx.device_error();
     if (all < 0) {
@@ -943,6 +948,7 @@ int llama_context_impl::enqueue_decode_step(int long_ctx) {
     h.logits = logits; h.probs = probs; h.n_vocab = p.n_vocab; h.temperature = opt.temperature;
     h.token_out = g.state + 2; h.next_ids = gpus.size() == 1 ? ids : nullptr;
     h.pos = g.state; h.advance = 1; h.log = log; h.step = g.state + 1; h.log_capacity = opt.context_len;
+    if (tells_host()) h.host_out = h_stage + 8;
     LCU_TRY(launch_logits_head(h, g.stream, pdl));
     if (opt.sampling)  // the reference's discrete_distribution over the probabilities (llama_cu.cu:1202-1203) instead of the argmax
       LCU_TRY(launch_sample(probs, p.n_vocab, opt.sample_seed, g.state, 0.f, g.state + 2, h.next_ids, log, g.state + 1, opt.context_len, g.stream));
@@ -1220,9 +1226,12 @@ int context::step(const short* tokens, int n, const int* want, int n_want, float
     LCU_REQUIRE(tokens[i] >= 0 && tokens[i] < c.n_vocab, "next_token: token id %d outside the vocabulary", tokens[i]);
   for (int i = 0; i < n_want; ++i) LCU_REQUIRE(want[i] >= 0 && want[i] < n, "step: place %d outside the %d tokens", want[i], n);
   LCU_REQUIRE(n_want == 0 || logits_out != nullptr, "step: no memory for the logits");
-  LCU_TRY(c.stage_inputs(tokens, n));
-  const bool single = n == 1 && !c.rows_only();
+  const bool single = n == 1 && !c.rows_only(), told = single && c.tells_host();
+  const bool in_place = told && c.dev_pos == c.start_pos && c.dev_token == tokens[0];
+  c.dev_pos = c.dev_token = -1;
+  if (!in_place) LCU_TRY(c.stage_inputs(tokens, n));
   if (single) {
+    if (told) *(volatile int*)(c.h_stage + 9) = context_impl::NOT_BACK;
     LCU_TRY(c.run_decode_step(c.start_pos + 1));
   } else {
     pass_request rq;
@@ -1234,12 +1243,23 @@ int context::step(const short* tokens, int n, const int* want, int n_want, float
   }
   c.last_row = n == 1 ? 0 : n - 1;
   device_guard dg(c.first().device);
-  LCU_TRY(c.read_back(c.last(), c.first().stream, c.h_stage + 2, 1, "next_token"));
-  LCU_TRY(finish_step(*this, "next_token"));
+  int* back = c.h_stage + (told ? 8 : 2);
+  bool came = false;
+  if (told) LCU_TRY(c.wait_for(back, c.first().stream, 1, "next_token", &came));
+  // (the words come from the step's last kernel, behind all of its results; a stream that has ended without them met an error)
+  if (!came) {
+    back = c.h_stage + 2;
+    LCU_TRY(c.read_back(c.last(), c.first().stream, back, 1, "next_token"));
+  }
+  LCU_TRY(finish_step(*this, back, "next_token"));
   c.start_pos += n;
+  if (told) {
+    c.dev_pos = c.start_pos;
+    c.dev_token = back[0];
+  }
   if (single)
     for (int i = 0; i < n_want; ++i) LCU_TRY(c.read_step_logits(logits_out + (size_t)i * c.n_vocab));
-  if (token_out) *token_out = c.h_stage[2];
+  if (token_out) *token_out = back[0];
   return LCU_OK;
 }
 
@@ -1250,6 +1270,7 @@ int context::decode_chained(short first_token, int n_steps, short* tokens_out, f
   LCU_REQUIRE(first_token >= 0 && first_token < c.n_vocab, "decode_chained: token id %d outside the vocabulary", first_token);
   LCU_REQUIRE(!c.rows_only(), "decode_chained: matmul_type 1 runs host-driven steps only (lcu_context_next_token)");
   LCU_TRY(c.settled("decode_chained"));
+  c.dev_pos = c.dev_token = -1;
   LCU_TRY(c.stage_inputs(&first_token, 1));
   device_guard dg(c.first().device);
   LCU_CUDA(cudaEventRecord(c.t0, c.first().stream));
@@ -1257,8 +1278,12 @@ int context::decode_chained(short first_token, int n_steps, short* tokens_out, f
   LCU_CUDA(cudaEventRecord(c.t1, c.first().stream));
   LCU_CUDA(cudaMemcpyAsync(c.h_ids, c.log, (size_t)n_steps * 2, cudaMemcpyDeviceToHost, c.first().stream));
   LCU_TRY(c.read_back(c.last(), c.first().stream, c.h_stage + 2, n_steps, "decode_chained"));
-  LCU_TRY(finish_step(*this, "decode_chained"));
+  LCU_TRY(finish_step(*this, c.h_stage + 2, "decode_chained"));
   c.start_pos += n_steps;
+  if (c.tells_host()) {
+    c.dev_pos = c.start_pos;
+    c.dev_token = c.h_stage[2];
+  }
   c.last_row = 0;
   memcpy(tokens_out, c.h_ids, (size_t)n_steps * 2);
   if (ms_out) LCU_CUDA(cudaEventElapsedTime(ms_out, c.t0, c.t1));
@@ -1315,6 +1340,7 @@ int llama_context_impl::bench_kernel(int which, int reps, float* ms_per_launch, 
   device_guard dg(g.device);
   c.h_stage[0] = 0;
   c.h_stage[1] = 0;
+  c.dev_pos = c.dev_token = -1;
   LCU_CUDA(cudaMemcpyAsync(g.state, c.h_stage, 8, cudaMemcpyHostToDevice, g.stream));
   int epi = 0;
   for (int i = 0; i < std::min(reps, 8); ++i) {  // warm-up

@@ -362,3 +362,38 @@ def test_a_wait_for_the_gpu_that_runs_out_is_an_error_and_not_the_end(lcu, famil
     finally:
         lcu.check(lcu.lib.lcu_set_tuning(b"host_wait_limit_ms", 600000))
     lcu.check(lcu.lib.lcu_synchronize())
+
+
+@pytest.mark.parametrize("bs", [0, 128])
+def test_single_steps_behind_other_calls(lcu, bs):
+    """A step that is fed the token before it copies nothing to the GPU: the same calls, each single step as a chained run of one (which always
+    copies), give the same tokens and probabilities bit for bit - behind prompts, other tokens, chained runs, cleared tokens, a sampler."""
+    model = lcu.Model.synthetic(dim=256, n_heads=2, n_layers=2, n_vocab=1000, block_size=bs, seed=9, scale=0.08)
+    runs = []
+    for single in (lambda c, t: c.next_token([t]), lambda c, t: int(c.decode_chained(t, 1)[0][0])):
+        ctx, seen = lcu.Context(model, context_len=64, temperature=0.8), []
+
+        def note(t):
+            seen.append((int(t), ctx.probs().tobytes()))
+            return int(t)
+
+        t = note(ctx.next_token([5, 6, 7, 8]))
+        for _ in range(3):
+            t = note(single(ctx, t))
+        note(single(ctx, 11))
+        t = note(single(ctx, 12))
+        t = int(ctx.decode_chained(t, 3)[0][-1])
+        t = note(single(ctx, t))
+        t = note(ctx.next_token([t, 9]))
+        t = note(single(ctx, t))
+        ctx.clear_tokens()
+        t = note(single(ctx, t))
+        ctx.set_sampling(1, 3)
+        ctx.next_token([t])
+        ctx.set_sampling(0)
+        t = note(single(ctx, 13))
+        note(single(ctx, t))
+        ctx.close()
+        runs.append(seen)
+    assert runs[0] == runs[1]
+    model.close()
