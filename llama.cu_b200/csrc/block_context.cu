@@ -340,7 +340,16 @@ int block_context<T>::mixer_rows(int run, int rows, int pos0) {
     const size_t stride = (size_t)rows_cap * K;
     const branch_spec& bs = ls.branches[0];
     LCU_TRY(launch_token_shift(h, K, runs[run].prev, L.mu, mix, stride, 5, rows, width, pos0, stream()));
-    for (int j = 0; j < 4; ++j) LCU_TRY(product(shifted[j], false, mix + j * stride, K, L.shifted[j], rows, L.shifted_rows[j], K));
+    bool stacked = !is_f32<T>() && rows > 1;  // matrices and results of the four lie one behind the other
+    for (int j = 1; j < 4 && stacked; ++j)
+      stacked = L.shifted_rows[j] == L.shifted_rows[0] && (T*)L.shifted[j] == (T*)L.shifted[0] + (size_t)j * L.shifted_rows[0] * K &&
+                shifted[j] == shifted[0] + (size_t)j * rows_cap * L.shifted_rows[0];
+    if (stacked) {
+      ++launches;
+      LCU_TRY(launch_gemm_tc_side_by_side(shifted[0], mix, K, L.shifted[0], 4, rows, rows_cap, L.shifted_rows[0], K, err(), stream()));
+    } else {
+      for (int j = 0; j < 4; ++j) LCU_TRY(product(shifted[j], false, mix + j * stride, K, L.shifted[j], rows, L.shifted_rows[j], K));
+    }
     LCU_TRY(product(low, true, mix + 4 * stride, K, L.shifted[4], rows, L.shifted_rows[4], K));
     size_t head_stride, row_stride, offset;
     scan_decay_layout(bs.dim, bs.vdim, rows, &head_stride, &row_stride, &offset);

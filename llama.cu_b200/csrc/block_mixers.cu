@@ -205,7 +205,10 @@ template <typename T>
 __device__ __forceinline__ void pool_block(const T* rows, int ld, int pool, const T* last, T* out, int dim) {
   for (int d = threadIdx.x; d < dim; d += blockDim.x) {
     float s = 0.f;
-    for (int j = 0; j < pool; ++j) s += to_f(last && j == pool - 1 ? last[d] : rows[(size_t)j * ld + d]);
+    const int stored = last ? pool - 1 : pool;
+#pragma unroll 8
+    for (int j = 0; j < stored; ++j) s += to_f(rows[(size_t)j * ld + d]);
+    if (last) s += to_f(last[d]);
     out[d] = from_f<T>(s / (float)pool);
   }
 }

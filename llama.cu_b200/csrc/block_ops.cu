@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(128) wkv_decay_kernel(float* w, size_t head_st
   for (int r = 0; r < WD_ROWS; ++r)
 #pragma unroll
     for (int c = 0; c < CH; ++c) acc[r][c] = w0[ch + c];
-#pragma unroll 2
+#pragma unroll 4
   for (int j = 0; j < rank; j += 4) {
     float a[4][CH];
 #pragma unroll

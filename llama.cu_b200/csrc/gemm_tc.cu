@@ -89,7 +89,15 @@ struct group_args {
   const int4* tiles = nullptr;
   const int* n_tiles = nullptr;
   const float* row_scale = nullptr;
+  int per = 0, stride = 0, rows = 0, total = 0;  // without a table: tiles per group, rows from group to group and of one, all tiles
 };
+__device__ __forceinline__ int group_tiles(const group_args& ga) { return ga.n_tiles ? *ga.n_tiles : ga.total; }
+template <int TILE_ROWS>
+__device__ __forceinline__ int4 group_tile(const group_args& ga, int i) {
+  if (ga.tiles) return ga.tiles[i];
+  const int g = i / ga.per, first = g * ga.stride;
+  return make_int4(first + (i - g * ga.per) * TILE_ROWS, first + ga.rows, g, 0);
+}
 constexpr int GM_NONE = 0, GM_PLAIN = 1, GM_GATED = 2;
 __device__ __forceinline__ void st_dsmem_f4(uint32_t addr, float a, float b, float c, float d) {
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
@@ -159,8 +167,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
   pdl_launch_dependents();
   pdl_wait();  // everything above ran under the previous kernel's tail; nothing before this line touches global memory
   if (GM != GM_NONE) {
-    if ((int)blockIdx.y < *ga.n_tiles) {
-      const int4 t = ga.tiles[blockIdx.y];
+    if ((int)blockIdx.y < group_tiles(ga)) {
+      const int4 t = group_tile<BM>(ga, blockIdx.y);
       m0 = t.x;
       m = t.y;
       n_w += t.z * N;
@@ -367,7 +375,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
   pdl_launch_dependents();
   pdl_wait();  // everything above ran under the previous kernel's tail; nothing before this line touches global memory
   if (GM != GM_NONE) {
-    tiles_m = *ga.n_tiles;
+    tiles_m = group_tiles(ga);
     n_tiles = tiles_m * (N / BN);
   }
 
@@ -379,7 +387,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
         int m0 = (t % tiles_m) * (2 * BM) + (int)rank * BM;
         int n0 = (t / tiles_m) * BN + (int)rank * (BN / 2);
         if (GM != GM_NONE) {
-          const int4 tile = ga.tiles[t % tiles_m];
+          const int4 tile = group_tile<2 * BM>(ga, t % tiles_m);
           m0 = tile.x + (int)rank * BM;
           n0 += tile.z * N;
         }
@@ -436,7 +444,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
       const int n0 = (t / tiles_m) * BN;
       float s = 1.f;
       if (GM != GM_NONE) {
-        const int4 tile = ga.tiles[t % tiles_m];
+        const int4 tile = group_tile<2 * BM>(ga, t % tiles_m);
         row = tile.x + (int)rank * BM + quad * 32 + lane;
         m = tile.y;
         if (GM == GM_GATED && row < m && ga.row_scale) s = ga.row_scale[row];
@@ -548,7 +556,7 @@ int launch_bn(void* out, const void* lhs, int ldx, const void* w, int m, int N, 
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(((N + BN - 1) / BN) * S, GM != GM_NONE ? gr->most_tiles : (m + BM - 1) / BM);
   group_args ga;
-  if (GM != GM_NONE) ga = group_args{gr->tiles, gr->n_tiles, gr->row_scale};
+  if (GM != GM_NONE) ga = group_args{gr->tiles, gr->n_tiles, gr->row_scale, gr->most_tiles / gr->groups, gr->stride, gr->group_rows, gr->most_tiles};
   cfg.blockDim = dim3(TC_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -603,7 +611,7 @@ int launch_pair(void* out, const void* lhs, int ldx, const void* w, int m, int N
   }
   const int tiles_m = GM != GM_NONE ? gr->most_tiles : (m + 2 * BM - 1) / (2 * BM), n_tiles = tiles_m * (N / BN);
   group_args ga;
-  if (GM != GM_NONE) ga = group_args{gr->tiles, gr->n_tiles, gr->row_scale};
+  if (GM != GM_NONE) ga = group_args{gr->tiles, gr->n_tiles, gr->row_scale, gr->most_tiles / gr->groups, gr->stride, gr->group_rows, gr->most_tiles};
   int clusters = gemv_sm_count() / 2;
   if (clusters > n_tiles) clusters = n_tiles;
   LCU_CUDA(launch_after(gemm_tc_pair_kernel<T, TO, BN, GM>, dim3(2 * clusters), dim3(TC_THREADS), smem, stream, map_a, map_b, (TO*)out, m, N, K, beta, nstages, tiles_m,
@@ -863,6 +871,27 @@ int launch_gemm_tc_grouped(tc_type type, void* out, const void* lhs, int ldx, co
   const int tile_m = std::min(rows, BM);
   if (gated) return launch_bn<T, T, 128, 1, GM_GATED>(out, lhs, ldx, w, rows, N, K, 0.f, err, stream, &g, tile_m);
   return launch_bn<T, float, 128, 1, GM_PLAIN>(out, lhs, ldx, w, rows, N, K, 0.f, err, stream, &g, tile_m);
+}
+
+// Four products of 2000 x 1024 x 1024: 9.6 us each, most of it a launch's start and its partial wave of tiles; side by side 21.4 in all.
+int launch_gemm_tc_side_by_side(void* out, const void* lhs, int ldx, const void* w, int groups, int rows, int stride, int N, int K, int* err,
+                                cudaStream_t stream) {
+  LCU_REQUIRE(groups >= 1 && rows >= 1 && rows <= stride && N % 128 == 0, "gemm_tc_side_by_side: %d groups of %d rows every %d, N=%d", groups, rows, stride, N);
+  const int all = (groups - 1) * stride + rows;
+  LCU_REQUIRE(gemm_tc_supported(all, N, K, ldx, lhs, w, out), "gemm_tc_side_by_side: unsupported shape m=%d N=%d K=%d", all, N, K);
+  using T = __nv_bfloat16;
+  gemm_groups g{};
+  g.groups = groups;
+  g.stride = stride;
+  g.group_rows = rows;
+  g.tile_rows = rows > BM ? 2 * BM : BM;
+  g.most_tiles = groups * ((rows + g.tile_rows - 1) / g.tile_rows);
+  if (g.tile_rows == BM) return launch_bn<T, T, 128, 1, GM_PLAIN>(out, lhs, ldx, w, all, N, K, 0.f, err, stream, &g, rows);
+  // whole pair tiles: a K step of 256 x 256 takes 0.39 us, of 256 x 128 0.225 (gemm_tc_plan_long), by waves
+  const long pairs = gemv_sm_count() / 2, wide = (long)g.most_tiles * (N / 256), narrow = (long)g.most_tiles * (N / 128);
+  if (N % 256 == 0 && (wide + pairs - 1) / pairs * 0.39 <= (narrow + pairs - 1) / pairs * 0.225)
+    return launch_pair<T, T, 256, GM_PLAIN>(out, lhs, ldx, w, all, N, K, 0.f, err, stream, &g);
+  return launch_pair<T, T, 128, GM_PLAIN>(out, lhs, ldx, w, all, N, K, 0.f, err, stream, &g);
 }
 
 }  // namespace lcu

@@ -36,7 +36,13 @@ struct gemm_groups {
   int tile_rows;            // 128 or 256 (gemm_tc_group_tile)
   int groups;
   const float* row_scale;
+  // tiles null: every group has `group_rows` rows, and group g starts at row g * stride (operand and result alike)
+  int stride = 0, group_rows = 0;
 };
+// several inputs with a matrix each, as one launch (a token-shifted mixer's projections): group g's rows g * stride .. + rows of x and out,
+// matrix w + g * N * K
+int launch_gemm_tc_side_by_side(void* out, const void* lhs, int ldx, const void* w, int groups, int rows, int stride, int N, int K, int* err,
+                                cudaStream_t stream);
 int gemm_tc_group_tile(int rows, int groups);  // for `rows` rows over all groups
 int& gemm_tc_group_mode();  // 128 / 256 = always that tile, 0 (default) = by the rows per group
 int launch_gemm_tc_grouped(tc_type type, void* out, const void* lhs, int ldx, const void* w, int rows, int N, int K, bool gated, const gemm_groups& g,

@@ -352,3 +352,15 @@ def test_single_rows_in_a_kernel_of_their_own(lcu, run, kind, width, streams):  
     finally:
         lcu.check(lcu.lib.lcu_set_tuning(b"block_row_single", 1))
     check(out[1], out[0], "bfloat16", 0.1)
+
+
+@pytest.mark.parametrize("heads", [2, 4])  # products of 128 and 256 columns: narrow and wide tiles
+@pytest.mark.parametrize("rows", [2, 17, 128, 129, 256, 257, 513])
+def test_projections_side_by_side_at_the_edges_of_tiles(run, rows, heads):  # noqa: F811
+    """The four products of a token-shifted mixer as one launch: rows that fill a tile, one more, parts of one, and tiles of 256 rows; the
+    rows behind a portion's last hold what a longer portion left there."""
+    cfg, W = B.case(seed=rows + heads, layers=("wkv",), width=64, ff=64, vocab=64, wkv=dict(heads=heads, dim=64))
+    t = B.tokens(cfg, rows, 2)
+    r = run(cfg, W, "bfloat16", context_len=1024)
+    r.feed(B.tokens(cfg, 700, 1), WHOLE)
+    check(r.feed(t, WHOLE), P.forward(t, cfg, W), "bfloat16")
