@@ -681,6 +681,123 @@ __device__ __forceinline__ float cluster_total(float v, float* slot) {
   return t;
 }
 
+// The keys of a slice, a running maximum, sum and output per warp: the warps of a CTA meet once (as the LLaMA family's decode
+// attention does).  Heads of up to 32 vectors of 16 bytes; a key is shared by `lanes` neighbouring lanes.  Rows that earlier steps
+// wrote are requested ahead of the wait.  Leaves maximum, sum and the value row in res. .
+constexpr int ST_KEYS = 4;  // keys of a group of lanes requested together
+template <typename T>
+__device__ __forceinline__ bool step_attend_suits(const attn_rows<T>& p) {
+  return (max(p.dim, p.vdim) + 7) / 8 * 8 <= 32 * (16 / (int)sizeof(T));
+}
+template <typename T>
+__device__ void step_attend(const attn_rows<T>& p, int head, int pos, int rank, float* part, float* res) {
+  constexpr int VEC = 16 / sizeof(T), WARPS = MX_THREADS / 32;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, kvh = head / (p.heads / p.kv_heads);
+  const int ldk = p.cache.ldk, ldv = p.cache.ldv, k_cols = (p.dim + 7) / 8 * 8, v_cols = (p.vdim + 7) / 8 * 8;
+  const int lanes = pow2_at_least((max(k_cols, v_cols) + VEC - 1) / VEC), groups = MX_THREADS / lanes, grp = tid / lanes, d = tid % lanes * VEC;
+  int lo, blocks;
+  window_of(pos, p.window, p.pool, lo, blocks);
+  const int total = blocks + pos + 1 - lo;
+  const int t0 = (int)((long long)total * rank / ST_CLUSTER), n = (int)((long long)total * (rank + 1) / ST_CLUSTER) - t0;
+  const T* kc = p.cache.k + kvh * p.cache.k_head;
+  const T* vc = p.cache.v + kvh * p.cache.v_head;
+  const T* kp = p.cache.kp + (size_t)kvh * p.cache.n_blocks * ldk;
+  const T* vp = p.cache.vp + (size_t)kvh * p.cache.n_blocks * ldv;
+  uint4 kr[ST_KEYS], vr[ST_KEYS];
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  auto fetch = [&](int base) {  // all but the token itself, which is the last key
+#pragma unroll
+    for (int i = 0; i < ST_KEYS; ++i) {
+      const int t = t0 + base + i * groups + grp, at = t < blocks ? t : lo + t - blocks;
+      const bool there = base + i * groups + grp < n && t + 1 < total;
+      kr[i] = there && d < k_cols ? __ldcg(reinterpret_cast<const uint4*>((t < blocks ? kp : kc) + (size_t)at * ldk + d)) : zero;
+      vr[i] = there && d < v_cols ? __ldcg(reinterpret_cast<const uint4*>((t < blocks ? vp : vc) + (size_t)at * ldv + d)) : zero;
+    }
+  };
+  fetch(0);
+  pdl_wait();
+  float q[VEC], acc[VEC] = {}, mx = -CUDART_INF_F, sum = 0.f;
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) q[e] = d + e < p.dim ? to_f(p.q[head * p.q_head + d + e]) : 0.f;
+  T ck[VEC], cv[VEC];  // the token's own key and value
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) {
+    ck[e] = d + e < p.dim ? p.k[kvh * p.dim + d + e] : from_f<T>(0.f);
+    cv[e] = d + e < p.vdim ? p.v[kvh * p.vdim + d + e] : from_f<T>(0.f);
+  }
+  const int rounds = (n + groups * ST_KEYS - 1) / (groups * ST_KEYS);  // (the same for every lane: the shuffles are warp-wide)
+  for (int rd = 0; rd < rounds; ++rd) {
+    const int base = rd * groups * ST_KEYS;
+    if (rd > 0) fetch(base);
+    float s[ST_KEYS], top = mx;
+#pragma unroll
+    for (int i = 0; i < ST_KEYS; ++i) {
+      const bool own = t0 + base + i * groups + grp + 1 == total;
+      s[i] = 0.f;
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) s[i] = fmaf(q[e], to_f(own ? ck[e] : reinterpret_cast<const T*>(&kr[i])[e]), s[i]);
+    }
+    for (int o = lanes >> 1; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < ST_KEYS; ++i) s[i] += __shfl_xor_sync(0xffffffffu, s[i], o);
+#pragma unroll
+    for (int i = 0; i < ST_KEYS; ++i) {
+      s[i] = base + i * groups + grp < n ? s[i] * p.scale : -CUDART_INF_F;
+      top = fmaxf(top, s[i]);
+    }
+    for (int o = lanes; o < 32; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    const float ref = top > -CUDART_INF_F ? top : 0.f, keep = expf(mx - ref);
+    mx = top;
+    sum *= keep;
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) acc[e] *= keep;
+#pragma unroll
+    for (int i = 0; i < ST_KEYS; ++i) {
+      const bool own = t0 + base + i * groups + grp + 1 == total;
+      const float w = expf(s[i] - ref);  // (0 for keys past the slice)
+      sum += w;
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) acc[e] = fmaf(w, to_f(own ? cv[e] : reinterpret_cast<const T*>(&vr[i])[e]), acc[e]);
+    }
+  }
+  for (int o = lanes; o < 32; o <<= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+  }
+  float* warp_max = part;  // [WARPS], [WARPS], [WARPS][lanes * VEC]
+  float* warp_total = part + WARPS;
+  float* rows = part + 2 * WARPS;
+  if (lane == 0) {
+    warp_max[warp] = mx;
+    warp_total[warp] = sum;
+  }
+  if (lane < lanes)
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) rows[warp * lanes * VEC + d + e] = acc[e];
+  __syncthreads();
+  float top = warp_max[0], f[WARPS];
+#pragma unroll
+  for (int x = 1; x < WARPS; ++x) top = fmaxf(top, warp_max[x]);
+#pragma unroll
+  for (int x = 0; x < WARPS; ++x) f[x] = warp_max[x] > -CUDART_INF_F ? expf(warp_max[x] - top) : 0.f;
+  for (int j = tid; j < p.vdim; j += MX_THREADS) {
+    float v = 0.f;
+#pragma unroll
+    for (int x = 0; x < WARPS; ++x)
+      if (f[x] > 0.f) v = fmaf(f[x], rows[x * lanes * VEC + j], v);
+    res[2 + j] = v;
+  }
+  if (tid == 0) {
+    float t = 0.f;
+#pragma unroll
+    for (int x = 0; x < WARPS; ++x)
+      if (f[x] > 0.f) t = fmaf(f[x], warp_total[x], t);
+    res[0] = top;
+    res[1] = t;
+  }
+}
+
 template <typename T>
 __device__ void step_attention(const step_branch<T>& b, int head, int rank, int pos, float* sm, float* red) {
   const attn_rows<T>& p = b.attn;
@@ -692,13 +809,19 @@ __device__ void step_attention(const step_branch<T>& b, int head, int rank, int 
   float* part = q + ldk;
   float* res = part + PART_FLOATS;
   float* sc = res + 2 + round_up_dev(p.vdim + 2, 4);
-  for (int d = tid; d < ldk; d += MX_THREADS) cur_k[d] = d < p.dim ? p.k[kvh * p.dim + d] : from_f<T>(0.f);
-  for (int d = tid; d < ldv; d += MX_THREADS) cur_v[d] = d < p.vdim ? p.v[kvh * p.vdim + d] : from_f<T>(0.f);
-  __syncthreads();
-  attend_slice(p, p.q, head, pos, rank, ST_CLUSTER, cur_k, cur_v, q, sc, part, red, res);
+  const bool one_pass = step_attend_suits(p);
+  const bool keeps = head % per == 0 && rank == 0;
+  if (one_pass) step_attend(p, head, pos, rank, part, res);
+  else pdl_wait();
+  if (!one_pass || keeps) {
+    for (int d = tid; d < ldk; d += MX_THREADS) cur_k[d] = d < p.dim ? p.k[kvh * p.dim + d] : from_f<T>(0.f);
+    for (int d = tid; d < ldv; d += MX_THREADS) cur_v[d] = d < p.vdim ? p.v[kvh * p.vdim + d] : from_f<T>(0.f);
+    __syncthreads();
+  }
+  if (!one_pass) attend_slice(p, p.q, head, pos, rank, ST_CLUSTER, cur_k, cur_v, q, sc, part, red, res);
   // the first query head of a group keeps the token: its cache rows, and the means of the block it completes (which no
   // position sees before the next step)
-  if (head % per == 0 && rank == 0) {
+  if (keeps) {
     const size_t row = (size_t)kvh * p.cache.ctx_len + pos;
     for (int d = tid; d < p.dim; d += MX_THREADS) p.cache.k[row * ldk + d] = cur_k[d];
     for (int d = tid; d < p.vdim; d += MX_THREADS) p.cache.v[row * ldv + d] = cur_v[d];
@@ -735,6 +858,10 @@ __device__ void step_attention(const step_branch<T>& b, int head, int rank, int 
   cluster_sync();
 }
 
+// What a step reads of weights, states and caches does not depend on the kernel before it (a step begins when the one before it has
+// ended), so the first of it - all of it at the usual sizes - is in registers when the wait ends.  Filulix step, four layers, attention in
+// one pass and this, at 40 / 430 positions, us: 1024 wide 132 -> 127 / 137 -> 128, 2048 wide 165 -> 163 / 171 -> 164.
+constexpr int ST_STATE = 8, ST_RANK = 16;  // state entries and weights of the decay's second product a thread holds
 template <typename T, bool WKV>
 __device__ void step_recurrence(const step_branch<T>& b, int head, int rank, int pos, float* sm, float* red) {
   const scan_rows<T>& p = b.scan;
@@ -746,13 +873,45 @@ __device__ void step_recurrence(const step_branch<T>& b, int head, int rank, int
   float* lows = part + MX_THREADS;
   __shared__ float s_slot;
   const int half = p.rot_dims >> 1;
+  // ---- ahead of the wait
+  const int v0 = DV * rank / ST_CLUSTER, nv = DV * (rank + 1) / ST_CLUSTER - v0;  // (at most 64 columns)
+  const int ng = nv > 0 ? MX_THREADS / nv : 0, grp = nv > 0 ? tid / nv : 0, j = tid - grp * nv;
+  const bool walks = nv > 0 && grp < ng;
+  float* st = p.state + (size_t)head * D * DV + v0 + j;
+  const float dec = WKV ? 0.f : p.decay[head];
+  const float* u = WKV ? p.u + head * D : nullptr;
+  float S0[ST_STATE], u0[WKV ? ST_STATE : 1];
+#pragma unroll
+  for (int s = 0; s < ST_STATE; ++s) {
+    const int i = grp + s * ng;
+    S0[s] = walks && i < D && pos > 0 ? __ldcg(st + (size_t)i * DV) : 0.f;
+    if (WKV) u0[s] = walks && i < D ? u[i] : 0.f;
+  }
+  const int ch_all = p.heads * D, ng2 = max(1, MX_THREADS / D), grp2 = tid / D, c2 = tid - grp2 * D;  // decays: groups of threads share the rank
+  float a0[WKV ? ST_RANK : 1], w0 = 0.f;
+  float2 cs = make_float2(1.f, 0.f);
+  if (WKV) {
+#pragma unroll
+    for (int s = 0; s < ST_RANK; ++s) {
+      const int r = grp2 + s * ng2;
+      a0[s] = D <= MX_THREADS && grp2 < ng2 && r < b.rank ? b.w2t[(size_t)r * ch_all + head * D + c2] : 0.f;
+    }
+    if (tid < D) w0 = b.w0[head * D + tid];
+  } else if (tid < p.rot_dims) {
+    cs = p.rope[(size_t)pos * half + (tid < half ? tid : tid - half)];
+  }
+  const int out_c = head * DV + v0 + tid;
+  const float gain = tid < nv && b.norm ? b.norm[out_c] : 1.f;
+  pdl_wait();
+  const float v = walks ? to_f(p.v[head * DV + v0 + j]) : 0.f;
+  const float gate = tid < nv ? to_f(b.g[out_c]) : 0.f;
   for (int d = tid; d < D; d += MX_THREADS) {
     const T *qr = p.q + head * D, *kr = p.k + head * D;
     float qv = to_f(qr[d]), kv = to_f(kr[d]);
     if (!WKV) {
       if (d < p.rot_dims) {
         const bool low = d < half;
-        const float2 cs = p.rope[(size_t)pos * half + (low ? d : d - half)];
+        if (d != tid) cs = p.rope[(size_t)pos * half + (low ? d : d - half)];
         const int pd = low ? d + half : d - half;
         const float qo = to_f(qr[pd]), ko = to_f(kr[pd]);
         qv = low ? qv * cs.x - qo * cs.y : qv * cs.x + qo * cs.y;
@@ -764,79 +923,73 @@ __device__ void step_recurrence(const step_branch<T>& b, int head, int rank, int
     k[d] = kv;
   }
   if (WKV) {
-    for (int j = tid; j < b.rank; j += MX_THREADS) lows[j] = tanhf(b.low[j]);
+    for (int r = tid; r < b.rank; r += MX_THREADS) lows[r] = tanhf(b.low[r]);
     __syncthreads();
-    const int ch_all = p.heads * D;
-    const int ng = max(1, MX_THREADS / D), grp = tid / D, c0 = tid - grp * D;
-    if (ng > 1) {  // groups of threads share the rank
+    if (ng2 > 1) {
       float a = 0.f;
-      if (grp < ng)
+      if (grp2 < ng2) {
+#pragma unroll
+        for (int s = 0; s < ST_RANK; ++s)
+          if (grp2 + s * ng2 < b.rank) a = fmaf(a0[s], lows[grp2 + s * ng2], a);
 #pragma unroll 8
-        for (int j = grp; j < b.rank; j += ng) a = fmaf(b.w2t[(size_t)j * ch_all + head * D + c0], lows[j], a);
+        for (int r = grp2 + ST_RANK * ng2; r < b.rank; r += ng2) a = fmaf(b.w2t[(size_t)r * ch_all + head * D + c2], lows[r], a);
+      }
       part[tid] = a;
       __syncthreads();
       if (tid < D) {
-        float z = b.w0[head * D + tid];
-        for (int g = 0; g < ng; ++g) z += part[g * D + tid];
+        float z = w0;
+        for (int g = 0; g < ng2; ++g) z += part[g * D + tid];
         w[tid] = expf(-expf(z));
       }
     } else {
       for (int c = tid; c < D; c += MX_THREADS) {
         float z = b.w0[head * D + c];
-        for (int j = 0; j < b.rank; ++j) z = fmaf(b.w2t[(size_t)j * ch_all + head * D + c], lows[j], z);
+        for (int r = 0; r < b.rank; ++r) z = fmaf(b.w2t[(size_t)r * ch_all + head * D + c], lows[r], z);
         w[c] = expf(-expf(z));
       }
     }
   }
   __syncthreads();
-  const int v0 = DV * rank / ST_CLUSTER, nv = DV * (rank + 1) / ST_CLUSTER - v0;  // (at most 64 columns)
-  float* st = p.state + (size_t)head * D * DV;
-  const float dec = WKV ? 0.f : p.decay[head];
-  const float* u = WKV ? p.u + head * D : nullptr;
   float o = 0.f;
   if (nv > 0) {
-    const int ng = MX_THREADS / nv, grp = tid / nv, j = tid - grp * nv;
     float acc = 0.f;
-    if (grp < ng) {
-      const float v = to_f(p.v[head * DV + v0 + j]);
-#pragma unroll 4
-      for (int i = grp; i < D; i += ng) {
-        float* s = st + (size_t)i * DV + v0 + j;
-        float S = pos > 0 ? *s : 0.f;
-        const float kv = k[i] * v;
-        if (WKV) {
-          acc = fmaf(q[i], fmaf(u[i], kv, S), acc);
-          S = fmaf(w[i], S, kv);
-        } else {
-          S = fmaf(dec, S, kv);
-          acc = fmaf(q[i], S, acc);
-        }
-        *s = S;
+    auto take = [&](int i, float S, float ui) {
+      const float kv = k[i] * v;
+      if (WKV) {
+        acc = fmaf(q[i], fmaf(ui, kv, S), acc);
+        S = fmaf(w[i], S, kv);
+      } else {
+        S = fmaf(dec, S, kv);
+        acc = fmaf(q[i], S, acc);
       }
+      st[(size_t)i * DV] = S;
+    };
+    if (walks) {
+#pragma unroll
+      for (int s = 0; s < ST_STATE; ++s)
+        if (grp + s * ng < D) take(grp + s * ng, S0[s], WKV ? u0[WKV ? s : 0] : 0.f);
+#pragma unroll 4
+      for (int i = grp + ST_STATE * ng; i < D; i += ng) take(i, pos > 0 ? st[(size_t)i * DV] : 0.f, WKV ? u[i] : 0.f);
     }
     part[tid] = acc;
     __syncthreads();
     if (tid < nv)
+#pragma unroll 8
       for (int g = 0; g < ng; ++g) o += part[g * nv + tid];
   }
-  const float ss = cluster_total(block_sum(o * o, red), &s_slot);
+  // (up to 32 columns - heads of up to 256 values - are the first warp's)
+  const float ss = cluster_total(DV <= 32 * ST_CLUSTER ? warp_sum(o * o) : block_sum(o * o, red), &s_slot);
   const float inv = 1.0f / sqrtf(ss / (float)DV + b.eps);
-  if (tid < nv) {
-    const int c = head * DV + v0 + tid;
-    float v = o * inv;
-    if (b.norm) v *= b.norm[c];
-    b.out[c] = from_f<T>(v * silu_f(to_f(b.g[c])) * b.out_scale);
-  }
+  if (tid < nv) b.out[out_c] = from_f<T>(o * inv * gain * silu_f(gate) * b.out_scale);
   cluster_sync();
 }
 
 // lines of the caches, states and weights this CTA will read, requested while the kernel before it ends
 template <typename T>
-__device__ __forceinline__ void step_lines(const step_branch<T>& b, int head, int rank, const int* pos_ptr) {
+__device__ __forceinline__ void step_lines(const step_branch<T>& b, int head, int rank, int pos) {
   const int tid = threadIdx.x;
   if (b.kind == BRANCH_WINDOW_ATTN) {
     const attn_rows<T>& p = b.attn;
-    const int pos = min(*(volatile const int*)pos_ptr, p.cache.ctx_len - 1);  // (may be the step before's: only lines are asked for)
     int lo, blocks;
     window_of(pos, p.window, p.pool, lo, blocks);
     const int kvh = head / (p.heads / p.kv_heads), total = blocks + pos + 1 - lo;
@@ -877,9 +1030,8 @@ __global__ void __launch_bounds__(MX_THREADS) mixer_step_kernel(const __grid_con
   const int bi = p.n_branches > 1 && cl >= p.b[1].first ? 1 : 0;
   const step_branch<T>& b = p.b[bi];
   const int head = cl - b.first;
-  step_lines(b, head, rank, p.pos);
-  pdl_wait();
-  const int pos = *p.pos;
+  const int pos = *p.pos;  // (settled before this step began)
+  step_lines(b, head, rank, pos);
   if (b.kind == BRANCH_WINDOW_ATTN) step_attention(b, head, rank, pos, sm, red);
   else if (b.kind == BRANCH_RETENTION) step_recurrence<T, false>(b, head, rank, pos, sm, red);
   else step_recurrence<T, true>(b, head, rank, pos, sm, red);
