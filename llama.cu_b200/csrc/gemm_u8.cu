@@ -76,7 +76,10 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
   uint8_t* smem = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t X_BLOCK = (uint32_t)t * (U8_KB * 2), STAGE = U8_Q_BYTES + 2 * X_BLOCK;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)nstages * STAGE);
-  uint64_t *full = bars, *empty = bars + U8_MAX_STAGES, *conv = empty + U8_MAX_STAGES, *freed = conv + U8_BUFS, *done = freed + U8_BUFS;
+  uint64_t *full = bars, *empty = bars + 2 * U8_MAX_STAGES, *conv = empty + U8_MAX_STAGES, *freed = conv + U8_BUFS, *done = freed + U8_BUFS;
+  // full: every slot has two barriers, used in turn.  A converting warpgroup looks at every other stage; with one barrier per slot and
+  // an odd number of slots it looked at that barrier every other time it was filled, and where a load was overtaken by the next
+  // stage's, the phase before the awaited one passed for it.
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   volatile float* failed = reinterpret_cast<volatile float*>(tmem_slot + 1);  // 1: a wait of this CTA ran out
 
@@ -87,10 +90,8 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
   const uint32_t idesc = (1u << 4) | ((uint32_t)(t >> 3) << 17) | ((uint32_t)(U8_ROWS >> 4) << 24);
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < nstages; ++i) {
-      mbar_init(smem_u32(&full[i]), 1);
-      mbar_init(smem_u32(&empty[i]), 1);
-    }
+    for (int i = 0; i < 2 * nstages; ++i) mbar_init(smem_u32(&full[i]), 1);
+    for (int i = 0; i < nstages; ++i) mbar_init(smem_u32(&empty[i]), 1);
     for (int i = 0; i < U8_BUFS; ++i) {
       mbar_init(smem_u32(&conv[i]), 4);
       mbar_init(smem_u32(&freed[i]), 1);
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
 #pragma unroll
     for (int i = 0; i < U8_AHEAD; ++i) ahead[i] = scales_of(group + i * U8_GROUPS);
     bool ok = true;
-    int s = group >> 1;
+    int s = group >> 1, f = s;
     uint32_t phase = 0;
     for (int b0 = group; b0 < n_blk && ok; b0 += U8_AHEAD * U8_GROUPS) {
 #pragma unroll
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
         if (blk >= n_blk) break;
         const uint32_t sw = ahead[u];
         ahead[u] = scales_of(blk + U8_AHEAD * U8_GROUPS);
-        ok = mbar_wait(smem_u32(&full[s]), phase, err, DEV_ERR_FULL_WAIT, HEED);
+        ok = mbar_wait(smem_u32(&full[f]), phase, err, DEV_ERR_FULL_WAIT, HEED);
         if (ok && blk >= U8_BUFS) ok = mbar_wait(smem_u32(&freed[buf]), (blk / U8_BUFS - 1) & 1, err, DEV_ERR_EMPTY_WAIT, HEED);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -163,8 +164,10 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&conv[buf]));
         s += U8_GROUPS / 2;
-        if (s >= nstages) {
-          s -= nstages;
+        if (s >= nstages) s -= nstages;
+        f += U8_GROUPS / 2;
+        if (f >= 2 * nstages) {
+          f -= 2 * nstages;
           phase ^= 1;
         }
       }
@@ -175,10 +178,10 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
     if (!go && lane == 0) *failed = 1.f;
   } else if (warp == U8_CONV_WARPS) {
     if (tc_elect()) {  // ---- TMA producer
-      tc_ring r;
-      for (int i = 0; i < n_st; ++i, r.step(nstages)) {
+      tc_ring r, f;
+      for (int i = 0; i < n_st; ++i, r.step(nstages), f.step(2 * nstages)) {
         if (!mbar_wait(smem_u32(&empty[r.slot]), r.phase ^ 1u, err, DEV_ERR_EMPTY_WAIT, HEED)) break;
-        const uint32_t bar = smem_u32(&full[r.slot]), dst = base + (uint32_t)r.slot * STAGE;
+        const uint32_t bar = smem_u32(&full[f.slot]), dst = base + (uint32_t)r.slot * STAGE;
         mbar_arrive_expect_tx(bar, STAGE);
         tma_load_2d(dst, &map_q, (st0 + i) * (U8_STAGE_K / 2), n0, bar);
         tma_load_3d(dst + U8_Q_BYTES, &map_x, 0, m0, (st0 + i) * 2, bar);
@@ -187,9 +190,9 @@ __global__ void __launch_bounds__(U8_THREADS, 1) gemm_u8_kernel(const __grid_con
     __syncwarp();
   } else {  // ---- MMA issuer
     bool ok = true;
-    tc_ring r, e;
-    for (int i = 0; i < n_st && ok; ++i, r.step(nstages)) {
-      ok = mbar_wait_warp(smem_u32(&full[r.slot]), r.phase, err, DEV_ERR_FULL_WAIT, HEED);
+    tc_ring r, f, e;
+    for (int i = 0; i < n_st && ok; ++i, r.step(nstages), f.step(2 * nstages)) {
+      ok = mbar_wait_warp(smem_u32(&full[f.slot]), f.phase, err, DEV_ERR_FULL_WAIT, HEED);
       if (!ok) break;
       const uint64_t x = smem_desc_sw128(base + (uint32_t)r.slot * STAGE + U8_Q_BYTES);
 #pragma unroll

@@ -176,6 +176,25 @@ def test_product_expands_8_bit_weights(lcu, m, k, n, beta, bs):
     assert (np.abs(f32(y_gemv) - exact) <= half + sums + 2.0 ** -11 * weight).all()
 
 
+@pytest.mark.parametrize("m", [48, 100, 200])  # tiles of 48, 112 and 208 rows: seven, five and three stages
+def test_product_with_8_bit_weights_from_a_cold_cache(lcu, m):
+    """Loads that arrive out of order: three copies of a matrix, more than the L2 cache holds, give the same bits every time."""
+    torch = pytest.importorskip("torch")
+    k, n, bs = 4096, 11008, 64
+    g = torch.Generator().manual_seed(m)
+    x = torch.randn((m, k), generator=g).half().cuda()
+    q = torch.randint(0, 256, (n, k), generator=g, dtype=torch.uint8).cuda()
+    s = (torch.rand((n, k // bs), generator=g) * 1e-3 + 1e-4).half().cuda()
+    copies = [(q.clone(), s.clone()) for _ in range(3)]
+    stream, first = torch.cuda.current_stream().cuda_stream, None
+    for i in range(30):
+        out = torch.full((m, n), float("nan"), dtype=torch.half, device="cuda")
+        cq, cs = copies[i % 3]
+        lcu.check(lcu.lib.lcu_matmul_nt_fp16u8(out.data_ptr(), x.data_ptr(), cq.data_ptr(), cs.data_ptr(), m, k, n, bs, 0.0, stream))
+        first = out if first is None else first
+        assert bool(torch.isfinite(out).all()) and torch.equal(out, first)
+
+
 @pytest.mark.parametrize("m,k,n", [(200, 512, 384), (9, 4096, 256)])  # one CTA per tile, and K split over a cluster
 def test_product_with_8_bit_weights_behind_an_earlier_error(lcu, m, k, n):
     """A code that another operator's launch left in the error word does not keep a product from its results, and is reported."""
