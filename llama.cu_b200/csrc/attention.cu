@@ -84,14 +84,15 @@ struct warp_rows {
 #pragma unroll
     for (int o = LPR; o < 32; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
     top = fmaxf(top, m);
-    const float keep = top > -CUDART_INF_F ? expf(m - top) : 1.f;
+    // (a score that is no number leaves the maximum alone but not the sum: without any maximum scores are taken as they are)
+    const float ref = top > -CUDART_INF_F ? top : 0.f, keep = expf(m - ref);
     m = top;
     sum *= keep;
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] *= keep;
 #pragma unroll
     for (int j = 0; j < ROUNDS; ++j) {
-      e[j] = valid(j) && m > -CUDART_INF_F ? expf(e[j] - m) : 0.f;
+      e[j] = expf(e[j] - ref);  // (0 for rows that do not exist)
       sum += e[j];
     }
   }
@@ -142,7 +143,7 @@ __device__ __forceinline__ void meet_and_store(const attn_params& p, meeting<HD>
     mt.warp_sum[warp] = w.sum;
   }
   bar_sync(1, ATT_THREADS);
-  // (an empty part has maximum -inf and adds nothing)
+  // (a part without rows has maximum -inf and sums 0; one whose scores are no numbers has sums that are none, whatever its weight)
   auto weight = [](float m, float top) { return m > -CUDART_INF_F ? expf(m - top) : 0.f; };
   asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // remote stores need the target CTA to have started
   if (tid < HD) {

@@ -468,6 +468,41 @@ def test_attention_slices_at_the_edges_of_chunks(lcu, T0, hd):
         assert np.abs(f32(outs[0]) - f32(oo)).max() <= 2.5e-3 + 2.0**-9, cluster
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("score", [np.nan, -np.inf])
+def test_attention_of_a_key_whose_score_is_no_number(lcu, hd, score):
+    """A cached key that overflowed, at every place of short slices and alone in its warp and CTA or not: a score that is NaN makes the whole
+    row NaN, as in the formula and in prompt attention; a score of -inf weighs nothing, unless there is no other (0 / 0).  Values stay
+    finite.  Bound of the rows that are numbers: as in the test of chunk edges."""
+    H = 2
+    rng = np.random.default_rng(hd)
+    for T0 in (0, 1, 6, 15, 38):
+        T, dim = T0 + 1, H * hd
+        q, k, v = rng.standard_normal((1, dim)), rng.standard_normal((T, dim)), f16(rng.standard_normal((T, dim)))
+        q[0, :2] = 1.0, -1.0
+        want = np.zeros((T, dim))  # by place of the key
+        for at in range(T):
+            kk = k.copy()
+            kk[at, :2] = (np.inf, np.inf) if np.isnan(score) else (-np.inf, 0.0)
+            qh, kh, vh = f32(f16(q)).reshape(H, hd), f32(f16(kk)).reshape(T, H, hd), f32(v).reshape(T, H, hd)
+            with np.errstate(invalid="ignore"):
+                s = (np.einsum("hd,thd->ht", qh, kh) / np.sqrt(hd)).astype(np.float16).astype(np.float64)
+                e = np.exp(s - s.max(1, keepdims=True))
+                want[at] = np.einsum("ht,thd->hd", e / e.sum(1, keepdims=True), vh).reshape(-1)
+            assert np.isnan(want[at, :hd]).all() == (np.isnan(score) or T == 1) and np.isfinite(want[at, hd:]).all()
+            got = [lcu.attention(f16(q), f16(kk), v, H, T0, 0)] if np.isnan(score) else []  # (prompt attention)
+            try:
+                for mode in (0, 1):
+                    lcu.check(lcu.lib.lcu_set_tuning(b"attn_stream", mode))
+                    got += [lcu.attention(f16(q), f16(kk), v, H, T0, cluster) for cluster in (1, 2, 8)]
+            finally:
+                lcu.check(lcu.lib.lcu_set_tuning(b"attn_stream", -1))
+            for i, g in enumerate(got):
+                g = f32(g)[0]
+                assert (np.isnan(g) == np.isnan(want[at])).all(), (T, at, i)
+                assert np.nanmax(np.abs(g - want[at]), initial=0) <= 2.5e-3 + 2.0**-9, (T, at, i)
+
+
 @pytest.mark.parametrize("m,T0,cluster", [(1, 50, 4), (70, 9, 0), (70, 9, -1), (300, 100, -1), (70, 9, -2), (300, 100, -2)])
 def test_attention_head_dim_64(lcu, m, T0, cluster):
     rng = np.random.default_rng(8)
