@@ -124,9 +124,10 @@ __device__ void attend_slice(const attn_rows<T>& p, const T* q_row, int head, in
   float mx = -CUDART_INF_F;
   for (int t = tid; t < n; t += MX_THREADS) mx = fmaxf(mx, sc[t]);
   mx = block_max(mx, red);
+  const float ref = mx > -CUDART_INF_F ? mx : 0.f;  // (scores of -inf alone weigh nothing; one that is no number reaches the sum either way)
   float sum = 0.f;
   for (int t = tid; t < n; t += MX_THREADS) {
-    const float e = expf(sc[t] - mx);
+    const float e = expf(sc[t] - ref);
     sc[t] = e;
     sum += e;
   }
@@ -828,20 +829,18 @@ __device__ void step_attend(const attn_rows<T>& p, int head, int pos, int rank, 
   float top = warp_max[0], f[WARPS];
 #pragma unroll
   for (int x = 1; x < WARPS; ++x) top = fmaxf(top, warp_max[x]);
-#pragma unroll
+#pragma unroll  // (a warp without keys has maximum -inf and sums 0; one whose scores are no numbers has sums that are none, whatever its factor)
   for (int x = 0; x < WARPS; ++x) f[x] = warp_max[x] > -CUDART_INF_F ? expf(warp_max[x] - top) : 0.f;
   for (int j = tid; j < p.vdim; j += MX_THREADS) {
     float v = 0.f;
 #pragma unroll
-    for (int x = 0; x < WARPS; ++x)
-      if (f[x] > 0.f) v = fmaf(f[x], rows[x * lanes * VEC + j], v);
+    for (int x = 0; x < WARPS; ++x) v = fmaf(f[x], rows[x * lanes * VEC + j], v);
     res[2 + j] = v;
   }
   if (tid == 0) {
     float t = 0.f;
 #pragma unroll
-    for (int x = 0; x < WARPS; ++x)
-      if (f[x] > 0.f) t = fmaf(f[x], warp_total[x], t);
+    for (int x = 0; x < WARPS; ++x) t = fmaf(f[x], warp_total[x], t);
     res[0] = top;
     res[1] = t;
   }
@@ -887,8 +886,8 @@ __device__ void step_attention(const step_branch<T>& b, int head, int rank, int 
 #pragma unroll
   for (int r = 0; r < ST_CLUSTER; ++r) {
     const float m = ld_dsmem_f32(mapa(smem_u32(res), r));
-    f[r] = m > -CUDART_INF_F ? expf(m - mx) : 0.f;
-    if (f[r] > 0.f) sum += f[r] * ld_dsmem_f32(mapa(smem_u32(res + 1), r));
+    f[r] = m > -CUDART_INF_F ? expf(m - mx) : 0.f;  // (an empty slice and one whose scores are no numbers: as the warps above)
+    sum += f[r] * ld_dsmem_f32(mapa(smem_u32(res + 1), r));
   }
   float inv = p.out_scale / sum;
   if (p.sink) {
@@ -900,8 +899,7 @@ __device__ void step_attention(const step_branch<T>& b, int head, int rank, int 
   for (int d = p.vdim * rank / ST_CLUSTER + tid; d < d1; d += MX_THREADS) {
     float v = 0.f;
 #pragma unroll
-    for (int r = 0; r < ST_CLUSTER; ++r)
-      if (f[r] > 0.f) v += f[r] * ld_dsmem_f32(mapa(smem_u32(res + 2 + d), r));
+    for (int r = 0; r < ST_CLUSTER; ++r) v += f[r] * ld_dsmem_f32(mapa(smem_u32(res + 2 + d), r));
     b.out[head * p.vdim + d] = from_f<T>(v * inv);
   }
   cluster_sync();

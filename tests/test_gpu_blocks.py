@@ -364,3 +364,30 @@ def test_projections_side_by_side_at_the_edges_of_tiles(run, rows, heads):  # no
     r = run(cfg, W, "bfloat16", context_len=1024)
     r.feed(B.tokens(cfg, 700, 1), WHOLE)
     check(r.feed(t, WHOLE), P.forward(t, cfg, W), "bfloat16")
+
+
+@pytest.mark.parametrize("dtype,dim,window", [("bfloat16", 24, 11), ("bfloat16", 24, 64), ("bfloat16", 264, 64), ("float32", 24, 64), ("float32", 136, 11)])
+def test_a_step_sees_a_key_whose_score_is_no_number(run, dtype, dim, window):  # noqa: F811
+    """One token's keys overflow (infinite in a channel where every query is zero, so that the score is NaN; values stay finite), at every
+    place: steps, whose keys are spread over warps and CTAs, give NaN for exactly the rows that see the token, as the formula and prompts do;
+    the others are what they are without it.  Heads of up to 32 vectors and longer ones take different paths."""
+    cfg, W = B.case(seed=3, layers=("parallel",), streams=1, mlp_none=(0,), mixer=dict(dim=dim, window=window))
+    m, j, odd, n, pool = cfg["layers"][0]["mixer"]["left"], 5, 7, 40, 4
+    W["embed"][:, j] = W["bigram"][:, j] = W["l0.norm1"][j] = 0
+    W["embed"][odd, j] = 4
+    W["l0.mix.left.q"].reshape(m["heads"], dim, -1)[:, 0] = 0
+    W["l0.mix.left.k"].reshape(m["kv_heads"], dim, -1)[:, 0] = 0
+    W["l0.mix.left.k"].reshape(m["kv_heads"], dim, -1)[:, 0, j] = 2.0**127
+    r = run(cfg, W, dtype)
+    t = B.tokens(cfg, n, 1)
+    t = [x if x != odd else odd + 1 for x in t]
+    i = np.arange(n)
+    for at in range(n):
+        with_odd = t[:at] + [odd] + t[at + 1:]
+        blocks = np.maximum(0, i + 1 - window) // pool  # means that row i sees in place of the tokens before its window
+        sees = (i >= at) & ((at > i - window) | (at // pool < blocks))
+        steps, whole = r.feed(with_odd, [1]), r.feed(with_odd, WHOLE)
+        assert (np.isnan(steps).all(1) == sees).all() and (np.isnan(steps).any(1) == sees).all(), at
+        assert (np.isnan(whole).all(1) == sees).all() and (np.isnan(whole).any(1) == sees).all(), at
+        if (~sees).any() and at % 8 == 0:
+            check(steps[~sees], whole[~sees], dtype, 2)
