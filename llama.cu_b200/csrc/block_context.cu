@@ -621,7 +621,7 @@ int block_context<T>::pick_token(bool advance_only, int advance, short* next, sh
   hp.log = log_at;
   hp.step = step;
   hp.log_capacity = log_cap;
-  if (next && tells_host()) hp.host_out = h_stage + 8;  // (a single-token step)
+  if (next && tells_host()) hp.host_out = h_words + TOLD;  // (a single-token step)
   ++launches;
   LCU_TRY(launch_logits_head(hp, g.stream, pdl));
   if (opt.sampling) {
@@ -702,7 +702,7 @@ int block_context<T>::enqueue_prefill(int m_rows, const pass_request& rq) {
       LCU_CUDA(cudaMemcpyAsync(row_list, h_rows, n * sizeof(int), cudaMemcpyHostToDevice, g.stream));
       LCU_TRY(rows_to_logits(done, row_list, 0, n));
       slab.resize((size_t)n * m->n_vocab_pad);
-      LCU_TRY(read_back(g, g.stream, h_stage + 4, 1, "step"));  // (a copy to pageable memory waits without a limit)
+      LCU_TRY(read_back(g, g.stream, BEFORE_LOGITS, 1, "step", nullptr));  // (a copy to pageable memory waits without a limit)
       LCU_CUDA(cudaMemcpyAsync(slab.data(), logits, slab.size() * 4, cudaMemcpyDeviceToHost, g.stream));
       LCU_CUDA(cudaStreamSynchronize(g.stream));
       for (int i = 0; i < n; ++i)

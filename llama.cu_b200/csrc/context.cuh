@@ -63,8 +63,9 @@ struct context_impl {
   short* ids = nullptr;                  // token ids on the embedding GPU [context_len]
   __half* probs = nullptr;               // on the output GPU
   short* log = nullptr;                  // generated tokens of a chained run [context_len]
-  int* h_stage = nullptr;                // pinned: [0] position, [1] zero, [2] token read-back, [3] error word; [4], [5] the same in front of logits;
-                                         // [8], [9] the same, written by the last kernel of a step itself (tells_host)
+  int* h_stage = nullptr;                // pinned: [0] position, [1] zero; h_words lies behind them
+  uint64_t* h_words = nullptr;           // pinned: step_words by place
+  enum words_place { COPIED, BEFORE_LOGITS, TOLD, WORDS };  // read back by a copy, the same in front of logits, written by a step's last kernel itself
   // what the position word and the first token id on the GPU hold (-1: not known): a step that finds both in place, as the one after
   // the token it is fed does, has nothing to copy
   int dev_pos = -1, dev_token = -1;
@@ -104,14 +105,13 @@ struct context_impl {
   int build_graph(int variant);
   int run_decode_step(int n_keys);
   int stage_inputs(const short* tokens, int n);
-  // a step's last kernel writes token and error word to h_stage[8], [9] (a sampler or another GPU's stage would come after it)
+  // a step's last kernel writes token and error word to h_words[TOLD] (a sampler or another GPU's stage would come after it)
   bool tells_host() const { return gpus.size() == 1 && !opt.sampling; }
-  // Two state words of `from` (token, error word) to pinned memory, and the wait for everything before them on `stream`: at most
+  // Token and error word of `from` to pinned memory, and the wait for everything before them on `stream`: at most
   // host_wait_limit_ms() for the call and again for every thousand steps in it, then LCU_ERR_DEVICE_WAIT.  (Kernels bound their
   // waits on barriers and flags themselves; this bounds whatever else keeps a stream from ending.)
-  int read_back(const gpu_state& from, cudaStream_t stream, int* to, int n_steps, const char* who);
-  static constexpr int NOT_BACK = -1;    // (error codes are positive)
-  int wait_for(int* to, cudaStream_t stream, int n_steps, const char* who, bool* came);  // until to[1] is no longer NOT_BACK
+  int read_back(const gpu_state& from, cudaStream_t stream, words_place place, int n_steps, const char* who, step_words* back);
+  int wait_for(words_place place, cudaStream_t stream, int n_steps, const char* who, step_words* back);  // until they come or the stream has ended
   bool running();                        // some stream has work left
   int settled(const char* who);          // after a wait that ran out: refuses until the streams are empty and the tokens cleared
 };

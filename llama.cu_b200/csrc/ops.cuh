@@ -51,7 +51,7 @@ struct head_params {
   short* log;
   int* step;
   int log_capacity;
-  int* host_out;            // optional, pinned host memory, 8-byte aligned: {token, the word behind token_out} in one store, last of all
+  uint64_t* host_out;       // optional, pinned host memory: token and the word behind token_out (step_words), last of all
 };
 #ifdef __CUDACC__
 __device__ __forceinline__ float head_logit(const head_params& p, int i) { return p.logits_f32 ? p.logits_f32[i] : __half2float(p.logits[i]); }

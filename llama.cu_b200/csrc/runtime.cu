@@ -512,11 +512,14 @@ context::~context() {
     impl.release();
     return;
   }
+  for (auto& gpu : c.gpus) {  // (a step that told its token may still be ending)
+    device_guard g(gpu.device);
+    cudaDeviceSynchronize();
+  }
   for (int v = 0; v < 2; ++v)
     if (c.graph[v]) cudaGraphExecDestroy(c.graph[v]);
   for (size_t i = 0; i < c.gpus.size(); ++i) {
     device_guard g(c.gpus[i].device);
-    cudaDeviceSynchronize();
     if (c.gpus[i].arena) cudaFree(c.gpus[i].arena);
     if (i < c.kv_arenas.size() && c.kv_arenas[i]) cudaFree(c.kv_arenas[i]);
     if (c.gpus[i].side) cudaStreamDestroy(c.gpus[i].side);
@@ -652,9 +655,11 @@ int model::new_context(std::unique_ptr<context_impl>& out, const context_options
 
 int context_impl::open_streams(int context_len) {
   device_guard dg(first().device);
+  static_assert((2 + 2 * WORDS) * sizeof(int) <= 64, "pinned words");
   LCU_CUDA(cudaMallocHost(&h_stage, 64));
   LCU_CUDA(cudaMallocHost(&h_ids, (size_t)context_len * 2));
   memset(h_stage, 0, 64);
+  h_words = reinterpret_cast<uint64_t*>(h_stage + 2);
   LCU_CUDA(cudaEventCreate(&t0));
   LCU_CUDA(cudaEventCreate(&t1));
   return LCU_OK;
@@ -733,28 +738,32 @@ int& host_wait_limit_ms() {
   return ms;
 }
 
-int context_impl::read_back(const gpu_state& from, cudaStream_t stream, int* to, int n_steps, const char* who) {
-  *(volatile int*)(to + 1) = NOT_BACK;
-  LCU_CUDA(cudaMemcpyAsync(to, from.state + 2, 8, cudaMemcpyDeviceToHost, stream));
-  LCU_TRY(wait_for(to, stream, n_steps, who, nullptr));
+int context_impl::read_back(const gpu_state& from, cudaStream_t stream, words_place place, int n_steps, const char* who, step_words* back) {
+  step_words seen;
+  clear_words(h_words + place);
+  LCU_CUDA(cudaMemcpyAsync(h_words + place, from.state + 2, 8, cudaMemcpyDeviceToHost, stream));
+  LCU_TRY(wait_for(place, stream, n_steps, who, &seen));
   LCU_CUDA(cudaStreamSynchronize(stream));
+  if (back) *back = read_words(h_words + place);
   return LCU_OK;
 }
 
-int context_impl::wait_for(int* to, cudaStream_t stream, int n_steps, const char* who, bool* came) {
-  volatile int* word = to + 1;
+int context_impl::wait_for(words_place place, cudaStream_t stream, int n_steps, const char* who, step_words* back) {
   const auto begin = std::chrono::steady_clock::now();
   const double limit = host_wait_limit_ms() * (1.0 + n_steps / 1000.0);
-  // the word itself is watched; the stream is asked now and then, for errors that keep the word from coming back
+  // the words themselves are watched; the stream is asked now and then, for errors that keep them from coming
   double next_query = limit > 0 && limit < 10 ? limit : 10;
-  while (*word == NOT_BACK) {
+  while (!(*back = read_words(h_words + place)).came()) {
     const double t = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - begin).count();
     if (t < next_query) continue;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // (another thread may be capturing)
     cudaThreadExchangeStreamCaptureMode(&mode);
     const cudaError_t e = cudaStreamQuery(stream);
     cudaThreadExchangeStreamCaptureMode(&mode);
-    if (e != cudaErrorNotReady) break;  // (done, or an error, which the synchronisation returns)
+    if (e != cudaErrorNotReady) {  // (done, or an error, which the synchronisation returns)
+      *back = read_words(h_words + place);
+      break;
+    }
     cudaGetLastError();
     if (limit > 0 && t > limit) {
       unfinished = place_lost = true;
@@ -764,7 +773,6 @@ int context_impl::wait_for(int* to, cudaStream_t stream, int n_steps, const char
     next_query = t + 1;
     std::this_thread::yield();
   }
-  if (came) *came = *word != NOT_BACK;
   return LCU_OK;
 }
 
@@ -795,11 +803,11 @@ int context_impl::settled(const char* who) {
   return LCU_OK;
 }
 
-// After the step's stream has been synchronised: the last stage's word came back behind the token (to[1]); with
-// more than one stage the other stages' words are read as well.
-static int finish_step(context& ctx, const int* to, const char* who) {
+// The last stage's words have come back (its stream has passed everything but the end of the kernel that told them); with
+// more than one stage, whose streams are synchronised, the other stages' words are read as well.
+static int finish_step(context& ctx, const step_words& back, const char* who) {
   context_impl& c = *ctx.impl;
-  int code = to[1];
+  int code = back.code;
   if (code != 0 || c.gpus.size() > 1) {
     const int all = ctx.device_error();
     if (all < 0) {
@@ -948,7 +956,7 @@ int llama_context_impl::enqueue_decode_step(int long_ctx) {
     h.logits = logits; h.probs = probs; h.n_vocab = p.n_vocab; h.temperature = opt.temperature;
     h.token_out = g.state + 2; h.next_ids = gpus.size() == 1 ? ids : nullptr;
     h.pos = g.state; h.advance = 1; h.log = log; h.step = g.state + 1; h.log_capacity = opt.context_len;
-    if (tells_host()) h.host_out = h_stage + 8;
+    if (tells_host()) h.host_out = h_words + TOLD;
     LCU_TRY(launch_logits_head(h, g.stream, pdl));
     if (opt.sampling)  // the reference's discrete_distribution over the probabilities (llama_cu.cu:1202-1203) instead of the argmax
       LCU_TRY(launch_sample(probs, p.n_vocab, opt.sample_seed, g.state, 0.f, g.state + 2, h.next_ids, log, g.state + 1, opt.context_len, g.stream));
@@ -1126,7 +1134,7 @@ int llama_context_impl::enqueue_prefill(int m_rows, const pass_request& rq) {
   }
   if (rq.n_want) {
     device_guard dg(last().device);
-    LCU_TRY(read_back(last(), last().stream, h_stage + 4, 1, "step"));
+    LCU_TRY(read_back(last(), last().stream, BEFORE_LOGITS, 1, "step", nullptr));
     LCU_TRY(read_step_logits(rq.logits_out));
   }
   return LCU_OK;
@@ -1231,7 +1239,7 @@ int context::step(const short* tokens, int n, const int* want, int n_want, float
   c.dev_pos = c.dev_token = -1;
   if (!in_place) LCU_TRY(c.stage_inputs(tokens, n));
   if (single) {
-    if (told) *(volatile int*)(c.h_stage + 9) = context_impl::NOT_BACK;
+    if (told) clear_words(c.h_words + context_impl::TOLD);
     LCU_TRY(c.run_decode_step(c.start_pos + 1));
   } else {
     pass_request rq;
@@ -1243,23 +1251,19 @@ int context::step(const short* tokens, int n, const int* want, int n_want, float
   }
   c.last_row = n == 1 ? 0 : n - 1;
   device_guard dg(c.first().device);
-  int* back = c.h_stage + (told ? 8 : 2);
-  bool came = false;
-  if (told) LCU_TRY(c.wait_for(back, c.first().stream, 1, "next_token", &came));
+  step_words back;
+  if (told) LCU_TRY(c.wait_for(context_impl::TOLD, c.first().stream, 1, "next_token", &back));
   // (the words come from the step's last kernel, behind all of its results; a stream that has ended without them met an error)
-  if (!came) {
-    back = c.h_stage + 2;
-    LCU_TRY(c.read_back(c.last(), c.first().stream, back, 1, "next_token"));
-  }
+  if (!back.came()) LCU_TRY(c.read_back(c.last(), c.first().stream, context_impl::COPIED, 1, "next_token", &back));
   LCU_TRY(finish_step(*this, back, "next_token"));
   c.start_pos += n;
   if (told) {
     c.dev_pos = c.start_pos;
-    c.dev_token = back[0];
+    c.dev_token = back.token;
   }
   if (single)
     for (int i = 0; i < n_want; ++i) LCU_TRY(c.read_step_logits(logits_out + (size_t)i * c.n_vocab));
-  if (token_out) *token_out = back[0];
+  if (token_out) *token_out = back.token;
   return LCU_OK;
 }
 
@@ -1277,12 +1281,13 @@ int context::decode_chained(short first_token, int n_steps, short* tokens_out, f
   for (int i = 0; i < n_steps; ++i) LCU_TRY(c.run_decode_step(c.start_pos + i + 1));
   LCU_CUDA(cudaEventRecord(c.t1, c.first().stream));
   LCU_CUDA(cudaMemcpyAsync(c.h_ids, c.log, (size_t)n_steps * 2, cudaMemcpyDeviceToHost, c.first().stream));
-  LCU_TRY(c.read_back(c.last(), c.first().stream, c.h_stage + 2, n_steps, "decode_chained"));
-  LCU_TRY(finish_step(*this, c.h_stage + 2, "decode_chained"));
+  step_words back;
+  LCU_TRY(c.read_back(c.last(), c.first().stream, context_impl::COPIED, n_steps, "decode_chained", &back));
+  LCU_TRY(finish_step(*this, back, "decode_chained"));
   c.start_pos += n_steps;
   if (c.tells_host()) {
     c.dev_pos = c.start_pos;
-    c.dev_token = c.h_stage[2];
+    c.dev_token = back.token;
   }
   c.last_row = 0;
   memcpy(tokens_out, c.h_ids, (size_t)n_steps * 2);

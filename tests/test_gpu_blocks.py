@@ -391,3 +391,41 @@ def test_a_step_sees_a_key_whose_score_is_no_number(run, dtype, dim, window):  #
         assert (np.isnan(whole).all(1) == sees).all() and (np.isnan(whole).any(1) == sees).all(), at
         if (~sees).any() and at % 8 == 0:
             check(steps[~sees], whole[~sees], dtype, 2)
+
+
+@pytest.mark.parametrize("family", ["recurrent", "latent"])
+def test_single_steps_behind_other_calls(run, family):  # noqa: F811
+    """A step that is fed the token before it copies nothing to the GPU and learns its token from the last kernel itself: the same calls with
+    each single step as a chained run of one, which copies both ways, give the same tokens and probabilities bit for bit - behind
+    prompts, other tokens, chained runs, logits, cleared tokens, a sampler."""
+    cfg, W = B.case(seed=3) if family == "recurrent" else B.latent_case(seed=3)
+    ctx, runs = run(cfg, W, "bfloat16", context_len=400).ctx, []
+    for single in (lambda t: ctx.next_token([t]), lambda t: int(ctx.decode_chained(t, 1)[0][0])):
+        ctx.clear_tokens()
+        seen = []
+
+        def note(t):
+            seen.append((int(t), ctx.probs().tobytes()))
+            return int(t)
+
+        t = note(ctx.next_token([5, 6, 7, 8]))
+        for _ in range(100):
+            t = note(single(t))
+        note(single(11))
+        t = note(single(12))
+        t = int(ctx.decode_chained(t, 3)[0][-1])
+        t = note(single(t))
+        logits, t = ctx.step([t], [0], token=True)
+        seen.append(logits.tobytes())
+        t = note(single(t))
+        t = note(ctx.next_token([t, 9]))
+        t = note(single(t))
+        ctx.clear_tokens()
+        t = note(single(t))
+        ctx.set_sampling(1, 3)
+        ctx.next_token([t])
+        ctx.set_sampling(0)
+        t = note(single(13))
+        note(single(t))
+        runs.append(seen)
+    assert runs[0] == runs[1]
