@@ -285,6 +285,10 @@ int lcu_plan_short_prompt_gemm(int n, int k, int sms, int* tile_n_out, int* spli
  * pair, 256 or 512 for the kernel that deals the K steps of the last wave's tiles evenly over the pairs, with tiles that wide
  * (estimates fitted to timings on B200). */
 int lcu_plan_long_prompt_gemm(int m, int n, int k, int sms, int* kernel_out);
+/* The launch of one product of a LLaMA decode step on a GPU of `sms` SMs: `mats` matrices of `rows` x k (1: wo, w2; 2: w1|w3; 3: wq|wk|wv),
+ * block_size 0 (fp16), 32, 64 or 128; tensor_parallel != 0: a launch of a tensor-parallel step.  *chunks_out = 4 KiB chunks of a row that
+ * a warp holds in registers, 0 where weights are streamed through shared memory; warps of a CTA that form products; CTAs. */
+int lcu_plan_decode_product(int k, int rows, int mats, int block_size, int tensor_parallel, int sms, int* chunks_out, int* warps_out, int* ctas_out);
 /* Products with 8-bit weights that are expanded inside (lcu_matmul_nt_fp16u8 from 2 rows): activation rows per tile (a multiple of 16
  * up to 224) and the CTAs that share a tile's K (1, 2, 4 or 8).  n even, k a multiple of 256. */
 int lcu_plan_u8_gemm(int m, int n, int k, int sms, int* tile_rows_out, int* splits_out);

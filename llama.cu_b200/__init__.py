@@ -62,6 +62,7 @@ _SIG = {
     "lcu_selftest_balanced_schedule": (C.c_int, [C.c_int, C.c_int, C.c_int]),
     "lcu_plan_long_prompt_gemm": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int)]),
     "lcu_plan_recurrence": (C.c_int, [C.c_int] * 6 + [C.POINTER(C.c_int)] * 4),
+    "lcu_plan_decode_product": (C.c_int, [C.c_int] * 6 + [C.POINTER(C.c_int)] * 3),
     "lcu_plan_u8_gemm": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "lcu_plan_short_prompt_gemm": (C.c_int, [C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "lcu_selftest_silu_arithmetic": (C.c_int, [C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]),

@@ -637,6 +637,21 @@ int lcu_plan_short_prompt_gemm(int n, int k, int sms, int* tile_n_out, int* spli
   gemm_tc_plan_short(n, k, sms, tile_n_out, split_out);
   return LCU_OK;
 }
+int lcu_plan_decode_product(int k, int rows, int mats, int block_size, int tensor_parallel, int sms, int* chunks_out, int* warps_out, int* ctas_out) {
+  LCU_REQUIRE(k >= 256 && k % 256 == 0 && rows >= 2 && rows % 2 == 0 && mats >= 1 && mats <= 3 && sms >= 1 && chunks_out && warps_out && ctas_out &&
+                  (block_size == 0 || block_size == 32 || block_size == 64 || block_size == 128),
+              "plan_decode_product: bad arguments");
+  int step_number = 0;
+  __half norm;
+  gemv_params p{};
+  p.K = k;
+  p.bs = block_size;
+  p.n_mats = mats;
+  p.rows_per_mat = rows;
+  p.norm_w = mats > 1 ? &norm : nullptr;  // (looked at, not read)
+  p.seq = tensor_parallel ? &step_number : nullptr;
+  return gemv_plan_single_row(p, mats == 1 ? EPI_PLAIN : mats == 2 ? EPI_SILU : EPI_ROPE_KV, sms, chunks_out, warps_out, ctas_out);
+}
 int lcu_plan_u8_gemm(int m, int n, int k, int sms, int* tile_rows_out, int* splits_out) {
   LCU_REQUIRE(m >= 2 && n >= 2 && n % 2 == 0 && k >= 256 && k % 256 == 0 && sms >= 1 && tile_rows_out && splits_out, "plan_u8_gemm: bad arguments");
   gemm_u8_plan(m, n, k, sms, tile_rows_out, splits_out);

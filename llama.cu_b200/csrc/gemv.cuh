@@ -111,8 +111,9 @@ void gemv_held_mode(int mode);
 
 // loads all single-row kernels on the current device ahead of their first launch
 int gemv_single_row_preload();
-// consumer warps of the single-row launch these arguments lead to
-int gemv_single_row_consumer_warps(const gemv_params& p);
+// the single-row launch these arguments lead to: 4 KiB chunks of a row that a warp holds in registers (0: streamed through a ring), warps
+// of a CTA that form products, CTAs
+int gemv_plan_single_row(const gemv_params& p, int epilogue, int sms, int* chunks, int* warps, int* grid);
 
 // single-row kernel (gemv1.cu); called by launch_gemv after argument checks
 int launch_gemv_single_row(const gemv_params& p, int epilogue, cudaStream_t stream, int pdl, int sms);

@@ -888,12 +888,14 @@ int g_held_mode = -1;  // -1 = by the rule, 0 = never
 // At most twelve warps per SM, one wave beside the kernels around it (4096 wide u8, 13.8 for wo: 2 % slower held).  Rows: a launch
 // between ring kernels gains nothing, so lengths stop where a model's other launches are too large - bfloat16 rows of 4 KiB
 // (Filulix, 2048 wide) 185 -> 188 us, rows of two chunks of 1536 wide fp16 (8 KiB) 152 -> 173, where 1024 wide ones (5.5 KiB), whose
-// step is held as a whole, gain 156 -> 143.  Tensor-parallel launches stay on the ring.
+// step is held as a whole, gain 156 -> 143.  Every launch of a tensor-parallel step (its step number is set) stays on the ring, the one
+// that neither waits for other GPUs nor publishes to them - layer 0's wq|wk|wv - too: ring kernels are loaded ahead of the first step, in
+// which other GPUs' bounded waits run while a launch stalls in loading its kernel.
 constexpr int HELD_WARPS_PER_SM = 12;
 template <class PairsOf>
 held_plan plan_held(int wt, int epi, const gemv_params& p, int n, PairsOf pairs_of, int sms) {
   held_plan h;
-  if (g_held_mode == 0 || wt == 1 || (wt == 2 && p.bs != 64 && p.bs != 128) || p.n_wait > 0 || p.done_count != nullptr || p.n_peer_out > 0) return h;
+  if (g_held_mode == 0 || wt == 1 || (wt == 2 && p.bs != 64 && p.bs != 128) || p.seq != nullptr) return h;
   const int rowbytes = p.K * (wt == 2 ? 1 : 2), chunks = (rowbytes + 4095) / 4096;
   if (rowbytes > (wt == 3 ? 3072 : epi == EPI_PLAIN ? 6144 : 4096)) return h;
   long long single = 0, two = 0;
@@ -978,12 +980,15 @@ int gemv_single_row_preload() {
   return LCU_OK;
 }
 
-// consumer warps of the launch launch_gemv would make for these arguments (each counts itself once on the waiting GPUs'
-// counters in tensor-parallel decode); 0 if the arguments cannot be launched
-int gemv_single_row_consumer_warps(const gemv_params& p) {
+int gemv_plan_single_row(const gemv_params& p, int epilogue, int sms, int* chunks, int* warps, int* grid) {
   gemv1_config c;
-  if (configure(p, gemv_sm_count(), c) != LCU_OK) return 0;
-  return c.grid * c.nw;
+  const int rc = configure(p, sms, c);
+  if (rc) return rc;
+  const held_plan h = plan_held(c.wt, epilogue, p, 1, [&](int) { return p.n_mats * p.rows_per_mat / 2; }, sms);
+  *chunks = h.chunks;
+  *warps = h.chunks ? h.warps : c.nw;
+  *grid = h.chunks ? h.grid : c.grid;
+  return LCU_OK;
 }
 
 // m == 1 entry used by launch_gemv (argument checks are done there)

@@ -143,6 +143,31 @@ def test_8_bit_product_plan_on_any_number_of_sms():
         plan(2, 64, 128)
 
 
+def test_tensor_parallel_steps_take_only_kernels_that_are_loaded_ahead():
+    """Host arithmetic behind the products of a decode step: small matrices are held in registers on one GPU, but no launch of a tensor-parallel
+    step is - wq|wk|wv of layer 0 neither, which waits for no other GPU - because the kernels that do so are not loaded ahead of it."""
+    lcu = load_package()
+
+    def plan(k, rows, mats, bs, tp):
+        out = [C.c_int(-1) for _ in range(3)]
+        lcu.check(lcu.lib.lcu_plan_decode_product(k, rows, mats, bs, tp, 148, *map(C.byref, out)))
+        return [o.value for o in out]
+
+    held = 0
+    for dim in (512, 1024, 2048, 4096, 5120, 8192):
+        for gpus in (2, 4, 8):
+            for bs in (0, 32, 64, 128):
+                for mats, rows in ((3, dim // gpus), (2, dim * 3 // gpus), (1, dim // gpus)):
+                    chunks, warps, ctas = plan(dim, rows, mats, bs, 1)
+                    assert chunks == 0 and warps in (4, 5) and 1 <= ctas <= 3 * 148, (dim, gpus, bs, mats)
+                    held += plan(dim, rows, mats, bs, 0)[0] > 0
+    assert held > 50
+    # one GPU: whole rows of up to a chunk (two for plain products) per warp, as many CTAs as the pairs need
+    assert plan(1024, 1024, 3, 0, 0) == [1, 6, 128] and plan(2816, 1024, 1, 0, 0) == [2, 4, 128] and plan(4096, 4096, 1, 128, 0)[0] == 0
+    with pytest.raises(lcu.LcuError):
+        plan(100, 2, 1, 0, 0)
+
+
 def test_recurrence_chunks_are_resident_at_once():
     """Host arithmetic behind the recurrences of block models: the CTAs of all chunks fit the SMs side by side (a second wave would be a
     second walk), on any number of SMs; chunks cover the rows in whole steps of 16."""
