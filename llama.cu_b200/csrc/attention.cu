@@ -340,16 +340,8 @@ __global__ void __launch_bounds__(AS_THREADS, 3) attn_stream_kernel(const attn_p
   meet_and_store(p, mt, w, head, qrow, rank, cs);
 }
 
-// positions a CTA's slice may hold (one half each within 200 KB beside the partial results)
 template <int HD>
-constexpr int most_positions() {
-  return (200 * 1024 - 16 - (int)sizeof(float) * (16 + 8 * HD + ATT_WARPS * HD + 2 * ATT_WARPS)) / 2;
-}
-
-template <int HD>
-int launch_hd(const attn_params& p, int m, int cs, int max_T, cudaStream_t stream, int pdl) {
-  const int chunk = (max_T + cs - 1) / cs;
-  LCU_REQUIRE(chunk <= most_positions<HD>(), "attention: %d positions per CTA do not fit in shared memory", chunk);
+int launch_hd(const attn_params& p, int m, int cs, cudaStream_t stream, int pdl) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cs, p.n_heads, m);
   cfg.blockDim = dim3(ATT_THREADS);
@@ -369,10 +361,8 @@ int launch_hd(const attn_params& p, int m, int cs, int max_T, cudaStream_t strea
 }
 
 template <int HD>
-int launch_stream_hd(const attn_params& p, int m, int cs, int max_T, cudaStream_t stream, int pdl) {
-  const int chunk = (max_T + cs - 1) / cs;
+int launch_stream_hd(const attn_params& p, int m, int cs, cudaStream_t stream, int pdl) {
   const size_t smem = (size_t)AS_NB * AS_CH * HD * 2;
-  LCU_REQUIRE(chunk <= most_positions<HD>() - AS_NB * AS_CH * HD, "attention: %d positions per CTA do not fit in shared memory", chunk);
   LCU_REQUIRE(p.err != nullptr, "attention: the streaming kernel needs a device error word");
   static bool attr_done[16] = {};
   int dev = 0;
@@ -421,11 +411,11 @@ int launch_attention(const attn_params& p, int m, int cluster, int max_T, cudaSt
   LCU_REQUIRE(max_T >= 1 && max_T <= p.ctx_len, "attention: %d positions exceed the context length %d", max_T, p.ctx_len);
   const bool streaming = p.err != nullptr && (g_attn_stream == 1 || (g_attn_stream < 0 && (max_T + cluster - 1) / cluster > AS_CH));
   if (streaming) {
-    if (p.head_dim == 128) return launch_stream_hd<128>(p, m, cluster, max_T, stream, pdl);
-    if (p.head_dim == 64) return launch_stream_hd<64>(p, m, cluster, max_T, stream, pdl);
+    if (p.head_dim == 128) return launch_stream_hd<128>(p, m, cluster, stream, pdl);
+    if (p.head_dim == 64) return launch_stream_hd<64>(p, m, cluster, stream, pdl);
   }
-  if (p.head_dim == 128) return launch_hd<128>(p, m, cluster, max_T, stream, pdl);
-  if (p.head_dim == 64) return launch_hd<64>(p, m, cluster, max_T, stream, pdl);
+  if (p.head_dim == 128) return launch_hd<128>(p, m, cluster, stream, pdl);
+  if (p.head_dim == 64) return launch_hd<64>(p, m, cluster, stream, pdl);
   LCU_REQUIRE(false, "attention: head_dim %d not supported (64 or 128)", p.head_dim);
 }
 

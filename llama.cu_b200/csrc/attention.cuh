@@ -30,8 +30,8 @@ struct attn_params {
   int exchanges_per_step;
 };
 
-// m query rows; `cluster` CTAs (1, 2, 4 or 8) share one (row, head); max_T bounds pos + m so that
-// shared memory can be sized without reading the device position.
+// m query rows; `cluster` CTAs (1, 2, 4 or 8) share one (row, head); max_T bounds pos + m (at most
+// ctx_len), so that the kernel can be chosen without reading the device position.
 int launch_attention(const attn_params& p, int m, int cluster, int max_T, cudaStream_t stream, int pdl);
 
 int attention_preload();

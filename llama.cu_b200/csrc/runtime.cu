@@ -941,7 +941,7 @@ int llama_context_impl::enqueue_decode_step(int long_ctx) {
     at.out = g.att; at.ldo = d;
     at.pos = g.state;
     at.ctx_len = opt.context_len; at.n_heads = p.n_heads; at.head_dim = hd; at.err = g.state + 3;
-    // max_T sizes the kernel's shared memory and picks its variant: up to 64 rows per CTA the register-path kernel
+    // max_T picks the kernel's variant: up to 64 rows per CTA the register-path kernel
     LCU_TRY(launch_attention(at, 1, opt.attn_cluster, long_ctx ? opt.context_len : std::min(opt.context_len, 64 * opt.attn_cluster), g.stream, pdl));
     LCU_TRY(launch_gemv(params_wo(l), EPI_PLAIN, g.stream, pdl));   // wo + residual (llama_cu.cu:1174)
     LCU_TRY(launch_gemv(params_w13(l), EPI_SILU, g.stream, pdl));   // RMSNorm + w1|w3 + SiLU gate (llama_cu.cu:1176-1183)

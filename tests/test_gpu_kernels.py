@@ -468,6 +468,27 @@ def test_attention_slices_at_the_edges_of_chunks(lcu, T0, hd):
         assert np.abs(f32(outs[0]) - f32(oo)).max() <= 2.5e-3 + 2.0**-9, cluster
 
 
+@pytest.mark.parametrize("hd,T", [(128, 73632), (64, 87968), (64, 110000)])
+def test_attention_over_more_positions_than_ever_fitted_in_shared_memory(lcu, hd, T):
+    """Nothing is kept per position: one CTA takes any slice, in both decode kernels, with equal bits.  Against binary64; bound: the result's
+    rounding to half (2^-11 of it); scores that round to another half (one of a thousand, by 2^-9 of its weight) and binary32 sums move a
+    row by less than 1e-6, a chunk of 64 rows too few by 1e-4."""
+    rng = np.random.default_rng(T)
+    q, k, v = f16(rng.standard_normal((1, hd))), f16(rng.standard_normal((T, hd))), f16(rng.standard_normal((T, hd)))
+    s = ((f32(k).astype(np.float64) @ f32(q)[0]) / np.sqrt(hd)).astype(np.float16).astype(np.float64)
+    e = np.exp(s - s.max())
+    want = (e / e.sum()) @ f32(v).astype(np.float64)
+    outs = []
+    try:
+        for mode in (0, 1):
+            lcu.check(lcu.lib.lcu_set_tuning(b"attn_stream", mode))
+            outs.append(lcu.attention(q, k, v, 1, T - 1, 1))
+    finally:
+        lcu.check(lcu.lib.lcu_set_tuning(b"attn_stream", -1))
+    assert (outs[0] == outs[1]).all() and 1e-3 < np.abs(want).max() < 0.1
+    assert np.abs(f32(outs[0])[0] - want).max() <= 2.0**-11 * np.abs(want).max() + 1e-6
+
+
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("score", [np.nan, -np.inf])
 def test_attention_of_a_key_whose_score_is_no_number(lcu, hd, score):
