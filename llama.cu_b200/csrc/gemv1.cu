@@ -277,9 +277,10 @@ __device__ __forceinline__ void row_sums8(const uint4& q, int i, int lane, float
 }
 // The row is in shared memory (each thread reads back the vectors it wrote itself, or all of them are visible): normalise
 // it and form its group sums.  K is a multiple of 256, so a warp's 32 vectors are all inside the row or all outside.
-template <int WT>
+// nw: norm weights of the thread's first NV vectors.
+template <int WT, int NV>
 __device__ __forceinline__ void row_finish(const gemv_params& p, bool norm, uint8_t* xs, float* xs64, float* squares, int tid, int threads,
-                                           const uint4 (&nw)[ROW_VEC], float inv_k) {
+                                           const uint4 (&nw)[NV], float inv_k) {
   const int vec = p.K >> 3, lane = tid & 31;
   float rinv = 1.f;
   if (norm) {
@@ -310,10 +311,10 @@ __device__ __forceinline__ void row_finish(const gemv_params& p, bool norm, uint
     if (tid < vec) finish(tid, nw[0]);
   } else if (norm) {
 #pragma unroll
-    for (int j = 0; j < ROW_VEC; ++j)
+    for (int j = 0; j < NV; ++j)
       if (tid + j * threads < vec) finish(tid + j * threads, nw[j]);
 #pragma unroll 1
-    for (int i = tid + ROW_VEC * threads; i < vec; i += threads) finish(i, *reinterpret_cast<const uint4*>(p.norm_w + i * 8));
+    for (int i = tid + NV * threads; i < vec; i += threads) finish(i, *reinterpret_cast<const uint4*>(p.norm_w + i * 8));
   } else if (WT == 2) {
 #pragma unroll 4
     for (int i = tid; i < vec; i += threads) finish(i, nw[0]);
@@ -403,7 +404,12 @@ __device__ __forceinline__ void store_pair(const gemv_params& p, const gemv_batc
 // 1024 + q (one PRMT per two weights) and the group sums of x coming from the prologue.  Mode 2 has
 // no per-weight rounding: it is closer to the exact product but is not the reference's rounding.  3 = bfloat16 weights and
 // activations: no fused norm or cache write; EPI_PLAIN runs the matrices of `bt`, each with its own vector, on runs of CTAs.
-template <int WT, int EPI, int NW>
+//
+// LONG: normalised fp16 rows of more than ROW_VEC vectors per thread (4096 values; the 13B and 65B models).  Their norm weights are requested
+// ahead of the wait as a whole, up to 8192 values; requested behind the row's sum, one after the other, every vector past the
+// fourth cost 0.25 to 0.3 us (wq|wk|wv of 6144 35.25 -> 34.74, of 8192 62.2 -> 61.0).  Code of its own, because the other launches pay for the fetch of instructions that they skip (with it in
+// their kernel a step of 2048 columns took 219.0 us for 215.6, u8 with blocks of 32 252 for 238 at 1024).
+template <int WT, int EPI, int NW, bool LONG = false>
 __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(const gemv_params p, const int sw, const int pf_bytes,
                                                                                         const __grid_constant__ gemv_batch bt) {
   constexpr int NCONS = NW * 32;
@@ -562,11 +568,12 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
   // The norm weights do not depend on the previous kernel: they are brought close while this one waits for it.
   const int vec = p.K >> 3;
   const bool norm = WT != 3 && p.norm_w != nullptr;
-  uint4 nw[ROW_VEC];
+  constexpr int NORM_VEC = LONG ? 2 * ROW_VEC : ROW_VEC;
+  uint4 nw[NORM_VEC];
   const float inv_k = 1.0f / p.K;
   if (norm) {
 #pragma unroll
-    for (int j = 0; j < ROW_VEC; ++j)
+    for (int j = 0; j < NORM_VEC; ++j)
       if (tid + j * NCONS < vec) nw[j] = *reinterpret_cast<const uint4*>(p.norm_w + (tid + j * NCONS) * 8);
   }
   pdl_wait();
@@ -577,7 +584,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 4 ? 3 : 2) gemv1_kernel(c
     // Rows of up to ROW_VEC vectors per thread are loaded by the threads themselves.  Longer rows come in as bulk copies of one
     // 512-element segment each: one trip to L2 whatever the row length, where per-thread loads would pay a round trip per
     // batch of vectors.  Both read past L1 (L2 is where another GPU's peer stores land).
-    if (vec <= ROW_VEC * NCONS) {
+    if (!LONG && vec <= ROW_VEC * NCONS) {
       if (p.n_wait > 0) {
         // tensor-parallel: parts of the row come from other GPUs; wait for their flags first
         if (tid < p.n_wait) flag_wait_at_least(p.wait_flags + tid, *p.seq * TP_EXCHANGES_PER_STEP + p.wait_id, p.err);
@@ -840,13 +847,13 @@ __global__ void __launch_bounds__(held_warps<NCH> * 32, NCH == 1 ? 2 : 3) gemv_h
   if (mine) store_pair<WT, EPI>(p, bt, bi, po, pr, v0, v1, pos, gate_scale);
 }
 
-template <int WT, int EPI, int NW>
+template <int WT, int EPI, int NW, bool LONG = false>
 int launch_one(const gemv_params& p, cudaStream_t stream, int pdl, size_t smem, int grid, int sw, int pf_bytes, const gemv_batch& bt = gemv_batch{}) {
   static bool attr_done[16] = {};
   int dev = 0;
   LCU_CUDA(cudaGetDevice(&dev));
   if (dev < 16 && !attr_done[dev]) {
-    LCU_CUDA(cudaFuncSetAttribute(gemv1_kernel<WT, EPI, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    LCU_CUDA(cudaFuncSetAttribute(gemv1_kernel<WT, EPI, NW, LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     attr_done[dev] = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -859,7 +866,7 @@ int launch_one(const gemv_params& p, cudaStream_t stream, int pdl, size_t smem, 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
-  LCU_CUDA(cudaLaunchKernelEx(&cfg, gemv1_kernel<WT, EPI, NW>, p, sw, pf_bytes, bt));
+  LCU_CUDA(cudaLaunchKernelEx(&cfg, gemv1_kernel<WT, EPI, NW, LONG>, p, sw, pf_bytes, bt));
   return LCU_OK;
 }
 
@@ -926,6 +933,7 @@ int launch_held(const held_plan& h, const gemv_params& p, cudaStream_t stream, i
 namespace {
 struct gemv1_config {
   int wt, nw, sw, grid, pf;
+  bool long_norm;  // a normalised fp16 row of more than ROW_VEC vectors per thread
   size_t smem;
 };
 int configure(const gemv_params& p, int sms, gemv1_config& c) {
@@ -947,13 +955,19 @@ int configure(const gemv_params& p, int sms, gemv1_config& c) {
   // when those fit (a long activation row: w2 of every model, every matrix of the larger models)
   int nw = 4;
   if (wt == 2 && cps < 3 && t.consumer_warps_int8 != 4 && fits(5, 2, cps)) nw = 5;
-  const int want_sw = wt == 2 ? t.warp_stages_int8 : t.warp_stages;
+  const bool long_norm = wt == 0 && norm && p.K > ROW_VEC * 8 * 4 * 32;
+  int want_sw = wt == 2 ? t.warp_stages_int8 : t.warp_stages;
+  // Normalised fp16 rows of more than 6144 values: two stages are enough, and with three the CTAs of an SM take all of its shared memory.
+  // Three / two, us: w1|w3 7168 wide 84.3 / 82.3, 8192 106.9 / 102.7, output matrix 78.4 / 75.5, a step of 4 layers 1114 / 1080; but 5120
+  // wide 44.9 / 46.8.
+  if (long_norm && p.K > 6144) want_sw = std::min(want_sw, 2);
   int sw = want_sw < 2 ? 2 : (want_sw > MAX_SW ? MAX_SW : want_sw);
   while (sw > 2 && !fits(nw, sw, cps)) --sw;
   const size_t smem = fixed + (size_t)nw * sw * stage_bytes;
   LCU_REQUIRE(smem <= 227 * 1024, "gemv: a row of K=%d does not fit in shared memory", p.K);
   const int pairs = p.n_mats * p.rows_per_mat / 2;
   c.wt = wt;
+  c.long_norm = long_norm;
   c.nw = nw;
   c.sw = sw;
   c.grid = sms * cps > pairs ? pairs : sms * cps;
@@ -977,6 +991,11 @@ int gemv_single_row_preload() {
   LCU_PRELOAD_E(EPI_SILU)
 #undef LCU_PRELOAD_E
 #undef LCU_PRELOAD
+#define LCU_PRELOAD_LONG(E) LCU_CUDA(cudaFuncGetAttributes(&fa, gemv1_kernel<0, E, 4, true>));
+  LCU_PRELOAD_LONG(EPI_PLAIN)
+  LCU_PRELOAD_LONG(EPI_ROPE_KV)
+  LCU_PRELOAD_LONG(EPI_SILU)
+#undef LCU_PRELOAD_LONG
   return LCU_OK;
 }
 
@@ -1011,6 +1030,7 @@ int launch_gemv_single_row(const gemv_params& p, int epilogue, cudaStream_t stre
   }
 #define LCU_GEMV1_CASE(E)                                                                  \
   case E:                                                                                  \
+    if (c.long_norm) return launch_one<0, E, 4, true>(p, stream, pdl, smem, grid, sw, pf); \
     if (wt == 0) return launch_one<0, E, 4>(p, stream, pdl, smem, grid, sw, pf);           \
     if (wt == 1) return launch_one<1, E, 4>(p, stream, pdl, smem, grid, sw, pf);           \
     if (nw == 5) return launch_one<2, E, 5>(p, stream, pdl, smem, grid, sw, pf);           \

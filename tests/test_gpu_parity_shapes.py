@@ -171,6 +171,30 @@ def test_one_layer_model_at_large_widths(lcu, dim, n_heads, mode):
     model.close()
 
 
+@pytest.mark.parametrize("dim", [4096, 4352, 6400, 8192, 8448])
+def test_norm_weights_of_rows_longer_than_the_first_vectors(lcu, dim):
+    """wq|wk|wv, w1|w3 and the output matrix with every norm weight of its own, where a thread's norm weights are its first four vectors of the
+    row, a fifth, all eight, and more: against the kernel that shares no code with it (16-row blocks).  Bound: between the two, sums differ
+    in their order only, so that halves rounded on the way move by one unit at most, three roundings in a chain - 2^-9 of the logits'
+    RMS; norm weights of one vector that belong to another move them by 1e-2."""
+    model = lcu.Model.synthetic(dim=dim, n_heads=dim // 128, n_layers=1, n_vocab=512, seed=7, scale=0.02)
+    rng = np.random.default_rng(dim)
+    for name in ("layers.0.attention_norm", "layers.0.ffn_norm", "norm"):
+        w = f16(rng.choice([-1.0, 1.0], dim) * rng.uniform(0.5, 1.5, dim))
+        ptr, size, _ = model.tensor(name, 0)
+        assert size == w.nbytes
+        lcu.check(lcu.lib.lcu_memcpy_h2d(ptr, w.ctypes.data, size))
+    rows = []
+    for variant in (0, 1):
+        with tuning(lcu, b"gemv_variant", variant, 1):
+            ctx = lcu.Context(model, context_len=16, temperature=0.8)
+            rows.append(np.concatenate([ctx.step([t], [0]) for t in (5, 9, 300)]).astype(np.float64))
+            ctx.close()
+    error = np.sqrt(((rows[1] - rows[0]) ** 2).mean(1)) / np.sqrt((rows[0] ** 2).mean(1))
+    assert np.isfinite(rows[1]).all() and error.max() <= 2.0 ** -9, error
+    model.close()
+
+
 # ------------------------------------------------------------------ matmul_type 1: the pedantic kernels
 @pytest.mark.parametrize("m,k,n,bs,beta", [(1, 256, 64, 0, 0.0), (3, 768, 130, 0, 1.0), (1, 4096, 512, 128, 0.0), (5, 512, 96, 64, 1.0),
                                            (2, 256, 33, 32, 0.0)])
