@@ -895,12 +895,18 @@ int g_held_mode = -1;  // -1 = by the rule, 0 = never
 // At most twelve warps per SM, one wave beside the kernels around it (4096 wide u8, 13.8 for wo: 2 % slower held).  Rows: a launch
 // between ring kernels gains nothing, so lengths stop where a model's other launches are too large - bfloat16 rows of 4 KiB
 // (Filulix, 2048 wide) 185 -> 188 us, rows of two chunks of 1536 wide fp16 (8 KiB) 152 -> 173, where 1024 wide ones (5.5 KiB), whose
-// step is held as a whole, gain 156 -> 143.  Every launch of a tensor-parallel step (its step number is set) stays on the ring, the one
+// step is held as a whole, gain 156 -> 143.  In between, two-byte weights are held in small launches only.  Steps in us, ring / held
+// (every multiple of 256 columns, 10 layers fp16, 4 bfloat16):
+//   two chunks, wo of fp16:   2304 wide 370 / 377, 2560 423 / 434, 3072 491 / 511: four warps per SM (w2 of 1024 columns has 3.5)
+//   rows of 2.5 and 3 KiB:    wo of 1280 239.1 / 241.7, of 1536 246.4 / 254.4 (but 3.5 and 4 KiB: 1792 281 / 274, 2048 298 / 290);
+//                             Filulix 1280 121 / 123, 1408 122 / 127, 1536 128 / 132, Zibovik 1280 154 / 156, 1408 159 / 162, 1536 168 / 170
+//                             (1152: 116.4 / 116.4 and 149.9 / 148.7): three, but for picked experts (Zibovik 768 140 / 125, 1024 145 / 131)
+// 8-bit weights gain or are level at every width.  Every launch of a tensor-parallel step (its step number is set) stays on the ring, the one
 // that neither waits for other GPUs nor publishes to them - layer 0's wq|wk|wv - too: ring kernels are loaded ahead of the first step, in
 // which other GPUs' bounded waits run while a launch stalls in loading its kernel.
-constexpr int HELD_WARPS_PER_SM = 12;
+constexpr int HELD_WARPS_PER_SM = 12, HELD_WARPS_TWO_CHUNKS = 4, HELD_WARPS_LONG_CHUNK = 3;
 template <class PairsOf>
-held_plan plan_held(int wt, int epi, const gemv_params& p, int n, PairsOf pairs_of, int sms) {
+held_plan plan_held(int wt, int epi, const gemv_params& p, int n, PairsOf pairs_of, int sms, bool picked = false) {
   held_plan h;
   if (g_held_mode == 0 || wt == 1 || (wt == 2 && p.bs != 64 && p.bs != 128) || p.seq != nullptr) return h;
   const int rowbytes = p.K * (wt == 2 ? 1 : 2), chunks = (rowbytes + 4095) / 4096;
@@ -912,7 +918,10 @@ held_plan plan_held(int wt, int epi, const gemv_params& p, int n, PairsOf pairs_
   }
   h.dual = rowbytes <= 2048 && single > 4 * sms;
   const long long units = h.dual ? two : single;
-  if (units > HELD_WARPS_PER_SM * sms) return h;
+  int most = HELD_WARPS_PER_SM;
+  if (wt != 2 && chunks == 2) most = HELD_WARPS_TWO_CHUNKS;
+  else if (wt != 2 && !picked && rowbytes > 2304 && rowbytes <= 3072) most = HELD_WARPS_LONG_CHUNK;
+  if (units > most * sms) return h;
   h.warps = std::max(((int)units + sms - 1) / sms, p.norm_w ? 4 : 2);
   h.warps = std::max(std::min(h.warps, chunks == 1 ? held_warps<1> : held_warps<2>), (p.K / 8 + ROW_VEC * 32 - 1) / (ROW_VEC * 32));
   if (h.warps > (chunks == 1 ? held_warps<1> : held_warps<2>)) return h;  // (a thread holds ROW_VEC vectors of the row)
@@ -1060,7 +1069,7 @@ int launch_gemv_bf16(const gemv_batch& b, int K, int* err, cudaStream_t stream, 
   p.m = 1;
   p.err = err;
   gemv_batch bt = b;
-  const held_plan h = plan_held(3, EPI_PLAIN, p, b.n, [&](int i) { return b.rows[i] / 2; }, gemv_sm_count());
+  const held_plan h = plan_held(3, EPI_PLAIN, p, b.n, [&](int i) { return b.rows[i] / 2; }, gemv_sm_count(), b.choice != nullptr);
   if (h.chunks) {
     bt.first_cta[0] = 0;
     for (int i = 0; i < b.n; ++i) bt.first_cta[i + 1] = bt.first_cta[i] + ((h.dual ? (b.rows[i] / 2 + 1) / 2 : b.rows[i] / 2) + h.warps - 1) / h.warps;
@@ -1118,7 +1127,7 @@ int launch_gemv_bf16_gated_picked(const gemv_batch& b, int f, int K, int* err, c
     bt.w[i] = b.w[0];
     bt.rows[i] = 2 * f;
   }
-  const held_plan h = plan_held(3, EPI_SILU, p, b.n, [&](int) { return f; }, gemv_sm_count());
+  const held_plan h = plan_held(3, EPI_SILU, p, b.n, [&](int) { return f; }, gemv_sm_count(), true);
   if (h.chunks) {
     for (int i = 0; i <= b.n; ++i) bt.first_cta[i] = i * (h.grid / b.n);
     return launch_held<3, EPI_SILU>(h, p, stream, pdl, bt);

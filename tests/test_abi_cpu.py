@@ -162,7 +162,14 @@ def test_tensor_parallel_steps_take_only_kernels_that_are_loaded_ahead():
                     assert chunks == 0 and warps in (4, 5) and 1 <= ctas <= 3 * 148, (dim, gpus, bs, mats)
                     held += plan(dim, rows, mats, bs, 0)[0] > 0
     assert held > 50
-    # one GPU: whole rows of up to a chunk (two for plain products) per warp, as many CTAs as the pairs need
+    # one GPU: the lines of the rule - whole steps of 1024 columns; wo alone at 1792 and 2048 but not at 1280, 1536 and from 2304 on
+    for dim, ffn in ((512, 1536), (768, 2048), (1024, 2816)):
+        assert all(plan(k, n, mats, 0, 0)[0] for k, n, mats in ((dim, dim, 3), (dim, dim, 1), (dim, ffn, 2), (ffn, dim, 1))), dim
+    assert [dim for dim in range(1280, 4097, 256) if plan(dim, dim, 1, 0, 0)[0]] == [1792, 2048]
+    assert plan(1280, 2 * 3 * 148, 1, 0, 0)[0] == 1 and plan(1280, 2 * 3 * 148 + 2, 1, 0, 0)[0] == 0
+    assert plan(2304, 2 * 4 * 148, 1, 0, 0)[0] == 2 and plan(2304, 2 * 4 * 148 + 2, 1, 0, 0)[0] == 0
+    assert [dim for dim in range(256, 5121, 256) if plan(dim, dim, 1, 128, 0)[0]] == list(range(256, 3329, 256))
+    # whole rows of up to a chunk (two for plain products) per warp, as many CTAs as the pairs need
     assert plan(1024, 1024, 3, 0, 0) == [1, 6, 128] and plan(2816, 1024, 1, 0, 0) == [2, 4, 128] and plan(4096, 4096, 1, 128, 0)[0] == 0
     with pytest.raises(lcu.LcuError):
         plan(100, 2, 1, 0, 0)

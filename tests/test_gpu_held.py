@@ -38,6 +38,11 @@ def test_products_have_the_same_bits(lcu, k, n, bs):
     assert np.isfinite(ring.view(np.float16).astype(np.float32)).all() and np.array_equal(ring, held)
 
 
+@pytest.mark.parametrize("k,n", [(1280, 888), (1280, 890), (1536, 600), (1792, 1792), (2304, 1184), (2304, 1186), (3072, 1000)])
+def test_fp16_products_on_both_sides_of_the_rule(lcu, k, n):
+    test_products_have_the_same_bits(lcu, k, n, 0)
+
+
 @pytest.mark.parametrize("dim,heads,bs", [(256, 2, 0), (512, 8, 64), (1024, 8, 0), (1024, 16, 128), (1280, 10, 0), (2048, 16, 128), (2048, 16, 0)])
 def test_decode_steps_have_the_same_bits(lcu, dim, heads, bs):
     """Norms, rotation and cache rows, gate and residual of a step: greedy tokens and the last probabilities."""
