@@ -536,6 +536,25 @@ def test_attention_head_dim_64(lcu, m, T0, cluster):
     assert np.abs(f32(out) - f32(oo)).max() <= 4e-3
 
 
+@pytest.mark.parametrize("vocab", [200, 255, 256, 1000, 32000])  # one CTA below 256, a cluster from there on
+def test_logits_head_of_rows_without_a_number(lcu, vocab):
+    """No probability is a number where a logit is NaN or infinite, or all are -inf: token 0, as std::max_element over such a row gives
+    (a chained step feeds it back, so it has to lie inside the embedding table)."""
+    rng = np.random.default_rng(vocab)
+    rows = [np.full(vocab, np.nan), np.full(vocab, -np.inf)]
+    for value in (np.nan, np.inf):
+        for at in (0, vocab // 2, vocab - 1):
+            rows.append(rng.standard_normal(vocab))
+            rows[-1][at] = value
+    for row in rows:
+        token, probs = lcu.logits_head(f16(row), 0.8)
+        assert token == 0 and np.isnan(f32(probs)).all()
+    row = rng.standard_normal(vocab)
+    row[vocab // 3:] = -np.inf  # (some of them: no reason to worry)
+    token, probs = lcu.logits_head(f16(row), 0.8)
+    assert token == f16(row).view(np.float16).argmax() and np.isfinite(f32(probs)).all()
+
+
 def test_logits_head_first_maximum_and_ties(lcu):
     rng = np.random.default_rng(9)
     V = 32000
