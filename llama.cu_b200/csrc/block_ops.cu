@@ -837,19 +837,15 @@ int launch_hyper_rows(const hyper_params<T>& p, int n_rows, cudaStream_t stream)
   LCU_REQUIRE(p.mix == nullptr || (n_rows == 1 && p.n_mix == HY_MIX), "hyper_rows: the token shift is fused for a single row of %d inputs", HY_MIX);
   LCU_REQUIRE(p.router == nullptr || n_rows == 1, "hyper_rows: experts are picked for a single row");
   const bool pre = p.y && (p.post_w || p.y_rows);
-  // One row of whole vectors, up to four streams: one CTA where a thread holds one vector (two of a single stream), else a cluster.
-  // (Router weights and the row of a router fit the default 48 KB then: 2048 columns and 1024 experts take 16.)
+  // One row of whole vectors, up to four streams: one CTA of one vector per thread up to 2048 columns, a cluster of two per thread up to
+  // 8192.  (Router weights and the row of a router fit the default 48 KB then: 2048 columns and 1024 experts take 16.)
   if (n_rows == 1 && p.streams <= 4 && p.width % 4 == 0 && p.width <= 8 * HY_CLUSTER * 128 && hyper_row_single()) {
-#define LCU_SINGLE(SM, CL, NT, V) \
-  return pre ? launch_hyper_single<T, SM, CL, NT, V, true>(p, stream) : launch_hyper_single<T, SM, CL, NT, V, false>(p, stream)
-    if (p.streams == 1) {
-      if (p.width <= 1024) LCU_SINGLE(1, 1, 256, 1);
-      if (p.width <= 2048) LCU_SINGLE(1, 1, 512, 1);
-      LCU_SINGLE(1, HY_CLUSTER, 128, 2);
-    }
-    if (p.width <= 1024) LCU_SINGLE(4, 1, 256, 1);
-    if (p.width <= 2048) LCU_SINGLE(4, 1, 512, 1);
-    LCU_SINGLE(4, HY_CLUSTER, 128, 2);
+#define LCU_SINGLE(CL, NT, V)                                                                                                              \
+  if (p.streams == 1) return pre ? launch_hyper_single<T, 1, CL, NT, V, true>(p, stream) : launch_hyper_single<T, 1, CL, NT, V, false>(p, stream); \
+  return pre ? launch_hyper_single<T, 4, CL, NT, V, true>(p, stream) : launch_hyper_single<T, 4, CL, NT, V, false>(p, stream)
+    if (p.width <= 1024) { LCU_SINGLE(1, 256, 1); }
+    if (p.width <= 2048) { LCU_SINGLE(1, 512, 1); }
+    LCU_SINGLE(HY_CLUSTER, 128, 2);
 #undef LCU_SINGLE
   }
   const int most = hyper_row_one_cta();  // (measured: 7 % of a step at 1024 columns, lost again where a CTA has four vectors per thread to load twice)
