@@ -365,27 +365,41 @@ def measure_decode(lcu, workload, K, W, prompt_len, world, dist, layer_gpus=None
     ms_all = reduce_max_time(ms, dist)
     value = world * K / (ms_all / 1e3)
 
-    # ---- end to end through the reference-facing call: host token in, host token out, every step
-    ctx.clear_tokens()
-    tok = ctx.next_token(prompt)
-    for _ in range(W):
-        tok = ctx.next_token([tok])
-    barrier_sync(dist, lcu)
-    t0 = time.perf_counter()
-    e2e_tokens = []
-    for _ in range(K):
-        tok = ctx.next_token([tok])
-        e2e_tokens.append(tok)
-    lcu.check(lcu.lib.lcu_synchronize())
-    e2e_ms = (time.perf_counter() - t0) * 1e3
-    barrier_sync(dist, lcu)
-    e2e_ms_all = reduce_max_time(e2e_ms, dist)
+    # ---- end to end through the reference-facing call: host token in, host token out, every step.  On one GPU a step that is fed the token
+    # before it copies nothing to the GPU ("in_place"); the end-to-end figure is taken with a context that copies every step's input.
+    def host_driven(c):
+        c.clear_tokens()
+        tok = c.next_token(prompt)
+        for _ in range(W):
+            tok = c.next_token([tok])
+        barrier_sync(dist, lcu)
+        t0 = time.perf_counter()
+        out = []
+        for _ in range(K):
+            tok = c.next_token([tok])
+            out.append(tok)
+        lcu.check(lcu.lib.lcu_synchronize())
+        wall_ms = (time.perf_counter() - t0) * 1e3
+        barrier_sync(dist, lcu)
+        return reduce_max_time(wall_ms, dist), out
+
+    e2e_ms_all, e2e_tokens = host_driven(ctx)
+    in_place = None
+    if layer_gpus is None:
+        in_place = {"value": round(world * K / (e2e_ms_all / 1e3), 2), "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 8}
+        lcu.check(lcu.lib.lcu_set_tuning(b"step_copies", 1))
+        copying = lcu.Context(model, context_len=ctx_len, temperature=TEMPERATURE)
+        lcu.check(lcu.lib.lcu_set_tuning(b"step_copies", 0))
+        first_tokens = e2e_tokens
+        e2e_ms_all, e2e_tokens = host_driven(copying)
+        copying.close()
+        in_place["tokens_equal"] = first_tokens == e2e_tokens
     e2e_value = world * K / (e2e_ms_all / 1e3)
     same_tokens = bool((np.array(e2e_tokens, np.int16) == tokens).all())
     res = {"workload": workload, "cfg": cfg, "ffn": ffn, "ctx_len": ctx_len, "gen_s": gen_s, "prefill_s": prefill_s, "value": value,
            "ms_per_step": ms_all / K, "first": int(first), "warm_tokens": [int(t) for t in warm_tokens], "tokens": [int(t) for t in tokens],
            "e2e": {"value": round(e2e_value, 2), "unit": "tok/s", "h2d_bytes_per_step": 10, "d2h_bytes_per_step": 8,
-                   "ms_per_step": round(e2e_ms_all / K, 5), "tokens_equal_chained_run": same_tokens},
+                   "ms_per_step": round(e2e_ms_all / K, 5), "tokens_equal_chained_run": same_tokens, "in_place": in_place},
            "kernels_per_step": ctx.kernels_per_step()}
 
     if forced is not None:  # top-1 agreement with another run's tokens, teacher-forced on them

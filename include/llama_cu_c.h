@@ -45,7 +45,9 @@ int lcu_set_matmul_type(int type);
  * single residual row of a block model takes the kernel of many rows), "block_row_one_cta" (there a single residual row
  * of a block model of up to this many columns is one CTA's work, a longer one a cluster's), "block_attn_mma" (0 = the per-row attention kernel for every pass of a block model),
  * "host_wait_limit_ms" (how long a call of lcu_context_* waits for the GPU to finish, again for every thousand steps of a chained call: 600000;
- * 0 = for ever), "use_graph", "use_pdl", "attn_cluster", "loader_staged" (lcu_model_load: 1 = pinned double-buffered asynchronous copies, 0 = a file mapping and one
+ * 0 = for ever), "use_graph", "use_pdl", "attn_cluster", "step_copies" (contexts made afterwards: 1 = a host-driven step copies its
+ * position and token to the GPU and token and error word back each time, as with a sampler; 0 = not where the GPU holds them already, and the
+ * step's last kernel writes the words to the host), "loader_staged" (lcu_model_load: 1 = pinned double-buffered asynchronous copies, 0 = a file mapping and one
  * blocking pageable copy per tensor as the reference does).  Unknown keys are rejected. */
 int lcu_set_tuning(const char* key, int value);
 

@@ -21,7 +21,7 @@
 using namespace lcu;
 
 namespace {
-context_options g_default_opts;  // "use_graph", "use_pdl", "attn_cluster" knobs apply to contexts created afterwards
+context_options g_default_opts;  // "use_graph", "use_pdl", "attn_cluster", "step_copies" knobs apply to contexts created afterwards
 
 int require_device() {
   int n = 0;
@@ -131,6 +131,7 @@ int lcu_set_tuning(const char* key, int value) {
   else if (k == "loader_staged") set_loader_staged(value);
   else if (k == "host_wait_limit_ms") host_wait_limit_ms() = value < 0 ? 0 : value;
   else if (k == "use_graph") g_default_opts.use_graph = value;
+  else if (k == "step_copies") g_default_opts.step_copies = value;
   else if (k == "use_pdl") g_default_opts.use_pdl = value;
   else if (k == "attn_cluster") g_default_opts.attn_cluster = value;
   else LCU_REQUIRE(false, "unknown tuning key %s", k.c_str());

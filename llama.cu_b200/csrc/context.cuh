@@ -106,7 +106,7 @@ struct context_impl {
   int run_decode_step(int n_keys);
   int stage_inputs(const short* tokens, int n);
   // a step's last kernel writes token and error word to h_words[TOLD] (a sampler or another GPU's stage would come after it)
-  bool tells_host() const { return gpus.size() == 1 && !opt.sampling; }
+  bool tells_host() const { return gpus.size() == 1 && !opt.sampling && !opt.step_copies; }
   // Token and error word of `from` to pinned memory, and the wait for everything before them on `stream`: at most
   // host_wait_limit_ms() for the call and again for every thousand steps in it, then LCU_ERR_DEVICE_WAIT.  (Kernels bound their
   // waits on barriers and flags themselves; this bounds whatever else keeps a stream from ending.)

@@ -163,6 +163,7 @@ struct context_options {
   int context_len = 2048;
   float temperature = 0.9f;
   int use_graph = 1;     // replay one CUDA graph per decode step
+  int step_copies = 0;   // host-driven single steps: 1 = position and token are copied to the GPU for every step, and its words back
   int use_pdl = 1;       // programmatic dependent launch between the kernels of a step
   int attn_cluster = 8;  // CTAs per (row, head) in decode attention
   int sampling = 0;      // 0 = greedy (first maximum, what the reference runs); 1 = multinomial over the fp16 probabilities

@@ -397,3 +397,22 @@ def test_single_steps_behind_other_calls(lcu, bs):
         runs.append(seen)
     assert runs[0] == runs[1]
     model.close()
+
+
+def test_steps_that_copy_their_inputs_give_the_same(lcu):
+    """A context made with "step_copies" = 1 copies position and token for every step and the words back: the same tokens and probabilities."""
+    model, runs = lcu.Model.synthetic(dim=256, n_heads=2, n_layers=2, n_vocab=1000, seed=9, scale=0.08), []
+    for copies in (0, 1):
+        lcu.check(lcu.lib.lcu_set_tuning(b"step_copies", copies))
+        try:
+            ctx = lcu.Context(model, context_len=64, temperature=0.8)
+        finally:
+            lcu.check(lcu.lib.lcu_set_tuning(b"step_copies", 0))
+        seen, t = [], ctx.next_token([5, 6, 7, 8])
+        for i in range(20):
+            t = ctx.next_token([t if i != 11 else 40])
+            seen.append((t, ctx.probs().tobytes()))
+        ctx.close()
+        runs.append(seen)
+    assert runs[0] == runs[1]
+    model.close()
