@@ -87,9 +87,9 @@ struct warp_rows {
     // (a score that is no number leaves the maximum alone but not the sum: without any maximum scores are taken as they are)
     const float ref = top > -CUDART_INF_F ? top : 0.f, keep = expf(m - ref);
     m = top;
-    sum *= keep;
+    sum = __fmul_rn(sum, keep);  // (rounded by itself, whatever the compiler makes of the additions behind it)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] *= keep;
+    for (int i = 0; i < 8; ++i) acc[i] = __fmul_rn(acc[i], keep);
 #pragma unroll
     for (int j = 0; j < ROUNDS; ++j) {
       e[j] = expf(e[j] - ref);  // (0 for rows that do not exist)
