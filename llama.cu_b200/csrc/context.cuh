@@ -63,11 +63,11 @@ struct context_impl {
   short* ids = nullptr;                  // token ids on the embedding GPU [context_len]
   __half* probs = nullptr;               // on the output GPU
   short* log = nullptr;                  // generated tokens of a chained run [context_len]
-  int* h_stage = nullptr;                // pinned: [0] position, [1] zero; h_words lies behind them
+  int* h_stage = nullptr;                // pinned: [0] position, [1] step count (log_or_tell); h_words lies behind them
   uint64_t* h_words = nullptr;           // pinned: step_words by place
   enum words_place { COPIED, BEFORE_LOGITS, TOLD, WORDS };  // read back by a copy, the same in front of logits, written by a step's last kernel itself
-  // what the position word and the first token id on the GPU hold (-1: not known): a step that finds both in place, as the one after
-  // the token it is fed does, has nothing to copy
+  // what the position word and the first token id on the GPU hold behind a single step (-1: not known, or a step of another kind): a
+  // single step that finds both in place, as the one after the token it is fed does, has nothing to copy
   int dev_pos = -1, dev_token = -1;
   short* h_ids = nullptr;                // pinned token staging [context_len]
   cudaEvent_t t0 = nullptr, t1 = nullptr;
@@ -104,7 +104,7 @@ struct context_impl {
   int open_streams(int context_len);     // pinned staging and events; gpus must be filled in
   int build_graph(int variant);
   int run_decode_step(int n_keys);
-  int stage_inputs(const short* tokens, int n);
+  int stage_inputs(const short* tokens, int n, int step);
   // a step's last kernel writes token and error word to h_words[TOLD] (a sampler or another GPU's stage would come after it)
   bool tells_host() const { return gpus.size() == 1 && !opt.sampling && !opt.step_copies; }
   // Token and error word of `from` to pinned memory, and the wait for everything before them on `stream`: at most

@@ -143,11 +143,7 @@ __global__ void __cluster_dims__(HC_CLUSTER, 1, 1) __launch_bounds__(HC_THREADS)
     if (p.token_out) *p.token_out = best_i;
     if (p.next_ids) p.next_ids[0] = (short)best_i;
     if (p.pos) *p.pos += p.advance;
-    if (p.log && p.step) {
-      if (*p.step < p.log_capacity) p.log[*p.step] = (short)best_i;
-      *p.step += 1;
-    }
-    if (p.host_out) tell_host(p.host_out, best_i, __ldcg(p.token_out + 1));
+    log_or_tell(p, best_i);
   }
 }
 

@@ -299,11 +299,7 @@ __global__ void __launch_bounds__(HEAD_THREADS) logits_head_kernel(const head_pa
     if (p.token_out) *p.token_out = best_i;
     if (p.next_ids) p.next_ids[0] = (short)best_i;
     if (p.pos) *p.pos += p.advance;
-    if (p.log && p.step) {
-      if (*p.step < p.log_capacity) p.log[*p.step] = (short)best_i;
-      *p.step += 1;
-    }
-    if (p.host_out) tell_host(p.host_out, best_i, __ldcg(p.token_out + 1));
+    log_or_tell(p, best_i);
   }
 }
 

@@ -51,9 +51,19 @@ struct head_params {
   short* log;
   int* step;
   int log_capacity;
-  uint64_t* host_out;       // optional, pinned host memory: token and the word behind token_out (step_words), last of all
+  uint64_t* host_out;       // optional, pinned host memory: token and the word behind token_out (step_words), where *step is negative
 };
 #ifdef __CUDACC__
+// The last of a step.  Steps of a chained run are counted from 0 and their tokens logged; a single step (a negative count) tells the host,
+// which waits for it.  (A chained step that told it too was 2.1 us longer: 51.2 us for 49.1 at 512 columns and 2 layers.)
+__device__ __forceinline__ void log_or_tell(const head_params& p, int token) {
+  const int step = p.step ? *p.step : 0;
+  if (p.log && p.step && step >= 0) {
+    if (step < p.log_capacity) p.log[step] = (short)token;
+    *p.step = step + 1;
+  }
+  if (p.host_out && step < 0) tell_host(p.host_out, token, __ldcg(p.token_out + 1));
+}
 __device__ __forceinline__ float head_logit(const head_params& p, int i) { return p.logits_f32 ? p.logits_f32[i] : __half2float(p.logits[i]); }
 #endif
 int launch_logits_head(const head_params& p, cudaStream_t stream, int pdl);

@@ -1195,10 +1195,10 @@ int context_impl::run_decode_step(int n_keys) {
   return enqueue_decode_step(variant);
 }
 
-// position word (and a zeroed step counter) to every stage, token ids to stage 0
-int context_impl::stage_inputs(const short* tokens, int n) {
+// position word and step count (0, or -1 for a single step that tells the host) to every stage, token ids to stage 0
+int context_impl::stage_inputs(const short* tokens, int n, int step) {
   h_stage[0] = start_pos;
-  h_stage[1] = 0;
+  h_stage[1] = step;
   for (size_t gi = 0; gi < gpus.size(); ++gi) {
     gpu_state& g = gpus[gi];
     device_guard dg(g.device);
@@ -1237,7 +1237,7 @@ int context::step(const short* tokens, int n, const int* want, int n_want, float
   const bool single = n == 1 && !c.rows_only(), told = single && c.tells_host();
   const bool in_place = told && c.dev_pos == c.start_pos && c.dev_token == tokens[0];
   c.dev_pos = c.dev_token = -1;
-  if (!in_place) LCU_TRY(c.stage_inputs(tokens, n));
+  if (!in_place) LCU_TRY(c.stage_inputs(tokens, n, told ? -1 : 0));
   if (single) {
     if (told) clear_words(c.h_words + context_impl::TOLD);
     LCU_TRY(c.run_decode_step(c.start_pos + 1));
@@ -1275,7 +1275,7 @@ int context::decode_chained(short first_token, int n_steps, short* tokens_out, f
   LCU_REQUIRE(!c.rows_only(), "decode_chained: matmul_type 1 runs host-driven steps only (lcu_context_next_token)");
   LCU_TRY(c.settled("decode_chained"));
   c.dev_pos = c.dev_token = -1;
-  LCU_TRY(c.stage_inputs(&first_token, 1));
+  LCU_TRY(c.stage_inputs(&first_token, 1, 0));
   device_guard dg(c.first().device);
   LCU_CUDA(cudaEventRecord(c.t0, c.first().stream));
   for (int i = 0; i < n_steps; ++i) LCU_TRY(c.run_decode_step(c.start_pos + i + 1));
@@ -1285,10 +1285,6 @@ int context::decode_chained(short first_token, int n_steps, short* tokens_out, f
   LCU_TRY(c.read_back(c.last(), c.first().stream, context_impl::COPIED, n_steps, "decode_chained", &back));
   LCU_TRY(finish_step(*this, back, "decode_chained"));
   c.start_pos += n_steps;
-  if (c.tells_host()) {
-    c.dev_pos = c.start_pos;
-    c.dev_token = back.token;
-  }
   c.last_row = 0;
   memcpy(tokens_out, c.h_ids, (size_t)n_steps * 2);
   if (ms_out) LCU_CUDA(cudaEventElapsedTime(ms_out, c.t0, c.t1));
